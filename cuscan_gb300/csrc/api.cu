@@ -5,6 +5,7 @@
 
 #include "common.cuh"
 #include "forest.cuh"
+#include "simt.cuh"
 #include "workspace.cuh"
 
 namespace cuscan {
@@ -140,8 +141,9 @@ int64_t cuscan_fit_workspace_bytes(int64_t n, int32_t d, int32_t min_samples, in
     size_t b = 4 * N * D + 8 * N * k + 5 * 4 * N;  // input copy, kNN lists, core/label/MST arrays
     b += 18 * 4 * N + 4 * N * D + 16 * N;          // forest arrays, sorted copy, 64-bit keys
     b += 2 * 4 * (N / 32 + 2) + 64 + sizeof(DevStatus) + 4 * (N / 1024 + 2);  // tiles, scan
-    // split-kNN partial lists: at most 2 * SMs + query blocks blocks of 128 rows
-    b += 8 * k * 128 * (size_t)(2 * 2 * kSMs + ceil_div(n, 128));
+    // split-kNN partial lists, one list per query row of every CTA
+    b += 8 * k * simt::QT *
+         (size_t)simt::split_plan_max_ctas(kSMs, ceil_div(n, (int64_t)simt::QT));
     if (precision == CUSCAN_PRECISION_BF16_REFINED || precision == CUSCAN_PRECISION_FP16_REFINED)
         b += refined_workspace_bytes(n, d, (int)k);
     else if (n >= 2048)  // exact rounds over a row subset: bounds, flags, positions, counts

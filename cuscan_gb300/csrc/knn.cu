@@ -4,255 +4,476 @@
 // squared distance is acc = fmaf(q_f - r_f, q_f - r_f, acc) over features in order, rows are
 // ordered by (distance, id), self is excluded by global id, empty slots hold (pad, nr).
 //
-// Layout: one thread owns one query row (its features staged once in shared memory as
-// [feature][query] so the per-feature reads are conflict free); reference rows stream through
-// a double-buffered shared tile [feature][RT] filled with 4-byte cp.async copies, and each
-// thread keeps RT running distances in registers. Per feature and per 4 references that is one
-// broadcast 16-byte shared load, four FADD and four FFMA. The running top-K list lives in
-// registers and is updated with a fully unrolled predicated insertion; after the first few
-// tiles almost every candidate fails the threshold test, so the list costs one compare per
-// pair. When there are too few query blocks to fill the 152 SMs the reference range is split
-// across blocks and the partial lists are merged by a second kernel.
+// The distances come from the register-tiled sweep of simt.cuh. A thread tests its 64 pairs of a
+// tile against its queries' thresholds (the k-th entry of each query's list) with one minimum per
+// query; the few pairs that pass go to the query's bucket in shared memory, and after the tile
+// each warp merges the buckets of its 16 queries into their sorted lists, all pairs of a bucket at
+// once and a lane per list slot. A list costs 8 k bytes of shared memory and no registers, so k
+// up to 256 takes the same kernel. The order of arrival does not matter: a list holds the k least
+// (distance, id) pairs seen.
+//
+// Measured on a GB300: 100,000 x 64 rows, k = 10: KNN_A ms against 128.0 ms for one query per
+// thread with register lists; 20,011 x 32, k = 50: KNN_B ms against 23.0 ms for per-thread lists
+// in global memory.
+//
+// When there are too few query tiles to fill the SMs the reference range is split across CTAs
+// and the partial lists are merged by a second kernel.
 #include <limits>
 
 #include "forest.cuh"
+#include "simt.cuh"
 
 namespace cuscan {
 namespace {
 
-constexpr int QB = 128;  // queries (threads) per block
-constexpr int RT = 32;   // references per shared tile
-constexpr int RTP = 36;  // padded tile row (keeps 16-byte alignment, spreads store banks)
+using simt::Packed;
+using simt::QT;
+using simt::RT;
+constexpr int BUCKET = 26;        // pairs a query's bucket holds between two merges
+constexpr int GROUPED_K = 32;     // largest k of the packed fits' kernels
+constexpr int TILED_K = 256;      // largest k of the tiled kernel
+constexpr int SEEDED_K = 32;      // largest k whose first thresholds come from group minima
 
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem, bool valid) {
-    unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    int src_size = valid ? 4 : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gmem),
-                 "r"(src_size));
+// Shared memory of one CTA after the sweep's stages (k entries per list). Up to k = 54 three
+// CTAs fit an SM.
+struct KnnShared {
+    float *thr;        // [QT] upper bound of the row's k-th distance
+    int32_t *row;      // [QT] query row in the query array
+    int *held;         // [QT] pairs pushed to the row's bucket (may exceed BUCKET)
+    float *bucket_d;   // [QT][BUCKET] (the first tile's group minima before)
+    uint8_t *bucket_r; // [QT][BUCKET] reference within the tile
+    float *list_d;     // [QT][k]
+    int32_t *list_i;   // [QT][k]
+};
+__host__ __device__ constexpr size_t knn_smem_bytes(int k) {
+    return sizeof(float) * (simt::STAGES * simt::STAGE_FLOATS + 3 * QT) + 5 * QT * BUCKET +
+           8 * (size_t)QT * k;
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+__device__ __forceinline__ KnnShared knn_shared(float *smem, int k) {
+    KnnShared s;
+    s.thr = smem + simt::STAGES * simt::STAGE_FLOATS;
+    s.row = reinterpret_cast<int32_t *>(s.thr + QT);
+    s.held = s.row + QT;
+    s.bucket_d = reinterpret_cast<float *>(s.held + QT);
+    s.bucket_r = reinterpret_cast<uint8_t *>(s.bucket_d + QT * BUCKET);
+    s.list_d = reinterpret_cast<float *>(s.bucket_r + QT * BUCKET);
+    s.list_i = reinterpret_cast<int32_t *>(s.list_d + (size_t)QT * k);
+    return s;
 }
 
-// Copy reference rows [r0, r0+RT) into tile[f*RTP + r] (zero fill past nr).
-__device__ __forceinline__ void load_ref_tile(float *tile, const float *ref, int64_t nr, int d,
-                                              int64_t r0) {
-    const int total = RT * d;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-        int r = e / d;
-        int f = e - r * d;
-        int64_t row = r0 + r;
-        bool valid = row < nr;
-        const float *src = valid ? ref + row * (int64_t)d + f : ref;
-        cp_async4(&tile[f * RTP + r], src, valid);
-    }
-}
-
-// Sorted register list insertion: (x, j) is known to beat slot K-1.
-template <int K>
-__device__ __forceinline__ void list_insert(float (&ld)[K], int (&li)[K], float x, int j) {
+// Merge the pairs (x, j) of the lanes in `hits` into a sorted list of k entries in shared memory;
+// one warp, slot s of the list in lane s % 32. Every pair's place is its rank in the list plus its
+// rank among the pairs, and a list entry moves by the pairs before it, so the pairs do not wait
+// for one another (inserting them one by one took about 900 cycles each at k = 50).
+template <int L>
+__device__ __forceinline__ void merge_hits(float *ld, int32_t *li, int k, float x, int32_t j,
+                                           unsigned hits) {
+    const int lane = threadIdx.x & 31;
+    float d[L];
+    int32_t id[L];
+    int shift[L];
 #pragma unroll
-    for (int s = K - 1; s >= 0; --s) {
-        bool here = knn_better(x, j, ld[s], li[s]);
-        bool prev = (s > 0) ? knn_better(x, j, ld[s > 0 ? s - 1 : 0], li[s > 0 ? s - 1 : 0]) : false;
-        if (here) {
-            if (prev) {
-                ld[s] = ld[s - 1 < 0 ? 0 : s - 1];
-                li[s] = li[s - 1 < 0 ? 0 : s - 1];
-            } else {
-                ld[s] = x;
-                li[s] = j;
-            }
+    for (int e = 0; e < L; ++e) {
+        const int s = lane + 32 * e;
+        d[e] = s < k ? ld[s] : CUSCAN_INF;
+        id[e] = s < k ? li[s] : -1;  // after every pair
+        shift[e] = 0;
+    }
+    int at = 0;  // this lane's pair
+    for (unsigned m = hits; m; m &= m - 1) {
+        const int from = __ffs(m) - 1;
+        const float xo = __shfl_sync(0xffffffffu, x, from);
+        const int32_t jo = __shfl_sync(0xffffffffu, j, from);
+        int before = 0;
+#pragma unroll
+        for (int e = 0; e < L; ++e) {
+            const bool b = knn_better(d[e], id[e], xo, jo);
+            before += __popc(__ballot_sync(0xffffffffu, b));
+            shift[e] += b ? 0 : 1;
+        }
+        if (lane == from) at += before;
+        else if (knn_better(xo, jo, x, j)) ++at;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < L; ++e) {
+        const int s = lane + 32 * e;
+        if (s < k && shift[e] && s + shift[e] < k) {
+            ld[s + shift[e]] = d[e];
+            li[s + shift[e]] = id[e];
         }
     }
+    if (((hits >> lane) & 1u) && at < k) {
+        ld[at] = x;
+        li[at] = j;
+    }
+    __syncwarp();
 }
 
-// One block: QB query rows [q0, q0 + QB) x reference rows [r_begin, r_end). Writes the K-best
-// list of each query (first k entries) to out_ids/out_dist rows of width k, at split * stride
-// (partial lists when split); with stride 0 a query qi goes to row qmap[qi] when qmap is set.
-template <int K>
+// First thresholds of the CTA's rows, before its first tile: each of a row's reference groups
+// (two per thread) has a minimum, and the k-th least of these minima bounds the row's k-th
+// distance, so that the first tile queues little more than k pairs per row instead of all 128.
+// minima: [QT][32] group minima (+inf for an empty group).
+__device__ __forceinline__ void seed_thresholds(const KnnShared &sh, const float *minima, int k) {
+    // two threads per row, 16 groups each: the group whose rank is k - 1
+    const int row = threadIdx.x >> 1, half = threadIdx.x & 1;
+    const float *m = minima + row * 32;
+    float v[32];
+#pragma unroll
+    for (int g = 0; g < 32; ++g) v[g] = m[g];
+#pragma unroll
+    for (int g = 0; g < 16; ++g) {
+        const float x = half ? v[16 + g] : v[g];
+        const int at = half ? 16 + g : g;
+        int rank = 0;
+#pragma unroll
+        for (int o = 0; o < 32; ++o) rank += (v[o] < x || (v[o] == x && o < at)) ? 1 : 0;
+        if (rank == k - 1 && sh.thr[row] == CUSCAN_INF) sh.thr[row] = x;
+    }
+}
+
+// One CTA: query rows [q0, q0 + 64) of nq against reference rows [r_begin, r_end) (r_begin a
+// multiple of the tile). Writes each query's sorted list (k entries) to out rows of width k, at
+// part * part_stride when the lists are partial, else to row qmap[qi] (or qi). root: distances
+// leave as their square roots.
+template <int L>
 __device__ __forceinline__ void knn_block(
     const float *__restrict__ query, int64_t nq, const float *__restrict__ ref, int64_t nr, int d,
     int k, int exclude_self, int64_t query_offset, float pad, int64_t q0, int64_t r_begin,
     int64_t r_end, int32_t *__restrict__ out_ids, float *__restrict__ out_dist,
-    int64_t out_split_stride, int64_t split, const int32_t *__restrict__ qmap, float *smem) {
-    float *qs = smem;                         // [d][QB]
-    float *tiles = smem + (size_t)d * QB;     // 2 x [d][RTP]
-    const int tid = threadIdx.x;
-    const int64_t qi = q0 + tid;
-
-    // stage this block's queries transposed (qmap selects a subset of query rows)
-    for (int e = tid; e < QB * d; e += QB) {
-        int q = e / d;
-        int f = e - q * d;
-        int64_t row = q0 + q;
-        int64_t src = row < nq ? (qmap ? (int64_t)qmap[row] : row) : 0;
-        qs[f * QB + q] = row < nq ? query[src * (int64_t)d + f] : 0.0f;
+    int64_t part_stride, int64_t part, bool root, const int32_t *__restrict__ qmap, float *smem) {
+    const KnnShared sh = knn_shared(smem, k);
+    const simt::Place p = simt::place();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid < QT) {
+        const int64_t qi = q0 + tid;
+        sh.row[tid] = qi < nq ? (qmap ? qmap[qi] : (int32_t)qi) : (qmap ? qmap[q0] : (int32_t)q0);
+        // rows past the end keep no pair
+        sh.thr[tid] = qi < nq ? CUSCAN_INF : -CUSCAN_INF;
     }
-
-    float ld[K];
-    int li[K];
-#pragma unroll
-    for (int s = 0; s < K; ++s) {
-        ld[s] = pad;
-        li[s] = (int)nr;
+    for (int e = tid; e < QT * k; e += simt::THREADS) {
+        sh.list_d[e] = pad;
+        sh.list_i[e] = (int32_t)nr;
     }
-    const int64_t self =
-        exclude_self ? (qmap ? (qi < nq ? (int64_t)qmap[qi] : -1) : query_offset + qi) : -1;
-
-    const int tile_floats = d * RTP;
-    int buf = 0;
-    if (r_begin < r_end) {
-        load_ref_tile(tiles, ref, r_end, d, r_begin);
-        cp_async_commit();
-    }
-    for (int64_t r0 = r_begin; r0 < r_end; r0 += RT) {
-        const int64_t next = r0 + RT;
-        if (next < r_end) {
-            load_ref_tile(tiles + (buf ^ 1) * tile_floats, ref, r_end, d, next);
-            cp_async_commit();
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        const float *tile = tiles + buf * tile_floats;
-        float acc[RT];
+    if (tid < QT) sh.held[tid] = 0;
+    __syncthreads();
+    bool first = true;
+    // pairs of the tile that may enter their query's list, one bit each (query i, reference j)
+    auto test = [&](const Packed(&acc)[8][4], int64_t r0, unsigned long long among) {
+        unsigned long long hits = 0;
+        const float4 ta = *reinterpret_cast<const float4 *>(sh.thr + p.tq * 4);
+        const float4 tb = *reinterpret_cast<const float4 *>(sh.thr + 32 + p.tq * 4);
+        const float thr[8] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
 #pragma unroll
-        for (int r = 0; r < RT; ++r) acc[r] = 0.0f;
-        const float *qcol = qs + tid;
-#pragma unroll 2
-        for (int f = 0; f < d; ++f) {
-            const float qv = qcol[f * QB];
-            const float4 *row4 = reinterpret_cast<const float4 *>(tile + f * RTP);
+        for (int i = 0; i < 8; ++i) {
+            float v[8];
+            simt::row_of(acc[i], v);
+            const float m = fminf(fminf(fminf(v[0], v[1]), fminf(v[2], v[3])),
+                                  fminf(fminf(v[4], v[5]), fminf(v[6], v[7])));
+            if (m <= thr[i]) {
+                const int32_t row = sh.row[simt::query_of(p, i)];
+                const int64_t self = exclude_self ? query_offset + row : -1;
 #pragma unroll
-            for (int r4 = 0; r4 < RT / 4; ++r4) {
-                const float4 v = row4[r4];
-                float t0 = qv - v.x, t1 = qv - v.y, t2 = qv - v.z, t3 = qv - v.w;
-                acc[4 * r4 + 0] = __fmaf_rn(t0, t0, acc[4 * r4 + 0]);
-                acc[4 * r4 + 1] = __fmaf_rn(t1, t1, acc[4 * r4 + 1]);
-                acc[4 * r4 + 2] = __fmaf_rn(t2, t2, acc[4 * r4 + 2]);
-                acc[4 * r4 + 3] = __fmaf_rn(t3, t3, acc[4 * r4 + 3]);
+                for (int j = 0; j < 8; ++j) {
+                    const int64_t r = r0 + simt::ref_of(p, j);
+                    if (v[j] <= thr[i] && r < r_end && r != self) hits |= 1ull << (8 * i + j);
+                }
             }
         }
+        return hits & among;
+    };
+    auto nothing = [](int64_t, int) {};
+    auto every = [](int64_t t) { return t; };
+    auto epilogue = [&](int64_t tile, int, const Packed(&acc)[8][4]) {
+        const int64_t r0 = tile * RT;
+        if (first && k > 1 && k <= SEEDED_K) {
+            float *minima = sh.bucket_d;  // [QT][32], the buckets are empty
+            static_assert(5 * BUCKET >= 4 * 32, "group minima fit the buckets");
 #pragma unroll
-        for (int r = 0; r < RT; ++r) {
-            const int64_t j = r0 + r;
-            const float x = acc[r];
-            if (j < r_end && j != self && knn_better(x, (int)j, ld[K - 1], li[K - 1]))
-                list_insert<K>(ld, li, x, (int)j);
-        }
-        __syncthreads();
-        buf ^= 1;
-    }
-    if (qi < nq) {
-        // partial lists (split > 1) stay compact; final rows go to their mapped row
-        const int64_t orow = (qmap && out_split_stride == 0) ? (int64_t)qmap[qi] : qi;
-        int32_t *oi = out_ids + split * out_split_stride + orow * k;
-        float *od = out_dist + split * out_split_stride + orow * k;
+            for (int i = 0; i < 8; ++i) {
+                const int q = simt::query_of(p, i);
+                const int64_t self = exclude_self ? query_offset + sh.row[q] : -1;
+                float v[8];
+                simt::row_of(acc[i], v);
 #pragma unroll
-        for (int s = 0; s < K; ++s) {
-            if (s < k) {
-                oi[s] = li[s];
-                od[s] = ld[s];
+                for (int g = 0; g < 2; ++g) {
+                    float m = CUSCAN_INF;
+#pragma unroll
+                    for (int j = 4 * g; j < 4 * g + 4; ++j) {
+                        const int64_t r = r0 + simt::ref_of(p, j);
+                        if (r < r_end && r != self) m = fminf(m, v[j]);
+                    }
+                    minima[q * 32 + p.tr * 2 + g] = m;
+                }
             }
+            __syncthreads();
+            seed_thresholds(sh, minima, k);
+            __syncthreads();
         }
+        first = false;
+        unsigned long long hits = test(acc, r0, ~0ull);
+        for (;;) {
+            if (hits) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (((hits >> (8 * i)) & 0xffull) == 0) continue;
+                    const int q = simt::query_of(p, i);
+                    float v[8];
+                    simt::row_of(acc[i], v);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if ((hits >> (8 * i + j)) & 1ull) {
+                            const int slot = atomicAdd(&sh.held[q], 1);
+                            if (slot < BUCKET) {
+                                sh.bucket_d[q * BUCKET + slot] = v[j];
+                                sh.bucket_r[q * BUCKET + slot] = (uint8_t)simt::ref_of(p, j);
+                                hits &= ~(1ull << (8 * i + j));
+                            }
+                        }
+                }
+            }
+            // pairs whose bucket was full wait for the merge below
+            const int more = __syncthreads_or(hits != 0);
+            const int held = lane < 16 ? sh.held[warp * 16 + lane] : 0;
+            for (unsigned rows = __ballot_sync(0xffffffffu, held > 0); rows; rows &= rows - 1) {
+                const int q = warp * 16 + __ffs(rows) - 1;
+                const int count = min(__shfl_sync(0xffffffffu, held, q & 15), BUCKET);
+                float x = 0.0f;
+                int32_t j = -1;
+                bool pass = false;
+                if (lane < count) {
+                    x = sh.bucket_d[q * BUCKET + lane];
+                    j = (int32_t)(r0 + sh.bucket_r[q * BUCKET + lane]);
+                    pass = true;
+                }
+                float *ld = sh.list_d + (size_t)q * k;
+                merge_hits<L>(ld, sh.list_i + (size_t)q * k, k, x, j,
+                              __ballot_sync(0xffffffffu, pass));
+                if (lane == 0) {
+                    const float kth = ld[k - 1];
+                    if (kth < sh.thr[q]) sh.thr[q] = kth;
+                    sh.held[q] = 0;
+                }
+            }
+            if (!more) break;  // the next tile's first barrier comes before its pushes
+            __syncthreads();
+            if (hits) hits = test(acc, r0, hits);  // against the tightened thresholds
+        }
+    };
+    if (r_begin < r_end)
+        simt::sweep(query, sh.row, ref, d, r_begin / RT, ceil_div(r_end, (int64_t)RT), r_end, smem,
+                    every, nothing, epilogue);
+    __syncthreads();
+    for (int e = tid; e < QT * k; e += simt::THREADS) {
+        const int q = e / k, s = e - q * k;
+        const int64_t qi = q0 + q;
+        if (qi >= nq) break;
+        const int64_t at = part_stride ? part * part_stride + qi * k + s
+                                       : (qmap ? (int64_t)qmap[qi] : qi) * k + s;
+        const float x = sh.list_d[e];
+        out_ids[at] = sh.list_i[e];
+        out_dist[at] = root ? sqrtf(x) : x;
     }
 }
 
-template <int K>
-__global__ void __launch_bounds__(QB) knn_fp32_kernel(
+// k = 1 (the cell assignment of the refined fits): the nearest reference of each query stays in
+// the registers of its threads, without lists or queues.
+__device__ __forceinline__ void nearest_block(
+    const float *__restrict__ query, int64_t nq, const float *__restrict__ ref, int64_t nr, int d,
+    int exclude_self, int64_t query_offset, float pad, int64_t q0, int64_t r_begin, int64_t r_end,
+    int32_t *__restrict__ out_ids, float *__restrict__ out_dist, int64_t part_stride,
+    int64_t part, bool root, const int32_t *__restrict__ qmap, float *smem) {
+    const KnnShared sh = knn_shared(smem, 1);
+    const simt::Place p = simt::place();
+    const int tid = threadIdx.x;
+    if (tid < QT) {
+        const int64_t qi = q0 + tid;
+        sh.row[tid] = qi < nq ? (qmap ? qmap[qi] : (int32_t)qi) : (qmap ? qmap[q0] : (int32_t)q0);
+    }
+    __syncthreads();
+    float bd[8];
+    int32_t bi[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        bd[i] = pad;
+        bi[i] = (int32_t)nr;
+    }
+    auto nothing = [](int64_t, int) {};
+    auto every = [](int64_t t) { return t; };
+    auto epilogue = [&](int64_t tile, int, const Packed(&acc)[8][4]) {
+        const int64_t r0 = tile * RT;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float v[8];
+            simt::row_of(acc[i], v);
+            const float m = fminf(fminf(fminf(v[0], v[1]), fminf(v[2], v[3])),
+                                  fminf(fminf(v[4], v[5]), fminf(v[6], v[7])));
+            if (!(m <= bd[i])) continue;
+            const int64_t self =
+                exclude_self ? query_offset + sh.row[simt::query_of(p, i)] : -1;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int64_t r = r0 + simt::ref_of(p, j);
+                if (r < r_end && r != self && knn_better(v[j], (int)r, bd[i], bi[i])) {
+                    bd[i] = v[j];
+                    bi[i] = (int32_t)r;
+                }
+            }
+        }
+    };
+    if (r_begin < r_end)
+        simt::sweep(query, sh.row, ref, d, r_begin / RT, ceil_div(r_end, (int64_t)RT), r_end, smem,
+                    every, nothing, epilogue);
+    // the 16 threads of a query: eight lanes of each of two warps
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const float od = __shfl_xor_sync(0xffffffffu, bd[i], o);
+            const int32_t oi = __shfl_xor_sync(0xffffffffu, bi[i], o);
+            if (knn_better(od, oi, bd[i], bi[i])) {
+                bd[i] = od;
+                bi[i] = oi;
+            }
+        }
+    __syncthreads();
+    if (tid >= 64 && (tid & 7) == 0)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            sh.bucket_d[simt::query_of(p, i)] = bd[i];
+            sh.list_i[simt::query_of(p, i)] = bi[i];
+        }
+    __syncthreads();
+    if (tid < 64 && (tid & 7) == 0)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int q = simt::query_of(p, i);
+            const int64_t qi = q0 + q;
+            if (qi >= nq) continue;
+            const float od = sh.bucket_d[q];
+            const int32_t oi = sh.list_i[q];
+            if (knn_better(od, oi, bd[i], bi[i])) {
+                bd[i] = od;
+                bi[i] = oi;
+            }
+            const int64_t at = part_stride ? part * part_stride + qi
+                                           : (qmap ? (int64_t)qmap[qi] : qi);
+            out_ids[at] = bi[i];
+            out_dist[at] = root ? sqrtf(bd[i]) : bd[i];
+        }
+}
+
+// L: list slots per lane (ceil(k / 32)); 0: k = 1.
+template <int L>
+__global__ void __launch_bounds__(simt::THREADS, simt::CTAS_PER_SM) knn_fp32_kernel(
     const float *__restrict__ query, int64_t nq, const float *__restrict__ ref, int64_t nr, int d,
     int k, int exclude_self, int64_t query_offset, float pad, int64_t ref_chunk,
-    int32_t *__restrict__ out_ids, float *__restrict__ out_dist, int64_t out_split_stride,
+    int32_t *__restrict__ out_ids, float *__restrict__ out_dist, int64_t part_stride, int root,
     const int32_t *__restrict__ qmap) {
     extern __shared__ __align__(16) float smem[];
     const int64_t r_begin = (int64_t)blockIdx.y * ref_chunk;
-    int64_t r_end = r_begin + ref_chunk;
-    if (r_end > nr) r_end = nr;
-    knn_block<K>(query, nq, ref, nr, d, k, exclude_self, query_offset, pad,
-                 (int64_t)blockIdx.x * QB, r_begin, r_end, out_ids, out_dist, out_split_stride,
-                 (int64_t)blockIdx.y, qmap, smem);
+    const int64_t r_end = r_begin + ref_chunk < nr ? r_begin + ref_chunk : nr;
+    if constexpr (L == 0)
+        nearest_block(query, nq, ref, nr, d, exclude_self, query_offset, pad,
+                      (int64_t)blockIdx.x * QT, r_begin, r_end, out_ids, out_dist, part_stride,
+                      (int64_t)blockIdx.y, root != 0, qmap, smem);
+    else
+        knn_block<L>(query, nq, ref, nr, d, k, exclude_self, query_offset, pad,
+                     (int64_t)blockIdx.x * QT, r_begin, r_end, out_ids, out_dist, part_stride,
+                     (int64_t)blockIdx.y, root != 0, qmap, smem);
 }
 
-// Packed fits: fit blockIdx.z, query block blockIdx.x, reference chunk blockIdx.y of `splits`
+// Packed fits: fit blockIdx.z, query tile blockIdx.x, reference chunk blockIdx.y of `splits`
 // (the self-kNN of launch_exact_knn_fp32: squared distances, self excluded, +inf padding).
-// Fits with k > K take the per-fit launch instead.
-template <int K>
-__global__ void __launch_bounds__(QB) pack_knn_kernel(const PackFit *__restrict__ fits,
-                                                      int splits) {
+// Fits with k > 32 take the per-fit launch instead.
+__global__ void __launch_bounds__(simt::THREADS, simt::CTAS_PER_SM)
+    pack_knn_kernel(const PackFit *__restrict__ fits, int splits) {
     extern __shared__ __align__(16) float smem[];
     const PackFit &f = fits[blockIdx.z];
-    const int64_t n = f.n, q0 = (int64_t)blockIdx.x * QB;
+    const int64_t n = f.n, q0 = (int64_t)blockIdx.x * QT;
     const int k = f.k;
-    if (k > K || q0 >= n) return;
+    if (k > GROUPED_K || q0 >= n) return;
     const int64_t chunk = ceil_div(ceil_div(n, (int64_t)splits), (int64_t)RT) * RT;
     const int64_t r_begin = (int64_t)blockIdx.y * chunk;
     const int64_t r_end = r_begin + chunk < n ? r_begin + chunk : n;
     if (splits > 1)
-        knn_block<K>(f.x, n, f.x, n, f.d, k, 1, 0, CUSCAN_INF, q0, r_begin, r_end, f.part_ids,
-                     f.part_dist, n * k, (int64_t)blockIdx.y, nullptr, smem);
+        knn_block<1>(f.x, n, f.x, n, f.d, k, 1, 0, CUSCAN_INF, q0, r_begin, r_end, f.part_ids,
+                     f.part_dist, n * k, (int64_t)blockIdx.y, false, nullptr, smem);
     else
-        knn_block<K>(f.x, n, f.x, n, f.d, k, 1, 0, CUSCAN_INF, q0, r_begin, r_end, f.ids, f.dsq,
-                     0, 0, nullptr, smem);
+        knn_block<1>(f.x, n, f.x, n, f.d, k, 1, 0, CUSCAN_INF, q0, r_begin, r_end, f.ids, f.dsq,
+                     0, 0, false, nullptr, smem);
 }
 
-// Merge `splits` sorted partial lists of query q into the final top-k (row orow).
-template <int K>
+// Merge `splits` sorted partial lists of query q into its final row (orow): one warp, the list in
+// shared memory. The entries are taken rank by rank, 32 lists at a time; a rank at which no list
+// can contribute ends the merge, so few of the splits * k entries are read.
+template <int L>
 __device__ __forceinline__ void knn_merge_row(const int32_t *__restrict__ part_ids,
                                               const float *__restrict__ part_dist, int64_t q,
                                               int64_t orow, int k, int splits,
-                                              int64_t split_stride, float pad, int64_t nr,
-                                              int squared, int32_t *__restrict__ ids,
-                                              float *__restrict__ dist) {
-    float ld[K];
-    int li[K];
-#pragma unroll
-    for (int s = 0; s < K; ++s) {
+                                              int64_t part_stride, float pad, int64_t nr,
+                                              bool root, int32_t *__restrict__ ids,
+                                              float *__restrict__ dist, float *ld, int32_t *li) {
+    const int lane = threadIdx.x & 31;
+    for (int s = lane; s < k; s += 32) {
         ld[s] = pad;
-        li[s] = (int)nr;
+        li[s] = (int32_t)nr;
     }
-    for (int sp = 0; sp < splits; ++sp) {
-        const int32_t *pi = part_ids + sp * split_stride + q * k;
-        const float *pd = part_dist + sp * split_stride + q * k;
-        for (int s = 0; s < k; ++s) {
-            float x = pd[s];
-            int j = pi[s];
-            if (knn_better(x, j, ld[K - 1], li[K - 1])) list_insert<K>(ld, li, x, j);
+    __syncwarp();
+    for (int s = 0; s < k; ++s) {
+        bool any = false;
+        for (int b = 0; b < splits; b += 32) {
+            const int sp = b + lane;
+            float x = pad;
+            int32_t j = (int32_t)nr;
+            if (sp < splits) {
+                x = part_dist[sp * part_stride + q * k + s];
+                j = part_ids[sp * part_stride + q * k + s];
+            }
+            const unsigned hits =
+                __ballot_sync(0xffffffffu, knn_better(x, j, ld[k - 1], li[k - 1]));
+            if (hits) {
+                any = true;
+                merge_hits<L>(ld, li, k, x, j, hits);
+            }
         }
+        if (!any) break;
     }
-#pragma unroll
-    for (int s = 0; s < K; ++s) {
-        if (s < k) {
-            ids[orow * k + s] = li[s];
-            float x = ld[s];
-            dist[orow * k + s] = squared ? x : sqrtf(x);
-        }
+    __syncwarp();
+    for (int s = lane; s < k; s += 32) {
+        ids[orow * k + s] = li[s];
+        dist[orow * k + s] = root ? sqrtf(ld[s]) : ld[s];
     }
 }
 
-template <int K>
-__global__ void knn_merge_kernel(const int32_t *__restrict__ part_ids,
-                                 const float *__restrict__ part_dist, int64_t nq, int k,
-                                 int splits, int64_t split_stride, float pad, int64_t nr,
-                                 int squared, int32_t *__restrict__ ids, float *__restrict__ dist,
-                                 const int32_t *__restrict__ qmap) {
-    int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+constexpr int MERGE_WARPS = 4;
+
+template <int L>
+__global__ void __launch_bounds__(32 * MERGE_WARPS)
+    knn_merge_kernel(const int32_t *__restrict__ part_ids, const float *__restrict__ part_dist,
+                     int64_t nq, int k, int splits, int64_t part_stride, float pad, int64_t nr,
+                     int root, int32_t *__restrict__ ids, float *__restrict__ dist,
+                     const int32_t *__restrict__ qmap) {
+    __shared__ float ld[MERGE_WARPS][32 * L];
+    __shared__ int32_t li[MERGE_WARPS][32 * L];
+    const int warp = threadIdx.x >> 5;
+    const int64_t q = (int64_t)blockIdx.x * MERGE_WARPS + warp;
     if (q >= nq) return;
-    knn_merge_row<K>(part_ids, part_dist, q, qmap ? (int64_t)qmap[q] : q, k, splits, split_stride,
-                     pad, nr, squared, ids, dist);
+    knn_merge_row<L>(part_ids, part_dist, q, qmap ? (int64_t)qmap[q] : q, k, splits, part_stride,
+                     pad, nr, root != 0, ids, dist, ld[warp], li[warp]);
 }
 
 // Packed fits: the partial lists of fit blockIdx.y merged into its kNN lists.
-template <int K>
-__global__ void pack_knn_merge_kernel(const PackFit *__restrict__ fits, int splits) {
+__global__ void __launch_bounds__(32 * MERGE_WARPS)
+    pack_knn_merge_kernel(const PackFit *__restrict__ fits, int splits) {
+    __shared__ float ld[MERGE_WARPS][32];
+    __shared__ int32_t li[MERGE_WARPS][32];
     const PackFit &f = fits[blockIdx.y];
-    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f.k > K || q >= f.n) return;
-    knn_merge_row<K>(f.part_ids, f.part_dist, q, q, f.k, splits, f.n * f.k, CUSCAN_INF, f.n, 1,
-                     f.ids, f.dsq);
+    const int warp = threadIdx.x >> 5;
+    const int64_t q = (int64_t)blockIdx.x * MERGE_WARPS + warp;
+    if (f.k > GROUPED_K || q >= f.n) return;
+    knn_merge_row<1>(f.part_ids, f.part_dist, q, q, f.k, splits, f.n * f.k, CUSCAN_INF, f.n, false,
+                     f.ids, f.dsq, ld[warp], li[warp]);
 }
 
 __global__ void sqrt_rows_kernel(float *dist, int64_t count) {
@@ -260,23 +481,46 @@ __global__ void sqrt_rows_kernel(float *dist, int64_t count) {
     if (i < count) dist[i] = sqrtf(dist[i]);
 }
 
-// General k: one thread per query keeps its list in the output row in global memory,
-// exactly like the reference's serial kernel (used for k > 32).
-__global__ void __launch_bounds__(QB) knn_fp32_wide_kernel(
+constexpr int WIDE_Q = 128, WIDE_T = 32, WIDE_TP = 36;
+
+__device__ __forceinline__ void cp_async4_zfill(void *smem, const void *gmem, bool valid) {
+    unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    int src_size = valid ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gmem),
+                 "r"(src_size));
+}
+// Copy reference rows [r0, r0+WIDE_T) into tile[f*WIDE_TP + r] (zero fill past nr).
+__device__ __forceinline__ void load_ref_tile(float *tile, const float *ref, int64_t nr, int d,
+                                              int64_t r0) {
+    const int total = WIDE_T * d;
+    for (int e = threadIdx.x; e < total; e += blockDim.x) {
+        int r = e / d;
+        int f = e - r * d;
+        int64_t row = r0 + r;
+        bool valid = row < nr;
+        const float *src = valid ? ref + row * (int64_t)d + f : ref;
+        cp_async4_zfill(&tile[f * WIDE_TP + r], src, valid);
+    }
+}
+
+// Any k: one thread per query keeps its list in the output row in global memory, like the
+// reference's serial kernel. Only k > 256 takes it, whose lists do not fit shared memory beside
+// the sweep's stages.
+__global__ void __launch_bounds__(WIDE_Q) knn_fp32_wide_kernel(
     const float *__restrict__ query, int64_t nq, const float *__restrict__ ref, int64_t nr, int d,
     int k, int exclude_self, int64_t query_offset, float pad, int32_t *__restrict__ ids,
     float *__restrict__ dist) {
     extern __shared__ __align__(16) float smem[];
     float *qs = smem;
-    float *tile = smem + (size_t)d * QB;
+    float *tile = smem + (size_t)d * WIDE_Q;
     const int tid = threadIdx.x;
-    const int64_t q0 = (int64_t)blockIdx.x * QB;
+    const int64_t q0 = (int64_t)blockIdx.x * WIDE_Q;
     const int64_t qi = q0 + tid;
-    for (int e = tid; e < QB * d; e += QB) {
+    for (int e = tid; e < WIDE_Q * d; e += WIDE_Q) {
         int q = e / d;
         int f = e - q * d;
         int64_t row = q0 + q;
-        qs[f * QB + q] = row < nq ? query[row * (int64_t)d + f] : 0.0f;
+        qs[f * WIDE_Q + q] = row < nq ? query[row * (int64_t)d + f] : 0.0f;
     }
     int32_t *li = ids + (qi < nq ? qi : 0) * (int64_t)k;
     float *ld = dist + (qi < nq ? qi : 0) * (int64_t)k;
@@ -288,20 +532,20 @@ __global__ void __launch_bounds__(QB) knn_fp32_wide_kernel(
     float worst_d = pad;
     int worst_i = (int)nr;
     const int64_t self = exclude_self ? query_offset + qi : -1;
-    for (int64_t r0 = 0; r0 < nr; r0 += RT) {
+    for (int64_t r0 = 0; r0 < nr; r0 += WIDE_T) {
         __syncthreads();
         load_ref_tile(tile, ref, nr, d, r0);
-        cp_async_commit();
-        cp_async_wait<0>();
+        simt::cp_async_commit();
+        simt::cp_async_wait<0>();
         __syncthreads();
-        float acc[RT];
+        float acc[WIDE_T];
 #pragma unroll
-        for (int r = 0; r < RT; ++r) acc[r] = 0.0f;
+        for (int r = 0; r < WIDE_T; ++r) acc[r] = 0.0f;
         for (int f = 0; f < d; ++f) {
-            const float qv = qs[f * QB + tid];
-            const float4 *row4 = reinterpret_cast<const float4 *>(tile + f * RTP);
+            const float qv = qs[f * WIDE_Q + tid];
+            const float4 *row4 = reinterpret_cast<const float4 *>(tile + f * WIDE_TP);
 #pragma unroll
-            for (int r4 = 0; r4 < RT / 4; ++r4) {
+            for (int r4 = 0; r4 < WIDE_T / 4; ++r4) {
                 const float4 v = row4[r4];
                 float t0 = qv - v.x, t1 = qv - v.y, t2 = qv - v.z, t3 = qv - v.w;
                 acc[4 * r4 + 0] = __fmaf_rn(t0, t0, acc[4 * r4 + 0]);
@@ -311,7 +555,7 @@ __global__ void __launch_bounds__(QB) knn_fp32_wide_kernel(
             }
         }
         if (qi < nq) {
-            for (int r = 0; r < RT; ++r) {
+            for (int r = 0; r < WIDE_T; ++r) {
                 const int64_t j = r0 + r;
                 const float x = acc[r];
                 if (j >= nr || j == self || !knn_better(x, (int)j, worst_d, worst_i)) continue;
@@ -330,42 +574,32 @@ __global__ void __launch_bounds__(QB) knn_fp32_wide_kernel(
     }
 }
 
-// Split the reference range when the query blocks alone cannot fill the GPU: `splits` CTAs per
-// query block, each over `chunk` references.
+// Split the reference range when the query tiles alone cannot fill the GPU: `splits` CTAs per
+// query tile, each over `chunk` references.
 void knn_split_plan(const cuscan_ctx *ctx, int64_t nq, int64_t nr, int64_t &splits,
-                    int64_t &chunk) {
-    const int64_t qblocks = ceil_div(nq, QB);
-    splits = 1;
-    const int64_t target = 2 * (int64_t)ctx->sm_count;
-    if (qblocks < target) splits = ceil_div(target, qblocks);
-    const int64_t max_splits = ceil_div(nr, (int64_t)RT * 8);
-    if (splits > max_splits) splits = max_splits;
-    if (splits > 1024) splits = 1024;
-    if (splits < 1) splits = 1;
-    chunk = ceil_div(ceil_div(nr, splits), RT) * RT;
-    splits = ceil_div(nr, chunk);
+                    int64_t &chunk, int d, int k) {
+    // every part fills lists of its own: about 4 k merged pairs per row, against 384 d cycles per
+    // tile (both per resident CTA)
+    simt::split_plan(ctx->sm_count, ceil_div(nq, (int64_t)QT), nr, 2,
+                     1.0 + 2.0 * (double)k / (double)d, splits, chunk);
 }
 
-template <int K>
+template <int L>
 int run_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, int64_t nr, int d,
             int k, int exclude_self, int64_t query_offset, int squared, int32_t *ids, float *dist,
             cudaStream_t s, Buffer &scratch_ids, Buffer &scratch_dist, const int32_t *qmap) {
     const float pad = squared ? std::numeric_limits<float>::infinity() : 3.40282346638528859812e+38f;
-    const int64_t qblocks = ceil_div(nq, QB);
     int64_t splits = 1, chunk = 0;
-    knn_split_plan(ctx, nq, nr, splits, chunk);
-    const size_t smem = ((size_t)d * QB + 2 * (size_t)d * RTP) * sizeof(float);
-    if (int rc = allow_dynamic_smem(ctx, knn_fp32_kernel<K>, smem)) return rc;
-    dim3 grid((unsigned)qblocks, (unsigned)splits);
+    knn_split_plan(ctx, nq, nr, splits, chunk, d, k);
+    const size_t smem = knn_smem_bytes(k);
+    if (int rc = allow_dynamic_smem(ctx, knn_fp32_kernel<L>, smem)) return rc;
+    const dim3 grid((unsigned)ceil_div(nq, (int64_t)QT), (unsigned)splits);
     if (splits == 1) {
-        CUSCAN_KERNEL(knn_fp32_kernel<K>, grid, QB, smem, s, query, nq, ref, nr, d, k,
-                      exclude_self, query_offset, pad, chunk, ids, dist, 0, qmap);
+        if (!squared && qmap)
+            return fail(ctx, CUSCAN_INVALID_INPUT, "row-subset kNN is squared only");
+        CUSCAN_KERNEL(knn_fp32_kernel<L>, grid, simt::THREADS, smem, s, query, nq, ref, nr, d, k,
+                      exclude_self, query_offset, pad, chunk, ids, dist, 0, squared ? 0 : 1, qmap);
         CUSCAN_LAUNCH(ctx, "knn_fp32_kernel");
-        if (!squared && nq * k > 0) {
-            if (qmap) return fail(ctx, CUSCAN_INVALID_INPUT, "row-subset kNN is squared only");
-            CUSCAN_KERNEL(sqrt_rows_kernel, (unsigned)ceil_div(nq * k, 256), 256, 0, s, dist, nq * k);
-            CUSCAN_LAUNCH(ctx, "sqrt_rows_kernel");
-        }
         return CUSCAN_OK;
     }
     const int64_t stride = nq * k;
@@ -373,85 +607,70 @@ int run_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, i
     if (rc) return rc;
     rc = ensure(ctx, scratch_dist, (size_t)(stride * splits) * sizeof(float), "kNN partial distances");
     if (rc) return rc;
-    CUSCAN_KERNEL(knn_fp32_kernel<K>, grid, QB, smem, s, query, nq, ref, nr, d, k, exclude_self,
-                  query_offset, pad, chunk, as<int32_t>(scratch_ids), as<float>(scratch_dist),
-                  stride, qmap);
+    CUSCAN_KERNEL(knn_fp32_kernel<L>, grid, simt::THREADS, smem, s, query, nq, ref, nr, d, k,
+                  exclude_self, query_offset, pad, chunk, as<int32_t>(scratch_ids),
+                  as<float>(scratch_dist), stride, 0, qmap);
     CUSCAN_LAUNCH(ctx, "knn_fp32_kernel");
-    CUSCAN_KERNEL(knn_merge_kernel<K>, (unsigned)ceil_div(nq, 128), 128, 0, s,
-                  as<int32_t>(scratch_ids), as<float>(scratch_dist), nq, k, (int)splits, stride,
-                  pad, nr, squared, ids, dist, qmap);
+    constexpr int M = L == 0 ? 1 : L;
+    CUSCAN_KERNEL(knn_merge_kernel<M>, (unsigned)ceil_div(nq, (int64_t)MERGE_WARPS),
+                  32 * MERGE_WARPS, 0, s, as<int32_t>(scratch_ids), as<float>(scratch_dist), nq, k,
+                  (int)splits, stride, pad, nr, squared ? 0 : 1, ids, dist, qmap);
     CUSCAN_LAUNCH(ctx, "knn_merge_kernel");
     return CUSCAN_OK;
 }
 
 }  // namespace
 
-size_t exact_knn_scratch_elems(const cuscan_ctx *ctx, int64_t nq, int64_t nr, int k) {
-    int64_t splits = 1, chunk = 0;
-    knn_split_plan(ctx, nq, nr, splits, chunk);
-    return splits > 1 ? (size_t)(nq * k * splits) : 0;
-}
-
 int launch_exact_knn_fp32(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref,
                           int64_t nr, int d, int k, int exclude_self, int64_t query_offset,
                           int squared, int32_t *ids, float *dist, cudaStream_t s,
                           Buffer &scratch_ids, Buffer &scratch_dist, const int32_t *qmap) {
     if (nq == 0) return CUSCAN_OK;
-    const size_t smem_needed = ((size_t)d * QB + 2 * (size_t)d * RTP) * sizeof(float);
-    if (smem_needed > 200 * 1024)
+    if (d > CUSCAN_PACK_MAX_FEATURES)
         return fail(ctx, CUSCAN_CAPACITY,
                     "feature count %d exceeds the shared-memory staging limit of the kNN kernel "
                     "(at most 256 features)", d);
-    if (k == 1)  // nearest row only (the cell assignment of the bf16-refined fits)
-        return run_knn<1>(ctx, query, nq, ref, nr, d, k, exclude_self, query_offset, squared, ids,
-                          dist, s, scratch_ids, scratch_dist, qmap);
-    if (k <= 8)
-        return run_knn<8>(ctx, query, nq, ref, nr, d, k, exclude_self, query_offset, squared, ids,
-                          dist, s, scratch_ids, scratch_dist, qmap);
-    if (k <= 16)
-        return run_knn<16>(ctx, query, nq, ref, nr, d, k, exclude_self, query_offset, squared,
-                           ids, dist, s, scratch_ids, scratch_dist, qmap);
-    if (k <= 32)
-        return run_knn<32>(ctx, query, nq, ref, nr, d, k, exclude_self, query_offset, squared,
-                           ids, dist, s, scratch_ids, scratch_dist, qmap);
-    if (qmap) return fail(ctx, CUSCAN_CAPACITY, "row-subset kNN supports k <= 32");
-    const float pad = squared ? std::numeric_limits<float>::infinity() : 3.40282346638528859812e+38f;
-    const size_t smem = ((size_t)d * QB + (size_t)d * RTP) * sizeof(float);
-    if (int rc = allow_dynamic_smem(ctx, knn_fp32_wide_kernel, smem)) return rc;
-    CUSCAN_KERNEL(knn_fp32_wide_kernel, (unsigned)ceil_div(nq, QB), QB, smem, s,
-        query, nq, ref, nr, d, k, exclude_self, query_offset, pad, ids, dist);
-    CUSCAN_LAUNCH(ctx, "knn_fp32_wide_kernel");
-    if (!squared) {
-        CUSCAN_KERNEL(sqrt_rows_kernel, (unsigned)ceil_div(nq * k, 256), 256, 0, s, dist, nq * k);
-        CUSCAN_LAUNCH(ctx, "sqrt_rows_kernel");
+    if (k > TILED_K) {
+        if (qmap) return fail(ctx, CUSCAN_CAPACITY, "row-subset kNN supports k <= 256");
+        const float pad = squared ? std::numeric_limits<float>::infinity() : 3.40282346638528859812e+38f;
+        const size_t smem = ((size_t)d * WIDE_Q + (size_t)d * WIDE_TP) * sizeof(float);
+        if (int rc = allow_dynamic_smem(ctx, knn_fp32_wide_kernel, smem)) return rc;
+        CUSCAN_KERNEL(knn_fp32_wide_kernel, (unsigned)ceil_div(nq, WIDE_Q), WIDE_Q, smem, s,
+            query, nq, ref, nr, d, k, exclude_self, query_offset, pad, ids, dist);
+        CUSCAN_LAUNCH(ctx, "knn_fp32_wide_kernel");
+        if (!squared) {
+            CUSCAN_KERNEL(sqrt_rows_kernel, (unsigned)ceil_div(nq * k, 256), 256, 0, s, dist, nq * k);
+            CUSCAN_LAUNCH(ctx, "sqrt_rows_kernel");
+        }
+        return CUSCAN_OK;
     }
-    return CUSCAN_OK;
-}
-
-template <int K>
-static int run_pack_knn(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max,
-                        int d_max, int splits, cudaStream_t s, int64_t &launches) {
-    const size_t smem = ((size_t)d_max * QB + 2 * (size_t)d_max * RTP) * sizeof(float);
-    if (int rc = allow_dynamic_smem(ctx, pack_knn_kernel<K>, smem)) return rc;
-    dim3 grid((unsigned)ceil_div(n_max, QB), (unsigned)splits, (unsigned)count);
-    CUSCAN_KERNEL(pack_knn_kernel<K>, grid, QB, smem, s, fits, splits);
-    ++launches;
-    if (splits > 1) {
-        dim3 mg((unsigned)ceil_div(n_max, 128), (unsigned)count);
-        CUSCAN_KERNEL(pack_knn_merge_kernel<K>, mg, 128, 0, s, fits, splits);
-        ++launches;
-    }
-    CUSCAN_LAUNCH(ctx, "pack_knn_kernel");
-    return CUSCAN_OK;
+#define CUSCAN_RUN_KNN(L)                                                                        \
+    run_knn<L>(ctx, query, nq, ref, nr, d, k, exclude_self, query_offset, squared, ids, dist, s, \
+               scratch_ids, scratch_dist, qmap)
+    if (k == 1) return CUSCAN_RUN_KNN(0);
+    if (k <= 32) return CUSCAN_RUN_KNN(1);
+    if (k <= 64) return CUSCAN_RUN_KNN(2);
+    if (k <= 128) return CUSCAN_RUN_KNN(4);
+    return CUSCAN_RUN_KNN(8);
+#undef CUSCAN_RUN_KNN
 }
 
 int launch_pack_knn(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int d_max,
                     int k_max, int splits, cudaStream_t s, int64_t &launches) {
-    if (((size_t)d_max * QB + 2 * (size_t)d_max * RTP) * sizeof(float) > 200 * 1024)
+    if (d_max > CUSCAN_PACK_MAX_FEATURES)
         return fail(ctx, CUSCAN_CAPACITY, "feature count %d exceeds the kNN staging limit", d_max);
-    if (k_max <= 8) return run_pack_knn<8>(ctx, fits, count, n_max, d_max, splits, s, launches);
-    if (k_max <= 16) return run_pack_knn<16>(ctx, fits, count, n_max, d_max, splits, s, launches);
-    return run_pack_knn<32>(ctx, fits, count, n_max, d_max, splits, s, launches);
+    const size_t smem = knn_smem_bytes(k_max);
+    if (int rc = allow_dynamic_smem(ctx, pack_knn_kernel, smem)) return rc;
+    const dim3 grid((unsigned)ceil_div(n_max, (int64_t)QT), (unsigned)splits, (unsigned)count);
+    CUSCAN_KERNEL(pack_knn_kernel, grid, simt::THREADS, smem, s, fits, splits);
+    ++launches;
+    if (splits > 1) {
+        const dim3 mg((unsigned)ceil_div(n_max, (int64_t)MERGE_WARPS), (unsigned)count);
+        CUSCAN_KERNEL(pack_knn_merge_kernel, mg, 32 * MERGE_WARPS, 0, s, fits, splits);
+        ++launches;
+    }
+    CUSCAN_LAUNCH(ctx, "pack_knn_kernel");
+    return CUSCAN_OK;
 }
 
 }  // namespace cuscan

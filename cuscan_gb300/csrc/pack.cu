@@ -38,6 +38,7 @@
 
 #include "common.cuh"
 #include "forest.cuh"
+#include "simt.cuh"
 #include "workspace.cuh"
 
 namespace cuscan {
@@ -52,7 +53,7 @@ struct PackWorkspace {
 
 namespace {
 
-constexpr int kKnnRows = 128;      // query rows per block of the kNN and candidate sweeps
+constexpr int kKnnRows = simt::QT;  // query rows per block of the kNN and candidate sweeps
 constexpr int kGroupedMaxK = 32;   // larger k takes the per-fit kNN launch
 constexpr int kFirstBatch = 3;     // rounds launched before the first host read
 constexpr int kNextBatch = 2;
@@ -127,7 +128,7 @@ struct PackLayout {
 // over (the plan of a fit alone), chunks of at least 256 rows.
 int64_t pack_splits(const cuscan_ctx *ctx, int count, int64_t n_max) {
     const int64_t blocks = (int64_t)count * ceil_div(n_max, kKnnRows);
-    const int64_t target = 2 * (int64_t)ctx->sm_count;
+    const int64_t target = (int64_t)simt::CTAS_PER_SM * ctx->sm_count;
     int64_t splits = blocks < target ? ceil_div(target, blocks) : 1;
     const int64_t cap = ceil_div(n_max, 256);
     if (splits > cap) splits = cap;

@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "forest.cuh"
+#include "simt.cuh"
 #include "workspace.cuh"
 
 struct cuscan_predictor {
@@ -637,7 +638,8 @@ int64_t cuscan_predict_workspace_bytes(const cuscan_predictor *p, int64_t m) {
     if (!p || m <= 0) return 0;
     const int64_t k = 2 * (int64_t)p->s;
     // query rows, candidate ids and distances, split-search partial lists
-    const int64_t split = 8 * k * 128 * (4 * (int64_t)kSMs + ceil_div(m, (int64_t)128));
+    const int64_t split = 8 * k * simt::QT *
+                          simt::split_plan_max_ctas(kSMs, ceil_div(m, (int64_t)simt::QT));
     return (int64_t)sizeof(float) * m * p->d + 8 * m * k + split + (1 << 20);
 }
 
