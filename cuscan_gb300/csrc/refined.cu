@@ -22,12 +22,13 @@
 // |x| into [2^14, 2^15)); and split bf16, x = hi + lo with hi = bf16(x) and lo = bf16(x - hi),
 // whose dot product hi.hi' + hi.lo' + lo.hi' (three K blocks per 64 features) misses x.y by
 // about 3 * 2^-16 |x||y| instead of 2^-7. A bf16-refined fit whose plain bf16 screen leaves too
-// many kNN rows inconclusive screens again with split bf16 (d <= 64, where a tile of hi and lo
-// blocks fits two pipeline stages) or with scaled fp16 operands (wider rows), and keeps that
-// format for its Borůvka rounds.
+// many kNN rows inconclusive screens again with split bf16 (d <= 64: three MMAs per block) or
+// with scaled fp16 operands (wider rows: one MMA per block), and keeps that format for its
+// Borůvka rounds. Rows of up to 256 features take the screens.
 #include <cuda_bf16.h>
 
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 #include "forest.cuh"
@@ -70,7 +71,7 @@ struct Params {
     const int32_t *tile_lo;   // [n_tiles] label range of 256-row tiles (Borůvka)
     const int32_t *tile_hi;
     int64_t n, n_tiles, n_qblocks, n_chunks;
-    int kblocks, stages;
+    int kblocks, stages, stage_blocks;  // stage_blocks: K blocks per ring stage (divides nbk)
     // one-sided Borůvka with fewer query blocks than SMs: CTAs per query block, each running one
     // contiguous part of the block's tile order (work item qi = block qi / splits, part qi %
     // splits; appends then take their slots with atomics and the row bounds are min-reduced)
@@ -514,10 +515,16 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t a_bytes = (uint32_t)P.nbk * KBLOCK_A;
-    const uint32_t b_bytes = (uint32_t)P.nbk * KBLOCK_B;
+    const uint32_t b_bytes = (uint32_t)P.nbk * KBLOCK_B;  // one tile of the copy
     uint8_t *sA = smem;
+    // Ring of reference tiles. A stage holds a whole tile of up to two 64-column K blocks, one
+    // block of a wider one, so that rows of up to 256 features (four blocks of A, 64 KB) still
+    // leave three stages. One wait and commit per block for every width measured 118.2 ms against
+    // 102.7 ms at 500,000 x 128: the MMAs of a tile start when its TMEM buffer frees, and the
+    // waits between them add to that chain.
     uint8_t *sB = smem + a_bytes;
-    float *pbuf = (float *)(sB + (size_t)P.stages * b_bytes);      // [EPI_WARPS][PB_STRIDE]
+    const uint32_t stage_bytes = (uint32_t)P.stage_blocks * KBLOCK_B;
+    float *pbuf = (float *)(sB + (size_t)P.stages * stage_bytes);  // [EPI_WARPS][PB_STRIDE]
     float *vstage = pbuf + EPI_WARPS * PB_STRIDE;                    // [EPI_WARPS][32][VSTRIDE]
     uint64_t *bars = (uint64_t *)(vstage + EPI_WARPS * 32 * VSTRIDE);
     uint64_t *full = bars;
@@ -615,18 +622,25 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
                     const int64_t t = ROT ? (int64_t)knn_tile((int32_t)P.n_tiles, (int32_t)wa, rot, (int32_t)i)
                                           : vis_tile<SYM>(P, qb, wa, i);
                     if (tile_skipped<BORUVKA>(P, t, qlo, qhi)) continue;
-                    if (!mbar_wait(&empty[stage], phase ^ 1, abort, P.error)) break;
-                    issued[stage] = 2u | phase;
-                    mbar_expect_tx(&full[stage], b_bytes);
                     const uint8_t *bsrc = P.xt + (uint64_t)t * (uint64_t)b_bytes;
-                    uint8_t *bdst = sB + (size_t)stage * b_bytes;
-                    for (int kb = 0; kb < P.nbk; ++kb)
-                        bulk_g2s(bdst + kb * KBLOCK_B, bsrc + (uint64_t)kb * KBLOCK_B, KBLOCK_B,
-                                 &full[stage]);
-                    if (++stage == P.stages) {
-                        stage = 0;
-                        phase ^= 1;
+                    bool ok = true;
+                    for (int k0 = 0; k0 < P.nbk; k0 += P.stage_blocks) {
+                        if (!mbar_wait(&empty[stage], phase ^ 1, abort, P.error)) {
+                            ok = false;
+                            break;
+                        }
+                        issued[stage] = 2u | phase;
+                        mbar_expect_tx(&full[stage], stage_bytes);
+                        uint8_t *bdst = sB + (size_t)stage * stage_bytes;
+                        for (int kb = 0; kb < P.stage_blocks; ++kb)
+                            bulk_g2s(bdst + kb * KBLOCK_B, bsrc + (uint64_t)(k0 + kb) * KBLOCK_B,
+                                     KBLOCK_B, &full[stage]);
+                        if (++stage == P.stages) {
+                            stage = 0;
+                            phase ^= 1;
+                        }
                     }
+                    if (!ok) break;
                     if (ROT) atomicAdd(P.cursor, 1ull);
                 }
             }
@@ -648,68 +662,98 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
             int stage = 0;
             uint32_t phase = 0, a_phase = 0;
             uint32_t tcount = 0, a_commits = 0;
-            const uint32_t a_base = smem_u32(sA), b_base = smem_u32(sB);
-            for (uint32_t li = 0; !*abort; ++li) {
-                int64_t qi = blockIdx.x + (int64_t)li * gridDim.x;
-                if (ROT) {  // kNN sweeps: the block the producer took
-                    const uint32_t rs = li & 3;
-                    if (!mbar_wait(&rot_full[rs], (li >> 2) & 1, abort, P.error)) break;
-                    qi = *(volatile int64_t *)&rot_blk[rs];
-                    mbar_arrive(&rot_empty[rs]);
-                }
-                if (qi >= P.n_qblocks * P.splits) break;
-                const int64_t qb = block_at<SYM>(P, qi / P.splits);
-                const int64_t part = qi % P.splits;
-                if (!mbar_wait(a_full, a_phase, abort, P.error)) break;
-                a_phase ^= 1;
-                fence_after();
-                int32_t qlo = 0, qhi = 0;
-                if (BORUVKA) qblock_range(P, qb, qlo, qhi);
-                const int64_t wa = window_start(P, qb);
-                const int64_t nvis = vis_count<SYM>(P, qb);
-                const int64_t i_hi = (part + 1) * nvis / P.splits;
-                bool ok = true;
-                for (int64_t i = part * nvis / P.splits; i < i_hi; ++i) {
-                    const int64_t t = vis_tile<SYM>(P, qb, wa, i);
-                    if (tile_skipped<BORUVKA>(P, t, qlo, qhi)) continue;
-                    const uint32_t b = tcount & 1, tp = (tcount >> 1) & 1;
-                    if (!mbar_wait(&t_empty[b], tp ^ 1, abort, P.error)) { ok = false; break; }
-                    fence_after();
-                    if (!mbar_wait(&full[stage], phase, abort, P.error)) { ok = false; break; }
-                    fence_after();
-                    const uint32_t d_tmem = tmem_base + b * BN;
-                    const uint32_t bstage = b_base + (uint32_t)stage * b_bytes;
-                    for (int kb = 0; kb < P.kblocks; ++kb) {
+            // Descriptors of the first K step of A and of ring stage 0; a K step is 32 bytes, a
+            // block of A KBLOCK_A, so each further descriptor is one addition (in 16-byte units).
+            const uint64_t a_desc = desc_sw128(smem_u32(sA)), b_desc = desc_sw128(smem_u32(sB));
+            // One tile's MMAs for KB K blocks (SB of them per ring stage), fully unrolled: they are
+            // issued when the tile's TMEM buffer frees, so every instruction between that and the
+            // last MMA adds to the chain MMA -> epilogue -> MMA. Split copies: a hi block of B
+            // meets the hi and the lo block of A, a lo block of B (j >= KB) the hi block.
+            auto issue = [&](auto kb_c, auto sb_c, auto split_c, uint32_t b, uint32_t tp) -> bool {
+                constexpr int KB = decltype(kb_c)::value, SB = decltype(sb_c)::value;
+                constexpr bool SPLIT = decltype(split_c)::value;
+                constexpr int NB = SPLIT ? 2 * KB : KB;
+                const uint32_t d_tmem = tmem_base + b * BN;
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {
-                            const uint64_t ad = desc_sw128(a_base + kb * KBLOCK_A + ks * 32);
-                            const uint64_t bd = desc_sw128(bstage + kb * KBLOCK_B + ks * 32);
-                            mma_16bit(d_tmem, ad, bd, P.idesc, (kb | ks) != 0);
-                        }
-                        if (P.split) {
-                            // lo x hi and hi x lo (blocks kblocks + kb hold the lo parts)
-                            const uint32_t lo = (uint32_t)(P.kblocks + kb);
+                for (int k0 = 0; k0 < NB; k0 += SB) {
+                    if (!mbar_wait(&full[stage], phase, abort, P.error)) return false;
+                    if (k0 == 0 && !mbar_wait(&t_empty[b], tp ^ 1, abort, P.error)) return false;
+                    fence_after();
+                    const uint64_t bd = b_desc + (uint32_t)stage * (SB * KBLOCK_B >> 4);
 #pragma unroll
-                            for (int ks = 0; ks < 4; ++ks) {
-                                mma_16bit(d_tmem, desc_sw128(a_base + lo * KBLOCK_A + ks * 32),
-                                          desc_sw128(bstage + kb * KBLOCK_B + ks * 32), P.idesc, 1u);
-                                mma_16bit(d_tmem, desc_sw128(a_base + kb * KBLOCK_A + ks * 32),
-                                          desc_sw128(bstage + lo * KBLOCK_B + ks * 32), P.idesc, 1u);
-                            }
+                    for (int j = k0; j < k0 + SB; ++j) {
+                        const int ja = j < KB ? j : j - KB;  // the hi block of A
+#pragma unroll
+                        for (int ks = 0; ks < 4; ++ks)
+                            mma_16bit(d_tmem, a_desc + ((ja * KBLOCK_A + ks * 32) >> 4),
+                                      bd + (((j - k0) * KBLOCK_B + ks * 32) >> 4), P.idesc,
+                                      (j | ks) != 0);
+                        if (SPLIT && j < KB) {
+#pragma unroll
+                            for (int ks = 0; ks < 4; ++ks)
+                                mma_16bit(d_tmem, a_desc + (((KB + j) * KBLOCK_A + ks * 32) >> 4),
+                                          bd + (((j - k0) * KBLOCK_B + ks * 32) >> 4), P.idesc,
+                                          1u);
                         }
                     }
                     mma_commit(&empty[stage]);
-                    mma_commit(&t_full[b]);
                     if (++stage == P.stages) {
                         stage = 0;
                         phase ^= 1;
                     }
-                    ++tcount;
                 }
-                mma_commit(a_empty);
-                ++a_commits;
-                if (!ok) break;
-            }
+                mma_commit(&t_full[b]);
+                return true;
+            };
+            auto blocks = [&](auto kb_c, auto sb_c, auto split_c) {
+                for (uint32_t li = 0; !*abort; ++li) {
+                    int64_t qi = blockIdx.x + (int64_t)li * gridDim.x;
+                    if (ROT) {  // kNN sweeps: the block the producer took
+                        const uint32_t rs = li & 3;
+                        if (!mbar_wait(&rot_full[rs], (li >> 2) & 1, abort, P.error)) break;
+                        qi = *(volatile int64_t *)&rot_blk[rs];
+                        mbar_arrive(&rot_empty[rs]);
+                    }
+                    if (qi >= P.n_qblocks * P.splits) break;
+                    const int64_t qb = block_at<SYM>(P, qi / P.splits);
+                    const int64_t part = qi % P.splits;
+                    if (!mbar_wait(a_full, a_phase, abort, P.error)) break;
+                    a_phase ^= 1;
+                    fence_after();
+                    int32_t qlo = 0, qhi = 0;
+                    if (BORUVKA) qblock_range(P, qb, qlo, qhi);
+                    const int64_t wa = window_start(P, qb);
+                    const int64_t nvis = vis_count<SYM>(P, qb);
+                    const int64_t i_hi = (part + 1) * nvis / P.splits;
+                    bool ok = true;
+                    for (int64_t i = part * nvis / P.splits; i < i_hi; ++i) {
+                        if (BORUVKA &&
+                            tile_skipped<BORUVKA>(P, vis_tile<SYM>(P, qb, wa, i), qlo, qhi))
+                            continue;
+                        if (!issue(kb_c, sb_c, split_c, tcount & 1, (tcount >> 1) & 1)) {
+                            ok = false;
+                            break;
+                        }
+                        ++tcount;
+                    }
+                    mma_commit(a_empty);
+                    ++a_commits;
+                    if (!ok) break;
+                }
+            };
+            using std::integral_constant;
+            constexpr integral_constant<int, 1> c1{};
+            constexpr integral_constant<int, 2> c2{};
+            if (P.split)  // d <= 64
+                blocks(c1, c2, std::true_type{});
+            else if (P.kblocks == 1)
+                blocks(c1, c1, std::false_type{});
+            else if (P.kblocks == 2)
+                blocks(c2, c2, std::false_type{});
+            else if (P.kblocks == 3)
+                blocks(integral_constant<int, 3>{}, c1, std::false_type{});
+            else
+                blocks(integral_constant<int, 4>{}, c1, std::false_type{});
             atomicAdd(reinterpret_cast<unsigned long long *>(P.error + 2),
                       (unsigned long long)tcount);
             // wait until every issued MMA has completed before TMEM can be released
@@ -1613,24 +1657,26 @@ float fp16_scale(float absmax) {
 int refined_available() { return 1; }
 
 struct Layout {
-    int d_pad, kblocks, stages;
+    int d_pad, kblocks, stages, stage_blocks;
     int nbk, split;  // K blocks per tile row of the copy; split bf16 copy
     int64_t n_pad, n_tiles, n_qblocks;
     size_t smem;
 };
 
-// Tiling of n rows of d features; split copies hold hi and lo blocks, so a tile (the unit of a
-// pipeline stage) is twice as large and fits two stages only for d <= 64.
+// Tiling of n rows of d features: up to four 64-column K blocks. Split copies hold hi and lo
+// blocks and cost three MMAs per block pair; they are used up to d = 64 (wider rows take scaled
+// fp16 operands, one MMA per block).
 static bool refined_layout(int64_t n, int d, Layout &L, bool split = false) {
     L.d_pad = (int)ceil_div(d, 64) * 64;
-    if (L.d_pad > 128) return false;
+    if (L.d_pad > (split ? 64 : 256)) return false;
     L.kblocks = L.d_pad / 64;
     L.split = split ? 1 : 0;
     L.nbk = split ? 2 * L.kblocks : L.kblocks;
     L.n_tiles = ceil_div(n, BN);
     L.n_pad = L.n_tiles * BN;
     L.n_qblocks = ceil_div(n, BM);
-    const size_t a = (size_t)L.nbk * KBLOCK_A, b = (size_t)L.nbk * KBLOCK_B;
+    L.stage_blocks = L.nbk <= 2 ? L.nbk : 1;
+    const size_t a = (size_t)L.nbk * KBLOCK_A, b = (size_t)L.stage_blocks * KBLOCK_B;
     const size_t fixed = a + (size_t)EPI_WARPS * (PB_STRIDE + 32 * VSTRIDE) * 4 +
                          256 + 1024;
     int st = (int)((227 * 1024 - fixed) / b);
@@ -1817,6 +1863,7 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
     P.nbk = L.nbk;
     P.split = L.split;
     P.stages = L.stages;
+    P.stage_blocks = L.stage_blocks;
     P.cursor = as<unsigned long long>(R.cursor);
     // parts of at least 128 tiles: the start of a work item (A tile, pipeline fill) stays small
     // against its tiles, and the fits of a serving stream (under 32,768 rows) keep one CTA per
