@@ -309,11 +309,9 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
                                    b.knn_ids_tmp, b.knn_dist_tmp);
     if (rc) return rc;
     CUSCAN_CUDA(ctx, cudaEventRecord(ev[1], s));
-    if ((rc = forest_core(ctx, knn_sq, n, k, min_samples, core_sq, s))) return rc;
-    CUSCAN_CUDA(ctx, cudaEventRecord(ev[2], s));
-    // ---- mst: kNN seed then Borůvka rounds (estimator.rs:689-874) ----
-    if ((rc = forest_seed(ctx, b, core_sq, knn_ids, knn_sq, n, k, label, mst_src, mst_dst,
-                          mst_wsq, s)))
+    // ---- core column; mst: kNN seed then Borůvka rounds (estimator.rs:689-874) ----
+    if ((rc = forest_seed(ctx, b, core_sq, knn_ids, knn_sq, n, k, min_samples, label, mst_src,
+                          mst_dst, mst_wsq, s)))
         return rc;
     DevStatus *hs = f->host_status;
     if ((rc = read_status(ctx, b.status, hs, s))) return rc;
@@ -332,9 +330,10 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
         if (rounds > 64) return fail(ctx, CUSCAN_NUMERICAL, "Boruvka did not converge");
         if ((rc = forest_sort_by_component(ctx, b, data, core_sq, label, n, d, s))) return rc;
         unsigned long long *row_keys = as<unsigned long long>(b.row_keys);
-        if ((rc = launch_fill_u64(ctx, row_keys, n, ~0ull, s))) return rc;
+        const bool small = forest_small(n);  // its sort clears the keys and fills the label ranges
+        if (!small && (rc = launch_fill_u64(ctx, row_keys, n, ~0ull, s))) return rc;
         CUSCAN_CUDA(ctx, cudaEventRecord(ev[4], s));
-        if (refined)
+        if (refined && !small)
             rc = launch_candidates_refined(ctx, b, n, d, knn_ids, knn_sq, k, core_sq, label, s,
                                            &boruvka_fallback_rows);
         else if (exact_rows)
@@ -343,7 +342,8 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
         else
             rc = launch_candidates_fp32(ctx, as<float>(b.xp), as<float>(b.corep),
                                         as<int32_t>(b.labp), as<int32_t>(b.perm), n, d, row_keys,
-                                        as<int32_t>(b.tile_lo), as<int32_t>(b.tile_hi), s);
+                                        as<int32_t>(b.tile_lo), as<int32_t>(b.tile_hi), s, nullptr,
+                                        0, 0, small);
         if (rc) return rc;
         CUSCAN_CUDA(ctx, cudaEventRecord(ev[5], s));
         if ((rc = forest_round(ctx, b, n, components, label, mst_src, mst_dst, mst_wsq, s,
@@ -373,8 +373,8 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
         return fail(ctx, CUSCAN_NUMERICAL, "Boruvka produced an incomplete spanning tree");
     if (n_edges) *n_edges = (int64_t)hs->edges;
     if (stats) {
-        stats->core_ms = elapsed(ev[0], ev[2]);
-        stats->mst_ms = elapsed(ev[2], ev[3]);
+        stats->core_ms = elapsed(ev[0], ev[1]);
+        stats->mst_ms = elapsed(ev[1], ev[3]);
         stats->knn_kernel_ms = elapsed(ev[0], ev[1]);
         stats->candidate_kernel_ms = cand_ms;
         stats->rounds = rounds;
@@ -475,9 +475,8 @@ int cuscan_shard_seed(cuscan_ctx *ctx, int64_t n, int32_t d, int32_t min_samples
     if (rc) return rc;
     const int k = (int)((int64_t)min_samples < n - 1 ? min_samples : n - 1);
     CUSCAN_CUDA(ctx, cudaMemsetAsync(b.status, 0, sizeof(DevStatus), s));
-    if ((rc = forest_core(ctx, knn_sq, n, k, min_samples, core_sq, s))) return rc;
-    if ((rc = forest_seed(ctx, b, core_sq, knn_ids, knn_sq, n, k, labels, mst_src, mst_dst,
-                          mst_wsq, s)))
+    if ((rc = forest_seed(ctx, b, core_sq, knn_ids, knn_sq, n, k, min_samples, labels, mst_src,
+                          mst_dst, mst_wsq, s)))
         return rc;
     DevStatus *hs = f->host_status;
     if ((rc = read_status(ctx, b.status, hs, s))) return rc;

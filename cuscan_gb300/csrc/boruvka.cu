@@ -62,7 +62,7 @@ constexpr size_t kCandSmem =
 // costs a three-way maximum, a label test, a select and a minimum; the exact (w, id) order is only
 // looked at where a query's minimum over its eight references reaches its best so far.
 // Measured on a GB300, the four rounds of the anisotropic 100,000 x 64 fit in plain f32:
-// CAND_A ms against 143.1 ms for one query per thread.
+// 86.7 ms against 143.1 ms for one query per thread.
 __device__ __forceinline__ void candidates_block(
     const float *__restrict__ data, const float *__restrict__ core,
     const int32_t *__restrict__ labels, const int32_t *__restrict__ ids, int64_t n, int d,
@@ -357,11 +357,12 @@ int launch_tile_ranges(cuscan_ctx *ctx, const int32_t *labels, int64_t n, int32_
 int launch_candidates_fp32(cuscan_ctx *ctx, const float *data, const float *core_sq,
                            const int32_t *labels, const int32_t *ids, int64_t n, int d,
                            unsigned long long *row_keys, int32_t *tile_lo, int32_t *tile_hi,
-                           cudaStream_t s, const int32_t *qmap, int64_t nq, int64_t qoff) {
+                           cudaStream_t s, const int32_t *qmap, int64_t nq, int64_t qoff,
+                           bool ranges_ready) {
     if (!qmap && qoff == 0 && nq == 0) nq = n;
     if (nq == 0) return CUSCAN_OK;
-    int rc = launch_tile_ranges(ctx, labels, n, tile_lo, tile_hi, s);
-    if (rc) return rc;
+    if (!ranges_ready)
+        if (int rc = launch_tile_ranges(ctx, labels, n, tile_lo, tile_hi, s)) return rc;
     if (d > CUSCAN_PACK_MAX_FEATURES)
         return fail(ctx, CUSCAN_CAPACITY,
                     "feature count %d exceeds the shared-memory staging limit of the Boruvka "

@@ -8,7 +8,10 @@
 
 #include <atomic>
 #include <cstdarg>
+#include <map>
+#include <mutex>
 #include <string>
+#include <utility>
 
 #include "cuscan_gb300.h"
 
@@ -76,23 +79,41 @@ inline int cuda_fail(cuscan_ctx *ctx, cudaError_t e, const char *what) {
         if (_e != cudaSuccess) return ::cuscan::cuda_fail((ctx), _e, what); \
     } while (0)
 
-// Raise a kernel's dynamic shared-memory cap to the device's opt-in limit. Every call sets the
-// same value, so a fit running on another host thread cannot lower the cap between this call
-// and a launch that needs more (the attribute belongs to the kernel, not to a stream).
-template <class Kernel>
-inline int allow_dynamic_smem(cuscan_ctx *ctx, Kernel kernel, size_t bytes) {
-    int optin = 0;
-    CUSCAN_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
-                                            ctx->device));
-    cudaFuncAttributes attr;
-    CUSCAN_CUDA(ctx, cudaFuncGetAttributes(&attr, (const void *)kernel));
-    const size_t cap = (size_t)optin - attr.sharedSizeBytes;
+// Raise a kernel's dynamic shared-memory cap to the device's opt-in limit, once per kernel and
+// device of the process (the attribute belongs to the kernel, not to a stream, and every caller
+// sets the same value). The cap is remembered, so that a launch costs a lookup instead of three
+// runtime calls.
+inline int allow_dynamic_smem_of(cuscan_ctx *ctx, const void *kernel, size_t bytes) {
+    static std::mutex mutex;
+    static std::map<std::pair<const void *, int>, size_t> caps;
+    size_t cap = 0;
+    {
+        std::lock_guard<std::mutex> lock(mutex);
+        auto it = caps.find({kernel, ctx->device});
+        if (it != caps.end()) cap = it->second;
+    }
+    if (cap == 0) {
+        int optin = 0;
+        CUSCAN_CUDA(ctx, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
+                                                ctx->device));
+        cudaFuncAttributes attr;
+        CUSCAN_CUDA(ctx, cudaFuncGetAttributes(&attr, kernel));
+        cap = (size_t)optin - attr.sharedSizeBytes;
+        if (bytes <= cap) {
+            CUSCAN_CUDA(ctx, cudaFuncSetAttribute(
+                                 kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+            std::lock_guard<std::mutex> lock(mutex);
+            caps[{kernel, ctx->device}] = cap;
+        }
+    }
     if (bytes > cap)
         return fail(ctx, CUSCAN_CAPACITY, "a kernel needs %zu bytes of shared memory, the device "
                     "allows %zu", bytes, cap);
-    CUSCAN_CUDA(ctx, cudaFuncSetAttribute((const void *)kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
     return CUSCAN_OK;
+}
+template <class Kernel>
+inline int allow_dynamic_smem(cuscan_ctx *ctx, Kernel kernel, size_t bytes) {
+    return allow_dynamic_smem_of(ctx, (const void *)kernel, bytes);
 }
 
 // Number of kernels this library has launched in the process (reported by
@@ -186,11 +207,12 @@ int launch_exact_knn_fp32(cuscan_ctx *ctx, const float *query, int64_t nq, const
 // output (NULL = identity). tile_lo/tile_hi are scratch of ceil(n/32) ints each.
 // With qmap, only the nq query positions qmap[0..nq) are scanned (against all n positions);
 // without it, the positions [qoff, qoff + nq) (all n positions when nq and qoff are 0).
+// ranges_ready: tile_lo/tile_hi already hold the label ranges.
 int launch_candidates_fp32(cuscan_ctx *ctx, const float *data, const float *core_sq,
                            const int32_t *labels, const int32_t *ids, int64_t n, int d,
                            unsigned long long *row_keys, int32_t *tile_lo, int32_t *tile_hi,
                            cudaStream_t s, const int32_t *qmap = nullptr, int64_t nq = 0,
-                           int64_t qoff = 0);
+                           int64_t qoff = 0, bool ranges_ready = false);
 // Label range (min, max) of every 32-row tile of `labels`.
 int launch_tile_ranges(cuscan_ctx *ctx, const int32_t *labels, int64_t n, int32_t *tile_lo,
                        int32_t *tile_hi, cudaStream_t s);

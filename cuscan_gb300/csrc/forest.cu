@@ -19,6 +19,14 @@
 namespace cuscan {
 namespace {
 
+constexpr int SMALL_RANGE = 32;  // rows per label range of the candidate sweep
+
+__device__ __forceinline__ int log2_ceil_dev(int64_t c) {
+    int l = 0;
+    while ((1ll << l) < c) ++l;
+    return l;
+}
+
 __device__ __forceinline__ bool active_node(const int32_t *label, int64_t s) {
     return label == nullptr || label[s] == (int32_t)s;
 }
@@ -75,18 +83,15 @@ __global__ void seed_kernel(const float *__restrict__ core, const int32_t *__res
                             const float *__restrict__ dsq, int64_t n, int k,
                             int32_t *__restrict__ next, uint32_t *__restrict__ esrc,
                             uint32_t *__restrict__ edst, float *__restrict__ ew,
-                            DevStatus *status) {
+                            int32_t *__restrict__ label, DevStatus *status) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) seed_at(i, core, ids, dsq, n, k, next, esrc, edst, ew, status);
-}
-
-__global__ void iota_kernel(int32_t *p, int64_t n) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = (int32_t)i;
+    if (i >= n) return;
+    seed_at(i, core, ids, dsq, n, k, next, esrc, edst, ew, status);
+    label[i] = (int32_t)i;  // every point is its own component before the merge
 }
 
 // Per-node steps of the cycle breaking and union (resolve_proposals). Each is run by one
-// thread per node, either as a kernel of its own or inside the single-CTA resolve_small_kernel;
+// thread per node, either as a kernel of its own or inside the single-CTA steps of small fits;
 // the step order and the barriers between them are the same in both.
 __device__ __forceinline__ void dbl_init_at(int64_t s, const int32_t *__restrict__ next,
                                             const int32_t *__restrict__ label,
@@ -378,7 +383,9 @@ constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
+template <int THREADS = SCAN_THREADS>
 __device__ __forceinline__ int block_exclusive_scan(int v, int *warp_sums, int &total) {
+    static_assert(THREADS <= 1024, "one warp scans the warp sums");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int x = v;
 #pragma unroll
@@ -389,17 +396,17 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *warp_sums, int &
     if (lane == 31) warp_sums[warp] = x;
     __syncthreads();
     if (warp == 0) {
-        int w = lane < (SCAN_THREADS / 32) ? warp_sums[lane] : 0;
+        int w = lane < (THREADS / 32) ? warp_sums[lane] : 0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             int y = __shfl_up_sync(0xffffffffu, w, o);
             if (lane >= o) w += y;
         }
-        if (lane < (SCAN_THREADS / 32)) warp_sums[lane] = w;
+        if (lane < (THREADS / 32)) warp_sums[lane] = w;
     }
     __syncthreads();
     int warp_prefix = warp > 0 ? warp_sums[warp - 1] : 0;
-    total = warp_sums[SCAN_THREADS / 32 - 1];
+    total = warp_sums[THREADS / 32 - 1];
     __syncthreads();
     return warp_prefix + x - v;
 }
@@ -446,28 +453,69 @@ __global__ void scan_add_kernel(int32_t *__restrict__ out, int64_t n,
     if (i < n) out[i] += sums[i / SCAN_TILE];
 }
 
-// resolve_proposals of up to SMALL_RESOLVE_ROWS nodes in one CTA: the same per-node steps in
-// the same order as the kernel sequence below, with block barriers where the sequence has
-// kernel boundaries (global writes of the block are visible to the whole block after
-// __syncthreads). One launch instead of about 33 per seed or round of a small fit. In a round
-// active_label and point_label are the same array (no __restrict__ on either).
-constexpr int64_t SMALL_RESOLVE_ROWS = 2048;
-constexpr int SMALL_ITEMS = (int)(SMALL_RESOLVE_ROWS / SCAN_THREADS);
-__device__ __forceinline__ void resolve_block(
-    const int32_t *__restrict__ next, const int32_t *active_label, int32_t *point_label, int64_t n,
-    int steps, int32_t *ja, int32_t *ma, int32_t *jb, int32_t *mb, int32_t *__restrict__ keep,
-    int32_t *__restrict__ pos, int32_t *__restrict__ kept_total, const uint32_t *__restrict__ esrc,
-    const uint32_t *__restrict__ edst, const float *__restrict__ ew, int32_t *parent,
-    int32_t *__restrict__ minlab, DevStatus *status, uint32_t *__restrict__ out_src,
-    uint32_t *__restrict__ out_dst, float *__restrict__ out_w, int64_t capacity,
-    int require_progress) {
-    __shared__ int warp_sums[SCAN_THREADS / 32];
+// ---- forests of fewer than 2048 points: each step of a fit in one CTA ----
+//
+// The same per-node steps in the same order as the kernel sequences below, with block barriers
+// where the sequences have kernel boundaries, on arrays in shared memory. What bounds them is the
+// chain of dependent loads and barriers (two per pointer-doubling or path-halving step, 24 steps
+// at 2,000 points), so the arrays sit where a load takes tens of cycles instead of an L2 trip, and
+// 1,024 threads take two nodes each. Measured in a pack of eight fits of 500 to 2,047 rows on a
+// GB300, against 256 threads on global arrays: seed 16.4 us (41.0), sort 10.9 us (18.6), merge
+// 11.2 us (26.3).
+constexpr int64_t SMALL_ROWS = 2048;  // nodes the arrays hold; fits of fewer points take this form
+constexpr int SMALL_THREADS = 1024;
+constexpr int SMALL_ITEMS = (int)(SMALL_ROWS / SMALL_THREADS);
+
+struct SmallForest {
+    unsigned long long *comp_keys;
+    int32_t *next, *ja, *ma, *jb, *mb, *keep, *pos, *parent, *minlab, *label;
+    uint32_t *esrc, *edst;
+    float *ew;
+};
+constexpr size_t kSmallSmem = (size_t)SMALL_ROWS * (8 + 13 * 4);
+__device__ __forceinline__ SmallForest small_forest(void *smem) {
+    SmallForest f;
+    f.comp_keys = reinterpret_cast<unsigned long long *>(smem);
+    int32_t *p = reinterpret_cast<int32_t *>(f.comp_keys + SMALL_ROWS);
+    auto take = [&p]() {
+        int32_t *at = p;
+        p += SMALL_ROWS;
+        return at;
+    };
+    f.next = take();
+    f.ja = take();
+    f.ma = take();
+    f.jb = take();
+    f.mb = take();
+    f.keep = take();
+    f.pos = take();
+    f.parent = take();
+    f.minlab = take();
+    f.label = take();
+    f.esrc = reinterpret_cast<uint32_t *>(take());
+    f.edst = reinterpret_cast<uint32_t *>(take());
+    f.ew = reinterpret_cast<float *>(take());
+    return f;
+}
+
+// Cycle breaking, emit and union of the proposals in F.next/esrc/edst/ew (resolve_proposals).
+// The points' labels are F.label, which are also the active labels of a round; the seed
+// (active_label null) starts from labels 0..n-1. New labels leave to point_label.
+__device__ __forceinline__ void resolve_block(const SmallForest &F, const int32_t *active_label,
+                                              int32_t *__restrict__ point_label, int64_t n,
+                                              int steps, DevStatus *status,
+                                              uint32_t *__restrict__ out_src,
+                                              uint32_t *__restrict__ out_dst,
+                                              float *__restrict__ out_w, int64_t capacity,
+                                              int require_progress) {
+    __shared__ int warp_sums[SMALL_THREADS / 32];
     const int tid = threadIdx.x;
+    int32_t *ja = F.ja, *ma = F.ma, *jb = F.jb, *mb = F.mb;
     // cycle breaking: pointer doubling with a running maximum, ping-pong buffers
-    for (int64_t s = tid; s < n; s += SCAN_THREADS) dbl_init_at(s, next, active_label, ja, ma);
+    for (int64_t s = tid; s < n; s += SMALL_THREADS) dbl_init_at(s, F.next, active_label, ja, ma);
     __syncthreads();
     for (int t = 0; t < steps; ++t) {
-        for (int64_t s = tid; s < n; s += SCAN_THREADS)
+        for (int64_t s = tid; s < n; s += SMALL_THREADS)
             dbl_step_at(s, ja, ma, active_label, jb, mb);
         __syncthreads();
         int32_t *tj = ja, *tm = ma;
@@ -476,7 +524,8 @@ __device__ __forceinline__ void resolve_block(
         jb = tj;
         mb = tm;
     }
-    for (int64_t s = tid; s < n; s += SCAN_THREADS) keep_at(s, next, ja, ma, active_label, keep, parent);
+    for (int64_t s = tid; s < n; s += SMALL_THREADS)
+        keep_at(s, F.next, ja, ma, active_label, F.keep, F.parent);
     __syncthreads();
     // exclusive scan of keep in node order: thread t holds nodes [t SMALL_ITEMS, +SMALL_ITEMS)
     int v[SMALL_ITEMS];
@@ -484,125 +533,86 @@ __device__ __forceinline__ void resolve_block(
     const int64_t base = (int64_t)tid * SMALL_ITEMS;
 #pragma unroll
     for (int u = 0; u < SMALL_ITEMS; ++u) {
-        v[u] = base + u < n ? keep[base + u] : 0;
+        v[u] = base + u < n ? F.keep[base + u] : 0;
         sum += v[u];
     }
     int total;
-    int prefix = block_exclusive_scan(sum, warp_sums, total);
+    int prefix = block_exclusive_scan<SMALL_THREADS>(sum, warp_sums, total);
 #pragma unroll
     for (int u = 0; u < SMALL_ITEMS; ++u) {
-        if (base + u < n) pos[base + u] = prefix;
+        if (base + u < n) F.pos[base + u] = prefix;
         prefix += v[u];
     }
     __syncthreads();
     // append the kept edges in node order after the edges emitted so far
     const int64_t edges = (int64_t)status->edges;
-    for (int64_t s = tid; s < n; s += SCAN_THREADS)
-        emit_at(s, keep, pos, esrc, edst, ew, edges, out_src, out_dst, out_w, capacity);
+    for (int64_t s = tid; s < n; s += SMALL_THREADS)
+        emit_at(s, F.keep, F.pos, F.esrc, F.edst, F.ew, edges, out_src, out_dst, out_w, capacity);
     __syncthreads();
     if (tid == 0) {
-        *kept_total = total;
-        status->edges += (unsigned long long)total;
+        status->edges = (unsigned long long)(edges + total);
         // "Boruvka round made no progress" (mst.rs:279-283)
         if (require_progress && total == 0) atomicCAS(&status->err_kind, 0, 4);
     }
     // union: path halving, smallest point of every tree, relabel, count the components
     for (int t = 0; t < steps; ++t) {
-        for (int64_t s = tid; s < n; s += SCAN_THREADS) jump_at(s, parent, active_label);
+        for (int64_t s = tid; s < n; s += SMALL_THREADS) jump_at(s, F.parent, active_label);
         __syncthreads();
     }
-    for (int64_t s = tid; s < n; s += SCAN_THREADS) minlab_init_at(s, parent, active_label, minlab);
+    for (int64_t s = tid; s < n; s += SMALL_THREADS)
+        minlab_init_at(s, F.parent, active_label, F.minlab);
     __syncthreads();
-    for (int64_t s = tid; s < n; s += SCAN_THREADS)
-        minlab_reduce_at(s, parent, active_label, minlab);
-    __syncthreads();
-    for (int64_t i = tid; i < n; i += SCAN_THREADS) relabel_at(i, point_label, parent, minlab);
+    for (int64_t s = tid; s < n; s += SMALL_THREADS)
+        minlab_reduce_at(s, F.parent, active_label, F.minlab);
     __syncthreads();
     int roots = 0;
-    for (int64_t i0 = 0; i0 < n; i0 += SCAN_THREADS) {
+    for (int64_t i0 = 0; i0 < n; i0 += SMALL_THREADS) {
         const int64_t i = i0 + tid;
-        roots += __syncthreads_count(i < n && point_label[i] == (int32_t)i);
+        int32_t l = -1;
+        if (i < n) {
+            l = F.minlab[F.parent[active_label ? F.label[i] : (int32_t)i]];
+            point_label[i] = l;
+        }
+        roots += __syncthreads_count(l == (int32_t)i);
     }
     if (tid == 0) status->components = (unsigned long long)roots;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS)
-    resolve_small_kernel(const int32_t *__restrict__ next, const int32_t *active_label,
-                         int32_t *point_label, int64_t n, int steps, int32_t *ja,
-                         int32_t *ma, int32_t *jb, int32_t *mb, int32_t *__restrict__ keep,
-                         int32_t *__restrict__ pos, int32_t *__restrict__ kept_total,
-                         const uint32_t *__restrict__ esrc, const uint32_t *__restrict__ edst,
-                         const float *__restrict__ ew, int32_t *parent,
-                         int32_t *__restrict__ minlab, DevStatus *status,
-                         uint32_t *__restrict__ out_src, uint32_t *__restrict__ out_dst,
-                         float *__restrict__ out_w, int64_t capacity, int require_progress) {
-    resolve_block(next, active_label, point_label, n, steps, ja, ma, jb, mb, keep, pos, kept_total,
-                  esrc, edst, ew, parent, minlab, status, out_src, out_dst, out_w, capacity,
-                  require_progress);
+// Core column, seed proposals and their merge (core_kernel, seed_kernel, resolve_proposals).
+__device__ __forceinline__ void small_seed(const PackFit &f, void *smem) {
+    const SmallForest F = small_forest(smem);
+    const int64_t n = f.n;
+    for (int64_t i = threadIdx.x; i < n; i += SMALL_THREADS)
+        core_at(i, f.dsq, n, f.k, f.min_samples, f.core);
+    __syncthreads();
+    for (int64_t i = threadIdx.x; i < n; i += SMALL_THREADS)
+        seed_at(i, f.core, f.ids, f.dsq, n, f.k, F.next, F.esrc, F.edst, F.ew, f.status);
+    __syncthreads();
+    resolve_block(F, nullptr, f.label, n, log2_ceil_dev(n > 1 ? n : 2) + 1, f.status, f.src, f.dst,
+                  f.w, n - 1, 0);
 }
 
-// A Borůvka round's winners and merge for at most SMALL_RESOLVE_ROWS points in one CTA: the
-// per-component minimum key (component_min_kernel's keys, reduced with block atomics), the
-// winners (winner_kernel), then resolve_block. One launch instead of four.
-__device__ __forceinline__ void round_block(
-    const int32_t *__restrict__ perm, const int32_t *__restrict__ labp,
-    const unsigned long long *__restrict__ row_keys, unsigned long long *__restrict__ comp_keys,
-    int allow_empty, int32_t *label, int64_t n, int steps, int32_t *next, int32_t *ja,
-    int32_t *ma, int32_t *jb, int32_t *mb, int32_t *__restrict__ keep, int32_t *__restrict__ pos,
-    int32_t *__restrict__ kept_total, uint32_t *esrc, uint32_t *edst, float *ew, int32_t *parent,
-    int32_t *__restrict__ minlab, DevStatus *status, uint32_t *__restrict__ out_src,
-    uint32_t *__restrict__ out_dst, float *__restrict__ out_w, int64_t capacity) {
+// Start of a round: counting sort by label (histogram, sum of squared sizes, exclusive scan and
+// scatter; the order of points within a label is free, as in scatter_kernel), the sorted labels
+// and core distances, cleared row keys and the label range of every 32-row tile.
+__device__ __forceinline__ void small_sort(const PackFit &f, void *smem) {
+    const SmallForest F = small_forest(smem);
+    int32_t *cnt = F.next, *start = F.ja, *fill = F.ma, *perm = F.jb, *labp = F.mb;
+    __shared__ int warp_sums[SMALL_THREADS / 32];
+    __shared__ double pair_sums[SMALL_THREADS / 32];
     const int tid = threadIdx.x;
-    for (int64_t i = tid; i < n; i += SCAN_THREADS) comp_keys[i] = ~0ull;
-    __syncthreads();
-    for (int64_t p = tid; p < n; p += SCAN_THREADS) {
-        const unsigned long long v = comp_key_at(p, perm, row_keys, status, allow_empty);
-        if (v != ~0ull) atomicMin(&comp_keys[labp[p]], v);
-    }
-    __syncthreads();
-    for (int64_t i = tid; i < n; i += SCAN_THREADS)
-        winner_at(i, label, comp_keys, row_keys, n, next, esrc, edst, ew, status);
-    __syncthreads();
-    resolve_block(next, label, label, n, steps, ja, ma, jb, mb, keep, pos, kept_total, esrc, edst,
-                  ew, parent, minlab, status, out_src, out_dst, out_w, capacity, 1);
-}
-
-__global__ void __launch_bounds__(SCAN_THREADS)
-    round_small_kernel(const int32_t *__restrict__ perm, const int32_t *__restrict__ labp,
-                       const unsigned long long *__restrict__ row_keys,
-                       unsigned long long *__restrict__ comp_keys, int allow_empty,
-                       int32_t *label, int64_t n, int steps, int32_t *next, int32_t *ja,
-                       int32_t *ma, int32_t *jb, int32_t *mb, int32_t *__restrict__ keep,
-                       int32_t *__restrict__ pos, int32_t *__restrict__ kept_total,
-                       uint32_t *esrc, uint32_t *edst, float *ew, int32_t *parent,
-                       int32_t *__restrict__ minlab, DevStatus *status,
-                       uint32_t *__restrict__ out_src, uint32_t *__restrict__ out_dst,
-                       float *__restrict__ out_w, int64_t capacity) {
-    round_block(perm, labp, row_keys, comp_keys, allow_empty, label, n, steps, next, ja, ma, jb,
-                mb, keep, pos, kept_total, esrc, edst, ew, parent, minlab, status, out_src,
-                out_dst, out_w, capacity);
-}
-
-// Counting sort by label for at most SMALL_RESOLVE_ROWS points in one CTA: histogram, sum of
-// squared sizes, exclusive scan and scatter (hist_kernel, same_pairs_kernel, scan_exclusive,
-// scatter_kernel). The order of points within a label is free, as in scatter_kernel.
-__device__ __forceinline__ void sort_block(const int32_t *__restrict__ label, int64_t n,
-                                           int32_t *__restrict__ cnt, int32_t *__restrict__ start,
-                                           int32_t *__restrict__ fill, int32_t *__restrict__ perm,
-                                           DevStatus *status) {
-    __shared__ int warp_sums[SCAN_THREADS / 32];
-    __shared__ double pair_sums[SCAN_THREADS / 32];
-    const int tid = threadIdx.x;
-    for (int64_t i = tid; i < n; i += SCAN_THREADS) {
+    const int64_t n = f.n;
+    for (int64_t i = tid; i < n; i += SMALL_THREADS) {
         cnt[i] = 0;
         fill[i] = 0;
+        F.label[i] = f.label[i];
     }
     __syncthreads();
-    for (int64_t i = tid; i < n; i += SCAN_THREADS) atomicAdd(&cnt[label[i]], 1);
+    for (int64_t i = tid; i < n; i += SMALL_THREADS) atomicAdd(&cnt[F.label[i]], 1);
     __syncthreads();
     // sum of squared sizes (exact in f64: integers below 2^53)
     double v = 0.0;
-    for (int64_t i = tid; i < n; i += SCAN_THREADS) {
+    for (int64_t i = tid; i < n; i += SMALL_THREADS) {
         const double c = (double)cnt[i];
         v += c * c;
     }
@@ -618,7 +628,7 @@ __device__ __forceinline__ void sort_block(const int32_t *__restrict__ label, in
         sum += c[u];
     }
     int total;
-    int prefix = block_exclusive_scan(sum, warp_sums, total);
+    int prefix = block_exclusive_scan<SMALL_THREADS>(sum, warp_sums, total);
 #pragma unroll
     for (int u = 0; u < SMALL_ITEMS; ++u) {
         if (base + u < n) start[base + u] = prefix;
@@ -626,21 +636,82 @@ __device__ __forceinline__ void sort_block(const int32_t *__restrict__ label, in
     }
     if (tid == 0) {
         double t = 0.0;
-        for (int w = 0; w < SCAN_THREADS / 32; ++w) t += pair_sums[w];
-        status->same_pairs = t;
+        for (int w = 0; w < SMALL_THREADS / 32; ++w) t += pair_sums[w];
+        f.status->same_pairs = t;
     }
     __syncthreads();
-    for (int64_t i = tid; i < n; i += SCAN_THREADS) {
-        const int32_t l = label[i];
+    for (int64_t i = tid; i < n; i += SMALL_THREADS) {
+        const int32_t l = F.label[i];
         perm[start[l] + atomicAdd(&fill[l], 1)] = (int32_t)i;
+    }
+    __syncthreads();
+    for (int64_t p = tid; p < n; p += SMALL_THREADS) {
+        const int32_t i = perm[p], l = F.label[i];
+        labp[p] = l;
+        f.perm[p] = i;
+        f.corep[p] = f.core[i];
+        f.labp[p] = l;
+        f.row_keys[p] = ~0ull;
+    }
+    __syncthreads();
+    const int64_t tiles = ceil_div(n, SMALL_RANGE);
+    for (int64_t t = tid; t < tiles; t += SMALL_THREADS) {
+        const int64_t a = t * SMALL_RANGE, b = a + SMALL_RANGE < n ? a + SMALL_RANGE : n;
+        int32_t mn = labp[a], mx = mn;
+        for (int64_t i = a + 1; i < b; ++i) {
+            const int32_t l = labp[i];
+            mn = l < mn ? l : mn;
+            mx = l > mx ? l : mx;
+        }
+        f.tile_lo[t] = mn;
+        f.tile_hi[t] = mx;
     }
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS)
-    sort_small_kernel(const int32_t *__restrict__ label, int64_t n, int32_t *__restrict__ cnt,
-                      int32_t *__restrict__ start, int32_t *__restrict__ fill,
-                      int32_t *__restrict__ perm, DevStatus *status) {
-    sort_block(label, n, cnt, start, fill, perm, status);
+// End of a round: the per-component minimum key (component_min_kernel's keys, reduced with
+// shared atomics), the winners (winner_kernel), then resolve_block over `components` components.
+__device__ __forceinline__ void small_merge(const PackFit &f, int64_t components, void *smem) {
+    const SmallForest F = small_forest(smem);
+    const int tid = threadIdx.x;
+    const int64_t n = f.n;
+    for (int64_t i = tid; i < n; i += SMALL_THREADS) {
+        F.comp_keys[i] = ~0ull;
+        F.label[i] = f.label[i];
+    }
+    __syncthreads();
+    for (int64_t p = tid; p < n; p += SMALL_THREADS) {
+        const unsigned long long v = comp_key_at(p, f.perm, f.row_keys, f.status, f.allow_empty);
+        if (v != ~0ull) atomicMin(&F.comp_keys[f.labp[p]], v);
+    }
+    __syncthreads();
+    for (int64_t i = tid; i < n; i += SMALL_THREADS)
+        winner_at(i, F.label, F.comp_keys, f.row_keys, n, F.next, F.esrc, F.edst, F.ew, f.status);
+    __syncthreads();
+    resolve_block(F, F.label, f.label, n, log2_ceil_dev(components > 1 ? components : 2) + 1,
+                  f.status, f.src, f.dst, f.w, n - 1, 1);
+}
+
+// One fit alone: its descriptor is a kernel argument.
+__global__ void __launch_bounds__(SMALL_THREADS) small_seed_kernel(const PackFit f) {
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    small_seed(f, small_smem);
+}
+__global__ void __launch_bounds__(SMALL_THREADS) small_sort_kernel(const PackFit f) {
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    small_sort(f, small_smem);
+}
+__global__ void __launch_bounds__(SMALL_THREADS)
+    small_merge_kernel(const PackFit f, int64_t components) {
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    small_merge(f, components, small_smem);
+}
+// Sorted copy of the rows only (labels and cores: small_sort).
+__global__ void gather_rows_kernel(const float *__restrict__ x, const int32_t *__restrict__ perm,
+                                   int64_t total, int d, float *__restrict__ xp) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= total) return;
+    const int64_t pos = e / d;
+    xp[e] = x[(int64_t)perm[pos] * d + (e - pos * d)];
 }
 
 inline unsigned blocks(int64_t n, int t = 256) { return (unsigned)ceil_div(n > 0 ? n : 1, t); }
@@ -656,13 +727,6 @@ int scan_exclusive(cuscan_ctx *ctx, const int32_t *in, int32_t *out, int64_t n,
     CUSCAN_KERNEL(scan_sums_kernel, 1, SCAN_THREADS, 0, s, as<int32_t>(tmp), tiles, grand_total);
     CUSCAN_KERNEL(scan_add_kernel, blocks(n), 256, 0, s, out, n, as<int32_t>(tmp));
     CUSCAN_LAUNCH(ctx, "scan_exclusive");
-    return CUSCAN_OK;
-}
-
-int forest_core(cuscan_ctx *ctx, const float *knn_sq, int64_t n, int k, int min_samples,
-                float *core, cudaStream_t s) {
-    CUSCAN_KERNEL(core_kernel, blocks(n), 256, 0, s, knn_sq, n, k, min_samples, core);
-    CUSCAN_LAUNCH(ctx, "core_kernel");
     return CUSCAN_OK;
 }
 
@@ -682,16 +746,6 @@ static int resolve_proposals(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int64
     int32_t *ja = as<int32_t>(b.jmp_a), *ma = as<int32_t>(b.mx_a);
     int32_t *jb = as<int32_t>(b.jmp_b), *mb = as<int32_t>(b.mx_b);
     const int steps = log2_ceil(active > 1 ? active : 2) + 1;
-    if (n <= SMALL_RESOLVE_ROWS) {
-        CUSCAN_KERNEL(resolve_small_kernel, 1, SCAN_THREADS, 0, s, next, active_label,
-                      point_label, n, steps, ja, ma, jb, mb, as<int32_t>(b.keep),
-                      as<int32_t>(b.pos), as<int32_t>(b.kept_total), as<uint32_t>(b.esrc),
-                      as<uint32_t>(b.edst), as<float>(b.ew), as<int32_t>(b.parent),
-                      as<int32_t>(b.minlab), b.status, out_src, out_dst, out_w, n - 1,
-                      require_progress);
-        CUSCAN_LAUNCH(ctx, "resolve_small_kernel");
-        return CUSCAN_OK;
-    }
     CUSCAN_KERNEL(dbl_init_kernel, blocks(n), 256, 0, s, next, active_label, n, ja, ma);
     for (int t = 0; t < steps; ++t) {
         CUSCAN_KERNEL(dbl_step_kernel, blocks(n), 256, 0, s, ja, ma, active_label, n, jb, mb);
@@ -721,29 +775,61 @@ static int resolve_proposals(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int64
     return CUSCAN_OK;
 }
 
-int forest_seed(cuscan_ctx *ctx, ForestBuffers &b, const float *core, const int32_t *ids,
-                const float *dsq, int64_t n, int k, int32_t *label, uint32_t *out_src,
-                uint32_t *out_dst, float *out_w, cudaStream_t s, int64_t active_bound) {
+// The descriptor of a fit alone (fewer than SMALL_ROWS points) for the one-CTA steps.
+static PackFit small_fit(ForestBuffers &b, int64_t n, int32_t *label, uint32_t *out_src,
+                         uint32_t *out_dst, float *out_w) {
+    PackFit f{};
+    f.n = n;
+    f.label = label;
+    f.src = out_src;
+    f.dst = out_dst;
+    f.w = out_w;
+    f.perm = as<int32_t>(b.perm);
+    f.labp = as<int32_t>(b.labp);
+    f.corep = as<float>(b.corep);
+    f.row_keys = as<unsigned long long>(b.row_keys);
+    f.tile_lo = as<int32_t>(b.tile_lo);
+    f.tile_hi = as<int32_t>(b.tile_hi);
+    f.status = b.status;
+    return f;
+}
+
+bool forest_small(int64_t n) { return n < SMALL_ROWS; }
+
+int forest_seed(cuscan_ctx *ctx, ForestBuffers &b, float *core, const int32_t *ids,
+                const float *dsq, int64_t n, int k, int min_samples, int32_t *label,
+                uint32_t *out_src, uint32_t *out_dst, float *out_w, cudaStream_t s) {
+    if (forest_small(n)) {
+        PackFit f = small_fit(b, n, label, out_src, out_dst, out_w);
+        f.k = k;
+        f.min_samples = min_samples;
+        f.core = core;
+        f.ids = const_cast<int32_t *>(ids);
+        f.dsq = const_cast<float *>(dsq);
+        if (int rc = allow_dynamic_smem(ctx, small_seed_kernel, kSmallSmem)) return rc;
+        CUSCAN_KERNEL(small_seed_kernel, 1, SMALL_THREADS, kSmallSmem, s, f);
+        CUSCAN_LAUNCH(ctx, "small_seed_kernel");
+        return CUSCAN_OK;
+    }
+    CUSCAN_KERNEL(core_kernel, blocks(n), 256, 0, s, dsq, n, k, min_samples, core);
     CUSCAN_KERNEL(seed_kernel, blocks(n), 256, 0, s, core, ids, dsq, n, k, as<int32_t>(b.next),
                                            as<uint32_t>(b.esrc), as<uint32_t>(b.edst),
-                                           as<float>(b.ew), b.status);
-    CUSCAN_KERNEL(iota_kernel, blocks(n), 256, 0, s, label, n);
+                                           as<float>(b.ew), label, b.status);
     CUSCAN_LAUNCH(ctx, "seed_kernel");
     // all points are active nodes of the seed graph (active_label == nullptr)
-    int rc = resolve_proposals(ctx, b, n, active_bound > 0 ? active_bound : n, nullptr, label,
-                               out_src, out_dst, out_w, 0, s);
-    if (rc) return rc;
-    return CUSCAN_OK;
+    return resolve_proposals(ctx, b, n, n, nullptr, label, out_src, out_dst, out_w, 0, s);
 }
 
 int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, const float *core,
                              const int32_t *label, int64_t n, int d, cudaStream_t s) {
     int32_t *cnt = as<int32_t>(b.cnt), *start = as<int32_t>(b.start), *fill = as<int32_t>(b.fill);
-    if (n <= SMALL_RESOLVE_ROWS) {
-        CUSCAN_KERNEL(sort_small_kernel, 1, SCAN_THREADS, 0, s, label, n, cnt, start, fill,
-                      as<int32_t>(b.perm), b.status);
-        CUSCAN_KERNEL(gather_kernel, blocks(n * d), 256, 0, s, x, core, label, as<int32_t>(b.perm),
-                      n, d, as<float>(b.xp), as<float>(b.corep), as<int32_t>(b.labp));
+    if (forest_small(n)) {
+        PackFit f = small_fit(b, n, const_cast<int32_t *>(label), nullptr, nullptr, nullptr);
+        f.core = const_cast<float *>(core);
+        if (int rc = allow_dynamic_smem(ctx, small_sort_kernel, kSmallSmem)) return rc;
+        CUSCAN_KERNEL(small_sort_kernel, 1, SMALL_THREADS, kSmallSmem, s, f);
+        CUSCAN_KERNEL(gather_rows_kernel, blocks(n * d), 256, 0, s, x, as<int32_t>(b.perm), n * d, d,
+                      as<float>(b.xp));
         CUSCAN_LAUNCH(ctx, "component sort");
         return CUSCAN_OK;
     }
@@ -767,17 +853,12 @@ int forest_round(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int64_t component
                  int32_t *label, uint32_t *out_src, uint32_t *out_dst, float *out_w,
                  cudaStream_t s, int allow_empty) {
     unsigned long long *comp_keys = as<unsigned long long>(b.comp_keys);
-    if (n <= SMALL_RESOLVE_ROWS) {
-        const int steps = log2_ceil(components > 1 ? components : 2) + 1;
-        CUSCAN_KERNEL(round_small_kernel, 1, SCAN_THREADS, 0, s, as<int32_t>(b.perm),
-                      as<int32_t>(b.labp), as<unsigned long long>(b.row_keys), comp_keys,
-                      allow_empty, label, n, steps, as<int32_t>(b.next), as<int32_t>(b.jmp_a),
-                      as<int32_t>(b.mx_a), as<int32_t>(b.jmp_b), as<int32_t>(b.mx_b),
-                      as<int32_t>(b.keep), as<int32_t>(b.pos), as<int32_t>(b.kept_total),
-                      as<uint32_t>(b.esrc), as<uint32_t>(b.edst), as<float>(b.ew),
-                      as<int32_t>(b.parent), as<int32_t>(b.minlab), b.status, out_src, out_dst,
-                      out_w, n - 1);
-        CUSCAN_LAUNCH(ctx, "round_small_kernel");
+    if (forest_small(n)) {
+        PackFit f = small_fit(b, n, label, out_src, out_dst, out_w);
+        f.allow_empty = allow_empty;
+        if (int rc = allow_dynamic_smem(ctx, small_merge_kernel, kSmallSmem)) return rc;
+        CUSCAN_KERNEL(small_merge_kernel, 1, SMALL_THREADS, kSmallSmem, s, f, components);
+        CUSCAN_LAUNCH(ctx, "small_merge_kernel");
         return CUSCAN_OK;
     }
     int rc = launch_fill_u64(ctx, comp_keys, n, ~0ull, s);
@@ -912,39 +993,21 @@ void forest_release(ForestBuffers &b) {
 // ---- packed small fits: the one-CTA steps of every fit of a pack, one launch each ----
 namespace {
 
-constexpr int kPackRowTile = 32;  // rows per label-range tile of the candidate sweep
-
-__device__ __forceinline__ int log2_ceil_dev(int64_t c) {
-    int l = 0;
-    while ((1ll << l) < c) ++l;
-    return l;
-}
-
-// Fit blockIdx.x: core column, seed proposals, labels 0..n-1 and the seed's merge; the kernels
-// core_kernel, seed_kernel, iota_kernel and resolve_small_kernel of the fit alone, with its
-// step count. Block 0 also clears the pack's per-round counters.
-__global__ void __launch_bounds__(SCAN_THREADS)
+// Fit blockIdx.x: core column, seed proposals, labels and the seed's merge (small_seed, as a fit
+// alone). Block 0 also clears the pack's per-round counters.
+__global__ void __launch_bounds__(SMALL_THREADS)
     pack_seed_kernel(const PackFit *__restrict__ fits, int *more) {
-    const PackFit &f = fits[blockIdx.x];
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    const PackFit f = fits[blockIdx.x];
     const int tid = threadIdx.x;
-    const int64_t n = f.n;
     DevStatus *st = f.status;
-    if (blockIdx.x == 0)
-        for (int r = tid; r < kPackMaxRounds + 2; r += SCAN_THREADS) more[r] = 0;
+    if (blockIdx.x == 0 && tid < kPackMaxRounds + 2) more[tid] = 0;
     if (tid == 0) {
         *st = DevStatus{};
         f.kept_total[1] = 0;
     }
-    for (int64_t i = tid; i < n; i += SCAN_THREADS) core_at(i, f.dsq, n, f.k, f.min_samples, f.core);
     __syncthreads();
-    for (int64_t i = tid; i < n; i += SCAN_THREADS) {
-        seed_at(i, f.core, f.ids, f.dsq, n, f.k, f.next, f.esrc, f.edst, f.ew, st);
-        f.label[i] = (int32_t)i;
-    }
-    __syncthreads();
-    resolve_block(f.next, nullptr, f.label, n, log2_ceil_dev(n > 1 ? n : 2) + 1, f.ja, f.ma,
-                  f.jb, f.mb, f.keep, f.pos, f.kept_total, f.esrc, f.edst, f.ew, f.parent,
-                  f.minlab, st, f.src, f.dst, f.w, n - 1, 0);
+    small_seed(f, small_smem);
     if (tid == 0) {
         st->seed_edges = st->edges;
         st->components_after_seed = st->components;
@@ -952,16 +1015,14 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 }
 
 // Start of round r of fit blockIdx.x: whether it runs (more than one component, no error,
-// within the round limit: the host driver's checks), then the component sort, the sorted labels
-// and core distances (gather_kernel; pack_gather_kernel copies the rows), cleared row keys and
-// the label range of every 32-row tile (tile_range_kernel).
-__global__ void __launch_bounds__(SCAN_THREADS) pack_sort_kernel(const PackFit *__restrict__ fits) {
-    const PackFit &f = fits[blockIdx.x];
-    const int tid = threadIdx.x;
-    const int64_t n = f.n;
+// within the round limit: the host driver's checks), then small_sort (pack_gather_kernel copies
+// the rows).
+__global__ void __launch_bounds__(SMALL_THREADS) pack_sort_kernel(const PackFit *__restrict__ fits) {
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    const PackFit f = fits[blockIdx.x];
     DevStatus *st = f.status;
     __shared__ int run;
-    if (tid == 0) {
+    if (threadIdx.x == 0) {
         int on = st->components > 1 && st->err_kind == 0;
         if (on && st->rounds > (unsigned long long)kPackMaxRounds) {
             st->err_kind = kPackErrNoConvergence;
@@ -972,27 +1033,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) pack_sort_kernel(const PackFit *
     }
     __syncthreads();
     if (!run) return;
-    sort_block(f.label, n, f.cnt, f.start, f.fill, f.perm, st);
-    __syncthreads();
-    for (int64_t p = tid; p < n; p += SCAN_THREADS) {
-        const int32_t i = f.perm[p];
-        f.corep[p] = f.core[i];
-        f.labp[p] = f.label[i];
-        f.row_keys[p] = ~0ull;
-    }
-    __syncthreads();
-    const int64_t tiles = ceil_div(n, kPackRowTile);
-    for (int64_t t = tid; t < tiles; t += SCAN_THREADS) {
-        const int64_t a = t * kPackRowTile, b = a + kPackRowTile < n ? a + kPackRowTile : n;
-        int32_t mn = f.labp[a], mx = mn;
-        for (int64_t i = a + 1; i < b; ++i) {
-            const int32_t l = f.labp[i];
-            mn = l < mn ? l : mn;
-            mx = l > mx ? l : mx;
-        }
-        f.tile_lo[t] = mn;
-        f.tile_hi[t] = mx;
-    }
+    small_sort(f, small_smem);
 }
 
 // Sorted copy of the rows of fit blockIdx.y whose round runs (gather_kernel's copy), spread over
@@ -1011,21 +1052,19 @@ __global__ void pack_gather_kernel(const PackFit *__restrict__ fits) {
     }
 }
 
-// End of round r of fit blockIdx.x: winners and merge (round_small_kernel), then the round's
+// End of round r of fit blockIdx.x: winners and merge (small_merge), then the round's
 // bookkeeping (rounds run, ordered cross pairs entering it) and whether another round is due.
-__global__ void __launch_bounds__(SCAN_THREADS)
+__global__ void __launch_bounds__(SMALL_THREADS)
     pack_merge_kernel(const PackFit *__restrict__ fits, int r, int *more) {
-    const PackFit &f = fits[blockIdx.x];
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    const PackFit f = fits[blockIdx.x];
     if (!*(volatile int32_t *)&f.kept_total[1]) return;
     const int tid = threadIdx.x;
     const int64_t n = f.n;
     DevStatus *st = f.status;
     const int64_t comps = (int64_t)st->components;
     __syncthreads();  // every thread has the count before the merge rewrites it
-    round_block(f.perm, f.labp, f.row_keys, f.comp_keys, f.allow_empty, f.label, n,
-                log2_ceil_dev(comps > 1 ? comps : 2) + 1, f.next, f.ja, f.ma, f.jb, f.mb, f.keep,
-                f.pos, f.kept_total, f.esrc, f.edst, f.ew, f.parent, f.minlab, st, f.src, f.dst,
-                f.w, n - 1);
+    small_merge(f, comps, small_smem);
     if (tid == 0) {
         st->rounds += 1;
         st->cross_pairs += (double)n * (double)n - st->same_pairs;
@@ -1073,20 +1112,23 @@ int pack_knn(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int
 }
 
 int pack_seed(cuscan_ctx *ctx, const PackFit *fits, int count, int *more, cudaStream_t s) {
-    CUSCAN_KERNEL(pack_seed_kernel, count, SCAN_THREADS, 0, s, fits, more);
+    if (int rc = allow_dynamic_smem(ctx, pack_seed_kernel, kSmallSmem)) return rc;
+    CUSCAN_KERNEL(pack_seed_kernel, count, SMALL_THREADS, kSmallSmem, s, fits, more);
     CUSCAN_LAUNCH(ctx, "pack_seed_kernel");
     return CUSCAN_OK;
 }
 
 int pack_round(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int d_max,
                int splits, int r, int *more, cudaStream_t s) {
-    CUSCAN_KERNEL(pack_sort_kernel, count, SCAN_THREADS, 0, s, fits);
+    if (int rc = allow_dynamic_smem(ctx, pack_sort_kernel, kSmallSmem)) return rc;
+    if (int rc = allow_dynamic_smem(ctx, pack_merge_kernel, kSmallSmem)) return rc;
+    CUSCAN_KERNEL(pack_sort_kernel, count, SMALL_THREADS, kSmallSmem, s, fits);
     CUSCAN_LAUNCH(ctx, "pack_sort_kernel");
     const dim3 gg((unsigned)std::min<int64_t>(ceil_div(n_max * d_max, 256), 128), (unsigned)count);
     CUSCAN_KERNEL(pack_gather_kernel, gg, 256, 0, s, fits);
     CUSCAN_LAUNCH(ctx, "pack_gather_kernel");
     if (int rc = launch_pack_candidates(ctx, fits, count, n_max, d_max, splits, s)) return rc;
-    CUSCAN_KERNEL(pack_merge_kernel, count, SCAN_THREADS, 0, s, fits, r, more);
+    CUSCAN_KERNEL(pack_merge_kernel, count, SMALL_THREADS, kSmallSmem, s, fits, r, more);
     CUSCAN_LAUNCH(ctx, "pack_merge_kernel");
     return CUSCAN_OK;
 }

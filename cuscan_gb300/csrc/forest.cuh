@@ -68,15 +68,15 @@ void forest_release(ForestBuffers &b);
 // Every device buffer of the forest and of the bf16 screen (out may be null); returns the count.
 constexpr int kForestBufferCount = 64;
 int forest_buffers(ForestBuffers &b, Buffer **out);
-int forest_core(cuscan_ctx *ctx, const float *knn_sq, int64_t n, int k, int min_samples,
-                float *core, cudaStream_t s);
-// Seed forest (mst.rs:368-420): appends the kept seed edges and labels points by the smallest
-// point of their tree; status->components is refreshed. active_bound (default n) bounds the
-// nodes of the seed graph for the pointer-doubling step count.
-int forest_seed(cuscan_ctx *ctx, ForestBuffers &b, const float *core, const int32_t *ids,
-                const float *dsq, int64_t n, int k, int32_t *label, uint32_t *out_src,
-                uint32_t *out_dst, float *out_w, cudaStream_t s, int64_t active_bound = -1);
-// Group points by label: perm, xp, corep, labp.
+// Whether a set of n points takes the one-CTA forest steps (fewer than 2048 points).
+bool forest_small(int64_t n);
+// Core column, then the seed forest (mst.rs:368-420): appends the kept seed edges and labels
+// points by the smallest point of their tree; status->components is refreshed.
+int forest_seed(cuscan_ctx *ctx, ForestBuffers &b, float *core, const int32_t *ids,
+                const float *dsq, int64_t n, int k, int min_samples, int32_t *label,
+                uint32_t *out_src, uint32_t *out_dst, float *out_w, cudaStream_t s);
+// Group points by label: perm, xp, corep, labp. Small sets (forest_small) also get cleared row keys
+// and the label range of every 32-row tile.
 int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, const float *core,
                              const int32_t *label, int64_t n, int d, cudaStream_t s);
 // Merge one round from the per-row candidate keys in b.row_keys.
@@ -105,13 +105,10 @@ struct PackFit {
     int32_t *label;
     uint32_t *src, *dst;
     float *w;
-    int32_t *next, *ja, *ma, *jb, *mb, *keep, *pos, *parent, *minlab;
-    int32_t *kept_total;  // [0] kept edges of the last merge, [1] this round runs (0/1)
-    uint32_t *esrc, *edst;
-    float *ew;
-    int32_t *cnt, *start, *fill, *perm, *labp;
+    int32_t *kept_total;  // [1]: this round runs (0/1)
+    int32_t *perm, *labp;
     float *xp, *corep;
-    unsigned long long *row_keys, *comp_keys;
+    unsigned long long *row_keys;
     int32_t *tile_lo, *tile_hi;
     int32_t *part_ids;  // kNN partial lists when the reference range is split
     float *part_dist;

@@ -111,8 +111,7 @@ float elapsed_ms(cudaEvent_t a, cudaEvent_t b) {
 struct FitLayout {
     size_t x;
     size_t status, core, src, dst, w, ids, dsq;
-    size_t label, next, ja, ma, jb, mb, keep, pos, parent, minlab, kept, esrc, edst, ew;
-    size_t cnt, start, fill, perm, labp, xp, corep, row_keys, comp_keys, tile_lo, tile_hi;
+    size_t label, kept, perm, labp, xp, corep, row_keys, tile_lo, tile_hi;
     size_t part_ids, part_dist;
 };
 
@@ -124,11 +123,12 @@ struct PackLayout {
     size_t total = 0;
 };
 
-// Reference-range chunks of the kNN and candidate sweeps: enough blocks to fill the GPU twice
-// over (the plan of a fit alone), chunks of at least 256 rows.
+// Reference-range chunks of the kNN and candidate sweeps, chunks of at least 256 rows.
 int64_t pack_splits(const cuscan_ctx *ctx, int count, int64_t n_max) {
     const int64_t blocks = (int64_t)count * ceil_div(n_max, kKnnRows);
-    const int64_t target = (int64_t)simt::CTAS_PER_SM * ctx->sm_count;
+    // four times over: the fits of a pack differ in size and the largest sets the pace, so its
+    // sweep is cut finer than filling the GPU needs
+    const int64_t target = 4 * (int64_t)simt::CTAS_PER_SM * ctx->sm_count;
     int64_t splits = blocks < target ? ceil_div(target, blocks) : 1;
     const int64_t cap = ceil_div(n_max, 256);
     if (splits > cap) splits = cap;
@@ -168,14 +168,10 @@ PackLayout make_layout(const cuscan_fit_item *items, int count, int64_t splits) 
         FitLayout &F = L.fit[i];
         if (!it.knn_ids) F.ids = take(4 * nk);
         if (!it.knn_sq) F.dsq = take(4 * nk);
-        for (size_t *p : {&F.label, &F.next, &F.ja, &F.ma, &F.jb, &F.mb, &F.keep, &F.pos,
-                          &F.parent, &F.minlab, &F.esrc, &F.edst, &F.ew, &F.cnt, &F.start,
-                          &F.fill, &F.perm, &F.labp, &F.corep})
-            *p = take(4 * n);
+        for (size_t *p : {&F.label, &F.perm, &F.labp, &F.corep}) *p = take(4 * n);
         F.kept = take(2 * sizeof(int32_t));
         F.xp = take(4 * nd);
         F.row_keys = take(8 * n);
-        F.comp_keys = take(8 * n);
         F.tile_lo = take(4 * (n / 32 + 1));
         F.tile_hi = take(4 * (n / 32 + 1));
         const size_t parts = splits > 1 && item_k(it) <= kGroupedMaxK ? nk * (size_t)splits : 0;
@@ -203,28 +199,12 @@ PackFit describe(const cuscan_fit_item &it, const FitLayout &F, char *base) {
     f.src = reinterpret_cast<uint32_t *>(base + F.src);
     f.dst = reinterpret_cast<uint32_t *>(base + F.dst);
     f.w = reinterpret_cast<float *>(base + F.w);
-    f.next = reinterpret_cast<int32_t *>(base + F.next);
-    f.ja = reinterpret_cast<int32_t *>(base + F.ja);
-    f.ma = reinterpret_cast<int32_t *>(base + F.ma);
-    f.jb = reinterpret_cast<int32_t *>(base + F.jb);
-    f.mb = reinterpret_cast<int32_t *>(base + F.mb);
-    f.keep = reinterpret_cast<int32_t *>(base + F.keep);
-    f.pos = reinterpret_cast<int32_t *>(base + F.pos);
-    f.parent = reinterpret_cast<int32_t *>(base + F.parent);
-    f.minlab = reinterpret_cast<int32_t *>(base + F.minlab);
     f.kept_total = reinterpret_cast<int32_t *>(base + F.kept);
-    f.esrc = reinterpret_cast<uint32_t *>(base + F.esrc);
-    f.edst = reinterpret_cast<uint32_t *>(base + F.edst);
-    f.ew = reinterpret_cast<float *>(base + F.ew);
-    f.cnt = reinterpret_cast<int32_t *>(base + F.cnt);
-    f.start = reinterpret_cast<int32_t *>(base + F.start);
-    f.fill = reinterpret_cast<int32_t *>(base + F.fill);
     f.perm = reinterpret_cast<int32_t *>(base + F.perm);
     f.labp = reinterpret_cast<int32_t *>(base + F.labp);
     f.xp = reinterpret_cast<float *>(base + F.xp);
     f.corep = reinterpret_cast<float *>(base + F.corep);
     f.row_keys = reinterpret_cast<unsigned long long *>(base + F.row_keys);
-    f.comp_keys = reinterpret_cast<unsigned long long *>(base + F.comp_keys);
     f.tile_lo = reinterpret_cast<int32_t *>(base + F.tile_lo);
     f.tile_hi = reinterpret_cast<int32_t *>(base + F.tile_hi);
     f.part_ids = reinterpret_cast<int32_t *>(base + F.part_ids);
