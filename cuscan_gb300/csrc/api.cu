@@ -330,8 +330,7 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
         if (rounds > 64) return fail(ctx, CUSCAN_NUMERICAL, "Boruvka did not converge");
         if ((rc = forest_sort_by_component(ctx, b, data, core_sq, label, n, d, s))) return rc;
         unsigned long long *row_keys = as<unsigned long long>(b.row_keys);
-        const bool small = forest_small(n);  // its sort clears the keys and fills the label ranges
-        if (!small && (rc = launch_fill_u64(ctx, row_keys, n, ~0ull, s))) return rc;
+        const bool small = forest_small(n);  // its sort also fills the label ranges
         CUSCAN_CUDA(ctx, cudaEventRecord(ev[4], s));
         if (refined && !small)
             rc = launch_candidates_refined(ctx, b, n, d, knn_ids, knn_sq, k, core_sq, label, s,

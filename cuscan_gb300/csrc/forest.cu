@@ -161,84 +161,114 @@ __device__ __forceinline__ void minlab_reduce_at(int64_t s, const int32_t *__res
     if (!active_node(label, s)) return;
     atomicMin(&minlab[parent[s]], (int32_t)s);
 }
-// label[i] <- smallest label of the tree that holds i's old component.
-__device__ __forceinline__ void relabel_at(int64_t i, int32_t *__restrict__ label,
-                                           const int32_t *__restrict__ parent,
-                                           const int32_t *__restrict__ minlab) {
-    label[i] = minlab[parent[label[i]]];
+// Eight doubling steps' worth of hops per launch: jout[s] is jin applied eight times, mout the
+// largest label on the way (three steps of the one-hop form, whose launches were a quarter of a
+// 9,001-point fit's). The first launch (jin null) starts from the proposals themselves.
+constexpr int HOPS = 8;
+__global__ void dbl_hops_kernel(const int32_t *__restrict__ next, const int32_t *__restrict__ jin,
+                                const int32_t *__restrict__ min_, const int32_t *__restrict__ label,
+                                int64_t n, int32_t *__restrict__ jout, int32_t *__restrict__ mout) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n || !active_node(label, s)) return;
+    int32_t j = (int32_t)s, m = (int32_t)s;
+#pragma unroll
+    for (int h = 0; h < HOPS; ++h) {
+        const int32_t a = jin ? min_[j] : j;
+        m = a > m ? a : m;
+        j = jin ? jin[j] : next[j];
+    }
+    jout[s] = j;
+    mout[s] = m;
 }
 
-__global__ void dbl_init_kernel(const int32_t *__restrict__ next, const int32_t *__restrict__ label,
-                                int64_t n, int32_t *__restrict__ jmp, int32_t *__restrict__ mx) {
-    int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n) dbl_init_at(s, next, label, jmp, mx);
-}
-
-__global__ void dbl_step_kernel(const int32_t *__restrict__ jin, const int32_t *__restrict__ min_,
-                                const int32_t *__restrict__ label, int64_t n,
-                                int32_t *__restrict__ jout, int32_t *__restrict__ mout) {
-    int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n) dbl_step_at(s, jin, min_, label, jout, mout);
-}
-
+// keep_at, and the label minima of the roots (their own label) for minlab_reduce_kernel.
 __global__ void keep_kernel(const int32_t *__restrict__ next, const int32_t *__restrict__ jmp,
                             const int32_t *__restrict__ mx, const int32_t *__restrict__ label,
-                            int64_t n, int32_t *__restrict__ keep, int32_t *__restrict__ parent) {
+                            int64_t n, int32_t *__restrict__ keep, int32_t *__restrict__ parent,
+                            int32_t *__restrict__ minlab) {
     int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n) keep_at(s, next, jmp, mx, label, keep, parent);
+    if (s >= n) return;
+    keep_at(s, next, jmp, mx, label, keep, parent);
+    if (!keep[s]) minlab[s] = (int32_t)s;  // a root (or an inactive node, whose entry is not read)
 }
 
 __global__ void emit_kernel(const int32_t *__restrict__ keep, const int32_t *__restrict__ pos,
-                            const uint32_t *__restrict__ esrc, const uint32_t *__restrict__ edst,
-                            const float *__restrict__ ew, int64_t n, const DevStatus *status,
-                            uint32_t *__restrict__ out_src, uint32_t *__restrict__ out_dst,
-                            float *__restrict__ out_w, int64_t capacity) {
+                            const int32_t *__restrict__ sums, const uint32_t *__restrict__ esrc,
+                            const uint32_t *__restrict__ edst, const float *__restrict__ ew,
+                            int64_t n, const DevStatus *status, uint32_t *__restrict__ out_src,
+                            uint32_t *__restrict__ out_dst, float *__restrict__ out_w,
+                            int64_t capacity) {
     int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n)
-        emit_at(s, keep, pos, esrc, edst, ew, (int64_t)status->edges, out_src, out_dst, out_w,
-                capacity);
+    if (s >= n) return;
+    emit_at(s, keep, pos, esrc, edst, ew, (int64_t)status->edges + sums[s / kScanTile], out_src,
+            out_dst, out_w, capacity);
 }
 
-__global__ void add_edges_kernel(DevStatus *status, const int32_t *kept_total,
-                                 int require_progress) {
-    status->edges += *kept_total;
-    // "Boruvka round made no progress" (mst.rs:279-283)
-    if (require_progress && *kept_total == 0) atomicCAS(&status->err_kind, 0, 4);
-}
-
-// Path halving toward the root, repeated a fixed number of times by the host.
+// Eight hops toward the root per launch, in place: a parent read while another thread moves it
+// is an ancestor either way, so every launch at least multiplies the depth covered by eight.
 __global__ void jump_kernel(int32_t *__restrict__ parent, const int32_t *__restrict__ label,
                             int64_t n) {
-    int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n) jump_at(s, parent, label);
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n || !active_node(label, s)) return;
+    const volatile int32_t *vp = parent;
+    const int32_t p = vp[s];
+    int32_t q = p;
+#pragma unroll
+    for (int h = 1; h < HOPS; ++h) {
+        const int32_t up = vp[q];
+        if (up == q) break;
+        q = up;
+    }
+    if (q != p) parent[s] = q;
 }
 
-__global__ void minlab_init_kernel(const int32_t *__restrict__ parent,
-                                   const int32_t *__restrict__ label, int64_t n,
-                                   int32_t *__restrict__ minlab) {
-    int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n) minlab_init_at(s, parent, label, minlab);
-}
-
+// minlab_reduce_at; one thread also adds the emitted edges to the status and clears the component
+// count for relabel_kernel.
 __global__ void minlab_reduce_kernel(const int32_t *__restrict__ parent,
                                      const int32_t *__restrict__ label, int64_t n,
-                                     int32_t *__restrict__ minlab) {
+                                     int32_t *__restrict__ minlab, DevStatus *status,
+                                     const int32_t *kept_total, int require_progress) {
     int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s < n) minlab_reduce_at(s, parent, label, minlab);
+    if (s == 0) {
+        status->edges += *kept_total;
+        status->components = 0;
+        // "Boruvka round made no progress" (mst.rs:279-283)
+        if (require_progress && *kept_total == 0) atomicCAS(&status->err_kind, 0, 4);
+    }
 }
 
+// label[i] <- smallest label of the tree that holds i's old component; counts the components (the
+// points that carry their own label).
 __global__ void relabel_kernel(int32_t *__restrict__ label, const int32_t *__restrict__ parent,
-                               const int32_t *__restrict__ minlab, int64_t n) {
+                               const int32_t *__restrict__ minlab, int64_t n, DevStatus *status) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) relabel_at(i, label, parent, minlab);
+    bool root = false;
+    if (i < n) {
+        const int32_t l = minlab[parent[label[i]]];
+        label[i] = l;
+        root = l == (int32_t)i;
+    }
+    const int roots = __syncthreads_count(root);
+    if (threadIdx.x == 0 && roots) atomicAdd(&status->components, (unsigned long long)roots);
 }
 
-__global__ void count_components_kernel(const int32_t *__restrict__ label, int64_t n,
-                                        DevStatus *status) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    bool root = i < n && label[i] == (int32_t)i;
-    unsigned m = __ballot_sync(0xffffffffu, root);
-    if ((threadIdx.x & 31) == 0 && m) atomicAdd(&status->components, (unsigned long long)__popc(m));
+// Start of a component sort: empty histogram and cursors, empty row and component keys for the
+// round that follows, the pair sum and the scan's ticket.
+__global__ void sort_clear_kernel(int32_t *__restrict__ cnt, int32_t *__restrict__ fill,
+                                  unsigned long long *__restrict__ row_keys,
+                                  unsigned long long *__restrict__ comp_keys, int64_t n,
+                                  DevStatus *status) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        status->same_pairs = 0.0;
+        status->scan_ticket = 0;
+    }
+    if (i >= n) return;
+    cnt[i] = 0;
+    fill[i] = 0;
+    row_keys[i] = ~0ull;
+    comp_keys[i] = ~0ull;
 }
 
 // Counting sort of points by label: histogram with warp-aggregated atomics.
@@ -250,21 +280,9 @@ __global__ void hist_kernel(const int32_t *__restrict__ label, int64_t n, int32_
     if (l >= 0 && lane == __ffs(peers) - 1) atomicAdd(&cnt[l], __popc(peers));
 }
 
-// Sum of squared component sizes (ordered same-component pairs) for the work counters.
-__global__ void same_pairs_kernel(const int32_t *__restrict__ cnt, int64_t n, DevStatus *status) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    double v = 0.0;
-    if (i < n) {
-        double c = (double)cnt[i];
-        v = c * c;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(&status->same_pairs, v);
-}
-
 __global__ void scatter_kernel(const int32_t *__restrict__ label, int64_t n,
-                               const int32_t *__restrict__ start, int32_t *__restrict__ fill,
+                               const int32_t *__restrict__ start,
+                               const int32_t *__restrict__ sums, int32_t *__restrict__ fill,
                                int32_t *__restrict__ perm) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int32_t l = i < n ? label[i] : -1;
@@ -276,7 +294,7 @@ __global__ void scatter_kernel(const int32_t *__restrict__ label, int64_t n,
     base = __shfl_sync(peers, base, leader);
     if (l < 0) return;
     int rank = __popc(peers & ((1u << lane) - 1u));
-    perm[start[l] + base + rank] = (int32_t)i;
+    perm[start[l] + sums[l / kScanTile] + base + rank] = (int32_t)i;
 }
 
 __global__ void gather_kernel(const float *__restrict__ x, const float *__restrict__ core,
@@ -378,10 +396,11 @@ __global__ void winner_kernel(const int32_t *__restrict__ label,
     if (s < n) winner_at(s, label, comp_keys, row_keys, n, next, esrc, edst, ew, status);
 }
 
-// ---- exclusive scan of int32 (three passes) ----
+// ---- exclusive scan of int32: one launch; readers add their tile's offset ----
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+static_assert(SCAN_TILE == kScanTile, "tile of the scan offsets");
 
 template <int THREADS = SCAN_THREADS>
 __device__ __forceinline__ int block_exclusive_scan(int v, int *warp_sums, int &total) {
@@ -411,16 +430,27 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *warp_sums, int &
     return warp_prefix + x - v;
 }
 
-__global__ void scan_tiles_kernel(const int32_t *__restrict__ in, int32_t *__restrict__ out,
-                                  int64_t n, int32_t *__restrict__ tile_sums) {
+// Every block scans one tile into out and its total into tile_sums; the block that finishes last
+// scans the totals (entry i's position is out[i] + tile_sums[i / kScanTile]). With `square_sum`
+// the sum of squared inputs is added to it (exact in f64: integers below 2^53). The ticket wraps
+// back to 0.
+__global__ void __launch_bounds__(SCAN_THREADS)
+    scan_kernel(const int32_t *__restrict__ in, int32_t *__restrict__ out, int64_t n,
+                int32_t *tile_sums, int32_t *__restrict__ grand_total, DevStatus *status,
+                double *square_sum) {
     __shared__ int warp_sums[SCAN_THREADS / 32];
-    const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
+    __shared__ double pair_sums[SCAN_THREADS / 32];
+    __shared__ bool last;
+    const int tid = threadIdx.x;
+    const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)tid * SCAN_ITEMS;
     int v[SCAN_ITEMS];
     int sum = 0;
+    double sq = 0.0;
 #pragma unroll
     for (int t = 0; t < SCAN_ITEMS; ++t) {
         v[t] = base + t < n ? in[base + t] : 0;
         sum += v[t];
+        sq += (double)v[t] * (double)v[t];
     }
     int total;
     int prefix = block_exclusive_scan(sum, warp_sums, total);
@@ -429,28 +459,35 @@ __global__ void scan_tiles_kernel(const int32_t *__restrict__ in, int32_t *__res
         if (base + t < n) out[base + t] = prefix;
         prefix += v[t];
     }
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
-}
-
-__global__ void scan_sums_kernel(int32_t *__restrict__ sums, int64_t tiles,
-                                 int32_t *__restrict__ grand_total) {
-    __shared__ int warp_sums[SCAN_THREADS / 32];
-    int carry = 0;
-    for (int64_t b = 0; b < tiles; b += SCAN_THREADS) {
-        int64_t i = b + threadIdx.x;
-        int v = i < tiles ? sums[i] : 0;
-        int total;
-        int p = block_exclusive_scan(v, warp_sums, total);
-        if (i < tiles) sums[i] = carry + p;
-        carry += total;
+    if (square_sum) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if ((tid & 31) == 0) pair_sums[tid >> 5] = sq;
+        __syncthreads();
+        if (tid == 0) {
+            double t = 0.0;
+            for (int w = 0; w < SCAN_THREADS / 32; ++w) t += pair_sums[w];
+            if (t != 0.0) atomicAdd(square_sum, t);
+        }
     }
-    if (threadIdx.x == 0 && grand_total) *grand_total = carry;
-}
-
-__global__ void scan_add_kernel(int32_t *__restrict__ out, int64_t n,
-                                const int32_t *__restrict__ sums) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] += sums[i / SCAN_TILE];
+    if (tid == 0) {
+        tile_sums[blockIdx.x] = total;
+        __threadfence();
+        last = atomicInc(&status->scan_ticket, gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    int carry = 0;
+    for (int64_t b = 0; b < gridDim.x; b += SCAN_THREADS) {
+        const int64_t i = b + tid;
+        const int x = i < gridDim.x ? __ldcg(tile_sums + i) : 0;
+        int sums;
+        const int p = block_exclusive_scan(x, warp_sums, sums);
+        if (i < gridDim.x) tile_sums[i] = carry + p;
+        carry += sums;
+    }
+    if (tid == 0 && grand_total) *grand_total = carry;
 }
 
 // ---- forests of fewer than 2048 points: each step of a fit in one CTA ----
@@ -718,15 +755,14 @@ inline unsigned blocks(int64_t n, int t = 256) { return (unsigned)ceil_div(n > 0
 
 }  // namespace
 
-int scan_exclusive(cuscan_ctx *ctx, const int32_t *in, int32_t *out, int64_t n,
-                   int32_t *grand_total, Buffer &tmp, cudaStream_t s) {
+int scan_exclusive(cuscan_ctx *ctx, ForestBuffers &b, const int32_t *in, int32_t *out, int64_t n,
+                   int32_t *grand_total, cudaStream_t s, double *square_sum) {
     const int64_t tiles = ceil_div(n > 0 ? n : 1, SCAN_TILE);
-    int rc = ensure(ctx, tmp, (size_t)tiles * sizeof(int32_t), "scan tile sums");
+    int rc = ensure(ctx, b.scan_tmp, (size_t)tiles * sizeof(int32_t), "scan tile sums");
     if (rc) return rc;
-    CUSCAN_KERNEL(scan_tiles_kernel, (unsigned)tiles, SCAN_THREADS, 0, s, in, out, n, as<int32_t>(tmp));
-    CUSCAN_KERNEL(scan_sums_kernel, 1, SCAN_THREADS, 0, s, as<int32_t>(tmp), tiles, grand_total);
-    CUSCAN_KERNEL(scan_add_kernel, blocks(n), 256, 0, s, out, n, as<int32_t>(tmp));
-    CUSCAN_LAUNCH(ctx, "scan_exclusive");
+    CUSCAN_KERNEL(scan_kernel, (unsigned)tiles, SCAN_THREADS, 0, s, in, out, n,
+                  as<int32_t>(b.scan_tmp), grand_total, b.status, square_sum);
+    CUSCAN_LAUNCH(ctx, "scan_kernel");
     return CUSCAN_OK;
 }
 
@@ -745,10 +781,11 @@ static int resolve_proposals(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int64
     int32_t *next = as<int32_t>(b.next);
     int32_t *ja = as<int32_t>(b.jmp_a), *ma = as<int32_t>(b.mx_a);
     int32_t *jb = as<int32_t>(b.jmp_b), *mb = as<int32_t>(b.mx_b);
-    const int steps = log2_ceil(active > 1 ? active : 2) + 1;
-    CUSCAN_KERNEL(dbl_init_kernel, blocks(n), 256, 0, s, next, active_label, n, ja, ma);
+    // launches of eight hops for 2^(log2(active) + 1) hops
+    const int steps = (log2_ceil(active > 1 ? active : 2) + 1 + 2) / 3;
     for (int t = 0; t < steps; ++t) {
-        CUSCAN_KERNEL(dbl_step_kernel, blocks(n), 256, 0, s, ja, ma, active_label, n, jb, mb);
+        CUSCAN_KERNEL(dbl_hops_kernel, blocks(n), 256, 0, s, next, t ? ja : nullptr,
+                      t ? ma : nullptr, active_label, n, jb, mb);
         int32_t *tj = ja, *tm = ma;
         ja = jb;
         ma = mb;
@@ -756,21 +793,20 @@ static int resolve_proposals(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int64
         mb = tm;
     }
     int32_t *keep = as<int32_t>(b.keep), *pos = as<int32_t>(b.pos), *parent = as<int32_t>(b.parent);
-    CUSCAN_KERNEL(keep_kernel, blocks(n), 256, 0, s, next, ja, ma, active_label, n, keep, parent);
-    CUSCAN_LAUNCH(ctx, "cycle breaking");
-    int rc = scan_exclusive(ctx, keep, pos, n, as<int32_t>(b.kept_total), b.scan_tmp, s);
-    if (rc) return rc;
-    CUSCAN_KERNEL(emit_kernel, blocks(n), 256, 0, s, keep, pos, as<uint32_t>(b.esrc), as<uint32_t>(b.edst),
-                                           as<float>(b.ew), n, b.status, out_src, out_dst, out_w,
-                                           n - 1);
-    CUSCAN_KERNEL(add_edges_kernel, 1, 1, 0, s, b.status, as<int32_t>(b.kept_total), require_progress);
-    for (int t = 0; t < steps; ++t) CUSCAN_KERNEL(jump_kernel, blocks(n), 256, 0, s, parent, active_label, n);
     int32_t *minlab = as<int32_t>(b.minlab);
-    CUSCAN_KERNEL(minlab_init_kernel, blocks(n), 256, 0, s, parent, active_label, n, minlab);
-    CUSCAN_KERNEL(minlab_reduce_kernel, blocks(n), 256, 0, s, parent, active_label, n, minlab);
-    CUSCAN_KERNEL(relabel_kernel, blocks(n), 256, 0, s, point_label, parent, minlab, n);
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(&b.status->components, 0, sizeof(unsigned long long), s));
-    CUSCAN_KERNEL(count_components_kernel, blocks(n), 256, 0, s, point_label, n, b.status);
+    CUSCAN_KERNEL(keep_kernel, blocks(n), 256, 0, s, next, ja, ma, active_label, n, keep, parent,
+                  minlab);
+    CUSCAN_LAUNCH(ctx, "cycle breaking");
+    int rc = scan_exclusive(ctx, b, keep, pos, n, as<int32_t>(b.kept_total), s);
+    if (rc) return rc;
+    CUSCAN_KERNEL(emit_kernel, blocks(n), 256, 0, s, keep, pos, as<int32_t>(b.scan_tmp),
+                  as<uint32_t>(b.esrc), as<uint32_t>(b.edst), as<float>(b.ew), n, b.status, out_src,
+                  out_dst, out_w, n - 1);
+    for (int t = 0; t < steps; ++t)
+        CUSCAN_KERNEL(jump_kernel, blocks(n), 256, 0, s, parent, active_label, n);
+    CUSCAN_KERNEL(minlab_reduce_kernel, blocks(n), 256, 0, s, parent, active_label, n, minlab,
+                  b.status, as<int32_t>(b.kept_total), require_progress);
+    CUSCAN_KERNEL(relabel_kernel, blocks(n), 256, 0, s, point_label, parent, minlab, n, b.status);
     CUSCAN_LAUNCH(ctx, "union/relabel");
     return CUSCAN_OK;
 }
@@ -833,15 +869,16 @@ int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, 
         CUSCAN_LAUNCH(ctx, "component sort");
         return CUSCAN_OK;
     }
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(cnt, 0, sizeof(int32_t) * n, s));
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(fill, 0, sizeof(int32_t) * n, s));
+    CUSCAN_KERNEL(sort_clear_kernel, blocks(n), 256, 0, s, cnt, fill,
+                  as<unsigned long long>(b.row_keys), as<unsigned long long>(b.comp_keys), n,
+                  b.status);
     CUSCAN_KERNEL(hist_kernel, blocks(n), 256, 0, s, label, n, cnt);
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(&b.status->same_pairs, 0, sizeof(double), s));
-    CUSCAN_KERNEL(same_pairs_kernel, blocks(n), 256, 0, s, cnt, n, b.status);
     CUSCAN_LAUNCH(ctx, "hist_kernel");
-    int rc = scan_exclusive(ctx, cnt, start, n, nullptr, b.scan_tmp, s);
+    // same_pairs: the sum of squared component sizes, for the work counters
+    int rc = scan_exclusive(ctx, b, cnt, start, n, nullptr, s, &b.status->same_pairs);
     if (rc) return rc;
-    CUSCAN_KERNEL(scatter_kernel, blocks(n), 256, 0, s, label, n, start, fill, as<int32_t>(b.perm));
+    CUSCAN_KERNEL(scatter_kernel, blocks(n), 256, 0, s, label, n, start, as<int32_t>(b.scan_tmp),
+                  fill, as<int32_t>(b.perm));
     CUSCAN_KERNEL(gather_kernel, blocks(n * d), 256, 0, s, x, core, label, as<int32_t>(b.perm), n, d,
                                                  as<float>(b.xp), as<float>(b.corep),
                                                  as<int32_t>(b.labp));
@@ -861,8 +898,6 @@ int forest_round(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int64_t component
         CUSCAN_LAUNCH(ctx, "small_merge_kernel");
         return CUSCAN_OK;
     }
-    int rc = launch_fill_u64(ctx, comp_keys, n, ~0ull, s);
-    if (rc) return rc;
     CUSCAN_KERNEL(component_min_kernel, blocks(n), 256, 0, s, as<int32_t>(b.perm),
                   as<int32_t>(b.labp), as<unsigned long long>(b.row_keys), n, comp_keys, b.status,
                   allow_empty);

@@ -11,7 +11,8 @@ struct DevStatus {
     unsigned long long edges;       // MST edges emitted so far
     double same_pairs;     // sum of squared component sizes entering the current round
     int err_kind;          // 0 ok, 1 numerical weight, 2 index out of range, 4 no progress
-    int pad[3];
+    unsigned int scan_ticket;  // blocks of the running scan that have finished (0 between scans)
+    int pad[2];
     double mst_weight;     // f64 total MST weight, written once after the last round
     // kept on the device by packed fits (no host read after every round): the seed's results,
     // rounds run and ordered cross pairs entering them
@@ -75,8 +76,8 @@ bool forest_small(int64_t n);
 int forest_seed(cuscan_ctx *ctx, ForestBuffers &b, float *core, const int32_t *ids,
                 const float *dsq, int64_t n, int k, int min_samples, int32_t *label,
                 uint32_t *out_src, uint32_t *out_dst, float *out_w, cudaStream_t s);
-// Group points by label: perm, xp, corep, labp. Small sets (forest_small) also get cleared row keys
-// and the label range of every 32-row tile.
+// Group points by label: perm, xp, corep, labp; clears the row and component keys. Small sets
+// (forest_small) also get the label range of every 32-row tile.
 int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, const float *core,
                              const int32_t *label, int64_t n, int d, cudaStream_t s);
 // Merge one round from the per-row candidate keys in b.row_keys.
@@ -89,8 +90,11 @@ int forest_round(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int64_t component
 // fixed order (deterministic for a given edge list).
 int forest_mst_weight(cuscan_ctx *ctx, ForestBuffers &b, const float *w, int64_t m,
                       cudaStream_t s);
-int scan_exclusive(cuscan_ctx *ctx, const int32_t *in, int32_t *out, int64_t n,
-                   int32_t *grand_total, Buffer &tmp, cudaStream_t s);
+// Exclusive scan in one launch: entry i's position is out[i] + scan_tmp[i / kScanTile]. The total
+// goes to grand_total and the sum of squares is added to square_sum (either may be null).
+constexpr int kScanTile = 1024;
+int scan_exclusive(cuscan_ctx *ctx, ForestBuffers &b, const int32_t *in, int32_t *out, int64_t n,
+                   int32_t *grand_total, cudaStream_t s, double *square_sum = nullptr);
 
 // ---- packed small fits (pack.cu): one launch per step for every fit of a pack ----
 // One fit of a pack: its sizes and every device buffer its steps use. An array of these sits

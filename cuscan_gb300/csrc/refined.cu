@@ -125,6 +125,10 @@ constexpr int RESCREEN_MIN_ROWS = 256;  // fewer inconclusive kNN rows go straig
 // A bf16-refined fit whose first kNN screen leaves more than this share of rows inconclusive
 // screens again with tighter operands (split bf16, or scaled fp16 for rows too wide to split).
 constexpr double TIGHTEN_TRIGGER = 0.15;
+// Status words of a screen: [0] error flag, [2..3] tile pairs (u64), [4] inconclusive rows listed by
+// the re-rank, [5] spare.
+constexpr int SCREEN_STATUS_WORDS = 8;
+constexpr int STATUS_FALLBACKS = 4;
 // Operand formats of the 16-bit copy.
 constexpr int FMT_BF16 = 0;
 constexpr int FMT_FP16 = 1;
@@ -274,65 +278,122 @@ __host__ __device__ __forceinline__ uint64_t tiled_offset(int64_t r, int f, int 
            (uint64_t)rr * 128 + (uint64_t)chunk * 16 + (uint64_t)(c & 7) * 2;
 }
 
-// 16-bit tiled copy of the (scaled) rows: bf16, fp16 of x * scale (scale a power of two), or
-// split bf16 (hi in columns [0, d_pad), lo = bf16(x - hi) in [d_pad, 2 d_pad)).
-// Row r of the copy is row rowmap[r] of x (r itself when rowmap is null); rows >= n are zero.
+// Order-preserving map of f32 values to u32 (for integer warp reductions) and back.
+__device__ __forceinline__ uint32_t f2ord(float f) {
+    const uint32_t u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float ord2f(uint32_t o) {
+    return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
+}
+// Everything a screen needs of a set of rows, one block per 256-row tile: the 16-bit tiled copy of
+// the (scaled) rows (bf16, fp16 of x * scale, scale a power of two, or split bf16: hi in columns
+// [0, d_pad), lo = bf16(x - hi) in [d_pad, 2 d_pad)), their squared norms and rounded-up norms, the
+// tile's largest norm and, with labels, the label ranges of its 32-row chunks and of the tile.
+// Row r is row rowmap[r] of x (r itself when rowmap is null); rows >= n are zero with norm +inf.
+// Eight lanes share a row, eight features each per step, so the rows are read once with
+// consecutive addresses; separate kernels for the copy, the norms (one thread per row), the
+// tile statistics and the label ranges took 22 us per round of a 9,001 x 32 fit.
+constexpr int PREP_THREADS = 1024;
 template <int FMT>
-__global__ void tile_16bit_kernel(const float *__restrict__ x, int64_t n, int d, int d_pad,
-                                  int64_t n_pad, float scale, const int32_t *__restrict__ rowmap,
-                                  uint8_t *__restrict__ xt) {
-    // one thread per (row, group of 8 features): 16 bytes out (32 for split)
-    const int groups = d_pad >> 3;
+__global__ void __launch_bounds__(PREP_THREADS)
+    prep_rows_kernel(const float *__restrict__ x, int64_t n, int d, int d_pad, float scale,
+                     const int32_t *__restrict__ rowmap, int vec4, uint8_t *__restrict__ xt,
+                     float *__restrict__ pnorm, float *__restrict__ mnorm,
+                     float *__restrict__ tile_mmax, const int32_t *__restrict__ label,
+                     int32_t *__restrict__ chunk_lo, int32_t *__restrict__ chunk_hi,
+                     int32_t *__restrict__ tile_lo, int32_t *__restrict__ tile_hi) {
+    __shared__ float warp_max[PREP_THREADS / 32];
+    __shared__ int32_t range_lo[BN / 32], range_hi[BN / 32];
+    const int tid = threadIdx.x, lane = tid & 31, sub = tid & 7;
+    const int64_t row0 = (int64_t)blockIdx.x * BN;
     const int d_eff = FMT == FMT_SPLIT ? 2 * d_pad : d_pad;
-    int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_pad * groups) return;
-    int64_t r = e / groups;
-    int g = (int)(e - r * groups);
-    const int64_t src = r < n ? (rowmap ? (int64_t)rowmap[r] : r) : 0;
-    __align__(16) uint16_t h[8];
-    __align__(16) uint16_t l[8];
+    float mmax = 0.0f;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        int f = g * 8 + q;
-        float v = (r < n && f < d) ? x[src * d + f] : 0.0f;
-        if constexpr (FMT == FMT_FP16) {
-            h[q] = __half_as_ushort(__float2half_rn(v * scale));
-        } else {
-            const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-            h[q] = __bfloat16_as_ushort(hi);
-            // v - hi is exact in f32 (hi is within a factor of two of v)
+    for (int rr = 0; rr < BN; rr += PREP_THREADS / 8) {
+        const int64_t r = row0 + rr + (tid >> 3);
+        const bool valid = r < n;
+        const float *src = x + (valid ? (rowmap ? (int64_t)rowmap[r] : r) : 0) * d;
+        float acc = 0.0f;
+        for (int g = sub; g < d_pad / 8; g += 8) {
+            const int f0 = g * 8;
+            float v[8];
+            if (vec4 && valid && f0 + 8 <= d) {
+                const float4 a = *reinterpret_cast<const float4 *>(src + f0);
+                const float4 b = *reinterpret_cast<const float4 *>(src + f0 + 4);
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+                v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] = valid && f0 + q < d ? src[f0 + q] : 0.0f;
+            }
+            __align__(16) uint16_t h[8];
+            __align__(16) uint16_t l[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const float sv = v[q] * scale;
+                acc = __fmaf_rn(sv, sv, acc);
+                if constexpr (FMT == FMT_FP16) {
+                    h[q] = __half_as_ushort(__float2half_rn(sv));
+                } else {
+                    const __nv_bfloat16 hi = __float2bfloat16_rn(v[q]);
+                    h[q] = __bfloat16_as_ushort(hi);
+                    // v - hi is exact in f32 (hi is within a factor of two of v)
+                    if constexpr (FMT == FMT_SPLIT)
+                        l[q] = __bfloat16_as_ushort(
+                            __float2bfloat16_rn(v[q] - __bfloat162float(hi)));
+                }
+            }
+            *reinterpret_cast<uint4 *>(xt + tiled_offset(r, f0, d_eff)) =
+                *reinterpret_cast<const uint4 *>(h);
             if constexpr (FMT == FMT_SPLIT)
-                l[q] = __bfloat16_as_ushort(__float2bfloat16_rn(v - __bfloat162float(hi)));
+                *reinterpret_cast<uint4 *>(xt + tiled_offset(r, d_pad + f0, d_eff)) =
+                    *reinterpret_cast<const uint4 *>(l);
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        // rounded-up norm, widened by 2^-20 so it bounds the true norm despite the f32 sum
+        const float m = valid ? __fmul_ru(__fsqrt_ru(acc), 1.0f + 0x1p-20f) : 0.0f;
+        if (sub == 0) {
+            pnorm[r] = valid ? acc : CUSCAN_INF;
+            mnorm[r] = m;
+        }
+        mmax = fmaxf(mmax, m);
+    }
+    if (tile_mmax) {
+        mmax = ord2f(__reduce_max_sync(0xffffffffu, f2ord(mmax)));
+        if (lane == 0) warp_max[tid >> 5] = mmax;
+        if (label && tid < BN) {
+            // a warp per 32-row chunk; chunks past the end have the empty range
+            const int64_t r = row0 + tid;
+            const int32_t l = r < n ? label[r] : 0;
+            const int32_t lo = __reduce_min_sync(0xffffffffu, r < n ? l : INT32_MAX);
+            const int32_t hi = __reduce_max_sync(0xffffffffu, r < n ? l : INT32_MIN);
+            if (lane == 0) {
+                range_lo[tid >> 5] = lo;
+                range_hi[tid >> 5] = hi;
+                if (r < n) {
+                    chunk_lo[r >> 5] = lo;
+                    chunk_hi[r >> 5] = hi;
+                }
+            }
+        }
+        __syncthreads();
+        if (tid == 0) {
+            float mx = 0.0f;
+            for (int w = 0; w < PREP_THREADS / 32; ++w) mx = fmaxf(mx, warp_max[w]);
+            tile_mmax[blockIdx.x] = mx;
+            if (label) {
+                int32_t lo = INT32_MAX, hi = INT32_MIN;
+                for (int c = 0; c < BN / 32; ++c) {
+                    lo = min(lo, range_lo[c]);
+                    hi = max(hi, range_hi[c]);
+                }
+                tile_lo[blockIdx.x] = lo;
+                tile_hi[blockIdx.x] = hi;
+            }
         }
     }
-    *reinterpret_cast<uint4 *>(xt + tiled_offset(r, g * 8, d_eff)) =
-        *reinterpret_cast<const uint4 *>(h);
-    if constexpr (FMT == FMT_SPLIT)
-        *reinterpret_cast<uint4 *>(xt + tiled_offset(r, d_pad + g * 8, d_eff)) =
-            *reinterpret_cast<const uint4 *>(l);
-}
-
-// Squared norms and rounded-up norms of the scaled rows (x * scale, exact for a power of two);
-// row r is row rowmap[r] of x when rowmap is given.
-__global__ void norms_kernel(const float *__restrict__ x, int64_t n, int d, int64_t n_pad,
-                             float scale, const int32_t *__restrict__ rowmap,
-                             float *__restrict__ pnorm, float *__restrict__ mnorm) {
-    int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_pad) return;
-    if (r >= n) {
-        pnorm[r] = CUSCAN_INF;
-        mnorm[r] = 0.0f;
-        return;
-    }
-    const int64_t src = rowmap ? (int64_t)rowmap[r] : r;
-    float acc = 0.0f;
-    for (int f = 0; f < d; ++f) {
-        float v = x[src * d + f] * scale;
-        acc = __fmaf_rn(v, v, acc);
-    }
-    pnorm[r] = acc;
-    // rounded-up norm, widened by 2^-20 so it bounds the true norm despite the f32 sum
-    mnorm[r] = __fmul_ru(__fsqrt_ru(acc), 1.0f + 0x1p-20f);
 }
 
 // Largest |x| over all coordinates (non-negative floats order like their bit patterns).
@@ -347,15 +408,27 @@ __global__ void absmax_kernel(const float *__restrict__ x, int64_t count,
     if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
 }
 
-// Column terms of one screen launch, computed once instead of by every epilogue warp that
+// Before a screen launch: its column terms, computed once instead of by every epilogue warp that
 // reads the columns: colp = (1 - C_B) p (+inf on padding rows), colc = core * s2 (Borůvka; 0
-// past n), and for every 32-column chunk (min colp, min colc) (0 for colc in the kNN modes).
-// One thread per padded row; n_pad is a multiple of the 256-thread block.
+// past n), and for every 32-column chunk (min colp, min colc) (0 for colc in the kNN modes); and
+// its cleared counters: the status words, the cursor, the append counts of the query rows and, for
+// split blocks, their bounds (+inf). One thread per padded row; n_pad is a multiple of the
+// 256-thread block.
 __global__ void screen_columns_kernel(const float *__restrict__ pnorm,
                                       const float *__restrict__ core, int64_t n,
                                       float one_minus_cb, float s2, float *__restrict__ colp,
-                                      float *__restrict__ colc, float2 *__restrict__ cmin) {
+                                      float *__restrict__ colc, float2 *__restrict__ cmin,
+                                      int *__restrict__ status,
+                                      unsigned long long *__restrict__ cursor,
+                                      int2 *__restrict__ rowcnt, float2 *__restrict__ rowlb,
+                                      int64_t nq) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < SCREEN_STATUS_WORDS) status[j] = 0;
+    if (j < 2) cursor[j] = 0ull;
+    if (j < nq) {
+        if (rowcnt) rowcnt[j] = make_int2(0, 0);
+        if (rowlb) rowlb[j] = make_float2(CUSCAN_INF, CUSCAN_INF);
+    }
     const float p = pnorm[j] * one_minus_cb;
     colp[j] = p;
     float c = 0.0f;
@@ -370,26 +443,6 @@ __global__ void screen_columns_kernel(const float *__restrict__ pnorm,
         cm = fminf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
     }
     if ((threadIdx.x & 31) == 0) cmin[j >> 5] = make_float2(pm, cm);
-}
-
-__global__ void tile_stats_kernel(const float *__restrict__ mnorm, const int32_t *__restrict__ chunk_lo,
-                                  const int32_t *__restrict__ chunk_hi, int64_t n_tiles,
-                                  int64_t n_chunks, float *__restrict__ tile_mmax,
-                                  int32_t *__restrict__ tile_lo, int32_t *__restrict__ tile_hi) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_tiles) return;
-    float mx = 0.0f;
-    for (int r = 0; r < BN; ++r) mx = fmaxf(mx, mnorm[t * BN + r]);
-    tile_mmax[t] = mx;
-    if (chunk_lo) {
-        int32_t lo = INT32_MAX, hi = INT32_MIN;
-        for (int64_t c = t * 8; c < t * 8 + 8 && c < n_chunks; ++c) {
-            lo = min(lo, chunk_lo[c]);
-            hi = max(hi, chunk_hi[c]);
-        }
-        tile_lo[t] = lo;
-        tile_hi[t] = hi;
-    }
 }
 
 // Order in which query block qb visits the reference tiles. Every order starts with a window of
@@ -408,14 +461,6 @@ __global__ void tile_stats_kernel(const float *__restrict__ mnorm, const int32_t
 // DRAM about a thousand times over.
 constexpr int64_t WARM = 4;
 
-// Order-preserving map of f32 values to u32 (for integer warp reductions) and back.
-__device__ __forceinline__ uint32_t f2ord(float f) {
-    const uint32_t u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float ord2f(uint32_t o) {
-    return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
-}
 __device__ __forceinline__ float warp_max_f(float v) {
     return ord2f(__reduce_max_sync(0xffffffffu, f2ord(v)));
 }
@@ -1449,6 +1494,7 @@ __global__ void rerank_boruvka_kernel(const float *__restrict__ xp, const float 
                                       const int32_t *__restrict__ rowcnt, int cap,
                                       const int32_t *__restrict__ colcnt,
                                       const int32_t *__restrict__ colbuf, int capc,
+                                      const float *__restrict__ lbtmp, float *__restrict__ rowlb,
                                       unsigned long long *__restrict__ row_keys,
                                       int32_t *__restrict__ fallback,
                                       int *__restrict__ fallback_count) {
@@ -1457,6 +1503,12 @@ __global__ void rerank_boruvka_kernel(const float *__restrict__ xp, const float 
     const int lane = threadIdx.x & 31;
     if (q >= nq) return;
     const int64_t pos = qpos ? (int64_t)qpos[q] : q;
+    // Fold the one-sided screen's bounds (two column halves per query row) into the per-row lower
+    // bounds, kept in original row order across rounds.
+    if (lbtmp && lane == 0) {
+        const int32_t orow = perm[pos];
+        rowlb[orow] = fmaxf(rowlb[orow], fminf(lbtmp[2 * q], lbtmp[2 * q + 1]));
+    }
     const int c0 = rowcnt[q * 2], c1 = rowcnt[q * 2 + 1];
     const int c2 = colcnt ? colcnt[pos] : 0;  // pairs other blocks appended for this row
     if (c0 > cap || c1 > cap || c2 > capc) {
@@ -1554,17 +1606,17 @@ __global__ void init_row_bounds_kernel(const uint32_t *__restrict__ cbound,
     if ((threadIdx.x & 31) == 0 && m) atomicAdd(unbounded, __popc(m));
 }
 
-// Fold the one-sided screen's bounds (two column halves per query row) into the per-row lower
-// bounds, kept in original row order across rounds.
-__global__ void update_row_lb_kernel(const float *__restrict__ lbtmp,
-                                     const int32_t *__restrict__ qpos,
-                                     const int32_t *__restrict__ perm, int64_t nq,
-                                     float *__restrict__ rowlb) {
-    int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nq) return;
-    const int64_t pos = qpos ? (int64_t)qpos[q] : q;
-    const int32_t orow = perm[pos];
-    rowlb[orow] = fmaxf(rowlb[orow], fminf(lbtmp[2 * q], lbtmp[2 * q + 1]));
+// Start of a screened round: no component bound, empty column-side buffers, zero counts and, in a
+// fit's first round (rowlb given), no row bounds.
+__global__ void round_clear_kernel(uint32_t *__restrict__ cbound, int32_t *__restrict__ colcnt,
+                                   float *__restrict__ rowlb, int32_t *__restrict__ count,
+                                   int64_t n) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 2) count[i] = 0;
+    if (i >= n) return;
+    cbound[i] = 0x7f800000u;
+    colcnt[i] = 0;
+    if (rowlb) rowlb[i] = 0.0f;
 }
 
 // Exact rounds: the weight of each scanned row's cheapest cross-component edge (the top half of
@@ -1585,10 +1637,11 @@ __global__ void row_lb_from_keys_kernel(const unsigned long long *__restrict__ r
 
 // Positions of the flagged rows, in order (idx is the exclusive scan of the flags).
 __global__ void compact_positions_kernel(const int32_t *__restrict__ flag,
-                                         const int32_t *__restrict__ idx, int64_t n,
+                                         const int32_t *__restrict__ idx,
+                                         const int32_t *__restrict__ sums, int64_t n,
                                          int32_t *__restrict__ out) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && flag[i]) out[idx[i]] = (int32_t)i;
+    if (i < n && flag[i]) out[idx[i] + sums[i / kScanTile]] = (int32_t)i;
 }
 
 __global__ void fill_u32_kernel(uint32_t *p, int64_t n, uint32_t v) {
@@ -1716,49 +1769,50 @@ size_t refined_workspace_bytes(int64_t n, int d, int k) {
     return b;
 }
 
-// 16-bit tiled copy and norms of n rows (row r = rowmap[r] of x, or r), padded to n_pad rows.
+// prep_rows_kernel over n_pad / 256 tiles in the fit's operand format.
 static int tile_rows(cuscan_ctx *ctx, const RefinedBuffers &R, const float *x, int64_t n, int d,
                      int d_pad, int64_t n_pad, const int32_t *rowmap, uint8_t *xt, float *pnorm,
-                     float *mnorm, cudaStream_t s) {
-    const int64_t groups = n_pad * (d_pad / 8);
-    const unsigned gb = (unsigned)ceil_div(groups, 256);
+                     float *mnorm, cudaStream_t s, float *tile_mmax = nullptr,
+                     const int32_t *label = nullptr, int32_t *chunk_lo = nullptr,
+                     int32_t *chunk_hi = nullptr, int32_t *tile_lo = nullptr,
+                     int32_t *tile_hi = nullptr) {
+    const unsigned tiles = (unsigned)(n_pad / BN);
+    const int vec4 = d % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0;  // aligned rows
     if (R.fp16)
-        CUSCAN_KERNEL(tile_16bit_kernel<FMT_FP16>, gb, 256, 0, s, x, n, d, d_pad, n_pad, R.scale,
-                      rowmap, xt);
+        CUSCAN_KERNEL(prep_rows_kernel<FMT_FP16>, tiles, PREP_THREADS, 0, s, x, n, d, d_pad, R.scale,
+                      rowmap, vec4, xt, pnorm, mnorm, tile_mmax, label, chunk_lo, chunk_hi, tile_lo,
+                      tile_hi);
     else if (R.split)
-        CUSCAN_KERNEL(tile_16bit_kernel<FMT_SPLIT>, gb, 256, 0, s, x, n, d, d_pad, n_pad, 1.0f,
-                      rowmap, xt);
+        CUSCAN_KERNEL(prep_rows_kernel<FMT_SPLIT>, tiles, PREP_THREADS, 0, s, x, n, d, d_pad, 1.0f,
+                      rowmap, vec4, xt, pnorm, mnorm, tile_mmax, label, chunk_lo, chunk_hi, tile_lo,
+                      tile_hi);
     else
-        CUSCAN_KERNEL(tile_16bit_kernel<FMT_BF16>, gb, 256, 0, s, x, n, d, d_pad, n_pad, 1.0f,
-                      rowmap, xt);
-    CUSCAN_KERNEL(norms_kernel, (unsigned)ceil_div(n_pad, 256), 256, 0, s, x, n, d, n_pad,
-                  R.fp16 ? R.scale : 1.0f, rowmap, pnorm, mnorm);
-    CUSCAN_LAUNCH(ctx, "16-bit tiles");
+        CUSCAN_KERNEL(prep_rows_kernel<FMT_BF16>, tiles, PREP_THREADS, 0, s, x, n, d, d_pad, 1.0f,
+                      rowmap, vec4, xt, pnorm, mnorm, tile_mmax, label, chunk_lo, chunk_hi, tile_lo,
+                      tile_hi);
+    CUSCAN_LAUNCH(ctx, "prep_rows_kernel");
     return CUSCAN_OK;
 }
 
+// Tiles, norms and statistics of the reference rows; with labels, their chunk and tile ranges.
 static int prep(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, const float *x, int64_t n,
-                int d, const int32_t *chunk_lo, const int32_t *chunk_hi, cudaStream_t s) {
+                int d, const int32_t *label, int32_t *chunk_lo, int32_t *chunk_hi,
+                cudaStream_t s) {
     int rc = ensure(ctx, R.xt, (size_t)L.n_tiles * L.nbk * KBLOCK_B, "16-bit tiles");
     if (!rc) rc = ensure(ctx, R.pnorm, sizeof(float) * L.n_pad, "norms");
     if (!rc) rc = ensure(ctx, R.mnorm, sizeof(float) * L.n_pad, "norms");
     if (!rc) rc = ensure(ctx, R.tile_mmax, sizeof(float) * L.n_tiles, "tile norms");
     if (!rc) rc = ensure(ctx, R.tile_lo, sizeof(int32_t) * L.n_tiles, "tile labels");
     if (!rc) rc = ensure(ctx, R.tile_hi, sizeof(int32_t) * L.n_tiles, "tile labels");
-    if (!rc) rc = ensure(ctx, R.error, 16, "error flag");
-    if (!rc) rc = ensure(ctx, R.count, 16, "fallback count");
+    if (!rc) rc = ensure(ctx, R.error, sizeof(int) * SCREEN_STATUS_WORDS, "screen status");
+    if (!rc) rc = ensure(ctx, R.count, 16, "row counts");
     if (!rc) rc = ensure(ctx, R.cursor, 16, "tile cursor");
     if (!rc) rc = ensure(ctx, R.fallback, sizeof(int32_t) * n, "fallback rows");
     if (!rc) rc = ensure(ctx, R.qthr, sizeof(float) * n, "fallback thresholds");
     if (rc) return rc;
-    if ((rc = tile_rows(ctx, R, x, n, d, L.d_pad, L.n_pad, nullptr, as<uint8_t>(R.xt),
-                        as<float>(R.pnorm), as<float>(R.mnorm), s)))
-        return rc;
-    CUSCAN_KERNEL(tile_stats_kernel, (unsigned)ceil_div(L.n_tiles, 128), 128, 0, s,
-                  as<float>(R.mnorm), chunk_lo, chunk_hi, L.n_tiles, ceil_div(n, 32),
-                  as<float>(R.tile_mmax), as<int32_t>(R.tile_lo), as<int32_t>(R.tile_hi));
-    CUSCAN_LAUNCH(ctx, "refined prep");
-    return CUSCAN_OK;
+    return tile_rows(ctx, R, x, n, d, L.d_pad, L.n_pad, nullptr, as<uint8_t>(R.xt),
+                     as<float>(R.pnorm), as<float>(R.mnorm), s, as<float>(R.tile_mmax), label,
+                     chunk_lo, chunk_hi, as<int32_t>(R.tile_lo), as<int32_t>(R.tile_hi));
 }
 
 // Operand format of this fit's screens: fp16 of x * scale when the caller asked for it and the
@@ -1896,7 +1950,6 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
         if (rc) return rc;
         P.cbound = as<uint32_t>(R.cbound);
         P.rowcnt = as<int32_t>(R.rowcnt);
-        CUSCAN_CUDA(ctx, cudaMemsetAsync(R.rowcnt.ptr, 0, sizeof(int32_t) * 2 * n, s));
     }
     if (MODE == MODE_BORUVKA_SYM) {
         P.urow = as<uint32_t>(R.urow);
@@ -1905,18 +1958,12 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
         P.capc = BORUVKA_COL_CAP;
     }
     if (MODE == MODE_BORUVKA) P.rowlb = Q.rowlb;
-    if (MODE == MODE_BORUVKA && P.splits > 1 && P.rowlb && P.nq > 0)
-        if (int rc = launch_fill_u64(ctx, reinterpret_cast<unsigned long long *>(P.rowlb), P.nq,
-                                     0x7f8000007f800000ull, s))  // +inf in both halves
-            return rc;
     if (MODE == MODE_KNN_THRESHOLD) {
         P.cap = KNN_CAP;
         P.cand_ids = Q.cand_ids;
         P.rowcnt = Q.rowcnt;
     }
     if (P.n_qblocks == 0) return CUSCAN_OK;
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(R.error.ptr, 0, 16, s));
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(R.cursor.ptr, 0, 16, s));
     // the column terms of this launch (its C_B and, for Borůvka, the core scale)
     if (int rc = ensure(ctx, R.colp, sizeof(float) * L.n_pad, "screen column norms")) return rc;
     if (BORUVKA)
@@ -1927,7 +1974,9 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
     P.cmin = as<float4>(R.cmin);
     CUSCAN_KERNEL(screen_columns_kernel, (unsigned)(L.n_pad / 256), 256, 0, s, P.pnorm,
                   BORUVKA ? core : nullptr, n, P.one_minus_cb, P.s2, as<float>(R.colp),
-                  BORUVKA ? as<float>(R.colc) : nullptr, as<float2>(R.cmin));
+                  BORUVKA ? as<float>(R.colc) : nullptr, as<float2>(R.cmin), P.error, P.cursor,
+                  BORUVKA ? reinterpret_cast<int2 *>(P.rowcnt) : nullptr,
+                  P.splits > 1 ? reinterpret_cast<float2 *>(P.rowlb) : nullptr, P.nq);
     CUSCAN_LAUNCH(ctx, "screen_columns_kernel");
     auto kernel = screen_kernel<M, MODE>;
     if (int rc = allow_dynamic_smem(ctx, kernel, L.smem)) return rc;
@@ -1939,17 +1988,16 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
 }
 
 static int read_screen_status(cuscan_ctx *ctx, RefinedBuffers &R, cudaStream_t s, int &fallbacks) {
-    unsigned long long status[2] = {0, 0};  // error flag, tile pairs
-    int count = 0;
-    CUSCAN_CUDA(ctx, cudaMemcpyAsync(status, R.error.ptr, 16, cudaMemcpyDeviceToHost, s));
-    CUSCAN_CUDA(ctx, cudaMemcpyAsync(&count, R.count.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
+    int status[SCREEN_STATUS_WORDS] = {0};
+    CUSCAN_CUDA(ctx, cudaMemcpyAsync(status, R.error.ptr, sizeof(status), cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
-    if ((int)(status[0] & 0xffffffffu))
+    if (status[0])
         return fail(ctx, CUSCAN_BACKEND_UNAVAILABLE,
                     "tensor-core screening timed out waiting on a pipeline barrier");
-    R.tile_pairs += (int64_t)status[1];
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(R.error.ptr, 0, 16, s));
-    fallbacks = count;
+    unsigned long long tiles;
+    memcpy(&tiles, status + 2, sizeof(tiles));
+    R.tile_pairs += (int64_t)tiles;
+    fallbacks = status[STATUS_FALLBACKS];
     return CUSCAN_OK;
 }
 
@@ -1963,7 +2011,7 @@ static int knn_list_pass(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, co
     // exact distance at k <= 32 for bf16 screens (the rest go to the threshold re-screen), and
     // each insertion shifts 22 registers; 20 and 24 entries measured slower
     constexpr int M = KNN_LIST;
-    if (int rc = prep(ctx, R, L, xs, n, d, nullptr, nullptr, s)) return rc;
+    if (int rc = prep(ctx, R, L, xs, n, d, nullptr, nullptr, nullptr, s)) return rc;
     for (cudaEvent_t &e : R.screen_ev)
         if (!e) CUSCAN_CUDA(ctx, cudaEventCreate(&e));
     CUSCAN_CUDA(ctx, cudaEventRecord(R.screen_ev[0], s));
@@ -1971,13 +2019,12 @@ static int knn_list_pass(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, co
         return rc;
     CUSCAN_CUDA(ctx, cudaEventRecord(R.screen_ev[1], s));
     R.screen_timed = true;
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(R.count.ptr, 0, sizeof(int), s));
     const size_t rr_smem = sizeof(float) * RERANK_WARPS * (size_t)rerank_warp_floats(d);
     if (int rc = allow_dynamic_smem(ctx, rerank_knn_kernel<M>, rr_smem)) return rc;
     CUSCAN_KERNEL(rerank_knn_kernel<M>, (unsigned)ceil_div(n, (int64_t)RERANK_WARPS),
                   32 * RERANK_WARPS, rr_smem, s, xs, perm, n, d,
                   k, as<int32_t>(R.cand_ids), as<float>(R.cand_lb), ids, dist,
-                  as<int32_t>(R.fallback), as<float>(R.qthr), as<int>(R.count));
+                  as<int32_t>(R.fallback), as<float>(R.qthr), as<int>(R.error) + STATUS_FALLBACKS);
     CUSCAN_LAUNCH(ctx, "rerank_knn_kernel");
     return read_screen_status(ctx, R, s, fallbacks);
 }
@@ -2068,13 +2115,12 @@ int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
         if ((rc = run_screen<M, MODE_KNN_THRESHOLD>(ctx, R, L, n, d, nullptr, nullptr, nullptr,
                                                    nullptr, s, nullptr, nullptr, Q)))
             return rc;
-        CUSCAN_CUDA(ctx, cudaMemsetAsync(R.count.ptr, 0, sizeof(int), s));
         if ((rc = allow_dynamic_smem(ctx, rerank_knn_threshold_kernel, rr_smem))) return rc;
         CUSCAN_KERNEL(rerank_knn_threshold_kernel, (unsigned)ceil_div(nq, (int64_t)RERANK_WARPS),
                       32 * RERANK_WARPS, rr_smem, s, xs,
                       perm, as<int32_t>(R.fallback), nq, d, k, as<int32_t>(R.cand2),
                       as<int32_t>(R.rowcnt2), KNN_CAP, ids, dist, as<int32_t>(R.fallback2),
-                      as<int>(R.count));
+                      as<int>(R.error) + STATUS_FALLBACKS);
         CUSCAN_LAUNCH(ctx, "rerank_knn_threshold_kernel");
         if ((rc = read_screen_status(ctx, R, s, exact))) return rc;
         if (rescreened_rows) *rescreened_rows += fallbacks;
@@ -2111,16 +2157,10 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
     if (rc) return rc;
     if (!R.range_ok)  // values large enough to overflow f32: the exact round decides alone
         return launch_candidates_fp32(ctx, xp, corep, labp, perm, n, d, row_keys, clo, chi, s);
-    rc = launch_tile_ranges(ctx, labp, n, clo, chi, s);
-    if (!rc) rc = prep(ctx, R, L, xp, n, d, clo, chi, s);
-    if (rc) return rc;
-    // component bounds: +inf, then the exact cross-component edges of the kNN rows
+    if ((rc = prep(ctx, R, L, xp, n, d, labp, clo, chi, s))) return rc;
+    // component bounds: +inf, then the exact cross-component edges of the kNN rows. Symmetric
+    // screen: per-row bounds start at the component bounds; empty column buffers
     if ((rc = ensure(ctx, R.cbound, sizeof(uint32_t) * n, "component bounds"))) return rc;
-    CUSCAN_KERNEL(fill_u32_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, as<uint32_t>(R.cbound), n,
-                  0x7f800000u);
-    CUSCAN_KERNEL(seed_bounds_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, knn_ids, knn_sq, k,
-                  core, label, n, as<uint32_t>(R.cbound));
-    // symmetric screen: per-row bounds start at the component bounds; empty column buffers
     if ((rc = ensure(ctx, R.urow, sizeof(uint32_t) * n, "row bounds"))) return rc;
     if ((rc = ensure(ctx, R.colcnt, sizeof(int32_t) * n, "column-side counts"))) return rc;
     if ((rc = ensure(ctx, R.colbuf, sizeof(int32_t) * n * BORUVKA_COL_CAP, "column-side candidates")))
@@ -2131,18 +2171,18 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
     if (!rc) rc = ensure(ctx, R.rowlb, sizeof(float) * n, "row lower bounds");
     if (!rc) rc = ensure(ctx, R.lbtmp, sizeof(float) * 2 * n, "row lower bounds");
     if (rc) return rc;
-    if (!R.lb_valid) {  // first round of the fit: no bounds yet
-        CUSCAN_CUDA(ctx, cudaMemsetAsync(R.rowlb.ptr, 0, sizeof(float) * n, s));
-        R.lb_valid = true;
-    }
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(R.colcnt.ptr, 0, sizeof(int32_t) * n, s));
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(R.count.ptr, 0, 2 * sizeof(int), s));
+    CUSCAN_KERNEL(round_clear_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, as<uint32_t>(R.cbound),
+                  as<int32_t>(R.colcnt), R.lb_valid ? nullptr : as<float>(R.rowlb),
+                  as<int32_t>(R.count), n);
+    R.lb_valid = true;
+    CUSCAN_KERNEL(seed_bounds_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, knn_ids, knn_sq, k,
+                  core, label, n, as<uint32_t>(R.cbound));
     CUSCAN_KERNEL(init_row_bounds_kernel, (unsigned)ceil_div(n, 256), 256, 0, s,
                   as<uint32_t>(R.cbound), labp, corep, as<float>(R.rowlb), perm, n,
                   as<uint32_t>(R.urow), as<int>(R.count), as<int32_t>(R.act_flag));
     CUSCAN_LAUNCH(ctx, "init_row_bounds_kernel");
-    if ((rc = scan_exclusive(ctx, as<int32_t>(R.act_flag), as<int32_t>(R.act_idx), n,
-                             as<int32_t>(R.count) + 1, b.scan_tmp, s)))
+    if ((rc = scan_exclusive(ctx, b, as<int32_t>(R.act_flag), as<int32_t>(R.act_idx), n,
+                             as<int32_t>(R.count) + 1, s)))
         return rc;
     int counts[2] = {0, 0};  // rows without a component bound, rows that can hold an edge
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(counts, R.count.ptr, sizeof(counts), cudaMemcpyDeviceToHost, s));
@@ -2174,7 +2214,8 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
         if (!rc) rc = ensure(ctx, R.mq, sizeof(float) * nq_pad, "subset norms");
         if (rc) return rc;
         CUSCAN_KERNEL(compact_positions_kernel, (unsigned)ceil_div(n, 256), 256, 0, s,
-                      as<int32_t>(R.act_flag), as<int32_t>(R.act_idx), n, as<int32_t>(R.act_pos));
+                      as<int32_t>(R.act_flag), as<int32_t>(R.act_idx),
+                      as<int32_t>(b.scan_tmp), n, as<int32_t>(R.act_pos));
         CUSCAN_LAUNCH(ctx, "compact_positions_kernel");
         qpos = as<int32_t>(R.act_pos);
         if ((rc = tile_rows(ctx, R, xp, nq, d, L.d_pad, nq_pad, qpos, as<uint8_t>(R.xq),
@@ -2196,14 +2237,8 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
         rc = run_screen<M, MODE_BORUVKA>(ctx, R, L, n, d, corep, labp, clo, chi, s, nullptr, nullptr, Q);
     }
     if (rc) return rc;
-    if (!sym && nq > 0) {
-        CUSCAN_KERNEL(update_row_lb_kernel, (unsigned)ceil_div(nq, 256), 256, 0, s,
-                      as<float>(R.lbtmp), qpos, perm, nq, as<float>(R.rowlb));
-        CUSCAN_LAUNCH(ctx, "update_row_lb_kernel");
-    }
     R.screened_rows += nq;
     if (sym) ++R.symmetric_rounds;
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(R.count.ptr, 0, sizeof(int), s));
     const size_t rr_smem = sizeof(float) * RERANK_WARPS * (size_t)rerank_warp_floats(d);
     if ((rc = allow_dynamic_smem(ctx, rerank_boruvka_kernel, rr_smem))) return rc;
     if (nq > 0) {
@@ -2211,15 +2246,16 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
                       32 * RERANK_WARPS, rr_smem, s, xp, corep, labp, perm, nq, qpos, d,
                       as<int32_t>(R.cand_ids), as<int32_t>(R.rowcnt), BORUVKA_CAP,
                       sym ? as<int32_t>(R.colcnt) : nullptr, as<int32_t>(R.colbuf),
-                      BORUVKA_COL_CAP, row_keys, as<int32_t>(R.fallback), as<int>(R.count));
+                      BORUVKA_COL_CAP, sym ? nullptr : as<float>(R.lbtmp), as<float>(R.rowlb),
+                      row_keys, as<int32_t>(R.fallback), as<int>(R.error) + STATUS_FALLBACKS);
         CUSCAN_LAUNCH(ctx, "rerank_boruvka_kernel");
     }
     int fallbacks = 0;
-    if ((rc = read_screen_status(ctx, R, s, fallbacks))) return rc;
+    if (nq > 0 && (rc = read_screen_status(ctx, R, s, fallbacks))) return rc;
     if (fallback_rows) *fallback_rows += fallbacks;
     if (fallbacks > 0)
         return launch_candidates_fp32(ctx, xp, corep, labp, perm, n, d, row_keys, clo, chi, s,
-                                      as<int32_t>(R.fallback), fallbacks);
+                                      as<int32_t>(R.fallback), fallbacks, 0, true);
     return CUSCAN_OK;
 }
 
@@ -2265,8 +2301,8 @@ int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, i
                   as<uint32_t>(R.cbound), labp, corep, as<float>(R.rowlb), perm, n,
                   as<uint32_t>(R.urow), as<int>(R.count), as<int32_t>(R.act_flag));
     CUSCAN_LAUNCH(ctx, "component bounds");
-    if ((rc = scan_exclusive(ctx, as<int32_t>(R.act_flag), as<int32_t>(R.act_idx), n,
-                             as<int32_t>(R.count) + 1, b.scan_tmp, s)))
+    if ((rc = scan_exclusive(ctx, b, as<int32_t>(R.act_flag), as<int32_t>(R.act_idx), n,
+                             as<int32_t>(R.count) + 1, s)))
         return rc;
     int counts[2] = {0, 0};  // rows without a component bound, rows that can hold an edge
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(counts, R.count.ptr, sizeof(counts), cudaMemcpyDeviceToHost, s));
@@ -2277,7 +2313,8 @@ int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, i
         rc = launch_candidates_fp32(ctx, xp, corep, labp, perm, n, d, row_keys, clo, chi, s);
     } else if (active > 0) {
         CUSCAN_KERNEL(compact_positions_kernel, (unsigned)ceil_div(n, 256), 256, 0, s,
-                      as<int32_t>(R.act_flag), as<int32_t>(R.act_idx), n, as<int32_t>(R.act_pos));
+                      as<int32_t>(R.act_flag), as<int32_t>(R.act_idx),
+                      as<int32_t>(b.scan_tmp), n, as<int32_t>(R.act_pos));
         CUSCAN_LAUNCH(ctx, "compact_positions_kernel");
         qpos = as<int32_t>(R.act_pos);
         rc = launch_candidates_fp32(ctx, xp, corep, labp, perm, n, d, row_keys, clo, chi, s, qpos,
@@ -2321,7 +2358,7 @@ int debug_screen_tile(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t
         return fail(ctx, CUSCAN_CAPACITY, "shape outside the tensor-core tiling%s",
                     R.split ? " (split copies need d <= 64)" : "");
     if (scale_out) *scale_out = R.fp16 ? R.scale : 1.0f;
-    rc = prep(ctx, R, L, x, n, d, nullptr, nullptr, s);
+    rc = prep(ctx, R, L, x, n, d, nullptr, nullptr, nullptr, s);
     if (!rc)
         rc = run_screen<32, MODE_KNN_LIST>(ctx, R, L, n, d, nullptr, nullptr, nullptr, nullptr, s,
                                            out, chunk_out);
@@ -2334,7 +2371,6 @@ int debug_screen_tile(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t
     }
     if (!rc) {
         int fallbacks = 0;
-        CUSCAN_CUDA(ctx, cudaMemsetAsync(R.count.ptr, 0, sizeof(int), s));
         rc = read_screen_status(ctx, R, s, fallbacks);
     }
     R.have_scale = false;
