@@ -4,6 +4,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "cells.cuh"
 #include "forest.cuh"
 #include "simt.cuh"
 #include "workspace.cuh"
@@ -22,7 +23,7 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
 int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d,
                                  const int32_t *knn_ids, const float *knn_sq, int k,
                                  const float *core, const int32_t *label, cudaStream_t s,
-                                 int64_t *screened_rows);
+                                 int64_t *screened_rows, const TileBounds *bounds);
 int debug_screen_tile(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, int d,
                       int operands, float *out, float *rows_out, float *chunk_out,
                       float *scale_out, cudaStream_t s);
@@ -33,7 +34,7 @@ size_t refined_workspace_bytes(int64_t n, int d, int k);
 static int workspace_buffers(FitWorkspace *f, Buffer **out) {
     Buffer *own[] = {&f->x, &f->ids, &f->dsq, &f->core, &f->label, &f->src, &f->dst, &f->w,
                      &f->op_keys, &f->op_tiles_lo, &f->op_tiles_hi, &f->op_partials,
-                     &f->op_knn_ids, &f->op_knn_dist, &f->pred_q, &f->pred_ids,
+                     &f->op_knn_ids, &f->op_knn_dist, &f->pred_q, &f->pred_order, &f->pred_ids,
                      &f->pred_dist};
     const int n_own = (int)(sizeof(own) / sizeof(own[0]));
     static_assert(sizeof(own) / sizeof(own[0]) == kOwnBufferCount, "buffer list");
@@ -146,8 +147,13 @@ int64_t cuscan_fit_workspace_bytes(int64_t n, int32_t d, int32_t min_samples, in
          (size_t)simt::split_plan_max_ctas(kSMs, ceil_div(n, (int64_t)simt::QT));
     if (precision == CUSCAN_PRECISION_BF16_REFINED || precision == CUSCAN_PRECISION_FP16_REFINED)
         b += refined_workspace_bytes(n, d, (int)k);
-    else if (n >= 2048)  // exact rounds over a row subset: bounds, flags, positions, counts
+    else if (n >= 2048) {  // exact rounds over a row subset: bounds, flags, positions, counts
         b += 7 * 4 * N + 64;
+        // rows in spatial order, bounds of their tiles, first thresholds
+        if (worth_pruning(n, n, d))
+            b += cells_workspace_bytes(n, d) + 4 * TileBounds::PARTS * (N / simt::RT + 1) * (D + 1) +
+                 8 * (size_t)padded_queries(n) + (size_t)kPrunedPartials;
+    }
     return (int64_t)b + (1 << 20);
 }
 
@@ -298,13 +304,29 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
     b.refined.lb_valid = false;
     b.refined.screen_timed = false;
 
+    const bool spatial = !refined && knn_pruned_shape(d, k) && worth_pruning(n, n, d);
+    TileBounds bounds;
     CUSCAN_CUDA(ctx, cudaMemsetAsync(b.status, 0, sizeof(DevStatus), s));
     CUSCAN_CUDA(ctx, cudaEventRecord(ev[0], s));
     // ---- core_distances: exact kNN sweep (estimator.rs:591-657) + core column ----
     if (refined)
         rc = launch_knn_refined(ctx, b, data, n, d, k, knn_ids, knn_sq, s, &refined_rows,
                                 &fallback_rows, &rescreened_rows);
-    else
+    else if (spatial) {
+        // plain f32 in spatial order: every distance that is formed is the same, and tiles whose
+        // every row is too far to matter are left out (here and in the rounds)
+        if ((rc = sort_by_cells(ctx, b, data, n, d, s))) return rc;
+        if ((rc = tile_bounds(ctx, as<float>(b.xp), n, d, b.refined.tile_centre,
+                              b.refined.tile_radius, bounds, s)))
+            return rc;
+        rc = ensure(ctx, b.refined.qorder, sizeof(int32_t) * padded_queries(n), "query order");
+        if (!rc) rc = order_positions(ctx, b, n, as<int32_t>(b.refined.qorder), s);
+        if (!rc)
+            rc = launch_knn_pruned(ctx, as<float>(b.xp), padded_queries(n), as<float>(b.xp), n, d, k,
+                                   1, knn_ids, knn_sq, s, b.knn_ids_tmp, b.knn_dist_tmp,
+                                   b.refined.thr0, bounds, as<int32_t>(b.perm),
+                                   as<int32_t>(b.refined.qorder), as<int32_t>(b.perm));
+    } else
         rc = launch_exact_knn_fp32(ctx, data, n, data, n, d, k, 1, 0, 1, knn_ids, knn_sq, s,
                                    b.knn_ids_tmp, b.knn_dist_tmp);
     if (rc) return rc;
@@ -328,7 +350,10 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
     while (components > 1) {
         const int64_t rows0 = b.refined.screened_rows, tiles0 = b.refined.tile_pairs;
         if (rounds > 64) return fail(ctx, CUSCAN_NUMERICAL, "Boruvka did not converge");
-        if ((rc = forest_sort_by_component(ctx, b, data, core_sq, label, n, d, s))) return rc;
+        // plain f32 in spatial order keeps that order; the others group the rows by component
+        rc = spatial ? forest_label_cells(ctx, b, core_sq, label, n, s)
+                     : forest_sort_by_component(ctx, b, data, core_sq, label, n, d, s);
+        if (rc) return rc;
         unsigned long long *row_keys = as<unsigned long long>(b.row_keys);
         const bool small = forest_small(n);  // its sort also fills the label ranges
         CUSCAN_CUDA(ctx, cudaEventRecord(ev[4], s));
@@ -337,7 +362,7 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
                                            &boruvka_fallback_rows);
         else if (exact_rows)
             rc = launch_candidates_exact_rows(ctx, b, n, d, knn_ids, knn_sq, k, core_sq, label, s,
-                                              &b.refined.screened_rows);
+                                              &b.refined.screened_rows, spatial ? &bounds : nullptr);
         else
             rc = launch_candidates_fp32(ctx, as<float>(b.xp), as<float>(b.corep),
                                         as<int32_t>(b.labp), as<int32_t>(b.perm), n, d, row_keys,

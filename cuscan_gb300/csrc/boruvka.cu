@@ -13,6 +13,7 @@
 // before any distance is computed; tile label ranges are precomputed per 32-row tile.
 #include <mutex>
 
+#include "cells.cuh"
 #include "forest.cuh"
 #include "simt.cuh"
 
@@ -52,9 +53,25 @@ struct CandShared {
     float q_core[QT];
     int32_t q_label[QT];
     int32_t q_range[2];
+    // pruned sweeps: what each query's cheapest edge has to beat, and the queries' ball
+    float thr[QT];
+    alignas(16) simt::QueryBalls balls;
 };
 constexpr size_t kCandSmem =
     sizeof(float) * simt::STAGES * simt::STAGE_FLOATS + sizeof(CandShared);
+
+// A pruned sweep: bounds of the reference tiles and the components' upper bounds (f32 bits, by
+// label). A pair is left out only when its weight exceeds both its query's best so far and the
+// bound of the query's component, so a query's key is its exact cheapest edge unless that exceeds
+// the component's bound (such a key, or none, cannot win the component).
+// The component bounds stay as the round starts with them: lowering them as the sweep finds
+// edges prunes more of a round (31.2 -> 26.3 ms at 100,000 x 64, round 2), but then fewer rows
+// leave a lower bound above their component's next bound, and the rounds after it scan more rows
+// (18,539 -> 75,251 in round 4): 66.6 ms became 74.7 ms over the fit's rounds.
+struct CandPrune {
+    TileBounds bounds;
+    const uint32_t *cbound;
+};
 
 // One CTA: 64 query rows [q0, q0 + 64) against rows [r_begin, r_end) (r_begin a multiple of the
 // reference tile); each query's cheapest cross-component key is folded into row_keys with
@@ -63,12 +80,14 @@ constexpr size_t kCandSmem =
 // looked at where a query's minimum over its eight references reaches its best so far.
 // Measured on a GB300, the four rounds of the anisotropic 100,000 x 64 fit in plain f32:
 // 86.7 ms against 143.1 ms for one query per thread.
+template <bool PRUNE = false>
 __device__ __forceinline__ void candidates_block(
     const float *__restrict__ data, const float *__restrict__ core,
     const int32_t *__restrict__ labels, const int32_t *__restrict__ ids, int64_t n, int d,
     const int32_t *__restrict__ tile_lo, const int32_t *__restrict__ tile_hi, int64_t q0,
     int64_t r_begin, int64_t r_end, unsigned long long *__restrict__ row_keys,
-    const int32_t *__restrict__ qmap, int64_t nq, int64_t qoff, float *smem) {
+    const int32_t *__restrict__ qmap, int64_t nq, int64_t qoff, float *smem,
+    const CandPrune &prune = CandPrune()) {
     CandShared &sh = *reinterpret_cast<CandShared *>(smem + simt::STAGES * simt::STAGE_FLOATS);
     const simt::Place p = simt::place();
     const int tid = threadIdx.x, lane = tid & 31;
@@ -88,8 +107,15 @@ __device__ __forceinline__ void candidates_block(
         sh.q_label[tid] = l;
         atomicMin(&sh.q_range[0], l);
         atomicMax(&sh.q_range[1], l);
+        if (PRUNE)
+            sh.thr[tid] = q0 + tid < nq ? __uint_as_float(prune.cbound[l]) : -CUSCAN_INF;
     }
     __syncthreads();
+    simt::PrunedWalk walk{};
+    if constexpr (PRUNE) {
+        simt::query_balls(sh.balls, data, sh.row, d);
+        walk.balls = &sh.balls;
+    }
     const int32_t qlo = sh.q_range[0];
     const bool q_uniform = qlo == sh.q_range[1];
     float qc[8], bw[8];
@@ -106,7 +132,7 @@ __device__ __forceinline__ void candidates_block(
     const int64_t t_end = ceil_div(r_end, (int64_t)simt::RT), ranges = ceil_div(n, (int64_t)RT);
     // A tile whose rows all carry the one label of the CTA's queries holds no cross pair. The
     // lanes of every warp look at 32 tiles at a time.
-    auto next = [&](int64_t t) -> int64_t {
+    auto other_component = [&](int64_t t) -> int64_t {
         if (!q_uniform) return t;
         while (t < t_end) {
             const int64_t mine = t + lane;
@@ -124,6 +150,17 @@ __device__ __forceinline__ void candidates_block(
         }
         return t_end;
     };
+    auto next = [&](int64_t t) -> int64_t {
+        if constexpr (PRUNE) {
+            for (;;) {
+                const int64_t a = other_component(t);
+                if (a >= t_end) return t_end;
+                t = walk.next(prune.bounds, d, a, t_end, sh.thr);
+                if (t == a || t >= t_end) return t;
+            }
+        }
+        return other_component(t);
+    };
     auto meta = [&](int64_t t, int slot) {
         int64_t row = t * simt::RT + tid;
         if (row >= r_end) row = r_end - 1;
@@ -136,6 +173,7 @@ __device__ __forceinline__ void candidates_block(
     };
     auto epilogue = [&](int64_t tile, int slot, const Packed(&acc)[8][4]) {
         const int64_t r0 = tile * simt::RT;
+        if (PRUNE) __syncthreads();  // every warp has walked before the thresholds move
         float rc[8];
         int32_t rl[8];
         bool ok[8];
@@ -169,6 +207,14 @@ __device__ __forceinline__ void candidates_block(
                     bw[i] = w[j];
                     bi[i] = id;
                 }
+            }
+            // weights are >= 0, so their bit patterns order like the values; rows past the end
+            // (-inf, above every weight as unsigned bits) take none
+            if (PRUNE) {
+                const int q = simt::query_of(p, i);
+                if (q0 + q < nq)
+                    atomicMin(reinterpret_cast<unsigned int *>(&sh.thr[q]),
+                              weight_key_bits(bw[i]));
             }
         }
     };
@@ -205,6 +251,19 @@ __global__ void __launch_bounds__(simt::THREADS, simt::CTAS_PER_SM) candidates_f
     const int64_t r_end = r_begin + ref_chunk < n ? r_begin + ref_chunk : n;
     candidates_block(data, core, labels, ids, n, d, tile_lo, tile_hi, (int64_t)blockIdx.x * QT,
                      r_begin, r_end, row_keys, qmap, nq, qoff, smem);
+}
+
+__global__ void __launch_bounds__(simt::THREADS, simt::CTAS_PER_SM) candidates_pruned_kernel(
+    const float *__restrict__ data, const float *__restrict__ core,
+    const int32_t *__restrict__ labels, const int32_t *__restrict__ ids, int64_t n, int d,
+    const int32_t *__restrict__ tile_lo, const int32_t *__restrict__ tile_hi, int64_t ref_chunk,
+    unsigned long long *__restrict__ row_keys, const int32_t *__restrict__ qmap, int64_t nq,
+    const CandPrune prune) {
+    extern __shared__ __align__(16) float smem[];
+    const int64_t r_begin = (int64_t)blockIdx.y * ref_chunk;
+    const int64_t r_end = r_begin + ref_chunk < n ? r_begin + ref_chunk : n;
+    candidates_block<true>(data, core, labels, ids, n, d, tile_lo, tile_hi, (int64_t)blockIdx.x * QT,
+                           r_begin, r_end, row_keys, qmap, nq, 0, smem, prune);
 }
 
 // Packed fits: fit blockIdx.z (skipped unless its round runs), query tile blockIdx.x,
@@ -358,7 +417,7 @@ int launch_candidates_fp32(cuscan_ctx *ctx, const float *data, const float *core
                            const int32_t *labels, const int32_t *ids, int64_t n, int d,
                            unsigned long long *row_keys, int32_t *tile_lo, int32_t *tile_hi,
                            cudaStream_t s, const int32_t *qmap, int64_t nq, int64_t qoff,
-                           bool ranges_ready) {
+                           bool ranges_ready, const TileBounds *bounds, const uint32_t *cbound) {
     if (!qmap && qoff == 0 && nq == 0) nq = n;
     if (nq == 0) return CUSCAN_OK;
     if (!ranges_ready)
@@ -372,6 +431,14 @@ int launch_candidates_fp32(cuscan_ctx *ctx, const float *data, const float *core
     simt::split_plan(ctx->sm_count, qtiles, n, 2, 1.0, splits, chunk);
     if (int rc = allow_dynamic_smem(ctx, candidates_fp32_kernel, kCandSmem)) return rc;
     const dim3 grid((unsigned)qtiles, (unsigned)splits);
+    if (bounds) {
+        if (int rc = allow_dynamic_smem(ctx, candidates_pruned_kernel, kCandSmem)) return rc;
+        CUSCAN_KERNEL(candidates_pruned_kernel, grid, simt::THREADS, kCandSmem, s, data, core_sq,
+                      labels, ids, n, d, tile_lo, tile_hi, chunk, row_keys, qmap, nq,
+                      CandPrune{*bounds, cbound});
+        CUSCAN_LAUNCH(ctx, "candidates_pruned_kernel");
+        return CUSCAN_OK;
+    }
     CUSCAN_KERNEL(candidates_fp32_kernel, grid, simt::THREADS, kCandSmem, s, data, core_sq, labels, ids, n, d,
                   tile_lo, tile_hi, chunk, row_keys, qmap, nq, qoff);
     CUSCAN_LAUNCH(ctx, "candidates_fp32_kernel");

@@ -1,0 +1,325 @@
+// Spatial order of a point set: cells of pivot rows along a tour of the pivots, rows far outside
+// their cell's scale last; and the bounds of its tiles.
+//
+// The sweeps of this library compare tiles of rows with tiles of rows. In this order a tile of
+// clustered data is a small ball, so a tile's nearest rows sit in a few other tiles: the screens
+// see them first, and the sweeps with bounds (cells.cuh) leave most of the others out. Nothing
+// but the order of work depends on it; every result is decided by exact distances.
+#include "cells.cuh"
+
+namespace cuscan {
+namespace {
+
+// Evenly spaced rows as cell pivots.
+__global__ void pick_pivots_kernel(const float *__restrict__ x, int64_t n, int d, int npiv,
+                                   float *__restrict__ piv) {
+    int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (int64_t)npiv * d) return;
+    const int64_t p = e / d;
+    const int f = (int)(e - p * d);
+    const int64_t r = (p * n) / npiv;
+    piv[e] = x[r * d + f];
+}
+
+// Squared distances of pivot blockIdx.x to every pivot, one warp per pair.
+__global__ void pivot_distances_kernel(const float *__restrict__ piv, int npiv, int d,
+                                       float *__restrict__ out) {
+    const float *a = piv + (int64_t)blockIdx.x * d;
+    const int lane = threadIdx.x & 31;
+    for (int j = threadIdx.x >> 5; j < npiv; j += blockDim.x >> 5) {
+        float sq = 0.0f;
+        for (int f = lane; f < d; f += 32) {
+            const float t = a[f] - piv[(int64_t)j * d + f];
+            sq = fmaf(t, t, sq);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if (lane == 0) out[blockIdx.x * npiv + j] = sq;
+    }
+}
+
+// Greedy tour of the pivots: from each to the nearest one not visited yet, so that the cells of
+// a cluster follow one another and few tiles straddle two clusters. One CTA, a thread per pivot;
+// a step is one row of the distance matrix and a block minimum. Also writes the pivots in tour
+// order.
+__global__ void __launch_bounds__(kMaxPivots)
+    pivot_tour_kernel(const float *__restrict__ piv, const float *__restrict__ dist, int npiv, int d,
+                      float *__restrict__ out) {
+    __shared__ unsigned long long best[2];
+    __shared__ int order[kMaxPivots];
+    const int t = threadIdx.x, lane = t & 31;
+    bool open = t < npiv && t != 0;
+    if (t == 0) {
+        order[0] = 0;
+        best[0] = best[1] = ~0ull;
+    }
+    __syncthreads();
+    int at = 0;
+    for (int s = 1; s < npiv; ++s) {
+        unsigned long long key = ~0ull;
+        if (open) {
+            const float v = dist[at * npiv + t];
+            // NaN and infinite distances come last, in index order
+            key = ((unsigned long long)__float_as_uint(v >= 0.0f ? v : CUSCAN_INF) << 32) | (unsigned)t;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long u = __shfl_xor_sync(0xffffffffu, key, o);
+            key = u < key ? u : key;
+        }
+        if (lane == 0 && key != ~0ull) atomicMin(&best[s & 1], key);
+        __syncthreads();
+        at = (int)(uint32_t)best[s & 1];
+        if (t == at) open = false;
+        if (t == 0) {
+            order[s] = at;
+            best[(s + 1) & 1] = ~0ull;
+        }
+        __syncthreads();
+    }
+    for (int64_t e = t; e < (int64_t)npiv * d; e += blockDim.x) {
+        const int64_t p = e / d;
+        out[e] = piv[(int64_t)order[p] * d + (e - p * d)];
+    }
+}
+
+// Per cell: rows with a positive distance and the sum of its inverse (their ratio is the cell's
+// scale, which a few far rows hardly move).
+__global__ void cell_scale_kernel(const int32_t *__restrict__ cell, const float *__restrict__ dist,
+                                  int64_t n, float *__restrict__ count, float *__restrict__ inv) {
+    __shared__ float c[kMaxPivots], v[kMaxPivots];
+    for (int i = threadIdx.x; i < kMaxPivots; i += blockDim.x) c[i] = v[i] = 0.0f;
+    __syncthreads();
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const float sq = dist[i];
+        if (sq > 1e-30f && sq < 1e30f) {
+            atomicAdd(&c[cell[i]], 1.0f);
+            atomicAdd(&v[cell[i]], 1.0f / sq);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kMaxPivots; i += blockDim.x)
+        if (c[i] != 0.0f) {
+            atomicAdd(&count[i], c[i]);
+            atomicAdd(&inv[i], v[i]);
+        }
+}
+
+// Rows whose squared distance to the pivot is over three times the cell's scale (harmonic mean) go
+// to a second run of cells after all others: a few noise rows would widen every tile they sit in.
+constexpr float FAR_ROWS = 3.0f;
+__global__ void far_rows_kernel(int32_t *__restrict__ cell, const float *__restrict__ dist,
+                                int64_t n, int npiv, const float *__restrict__ count,
+                                const float *__restrict__ inv) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int32_t c = cell[i];
+    if (dist[i] * inv[c] > FAR_ROWS * count[c]) cell[i] = c + npiv;
+}
+
+// Start of every cell in a padded order (kMaxCells threads), from its row count.
+__device__ __forceinline__ int padded_start(int count, int *warp_sums) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int mine = (count + kBallRows - 1) / kBallRows * kBallRows;
+    int x = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_sums[warp] = x;
+    __syncthreads();
+    int before = 0;
+    for (int w = 0; w < warp; ++w) before += warp_sums[w];
+    return before + x - mine;
+}
+
+// Padded order of m query rows by cell, one CTA; the order within a cell is free.
+__global__ void __launch_bounds__(kMaxCells)
+    order_queries_kernel(const int32_t *__restrict__ cell, int64_t m, int64_t padded,
+                         int32_t *__restrict__ order) {
+    __shared__ int start[kMaxCells];
+    __shared__ int warp_sums[kMaxCells / 32];
+    const int t = threadIdx.x;
+    start[t] = 0;
+    for (int64_t i = t; i < padded; i += kMaxCells) order[i] = -1;
+    __syncthreads();
+    for (int64_t i = t; i < m; i += kMaxCells) atomicAdd(&start[cell[i]], 1);
+    __syncthreads();
+    const int at = padded_start(start[t], warp_sums);
+    start[t] = at;
+    __syncthreads();
+    for (int64_t i = t; i < m; i += kMaxCells) order[atomicAdd(&start[cell[i]], 1)] = (int32_t)i;
+}
+
+// The same of a sorted set's positions: shift[c] is what a position of cell c moves by.
+__global__ void __launch_bounds__(kMaxCells)
+    cell_shift_kernel(const int32_t *__restrict__ cnt, const int32_t *__restrict__ start,
+                      const int32_t *__restrict__ sums, int32_t *__restrict__ shift) {
+    __shared__ int warp_sums[kMaxCells / 32];
+    const int t = threadIdx.x;
+    const int at = padded_start(cnt[t], warp_sums);
+    shift[t] = at - (start[t] + sums[t / kScanTile]);
+}
+__global__ void order_positions_kernel(const int32_t *__restrict__ cell,
+                                       const int32_t *__restrict__ shift, int64_t n,
+                                       int32_t *__restrict__ order) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < n) order[p + shift[cell[p]]] = (int32_t)p;
+}
+
+// Upper bounds of the components' cheapest edges from the pivot rows: a pair of pivots in two
+// components is an edge of known weight, up to the rounding of the pivot distances (their sums
+// run in another order than the reference's; both are within 2e-5 of exact). Block p: pivot p.
+__global__ void pivot_bounds_kernel(const float *__restrict__ dist, int npiv, int64_t n,
+                                    const float *__restrict__ core,
+                                    const int32_t *__restrict__ label,
+                                    uint32_t *__restrict__ cbound) {
+    const int64_t row = ((int64_t)blockIdx.x * n) / npiv;
+    const int32_t l = label[row];
+    float best = CUSCAN_INF;
+    for (int j = threadIdx.x; j < npiv; j += 32) {
+        const int64_t other = ((int64_t)j * n) / npiv;
+        if (label[other] == l) continue;
+        const float v = dist[blockIdx.x * npiv + j] * (1.0f + 1e-4f) + 1e-30f;
+        best = fminf(best, fmaxf(fmaxf(v, core[row]), core[other]));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) best = fminf(best, __shfl_xor_sync(0xffffffffu, best, o));
+    if (threadIdx.x == 0 && best < CUSCAN_INF) atomicMin(&cbound[l], __float_as_uint(best));
+}
+
+// Centre and radius of half blockIdx.y of tile blockIdx.x (simt::RT rows).
+__global__ void __launch_bounds__(simt::RT)
+    tile_bounds_kernel(const float *__restrict__ x, int64_t n, int d, int64_t tiles,
+                       float *__restrict__ centre, float *__restrict__ radius) {
+    __shared__ float c[CUSCAN_PACK_MAX_FEATURES];
+    __shared__ float worst[simt::RT / 32];
+    constexpr int ROWS = simt::RT / TileBounds::PARTS;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t row0 = (int64_t)blockIdx.x * simt::RT + blockIdx.y * ROWS;
+    const int64_t at = (int64_t)blockIdx.y * tiles + blockIdx.x, stride = TileBounds::PARTS * tiles;
+    const int rows = (int)(n - row0 < ROWS ? n - row0 : ROWS);
+    if (rows <= 0) {  // the last tile's second half may be empty: beyond every threshold
+        for (int f = tid; f < d; f += simt::RT) centre[(int64_t)f * stride + at] = 0.0f;
+        if (tid == 0) radius[at] = -CUSCAN_INF;
+        return;
+    }
+    for (int f = tid; f < d; f += simt::RT) {
+        float sum = 0.0f;
+#pragma unroll 8
+        for (int r = 0; r < rows; ++r) sum += x[(row0 + r) * d + f];
+        c[f] = sum / (float)rows;
+        centre[(int64_t)f * stride + at] = c[f];
+    }
+    __syncthreads();
+    float m = 0.0f;
+    for (int r = warp; r < rows; r += simt::RT / 32) {
+        float sq = 0.0f;
+        for (int f = lane; f < d; f += 32) {
+            const float t = x[(row0 + r) * d + f] - c[f];
+            sq = fmaf(t, t, sq);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        m = fmaxf(m, sq == sq ? sq : CUSCAN_INF);
+    }
+    if (lane == 0) worst[warp] = m;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < simt::RT / 32; ++w) m = fmaxf(m, worst[w]);
+        radius[at] = bound_radius(m);
+    }
+}
+
+}  // namespace
+
+int sort_by_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, int d,
+                  cudaStream_t s) {
+    RefinedBuffers &R = b.refined;
+    const int npiv = cell_pivots(n);
+    int rc = ensure(ctx, R.pivots, sizeof(float) * 2 * npiv * d, "cell pivots");
+    if (!rc) rc = ensure(ctx, R.pivot_d, sizeof(float) * npiv * npiv, "pivot distances");
+    if (!rc) rc = ensure(ctx, R.cells, sizeof(int32_t) * n, "cells");
+    if (!rc) rc = ensure(ctx, R.cell_d, sizeof(float) * n, "cell distances");
+    if (!rc) rc = ensure(ctx, R.cell_scale, sizeof(float) * 2 * kMaxPivots, "cell scales");
+    if (rc) return rc;
+    float *toured = as<float>(R.pivots), *picked = toured + (size_t)npiv * d;
+    CUSCAN_KERNEL(pick_pivots_kernel, (unsigned)ceil_div((int64_t)npiv * d, 256), 256, 0, s, x, n, d,
+                  npiv, picked);
+    CUSCAN_KERNEL(pivot_distances_kernel, npiv, 256, 0, s, picked, npiv, d, as<float>(R.pivot_d));
+    CUSCAN_KERNEL(pivot_tour_kernel, 1, kMaxPivots, 0, s, picked, as<float>(R.pivot_d), npiv, d,
+                  toured);
+    CUSCAN_LAUNCH(ctx, "cell pivots");
+    if ((rc = launch_exact_knn_fp32(ctx, x, n, toured, npiv, d, 1, 0, 0, 1, as<int32_t>(R.cells),
+                                    as<float>(R.cell_d), s, b.knn_ids_tmp, b.knn_dist_tmp)))
+        return rc;
+    float *count = as<float>(R.cell_scale), *inv = count + kMaxPivots;
+    CUSCAN_CUDA(ctx, cudaMemsetAsync(count, 0, sizeof(float) * 2 * kMaxPivots, s));
+    int64_t grid = ceil_div(n, 1024);
+    if (grid > 2 * (int64_t)ctx->sm_count) grid = 2 * (int64_t)ctx->sm_count;
+    CUSCAN_KERNEL(cell_scale_kernel, (unsigned)grid, 256, 0, s, as<int32_t>(R.cells),
+                  as<float>(R.cell_d), n, count, inv);
+    CUSCAN_KERNEL(far_rows_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, as<int32_t>(R.cells),
+                  as<float>(R.cell_d), n, npiv, count, inv);
+    CUSCAN_LAUNCH(ctx, "cell scales");
+    return forest_sort_by_component(ctx, b, x, nullptr, as<int32_t>(R.cells), n, d, s);
+}
+
+int order_queries(cuscan_ctx *ctx, ForestBuffers &b, const float *pivots, int npiv, const float *q,
+                  int64_t m, int d, int32_t *order, cudaStream_t s) {
+    RefinedBuffers &R = b.refined;
+    int rc = ensure(ctx, R.cells, sizeof(int32_t) * m, "cells");
+    if (!rc) rc = ensure(ctx, R.cell_d, sizeof(float) * m, "cell distances");
+    if (rc) return rc;
+    if ((rc = launch_exact_knn_fp32(ctx, q, m, pivots, npiv, d, 1, 0, 0, 1, as<int32_t>(R.cells),
+                                    as<float>(R.cell_d), s, b.knn_ids_tmp, b.knn_dist_tmp)))
+        return rc;
+    CUSCAN_KERNEL(order_queries_kernel, 1, (unsigned)kMaxCells, 0, s, as<int32_t>(R.cells), m,
+                  padded_queries(m), order);
+    CUSCAN_LAUNCH(ctx, "order_queries_kernel");
+    return CUSCAN_OK;
+}
+
+int order_positions(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int32_t *order, cudaStream_t s) {
+    // the sort left its histogram, its scan and the cell of every position; the histogram's array
+    // holds at least 2048 entries and the cells are below kMaxCells
+    int32_t *shift = as<int32_t>(b.fill);  // the sort's cursors, idle now
+    CUSCAN_CUDA(ctx, cudaMemsetAsync(order, 0xff, sizeof(int32_t) * padded_queries(n), s));
+    CUSCAN_KERNEL(cell_shift_kernel, 1, (unsigned)kMaxCells, 0, s, as<int32_t>(b.cnt),
+                  as<int32_t>(b.start), as<int32_t>(b.scan_tmp), shift);
+    CUSCAN_KERNEL(order_positions_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, as<int32_t>(b.labp),
+                  shift, n, order);
+    CUSCAN_LAUNCH(ctx, "order_positions_kernel");
+    return CUSCAN_OK;
+}
+
+int pivot_component_bounds(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, const float *core,
+                           const int32_t *label, uint32_t *cbound, cudaStream_t s) {
+    const int npiv = cell_pivots(n);
+    CUSCAN_KERNEL(pivot_bounds_kernel, npiv, 32, 0, s, as<float>(b.refined.pivot_d), npiv, n, core,
+                  label, cbound);
+    CUSCAN_LAUNCH(ctx, "pivot_bounds_kernel");
+    return CUSCAN_OK;
+}
+
+int tile_bounds(cuscan_ctx *ctx, const float *x, int64_t n, int d, Buffer &centre, Buffer &radius,
+                TileBounds &out, cudaStream_t s) {
+    const int64_t tiles = ceil_div(n, (int64_t)simt::RT);
+    constexpr int PARTS = TileBounds::PARTS;
+    int rc = ensure(ctx, centre, sizeof(float) * PARTS * tiles * d, "tile centres");
+    if (!rc) rc = ensure(ctx, radius, sizeof(float) * PARTS * tiles, "tile radii");
+    if (rc) return rc;
+    const dim3 grid((unsigned)tiles, PARTS);
+    CUSCAN_KERNEL(tile_bounds_kernel, grid, simt::RT, 0, s, x, n, d, tiles,
+                  as<float>(centre), as<float>(radius));
+    CUSCAN_LAUNCH(ctx, "tile_bounds_kernel");
+    out.centre = as<float>(centre);
+    out.radius = as<float>(radius);
+    out.tiles = tiles;
+    out.stride = PARTS * tiles;
+    return CUSCAN_OK;
+}
+
+}  // namespace cuscan

@@ -192,6 +192,8 @@ __device__ __forceinline__ bool numerical_bits(uint32_t bits) {
 // Kernel launchers shared between translation units.
 namespace cuscan {
 
+struct TileBounds;  // cells.cuh
+
 // kNN (knn.cu). All pointers are device pointers. With qmap (squared, k <= 32 only), query row
 // i is row qmap[i] of `query`, excludes reference qmap[i] as itself and is written to output
 // row qmap[i].
@@ -207,12 +209,15 @@ int launch_exact_knn_fp32(cuscan_ctx *ctx, const float *query, int64_t nq, const
 // output (NULL = identity). tile_lo/tile_hi are scratch of ceil(n/32) ints each.
 // With qmap, only the nq query positions qmap[0..nq) are scanned (against all n positions);
 // without it, the positions [qoff, qoff + nq) (all n positions when nq and qoff are 0).
-// ranges_ready: tile_lo/tile_hi already hold the label ranges.
+// ranges_ready: tile_lo/tile_hi already hold the label ranges. With bounds (of the rows of data) and
+// cbound (per label, an upper bound of the component's cheapest edge, f32 bits) tiles that cannot
+// hold an edge of either kind are left out (CandPrune, boruvka.cu).
 int launch_candidates_fp32(cuscan_ctx *ctx, const float *data, const float *core_sq,
                            const int32_t *labels, const int32_t *ids, int64_t n, int d,
                            unsigned long long *row_keys, int32_t *tile_lo, int32_t *tile_hi,
                            cudaStream_t s, const int32_t *qmap = nullptr, int64_t nq = 0,
-                           int64_t qoff = 0, bool ranges_ready = false);
+                           int64_t qoff = 0, bool ranges_ready = false,
+                           const TileBounds *bounds = nullptr, const uint32_t *cbound = nullptr);
 // Label range (min, max) of every 32-row tile of `labels`.
 int launch_tile_ranges(cuscan_ctx *ctx, const int32_t *labels, int64_t n, int32_t *tile_lo,
                        int32_t *tile_hi, cudaStream_t s);

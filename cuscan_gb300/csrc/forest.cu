@@ -271,6 +271,23 @@ __global__ void sort_clear_kernel(int32_t *__restrict__ cnt, int32_t *__restrict
     comp_keys[i] = ~0ull;
 }
 
+// Labels and cores in the fit's spatial order, and the histogram of the labels.
+__global__ void label_cells_kernel(const int32_t *__restrict__ label, const float *__restrict__ core,
+                                   const int32_t *__restrict__ perm, int64_t n,
+                                   int32_t *__restrict__ cnt, int32_t *__restrict__ labp,
+                                   float *__restrict__ corep) {
+    const int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int32_t l = -1;
+    if (pos < n) {
+        const int32_t i = perm[pos];
+        l = label[i];
+        labp[pos] = l;
+        corep[pos] = core[i];
+    }
+    const unsigned peers = __match_any_sync(0xffffffffu, l);
+    if (l >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&cnt[l], __popc(peers));
+}
+
 // Counting sort of points by label: histogram with warp-aggregated atomics.
 __global__ void hist_kernel(const int32_t *__restrict__ label, int64_t n, int32_t *__restrict__ cnt) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -886,6 +903,18 @@ int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, 
     return CUSCAN_OK;
 }
 
+int forest_label_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *core, const int32_t *label,
+                       int64_t n, cudaStream_t s) {
+    int32_t *cnt = as<int32_t>(b.cnt);
+    CUSCAN_KERNEL(sort_clear_kernel, blocks(n), 256, 0, s, cnt, as<int32_t>(b.fill),
+                  as<unsigned long long>(b.row_keys), as<unsigned long long>(b.comp_keys), n,
+                  b.status);
+    CUSCAN_KERNEL(label_cells_kernel, blocks(n), 256, 0, s, label, core, as<int32_t>(b.perm), n, cnt,
+                  as<int32_t>(b.labp), as<float>(b.corep));
+    CUSCAN_LAUNCH(ctx, "label_cells_kernel");
+    return scan_exclusive(ctx, b, cnt, as<int32_t>(b.start), n, nullptr, s, &b.status->same_pairs);
+}
+
 int forest_round(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int64_t components,
                  int32_t *label, uint32_t *out_src, uint32_t *out_dst, float *out_w,
                  cudaStream_t s, int allow_empty) {
@@ -1010,7 +1039,8 @@ int forest_buffers(ForestBuffers &b, Buffer **out) {
                      &r.cbound, &r.rowcnt, &r.pivots, &r.cells, &r.cell_d, &r.absmax,
                      &r.qthr, &r.xq, &r.pq, &r.mq, &r.cand2, &r.rowcnt2, &r.fallback2,
                      &r.urow, &r.colcnt, &r.colbuf, &r.act_flag, &r.act_idx, &r.act_pos,
-                     &r.rowlb, &r.lbtmp, &r.cursor, &r.colp, &r.colc, &r.cmin};
+                     &r.rowlb, &r.lbtmp, &r.cursor, &r.colp, &r.colc, &r.cmin, &r.pivot_d,
+                     &r.cell_scale, &r.tile_centre, &r.tile_radius, &r.thr0, &r.qorder};
     static_assert(sizeof(all) / sizeof(all[0]) == kForestBufferCount, "buffer list");
     const int count = (int)(sizeof(all) / sizeof(all[0]));
     if (out)

@@ -26,6 +26,9 @@ struct DevStatus {
 struct RefinedBuffers {
     Buffer xt, pnorm, mnorm, tile_mmax, tile_lo, tile_hi, cand_ids, cand_lb, fallback, count;
     Buffer error, cbound, rowcnt, pivots, cells, cell_d, absmax;
+    Buffer pivot_d, cell_scale;  // pivot distances, per-cell scales (sort_by_cells)
+    // pruned sweeps: tile bounds, first thresholds, padded query order
+    Buffer tile_centre, tile_radius, thr0, qorder;
     Buffer qthr, xq, pq, mq, cand2, rowcnt2, fallback2;  // threshold re-screen of kNN rows
     Buffer urow, colcnt, colbuf;  // symmetric Borůvka: row bounds, column-side buffers
     Buffer act_flag, act_idx, act_pos;  // Borůvka rows that can hold their component's edge
@@ -67,7 +70,7 @@ struct ForestBuffers {
 int forest_reserve(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d);
 void forest_release(ForestBuffers &b);
 // Every device buffer of the forest and of the bf16 screen (out may be null); returns the count.
-constexpr int kForestBufferCount = 64;
+constexpr int kForestBufferCount = 70;
 int forest_buffers(ForestBuffers &b, Buffer **out);
 // Whether a set of n points takes the one-CTA forest steps (fewer than 2048 points).
 bool forest_small(int64_t n);
@@ -80,6 +83,10 @@ int forest_seed(cuscan_ctx *ctx, ForestBuffers &b, float *core, const int32_t *i
 // (forest_small) also get the label range of every 32-row tile.
 int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, const float *core,
                              const int32_t *label, int64_t n, int d, cudaStream_t s);
+// The same for a fit whose rounds keep the order of sort_by_cells (b.perm, b.xp stay): labels and
+// cores in that order, cleared keys.
+int forest_label_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *core, const int32_t *label,
+                       int64_t n, cudaStream_t s);
 // Merge one round from the per-row candidate keys in b.row_keys.
 // allow_empty: rows may lack a candidate (the bf16 screen appends only pairs that can reach
 // their component's cheapest edge).

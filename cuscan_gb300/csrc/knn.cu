@@ -20,6 +20,7 @@
 // and the partial lists are merged by a second kernel.
 #include <limits>
 
+#include "cells.cuh"
 #include "forest.cuh"
 #include "simt.cuh"
 
@@ -35,7 +36,7 @@ constexpr int TILED_K = 256;      // largest k of the tiled kernel
 constexpr int SEEDED_K = 32;      // largest k whose first thresholds come from group minima
 
 // Shared memory of one CTA after the sweep's stages (k entries per list). Up to k = 54 three
-// CTAs fit an SM.
+// CTAs fit an SM (52 with the ball of a pruned sweep).
 struct KnnShared {
     float *thr;        // [QT] upper bound of the row's k-th distance
     int32_t *row;      // [QT] query row in the query array
@@ -45,9 +46,14 @@ struct KnnShared {
     float *list_d;     // [QT][k]
     int32_t *list_i;   // [QT][k]
 };
-__host__ __device__ constexpr size_t knn_smem_bytes(int k) {
+__host__ __device__ constexpr size_t knn_smem_bytes(int k, bool pruned = false) {
     return sizeof(float) * (simt::STAGES * simt::STAGE_FLOATS + 3 * QT) + 5 * QT * BUCKET +
-           8 * (size_t)QT * k;
+           8 * (size_t)QT * k + (pruned ? sizeof(simt::QueryBalls) + 16 : 0);
+}
+__device__ __forceinline__ KnnShared knn_shared(float *smem, int k);
+__device__ __forceinline__ simt::QueryBalls *knn_balls(const KnnShared &s, int k) {
+    const uintptr_t end = reinterpret_cast<uintptr_t>(s.list_i + (size_t)QT * k);
+    return reinterpret_cast<simt::QueryBalls *>((end + 15) & ~(uintptr_t)15);
 }
 __device__ __forceinline__ KnnShared knn_shared(float *smem, int k) {
     KnnShared s;
@@ -132,24 +138,59 @@ __device__ __forceinline__ void seed_thresholds(const KnnShared &sh, const float
     }
 }
 
+// A pruned sweep: bounds of the reference tiles, an upper bound of every query's k-th distance
+// (from its nearest tile, may be +inf), and the ids and output rows of a spatially ordered set
+// (null: positions). thr_out: write only the k-th distance of each query there, over the BALLS
+// reference tiles listed in `tiles`.
+struct KnnPrune {
+    TileBounds bounds;
+    const float *thr0;
+    const int32_t *ids;
+    const int32_t *out_rows;
+    float *thr_out;
+};
+
+// Padded orders (PRUNE; qmap is never null there): whether a tile holds no row (padding follows a
+// cell's rows and the order's end), and the row that entry `i` of a tile stands for: padding repeats
+// the first row of its ball, an empty ball the first row of the tile that there is.
+__device__ __forceinline__ bool padded_tile_empty(const int32_t *__restrict__ qmap, int64_t q0,
+                                                  int64_t nq) {
+    for (int b = 0; b < QT; b += kBallRows)
+        if (q0 + b < nq && qmap[q0 + b] >= 0) return false;
+    return true;
+}
+__device__ __forceinline__ int32_t padded_row(const int32_t *__restrict__ qmap, int64_t q0, int64_t nq,
+                                              int i) {
+    int32_t row = q0 + i < nq ? qmap[q0 + i] : -1;
+    if (row < 0) row = q0 + i / kBallRows * kBallRows < nq ? qmap[q0 + i / kBallRows * kBallRows] : -1;
+    for (int b = 0; row < 0 && b < QT; b += kBallRows)
+        if (q0 + b < nq) row = qmap[q0 + b];
+    return row;
+}
+
 // One CTA: query rows [q0, q0 + 64) of nq against reference rows [r_begin, r_end) (r_begin a
 // multiple of the tile). Writes each query's sorted list (k entries) to out rows of width k, at
 // part * part_stride when the lists are partial, else to row qmap[qi] (or qi). root: distances
 // leave as their square roots.
-template <int L>
+template <int L, bool PRUNE = false>
 __device__ __forceinline__ void knn_block(
     const float *__restrict__ query, int64_t nq, const float *__restrict__ ref, int64_t nr, int d,
     int k, int exclude_self, int64_t query_offset, float pad, int64_t q0, int64_t r_begin,
     int64_t r_end, int32_t *__restrict__ out_ids, float *__restrict__ out_dist,
-    int64_t part_stride, int64_t part, bool root, const int32_t *__restrict__ qmap, float *smem) {
+    int64_t part_stride, int64_t part, bool root, const int32_t *__restrict__ qmap, float *smem,
+    const KnnPrune &prune = KnnPrune(), const int64_t *tiles = nullptr) {
     const KnnShared sh = knn_shared(smem, k);
     const simt::Place p = simt::place();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (PRUNE && padded_tile_empty(qmap, q0, nq)) return;
     if (tid < QT) {
         const int64_t qi = q0 + tid;
-        sh.row[tid] = qi < nq ? (qmap ? qmap[qi] : (int32_t)qi) : (qmap ? qmap[q0] : (int32_t)q0);
-        // rows past the end keep no pair
-        sh.thr[tid] = qi < nq ? CUSCAN_INF : -CUSCAN_INF;
+        const bool valid = qi < nq && !(PRUNE && qmap[qi] < 0);
+        sh.row[tid] = PRUNE  ? padded_row(qmap, q0, nq, tid)
+                      : valid ? (qmap ? qmap[qi] : (int32_t)qi)
+                              : (qmap ? qmap[q0] : (int32_t)q0);
+        // rows past the end and padding keep no pair
+        sh.thr[tid] = !valid ? -CUSCAN_INF : PRUNE && prune.thr0 ? prune.thr0[qi] : CUSCAN_INF;
     }
     for (int e = tid; e < QT * k; e += simt::THREADS) {
         sh.list_d[e] = pad;
@@ -183,7 +224,24 @@ __device__ __forceinline__ void knn_block(
         return hits & among;
     };
     auto nothing = [](int64_t, int) {};
-    auto every = [](int64_t t) { return t; };
+    const int64_t t_end = ceil_div(r_end, (int64_t)RT);
+    simt::PrunedWalk walk{};
+    if constexpr (PRUNE) {
+        simt::QueryBalls &balls = *knn_balls(sh, k);
+        if (!tiles) simt::query_balls(balls, query, sh.row, d);
+        walk.balls = &balls;
+    }
+    auto visit = [&](int64_t t) -> int64_t {
+        if constexpr (PRUNE) {
+            if (!tiles) return walk.next(prune.bounds, d, t, t_end, sh.thr);
+            int64_t to = t_end;  // the least listed tile at or after t
+#pragma unroll
+            for (int b = 0; b < simt::BALLS; ++b)
+                if (tiles[b] >= t && tiles[b] < to) to = tiles[b];
+            return to;
+        }
+        return t;
+    };
     auto epilogue = [&](int64_t tile, int, const Packed(&acc)[8][4]) {
         const int64_t r0 = tile * RT;
         if (first && k > 1 && k <= SEEDED_K) {
@@ -244,6 +302,7 @@ __device__ __forceinline__ void knn_block(
                 if (lane < count) {
                     x = sh.bucket_d[q * BUCKET + lane];
                     j = (int32_t)(r0 + sh.bucket_r[q * BUCKET + lane]);
+                    if (PRUNE && prune.ids) j = prune.ids[j];
                     pass = true;
                 }
                 float *ld = sh.list_d + (size_t)q * k;
@@ -261,15 +320,21 @@ __device__ __forceinline__ void knn_block(
         }
     };
     if (r_begin < r_end)
-        simt::sweep(query, sh.row, ref, d, r_begin / RT, ceil_div(r_end, (int64_t)RT), r_end, smem,
-                    every, nothing, epilogue);
+        simt::sweep(query, sh.row, ref, d, r_begin / RT, t_end, r_end, smem, visit, nothing,
+                    epilogue);
     __syncthreads();
+    if (PRUNE && prune.thr_out) {
+        if (tid < QT && q0 + tid < nq) prune.thr_out[q0 + tid] = sh.list_d[(size_t)tid * k + k - 1];
+        return;  // (entries of padding are not read)
+    }
     for (int e = tid; e < QT * k; e += simt::THREADS) {
         const int q = e / k, s = e - q * k;
         const int64_t qi = q0 + q;
         if (qi >= nq) break;
-        const int64_t at = part_stride ? part * part_stride + qi * k + s
-                                       : (qmap ? (int64_t)qmap[qi] : qi) * k + s;
+        int64_t row = qmap ? (int64_t)qmap[qi] : qi;
+        if (PRUNE && row < 0) continue;
+        if (PRUNE && prune.out_rows) row = prune.out_rows[row];
+        const int64_t at = part_stride ? part * part_stride + qi * k + s : row * k + s;
         const float x = sh.list_d[e];
         out_ids[at] = sh.list_i[e];
         out_dist[at] = root ? sqrtf(x) : x;
@@ -383,6 +448,65 @@ __global__ void __launch_bounds__(simt::THREADS, simt::CTAS_PER_SM) knn_fp32_ker
                      (int64_t)blockIdx.y, root != 0, qmap, smem);
 }
 
+// First thresholds of a pruned sweep: each query tile against its own position's reference tile
+// (self) or against the tiles nearest to the centres of its balls.
+template <int L>
+__global__ void __launch_bounds__(simt::THREADS, simt::CTAS_PER_SM) knn_thresholds_kernel(
+    const float *__restrict__ query, int64_t nq, const float *__restrict__ ref, int64_t nr, int d,
+    int k, int self, float pad, const int32_t *__restrict__ qmap, const KnnPrune prune) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ unsigned long long nearest[simt::BALLS];
+    __shared__ int64_t tiles[simt::BALLS];
+    __shared__ int32_t rows[QT];
+    const int tid = threadIdx.x;
+    const int64_t q0 = (int64_t)blockIdx.x * QT;
+    if (padded_tile_empty(qmap, q0, nq)) return;
+    if (!self) {
+        simt::QueryBalls &balls = *knn_balls(knn_shared(smem, k), k);
+        if (tid < simt::BALLS) nearest[tid] = ~0ull;
+        if (tid < QT) rows[tid] = padded_row(qmap, q0, nq, tid);
+        __syncthreads();
+        simt::query_balls(balls, query, rows, d);
+        unsigned long long best[simt::BALLS] = {~0ull, ~0ull, ~0ull, ~0ull};
+        for (int64_t part = tid; part < prune.bounds.stride; part += simt::THREADS) {
+            if (!(prune.bounds.radius[part] >= 0.0f)) continue;  // an empty half
+            float sq[simt::BALLS];
+            simt::centre_distances(sq, balls, prune.bounds, d, part);
+            const uint32_t t = (uint32_t)(part % prune.bounds.tiles);
+#pragma unroll
+            for (int b = 0; b < simt::BALLS; ++b) {
+                const float v = sq[b] == sq[b] ? sq[b] : CUSCAN_INF;
+                const unsigned long long key = ((unsigned long long)__float_as_uint(v) << 32) | t;
+                best[b] = key < best[b] ? key : best[b];
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < simt::BALLS; ++b) atomicMin(&nearest[b], best[b]);
+        __syncthreads();
+    }
+    // self: the tile of each ball's first position
+    if (tid < simt::BALLS)
+        tiles[tid] = self ? padded_row(qmap, q0, nq, tid * kBallRows) / RT
+                          : (int64_t)(uint32_t)nearest[tid];
+    __syncthreads();
+    knn_block<L, true>(query, nq, ref, nr, d, k, self, 0, pad, q0, 0, nr, nullptr, nullptr, 0, 0,
+                       false, qmap, smem, prune, tiles);
+}
+
+template <int L>
+__global__ void __launch_bounds__(simt::THREADS, simt::CTAS_PER_SM) knn_pruned_kernel(
+    const float *__restrict__ query, int64_t nq, const float *__restrict__ ref, int64_t nr, int d,
+    int k, int self, float pad, int64_t ref_chunk, int32_t *__restrict__ out_ids,
+    float *__restrict__ out_dist, int64_t part_stride, const int32_t *__restrict__ qmap,
+    const KnnPrune prune) {
+    extern __shared__ __align__(16) float smem[];
+    const int64_t r_begin = (int64_t)blockIdx.y * ref_chunk;
+    const int64_t r_end = r_begin + ref_chunk < nr ? r_begin + ref_chunk : nr;
+    knn_block<L, true>(query, nq, ref, nr, d, k, self, 0, pad, (int64_t)blockIdx.x * QT, r_begin,
+                       r_end, out_ids, out_dist, part_stride, (int64_t)blockIdx.y, false, qmap, smem,
+                       prune);
+}
+
 // Packed fits: fit blockIdx.z, query tile blockIdx.x, reference chunk blockIdx.y of `splits`
 // (the self-kNN of launch_exact_knn_fp32: squared distances, self excluded, +inf padding).
 // Fits with k > 32 take the per-fit launch instead.
@@ -453,14 +577,17 @@ __global__ void __launch_bounds__(32 * MERGE_WARPS)
     knn_merge_kernel(const int32_t *__restrict__ part_ids, const float *__restrict__ part_dist,
                      int64_t nq, int k, int splits, int64_t part_stride, float pad, int64_t nr,
                      int root, int32_t *__restrict__ ids, float *__restrict__ dist,
-                     const int32_t *__restrict__ qmap) {
+                     const int32_t *__restrict__ qmap, const int32_t *__restrict__ out_rows) {
     __shared__ float ld[MERGE_WARPS][32 * L];
     __shared__ int32_t li[MERGE_WARPS][32 * L];
     const int warp = threadIdx.x >> 5;
     const int64_t q = (int64_t)blockIdx.x * MERGE_WARPS + warp;
     if (q >= nq) return;
-    knn_merge_row<L>(part_ids, part_dist, q, qmap ? (int64_t)qmap[q] : q, k, splits, part_stride,
-                     pad, nr, root != 0, ids, dist, ld[warp], li[warp]);
+    int64_t row = qmap ? (int64_t)qmap[q] : q;
+    if (row < 0) return;  // padding of a query order
+    if (out_rows) row = out_rows[row];
+    knn_merge_row<L>(part_ids, part_dist, q, row, k, splits, part_stride, pad, nr, root != 0, ids,
+                     dist, ld[warp], li[warp]);
 }
 
 // Packed fits: the partial lists of fit blockIdx.y merged into its kNN lists.
@@ -614,7 +741,57 @@ int run_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, i
     constexpr int M = L == 0 ? 1 : L;
     CUSCAN_KERNEL(knn_merge_kernel<M>, (unsigned)ceil_div(nq, (int64_t)MERGE_WARPS),
                   32 * MERGE_WARPS, 0, s, as<int32_t>(scratch_ids), as<float>(scratch_dist), nq, k,
-                  (int)splits, stride, pad, nr, squared ? 0 : 1, ids, dist, qmap);
+                  (int)splits, stride, pad, nr, squared ? 0 : 1, ids, dist, qmap, nullptr);
+    CUSCAN_LAUNCH(ctx, "knn_merge_kernel");
+    return CUSCAN_OK;
+}
+
+template <int L>
+int run_knn_pruned(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, int64_t nr,
+                   int d, int k, int self, int32_t *ids, float *dist, cudaStream_t s,
+                   Buffer &scratch_ids, Buffer &scratch_dist, Buffer &thr0,
+                   const TileBounds &bounds, const int32_t *ref_ids, const int32_t *qmap,
+                   const int32_t *out_rows) {
+    const float pad = std::numeric_limits<float>::infinity();
+    if (int rc = ensure(ctx, thr0, sizeof(float) * nq, "first thresholds")) return rc;
+    const size_t smem = knn_smem_bytes(k, true);
+    if (int rc = allow_dynamic_smem(ctx, knn_thresholds_kernel<L>, smem)) return rc;
+    if (int rc = allow_dynamic_smem(ctx, knn_pruned_kernel<L>, smem)) return rc;
+    const unsigned qtiles = (unsigned)ceil_div(nq, (int64_t)QT);
+    KnnPrune prune{bounds, nullptr, ref_ids, out_rows, as<float>(thr0)};
+    CUSCAN_KERNEL(knn_thresholds_kernel<L>, qtiles, simt::THREADS, smem, s, query, nq, ref, nr, d, k,
+                  self, pad, qmap, prune);
+    CUSCAN_LAUNCH(ctx, "knn_thresholds_kernel");
+    prune.thr0 = as<float>(thr0);
+    prune.thr_out = nullptr;
+    // A query tile among far rows visits every reference tile, one in a cluster a few per cent of
+    // them, so the longest CTA sets the end of the launch: parts of at least 32 tiles, 16 at most,
+    // within kPrunedPartials of partial lists (100,000 x 64: 16.3 ms in one part, 11.1 ms in 16).
+    const int64_t tiles = ceil_div(nr, (int64_t)RT);
+    int64_t splits = tiles / 32 < 16 ? tiles / 32 : 16;
+    const int64_t room = kPrunedPartials / (8 * nq * k);
+    if (splits > room) splits = room;
+    if (splits < 1) splits = 1;
+    const int64_t chunk = ceil_div(tiles, splits) * RT;
+    splits = ceil_div(nr, chunk);
+    const dim3 grid(qtiles, (unsigned)splits);
+    if (splits == 1) {
+        CUSCAN_KERNEL(knn_pruned_kernel<L>, grid, simt::THREADS, smem, s, query, nq, ref, nr, d, k,
+                      self, pad, chunk, ids, dist, 0, qmap, prune);
+        CUSCAN_LAUNCH(ctx, "knn_pruned_kernel");
+        return CUSCAN_OK;
+    }
+    const int64_t stride = nq * k;
+    int rc = ensure(ctx, scratch_ids, (size_t)(stride * splits) * sizeof(int32_t), "kNN partial ids");
+    if (!rc) rc = ensure(ctx, scratch_dist, (size_t)(stride * splits) * sizeof(float),
+                         "kNN partial distances");
+    if (rc) return rc;
+    CUSCAN_KERNEL(knn_pruned_kernel<L>, grid, simt::THREADS, smem, s, query, nq, ref, nr, d, k, self,
+                  pad, chunk, as<int32_t>(scratch_ids), as<float>(scratch_dist), stride, qmap, prune);
+    CUSCAN_LAUNCH(ctx, "knn_pruned_kernel");
+    CUSCAN_KERNEL(knn_merge_kernel<L>, (unsigned)ceil_div(nq, (int64_t)MERGE_WARPS),
+                  32 * MERGE_WARPS, 0, s, as<int32_t>(scratch_ids), as<float>(scratch_dist), nq, k,
+                  (int)splits, stride, pad, nr, 0, ids, dist, qmap, out_rows);
     CUSCAN_LAUNCH(ctx, "knn_merge_kernel");
     return CUSCAN_OK;
 }
@@ -648,6 +825,24 @@ int launch_exact_knn_fp32(cuscan_ctx *ctx, const float *query, int64_t nq, const
     run_knn<L>(ctx, query, nq, ref, nr, d, k, exclude_self, query_offset, squared, ids, dist, s, \
                scratch_ids, scratch_dist, qmap)
     if (k == 1) return CUSCAN_RUN_KNN(0);
+    if (k <= 32) return CUSCAN_RUN_KNN(1);
+    if (k <= 64) return CUSCAN_RUN_KNN(2);
+    if (k <= 128) return CUSCAN_RUN_KNN(4);
+    return CUSCAN_RUN_KNN(8);
+#undef CUSCAN_RUN_KNN
+}
+
+bool knn_pruned_shape(int d, int k) { return d <= CUSCAN_PACK_MAX_FEATURES && k <= TILED_K; }
+
+int launch_knn_pruned(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, int64_t nr,
+                      int d, int k, int self, int32_t *ids, float *dist, cudaStream_t s,
+                      Buffer &scratch_ids, Buffer &scratch_dist, Buffer &thr0,
+                      const TileBounds &bounds, const int32_t *ref_ids, const int32_t *qmap,
+                      const int32_t *out_rows) {
+#define CUSCAN_RUN_KNN(L)                                                                       \
+    run_knn_pruned<L>(ctx, query, nq, ref, nr, d, k, self, ids, dist, s, scratch_ids,           \
+                      scratch_dist, thr0, bounds, ref_ids, qmap, out_rows)
+    if (nq == 0) return CUSCAN_OK;
     if (k <= 32) return CUSCAN_RUN_KNN(1);
     if (k <= 64) return CUSCAN_RUN_KNN(2);
     if (k <= 128) return CUSCAN_RUN_KNN(4);

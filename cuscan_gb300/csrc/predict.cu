@@ -23,6 +23,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "cells.cuh"
 #include "common.cuh"
 #include "forest.cuh"
 #include "simt.cuh"
@@ -43,10 +44,54 @@ struct cuscan_predictor {
     std::vector<double> point_departure;
     std::vector<double> cores;   // prediction core distances (Euclidean, f64)
     float *train = nullptr;      // device copy of the finite training rows [n_finite, d]
+    // the same rows in spatial order, their compact ids, the toured pivots and the tile bounds:
+    // large batches search only the tiles near their queries (empty below kSpatialWork)
+    cuscan::Buffer rows, ids, pivots, centre, radius;
+    int npiv = 0;
+    cuscan::TileBounds bounds;
 };
 
 namespace cuscan {
 namespace {
+
+// Work (query rows x training rows x features) of a batch from which its search runs in spatial
+// order. Ordering the batch costs about 50 us, the plain search about 1 s per 13e12:
+// 4,096 queries against 100,000 x 64 rows (2.6e10) take 1.1 ms instead of 2.4 ms, 63 queries
+// (4e8) 0.09 ms in the plain search.
+constexpr double kSpatialWork = 2e9;
+constexpr int64_t kSpatialQueries = 256;  // fewer queries are few tiles, each spread over the data
+
+void free_rows(cuscan_predictor &P) {
+    if (P.train) cudaFree(P.train);
+    P.train = nullptr;
+    for (Buffer *b : {&P.rows, &P.ids, &P.pivots, &P.centre, &P.radius}) release(*b);
+    P.bounds = TileBounds();
+}
+
+// The spatial copy of the training rows, when a batch of 4,096 queries would use it.
+int build_spatial(cuscan_ctx *ctx, cuscan_predictor &P) {
+    const int64_t n = P.n_finite;
+    const int d = P.d;
+    if (n < 2048 || !knn_pruned_shape(d, 2 * P.s) ||
+        4096.0 * (double)n * (double)d < kSpatialWork)
+        return CUSCAN_OK;
+    ForestBuffers &b = ctx->fit->forest;
+    cudaStream_t s = ctx->stream;
+    int rc = forest_reserve(ctx, b, n, d);
+    if (!rc) rc = sort_by_cells(ctx, b, P.train, n, d, s);
+    P.npiv = cell_pivots(n);
+    if (!rc) rc = ensure(ctx, P.rows, sizeof(float) * n * d, "predictor rows");
+    if (!rc) rc = ensure(ctx, P.ids, sizeof(int32_t) * n, "predictor ids");
+    if (!rc) rc = ensure(ctx, P.pivots, sizeof(float) * P.npiv * d, "predictor pivots");
+    if (rc) return rc;
+    CUSCAN_CUDA(ctx, cudaMemcpyAsync(P.rows.ptr, b.xp.ptr, sizeof(float) * n * d,
+                                     cudaMemcpyDeviceToDevice, s));
+    CUSCAN_CUDA(ctx, cudaMemcpyAsync(P.ids.ptr, b.perm.ptr, sizeof(int32_t) * n,
+                                     cudaMemcpyDeviceToDevice, s));
+    CUSCAN_CUDA(ctx, cudaMemcpyAsync(P.pivots.ptr, b.refined.pivots.ptr,
+                                     sizeof(float) * P.npiv * d, cudaMemcpyDeviceToDevice, s));
+    return tile_bounds(ctx, as<float>(P.rows), n, d, P.centre, P.radius, P.bounds, s);
+}
 
 int invalid(cuscan_ctx *ctx, const std::string &msg) {
     return fail(ctx, CUSCAN_INVALID_INPUT, "%s", msg.c_str());
@@ -340,11 +385,9 @@ static int create_predictor(cuscan_ctx *ctx, const float *train, int64_t n_finit
         }
         P->device = ctx->device;
         std::unique_ptr<cuscan_predictor, void (*)(cuscan_predictor *)> guard(
-            P.get(), [](cuscan_predictor *q) {
-                if (q->train) cudaFree(q->train);
-                q->train = nullptr;
-            });
+            P.get(), [](cuscan_predictor *q) { free_rows(*q); });
         CUSCAN_CUDA(ctx, cudaMemcpyAsync(P->train, train, bytes, cudaMemcpyHostToDevice, s));
+        if ((rc = build_spatial(ctx, *P))) return rc;
         if (!prediction_core) {
             // training cores: self-inclusive rows of width s, Euclidean value at rank s - 1
             P->cores.assign(n_finite, 0.0);
@@ -402,7 +445,7 @@ void cuscan_predictor_destroy(cuscan_predictor *p) {
     if (!p) return;
     if (p->train) {
         cudaSetDevice(p->device);
-        cudaFree(p->train);
+        free_rows(*p);
     }
     delete p;
 }
@@ -615,10 +658,14 @@ int cuscan_predictor_from_state(cuscan_ctx *ctx, const float *geometry, int64_t 
     }
     P->device = ctx->device;
     e = cudaMemcpyAsync(P->train, geometry, bytes, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess && (rc = build_spatial(ctx, *P))) {
+        cudaStreamSynchronize(ctx->stream);
+        free_rows(*P);
+        return finish(rc);
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
-        cudaFree(P->train);
-        P->train = nullptr;
+        free_rows(*P);
         return finish(cuda_fail(ctx, e, "predictor geometry upload"));
     }
     *out = P.release();
@@ -638,9 +685,13 @@ int64_t cuscan_predict_workspace_bytes(const cuscan_predictor *p, int64_t m) {
     if (!p || m <= 0) return 0;
     const int64_t k = 2 * (int64_t)p->s;
     // query rows, candidate ids and distances, split-search partial lists
-    const int64_t split = 8 * k * simt::QT *
-                          simt::split_plan_max_ctas(kSMs, ceil_div(m, (int64_t)simt::QT));
-    return (int64_t)sizeof(float) * m * p->d + 8 * m * k + split + (1 << 20);
+    int64_t split = 8 * k * simt::QT *
+                    simt::split_plan_max_ctas(kSMs, ceil_div(m, (int64_t)simt::QT));
+    const int64_t pruned = 16 * 8 * k * padded_queries(m);  // at most 16 parts
+    if (pruned > split) split = pruned < kPrunedPartials ? pruned : kPrunedPartials;
+    // queries in spatial order: cells, distances, order, first thresholds
+    return (int64_t)sizeof(float) * m * p->d + 8 * m * k + split + 16 * padded_queries(m) +
+           (1 << 20);
 }
 
 int cuscan_predictor_no_cluster_tree(const cuscan_predictor *p) {
@@ -722,10 +773,25 @@ int predict_queries(cuscan_ctx *ctx, const cuscan_predictor *p, const float *que
     if (rc) return rc;
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(f->pred_q.ptr, queries, sizeof(float) * m * p->d,
                                      cudaMemcpyHostToDevice, s));
-    if ((rc = launch_exact_knn_fp32(ctx, as<float>(f->pred_q), m, p->train, p->n_finite, p->d, k,
-                                    0, 0, 1, as<int32_t>(f->pred_ids), as<float>(f->pred_dist), s,
-                                    f->op_knn_ids, f->op_knn_dist)))
-        return rc;
+    if (p->bounds.centre && m >= kSpatialQueries &&
+        (double)m * (double)p->n_finite * (double)p->d >= kSpatialWork) {
+        rc = ensure(ctx, f->pred_order, sizeof(int32_t) * padded_queries(m), "query order");
+        if (!rc)
+            rc = order_queries(ctx, f->forest, reinterpret_cast<const float *>(p->pivots.ptr), p->npiv,
+                               as<float>(f->pred_q), m, p->d, as<int32_t>(f->pred_order), s);
+        if (!rc)
+            rc = launch_knn_pruned(ctx, as<float>(f->pred_q), padded_queries(m),
+                                   reinterpret_cast<const float *>(p->rows.ptr), p->n_finite, p->d, k,
+                                   0, as<int32_t>(f->pred_ids), as<float>(f->pred_dist), s,
+                                   f->op_knn_ids, f->op_knn_dist, f->forest.refined.thr0, p->bounds,
+                                   reinterpret_cast<const int32_t *>(p->ids.ptr),
+                                   as<int32_t>(f->pred_order), nullptr);
+    } else {
+        rc = launch_exact_knn_fp32(ctx, as<float>(f->pred_q), m, p->train, p->n_finite, p->d, k, 0, 0,
+                                   1, as<int32_t>(f->pred_ids), as<float>(f->pred_dist), s,
+                                   f->op_knn_ids, f->op_knn_dist);
+    }
+    if (rc) return rc;
     std::vector<int32_t> ids((size_t)m * k);
     std::vector<float> sq((size_t)m * k);
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(ids.data(), f->pred_ids.ptr, sizeof(int32_t) * ids.size(),

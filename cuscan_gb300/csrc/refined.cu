@@ -30,6 +30,7 @@
 #include <cmath>
 #include <type_traits>
 
+#include "cells.cuh"
 #include "common.cuh"
 #include "forest.cuh"
 
@@ -1568,17 +1569,6 @@ __global__ void seed_bounds_kernel(const int32_t *__restrict__ knn_ids,
     if (best < CUSCAN_INF) atomicMin(&cbound[li], __float_as_uint(best));
 }
 
-// Evenly spaced rows as cell pivots.
-__global__ void pick_pivots_kernel(const float *__restrict__ x, int64_t n, int d, int npiv,
-                                   float *__restrict__ piv) {
-    int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (int64_t)npiv * d) return;
-    const int64_t p = e / d;
-    const int f = (int)(e - p * d);
-    const int64_t r = (p * n) / npiv;
-    piv[e] = x[r * d + f];
-}
-
 // Per-row bounds of the symmetric screen: the bound of the row's component.
 // Also counts the rows whose component has no bound yet.
 // Row bounds of the symmetric screen (the component bounds), the count of rows without one, and
@@ -1625,13 +1615,17 @@ __global__ void round_clear_kernel(uint32_t *__restrict__ cbound, int32_t *__res
 __global__ void row_lb_from_keys_kernel(const unsigned long long *__restrict__ row_keys,
                                         const int32_t *__restrict__ qpos,
                                         const int32_t *__restrict__ perm, int64_t nq,
+                                        const int32_t *__restrict__ labp,
+                                        const uint32_t *__restrict__ cbound,
                                         float *__restrict__ rowlb) {
     int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nq) return;
     const int64_t pos = qpos ? (int64_t)qpos[q] : q;
     const int32_t orow = perm[pos];
     const unsigned long long key = row_keys[orow];  // keys are kept by original row
-    const float w = key == ~0ull ? CUSCAN_INF : __uint_as_float((uint32_t)(key >> 32));
+    float w = key == ~0ull ? CUSCAN_INF : __uint_as_float((uint32_t)(key >> 32));
+    // a pruned round left out pairs above both the row's best and its component's bound
+    if (cbound) w = fminf(w, __uint_as_float(cbound[labp[pos]]));
     rowlb[orow] = fmaxf(rowlb[orow], w);
 }
 
@@ -1757,7 +1751,7 @@ size_t refined_workspace_bytes(int64_t n, int d, int k) {
     b += sizeof(int32_t) * (size_t)n;                                                 // fallback
     b += 2 * 4 * (size_t)n * 2 * M;                  // candidate ids and bounds (two lists of M)
     b += sizeof(uint32_t) * (size_t)n + 2 * sizeof(int32_t) * (size_t)n;  // cbound, rowcnt
-    b += 256 * sizeof(float) * (size_t)d + 8 * (size_t)n;                 // pivots, cells
+    b += cells_workspace_bytes(n, d);
     // threshold re-screen of inconclusive kNN rows (at most all n): thresholds, tiles, norms,
     // candidates, counts, fallback list
     b += 4 * (size_t)n + (size_t)L.n_pad * copy_cols * 2 + 2 * sizeof(float) * (size_t)L.n_pad;
@@ -2045,22 +2039,8 @@ int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
     if (!R.range_ok)  // values large enough to overflow f32: the exact sweep decides alone
         return launch_exact_knn_fp32(ctx, x, n, x, n, d, k, 1, 0, 1, ids, dist, s, b.knn_ids_tmp,
                                      b.knn_dist_tmp);
-    // 1. cells: nearest of npiv evenly spaced pivot rows (exact f32, k = 1)
-    const int npiv = (int)(n / 256 < 256 ? (n / 256 < 1 ? 1 : n / 256) : 256);
-    rc = ensure(ctx, R.pivots, sizeof(float) * npiv * d, "cell pivots");
-    if (!rc) rc = ensure(ctx, R.cells, sizeof(int32_t) * n, "cells");
-    if (!rc) rc = ensure(ctx, R.cell_d, sizeof(float) * n, "cell distances");
-    if (rc) return rc;
-    CUSCAN_KERNEL(pick_pivots_kernel, (unsigned)ceil_div((int64_t)npiv * d, 256), 256, 0, s, x, n,
-                  d, npiv, as<float>(R.pivots));
-    CUSCAN_LAUNCH(ctx, "pick_pivots_kernel");
-    if ((rc = launch_exact_knn_fp32(ctx, x, n, as<float>(R.pivots), npiv, d, 1, 0, 0, 1,
-                                    as<int32_t>(R.cells), as<float>(R.cell_d), s, b.knn_ids_tmp,
-                                    b.knn_dist_tmp)))
-        return rc;
-    // 2. rows sorted by cell (b.perm, b.xp)
-    if ((rc = forest_sort_by_component(ctx, b, x, nullptr, as<int32_t>(R.cells), n, d, s)))
-        return rc;
+    // 1, 2. rows in spatial order (b.perm, b.xp)
+    if ((rc = sort_by_cells(ctx, b, x, n, d, s))) return rc;
     const float *xs = as<float>(b.xp);
     const int32_t *perm = as<int32_t>(b.perm);
     // 3. screen + exact re-rank in sorted positions, outputs in original rows
@@ -2272,7 +2252,7 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
 int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d,
                                  const int32_t *knn_ids, const float *knn_sq, int k,
                                  const float *core, const int32_t *label, cudaStream_t s,
-                                 int64_t *screened_rows) {
+                                 int64_t *screened_rows, const TileBounds *bounds) {
     const float *xp = as<float>(b.xp);
     const float *corep = as<float>(b.corep);
     const int32_t *labp = as<int32_t>(b.labp);
@@ -2296,6 +2276,11 @@ int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, i
                   0x7f800000u);
     CUSCAN_KERNEL(seed_bounds_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, knn_ids, knn_sq, k,
                   core, label, n, as<uint32_t>(R.cbound));
+    // a component whose neighbours are all its own has no bound from them; in spatial order the
+    // pivots give it one, and the walk something to beat
+    if (bounds &&
+        (rc = pivot_component_bounds(ctx, b, n, core, label, as<uint32_t>(R.cbound), s)))
+        return rc;
     CUSCAN_CUDA(ctx, cudaMemsetAsync(R.count.ptr, 0, 2 * sizeof(int), s));
     CUSCAN_KERNEL(init_row_bounds_kernel, (unsigned)ceil_div(n, 256), 256, 0, s,
                   as<uint32_t>(R.cbound), labp, corep, as<float>(R.rowlb), perm, n,
@@ -2309,8 +2294,10 @@ int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, i
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
     const int64_t active = counts[1];
     const int32_t *qpos = nullptr;
+    const uint32_t *cbound = bounds ? as<uint32_t>(R.cbound) : nullptr;
     if (active == n) {
-        rc = launch_candidates_fp32(ctx, xp, corep, labp, perm, n, d, row_keys, clo, chi, s);
+        rc = launch_candidates_fp32(ctx, xp, corep, labp, perm, n, d, row_keys, clo, chi, s, nullptr,
+                                    0, 0, false, bounds, cbound);
     } else if (active > 0) {
         CUSCAN_KERNEL(compact_positions_kernel, (unsigned)ceil_div(n, 256), 256, 0, s,
                       as<int32_t>(R.act_flag), as<int32_t>(R.act_idx),
@@ -2318,12 +2305,12 @@ int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, i
         CUSCAN_LAUNCH(ctx, "compact_positions_kernel");
         qpos = as<int32_t>(R.act_pos);
         rc = launch_candidates_fp32(ctx, xp, corep, labp, perm, n, d, row_keys, clo, chi, s, qpos,
-                                    active);
+                                    active, 0, false, bounds, cbound);
     }
     if (rc) return rc;
     if (active > 0) {
         CUSCAN_KERNEL(row_lb_from_keys_kernel, (unsigned)ceil_div(active, 256), 256, 0, s, row_keys,
-                      qpos, perm, active, as<float>(R.rowlb));
+                      qpos, perm, active, labp, cbound, as<float>(R.rowlb));
         CUSCAN_LAUNCH(ctx, "row_lb_from_keys_kernel");
     }
     if (screened_rows) *screened_rows += active;

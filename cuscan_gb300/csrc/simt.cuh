@@ -145,9 +145,11 @@ __device__ __forceinline__ void row_of(const Packed (&a)[4], float (&v)[8]) {
 }
 
 // The sweep of 64 query rows over the tiles of [t_begin, t_end) that `next` visits (next(t) is
-// the first visited tile at or after t), references below r_end. meta(tile, slot) copies a tile's
-// row data (cp.async) into slot 0..3 with the tile's first chunk; epilogue(tile, slot, acc) runs
-// once per tile, in order. Every thread of the CTA takes part.
+// the first visited tile at or after t, at least t_end when none is left), references below r_end.
+// next is called once per visited tile, by the copy side (up to two tiles ahead), right after a
+// barrier and before the following one. meta(tile, slot) copies a tile's row data (cp.async)
+// into slot 0..3 with the tile's first chunk; epilogue(tile, slot, acc) runs once per tile, in
+// order. Every thread of the CTA takes part.
 template <class Next, class Meta, class Epilogue>
 __device__ __forceinline__ void sweep(const float *__restrict__ query, const int32_t *rows_s,
                                       const float *__restrict__ ref, int d, int64_t t_begin,
@@ -155,7 +157,9 @@ __device__ __forceinline__ void sweep(const float *__restrict__ query, const int
                                       Meta meta, Epilogue epilogue) {
     const Place p = place();
     const int chunks = (d + KC - 1) / KC;
-    int64_t lt = next(t_begin), ct = lt;  // tiles of the copy and of the compute side
+    int64_t lt = next(t_begin);  // tile of the copy side
+    int64_t ahead[STAGES - 1];   // tiles whose copies have begun after the compute side's tile
+    int waiting = 0;
     int lc = 0, lstage = 0, stage = 0;
     int lslot = 0, slot = 0;
     auto load = [&]() {
@@ -164,7 +168,14 @@ __device__ __forceinline__ void sweep(const float *__restrict__ query, const int
             const int f0 = lc * KC, kc = d - f0 < KC ? d - f0 : KC;
             copy_queries(s, query, rows_s, d, f0, kc);
             copy_refs(s + KC * QS, ref, lt * RT, r_end, d, f0, kc);
-            if (lc == 0) meta(lt, lslot);
+            if (lc == 0) {
+                meta(lt, lslot);
+                // (unrolled: the queue stays in registers)
+#pragma unroll
+                for (int i = 0; i < STAGES - 1; ++i)
+                    if (i == waiting) ahead[i] = lt;
+                ++waiting;
+            }
             if (++lc == chunks) {
                 lc = 0;
                 lslot = (lslot + 1) & 3;
@@ -176,7 +187,11 @@ __device__ __forceinline__ void sweep(const float *__restrict__ query, const int
     };
 #pragma unroll
     for (int i = 0; i < STAGES - 1; ++i) load();
-    while (ct < t_end) {
+    while (waiting > 0) {
+        const int64_t ct = ahead[0];
+#pragma unroll
+        for (int i = 0; i + 1 < STAGES - 1; ++i) ahead[i] = ahead[i + 1];
+        --waiting;
         Packed acc[8][4];
 #pragma unroll
         for (int i = 0; i < 8; ++i)
@@ -193,7 +208,6 @@ __device__ __forceinline__ void sweep(const float *__restrict__ query, const int
         }
         epilogue(ct, slot, acc);
         slot = (slot + 1) & 3;
-        ct = next(ct + 1);
     }
     cp_async_wait<0>();
 }

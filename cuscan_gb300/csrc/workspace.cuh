@@ -16,7 +16,8 @@ struct FitWorkspace {
     ForestBuffers forest;
     Buffer x, ids, dsq, core, label, src, dst, w;  // device copies for the host-pointer entry
     Buffer op_keys, op_tiles_lo, op_tiles_hi, op_partials, op_knn_ids, op_knn_dist;
-    Buffer pred_q, pred_ids, pred_dist;            // approximate_predict queries and candidates
+    // approximate_predict queries, their spatial order and their candidates
+    Buffer pred_q, pred_order, pred_ids, pred_dist;
     DevStatus *host_status = nullptr;              // pinned
     cudaEvent_t ev[6] = {};
     PackWorkspace *pack = nullptr;                 // created by the first packed call
@@ -29,6 +30,6 @@ struct FitWorkspace {
     double round_ms[kMaxRoundLog] = {};
     double round_cross[kMaxRoundLog] = {};
 };
-constexpr int kOwnBufferCount = 17;
+constexpr int kOwnBufferCount = 18;
 
 }  // namespace cuscan

@@ -54,7 +54,8 @@ typedef enum cuscan_status {
 } cuscan_status;
 
 /* Arithmetic used by the distance sweeps of cuscan_fit_core. All give bit-identical results:
- * PLAIN evaluates every pair with exact f32 direct differences on the SIMT cores;
+ * PLAIN evaluates pairs with exact f32 direct differences on the SIMT cores (every pair, or for
+ * large sets every pair of tiles that the triangle inequality cannot rule out);
  * BF16_REFINED screens pairs with bf16 tensor-core GEMM tiles (f32 accumulation) and
  * re-evaluates every pair that the proven error bound cannot rule out with the same exact f32
  * direct differences; FP16_REFINED does the same with fp16 operands of x * 2^k (k chosen from
