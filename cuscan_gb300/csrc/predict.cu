@@ -313,6 +313,18 @@ int predict_row(cuscan_ctx *ctx, const cuscan_predictor &P, const int32_t *ids,
     return CUSCAN_OK;
 }
 
+// The largest magnitude's bit pattern decides: an integer maximum, which compiles to vector code.
+bool all_finite(const float *x, int64_t count) {
+    uint32_t most = 0;
+    for (int64_t i = 0; i < count; ++i) {
+        uint32_t bits;
+        std::memcpy(&bits, x + i, sizeof(bits));
+        bits &= 0x7fffffffu;
+        most = bits > most ? bits : most;
+    }
+    return most < 0x7f800000u;
+}
+
 int euclidean(cuscan_ctx *ctx, float sq, double *out) {
     if (!std::isfinite(sq) || sq < 0.0f)
         return fail(ctx, CUSCAN_NUMERICAL, "neighbor search returned invalid squared distance %g",
@@ -645,9 +657,8 @@ int cuscan_predictor_from_state(cuscan_ctx *ctx, const float *geometry, int64_t 
         *out = P.release();
         return CUSCAN_OK;
     }
-    for (int64_t i = 0; i < n_finite * (int64_t)d; ++i)
-        if (!std::isfinite(geometry[i]))
-            return finish(invalid(ectx, "predictor geometry must be finite"));
+    if (!all_finite(geometry, n_finite * (int64_t)d))
+        return finish(invalid(ectx, "predictor geometry must be finite"));
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     const size_t bytes = sizeof(float) * (size_t)n_finite * d;
     cudaError_t e = cudaMalloc(&P->train, bytes);
@@ -760,9 +771,8 @@ int predict_queries(cuscan_ctx *ctx, const cuscan_predictor *p, const float *que
     }
     if (!p->train || p->device != ctx->device)
         return fail(ctx, CUSCAN_INVALID_INPUT, "the predictor's training rows are not on this device");
-    for (int64_t i = 0; i < m * (int64_t)p->d; ++i)
-        if (!std::isfinite(queries[i]))
-            return fail(ctx, CUSCAN_INVALID_INPUT, "X must contain only finite values");
+    if (!all_finite(queries, m * (int64_t)p->d))
+        return fail(ctx, CUSCAN_INVALID_INPUT, "X must contain only finite values");
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
     FitWorkspace *f = ctx->fit;
