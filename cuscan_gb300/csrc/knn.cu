@@ -502,9 +502,10 @@ __global__ void __launch_bounds__(simt::THREADS, simt::CTAS_PER_SM) knn_pruned_k
     extern __shared__ __align__(16) float smem[];
     const int64_t r_begin = (int64_t)blockIdx.y * ref_chunk;
     const int64_t r_end = r_begin + ref_chunk < nr ? r_begin + ref_chunk : nr;
-    knn_block<L, true>(query, nq, ref, nr, d, k, self, 0, pad, (int64_t)blockIdx.x * QT, r_begin,
-                       r_end, out_ids, out_dist, part_stride, (int64_t)blockIdx.y, false, qmap, smem,
-                       prune);
+    // the last query tiles first: far rows are ordered last and visit the most tiles
+    const int64_t q0 = (int64_t)(gridDim.x - 1 - blockIdx.x) * QT;
+    knn_block<L, true>(query, nq, ref, nr, d, k, self, 0, pad, q0, r_begin, r_end, out_ids, out_dist,
+                       part_stride, (int64_t)blockIdx.y, false, qmap, smem, prune);
 }
 
 // Packed fits: fit blockIdx.z, query tile blockIdx.x, reference chunk blockIdx.y of `splits`
