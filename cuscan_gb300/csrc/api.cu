@@ -254,6 +254,9 @@ static int status_error(cuscan_ctx *ctx, int kind) {
     }
 }
 
+// Fewer norm levels than this per component do not narrow a 32-row chunk's norms.
+constexpr int NORM_LEVELS_MIN = 8;
+
 static float elapsed(cudaEvent_t a, cudaEvent_t b) {
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, a, b);
@@ -302,6 +305,7 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
     b.refined.screened_rows = 0;
     b.refined.symmetric_rounds = 0;
     b.refined.lb_valid = false;
+    b.refined.pivots_valid = false;
     b.refined.screen_timed = false;
 
     const bool spatial = !refined && knn_pruned_shape(d, k) && worth_pruning(n, n, d);
@@ -351,8 +355,17 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
         const int64_t rows0 = b.refined.screened_rows, tiles0 = b.refined.tile_pairs;
         if (rounds > 64) return fail(ctx, CUSCAN_NUMERICAL, "Boruvka did not converge");
         // plain f32 in spatial order keeps that order; the others group the rows by component
-        rc = spatial ? forest_label_cells(ctx, b, core_sq, label, n, s)
-                     : forest_sort_by_component(ctx, b, data, core_sq, label, n, d, s);
+        if (spatial) {
+            rc = forest_label_cells(ctx, b, core_sq, label, n, s);
+        } else if (b.refined.pivots_valid && norm_levels(n, components) >= NORM_LEVELS_MIN) {
+            // screened rounds: by norm within a component (see sort_by_cells)
+            rc = forest_norm_keys(ctx, b, label, n, components, s);
+            if (!rc)
+                rc = forest_sort_by_component(ctx, b, data, core_sq, label, n, d, s,
+                                              as<int32_t>(b.refined.key));
+        } else {
+            rc = forest_sort_by_component(ctx, b, data, core_sq, label, n, d, s);
+        }
         if (rc) return rc;
         unsigned long long *row_keys = as<unsigned long long>(b.row_keys);
         const bool small = forest_small(n);  // its sort also fills the label ranges

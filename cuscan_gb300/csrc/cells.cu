@@ -109,6 +109,8 @@ __global__ void cell_scale_kernel(const int32_t *__restrict__ cell, const float 
 // Rows whose squared distance to the pivot is over three times the cell's scale (harmonic mean) go
 // to a second run of cells after all others: a few noise rows would widen every tile they sit in.
 constexpr float FAR_ROWS = 3.0f;
+// Norm levels per cell: 2 * npiv cells of 64 levels are at most n / 2 keys.
+constexpr int CELL_LEVELS = 64;
 __global__ void far_rows_kernel(int32_t *__restrict__ cell, const float *__restrict__ dist,
                                 int64_t n, int npiv, const float *__restrict__ count,
                                 const float *__restrict__ inv) {
@@ -153,14 +155,18 @@ __global__ void __launch_bounds__(kMaxCells)
     for (int64_t i = t; i < m; i += kMaxCells) order[atomicAdd(&start[cell[i]], 1)] = (int32_t)i;
 }
 
-// The same of a sorted set's positions: shift[c] is what a position of cell c moves by.
+// The same of a sorted set's positions: shift[c] is what a position of cell c moves by. The cells
+// were sorted by keys of `levels` levels each; key k starts at start[k] + sums[k / kScanTile].
 __global__ void __launch_bounds__(kMaxCells)
-    cell_shift_kernel(const int32_t *__restrict__ cnt, const int32_t *__restrict__ start,
-                      const int32_t *__restrict__ sums, int32_t *__restrict__ shift) {
+    cell_shift_kernel(const int32_t *__restrict__ start, const int32_t *__restrict__ sums, int64_t n,
+                      int levels, int32_t *__restrict__ shift) {
     __shared__ int warp_sums[kMaxCells / 32];
     const int t = threadIdx.x;
-    const int at = padded_start(cnt[t], warp_sums);
-    shift[t] = at - (start[t] + sums[t / kScanTile]);
+    auto begin = [&](int64_t key) { return key < n ? start[key] + sums[key / kScanTile] : (int)n; };
+    const int64_t key = (int64_t)t * levels;
+    const int from = begin(key), to = t + 1 < (int)kMaxCells ? begin(key + levels) : (int)n;
+    const int at = padded_start(to - from, warp_sums);
+    shift[t] = at - from;
 }
 __global__ void order_positions_kernel(const int32_t *__restrict__ cell,
                                        const int32_t *__restrict__ shift, int64_t n,
@@ -188,6 +194,36 @@ __global__ void pivot_bounds_kernel(const float *__restrict__ dist, int npiv, in
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) best = fminf(best, __shfl_xor_sync(0xffffffffu, best, o));
     if (threadIdx.x == 0 && best < CUSCAN_INF) atomicMin(&cbound[l], __float_as_uint(best));
+}
+
+// Squared norms of the rows and their range (f32 bits; range[0] starts at the largest pattern).
+// Eight lanes per row.
+__global__ void row_norms_kernel(const float *__restrict__ x, int64_t n, int d,
+                                 float *__restrict__ out, unsigned int *__restrict__ range) {
+    const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int sub = threadIdx.x & 7;
+    float sq = 0.0f;
+    if (r < n)
+        for (int f = sub; f < d; f += 8) {
+            const float v = x[r * d + f];
+            sq = fmaf(v, v, sq);
+        }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    if (r < n && sub == 0) out[r] = sq;
+    const unsigned bits = __float_as_uint(sq);
+    const unsigned lo = __reduce_min_sync(0xffffffffu, r < n ? bits : 0xffffffffu);
+    const unsigned hi = __reduce_max_sync(0xffffffffu, r < n ? bits : 0u);
+    if ((threadIdx.x & 31) == 0) {
+        if (lo < *(volatile unsigned int *)&range[0]) atomicMin(&range[0], lo);
+        if (hi > *(volatile unsigned int *)&range[1]) atomicMax(&range[1], hi);
+    }
+}
+__global__ void clear_range_kernel(unsigned int *__restrict__ range, float *__restrict__ scale) {
+    const int t = threadIdx.x;
+    if (t == 0) range[0] = 0xffffffffu;
+    if (t == 1) range[1] = 0u;
+    for (int i = t; i < 2 * kMaxPivots; i += blockDim.x) scale[i] = 0.0f;
 }
 
 // Centre and radius of half blockIdx.y of tile blockIdx.x (simt::RT rows).
@@ -256,7 +292,12 @@ int sort_by_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, 
                                     as<float>(R.cell_d), s, b.knn_ids_tmp, b.knn_dist_tmp)))
         return rc;
     float *count = as<float>(R.cell_scale), *inv = count + kMaxPivots;
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(count, 0, sizeof(float) * 2 * kMaxPivots, s));
+    if ((rc = ensure(ctx, R.rnorm, sizeof(float) * n, "row norms"))) return rc;
+    if ((rc = ensure(ctx, R.norm_range, 16, "norm range"))) return rc;
+    unsigned int *range = as<unsigned int>(R.norm_range);
+    CUSCAN_KERNEL(clear_range_kernel, 1, 256, 0, s, range, count);
+    CUSCAN_KERNEL(row_norms_kernel, (unsigned)ceil_div(8 * n, 256), 256, 0, s, x, n, d,
+                  as<float>(R.rnorm), range);
     int64_t grid = ceil_div(n, 1024);
     if (grid > 2 * (int64_t)ctx->sm_count) grid = 2 * (int64_t)ctx->sm_count;
     CUSCAN_KERNEL(cell_scale_kernel, (unsigned)grid, 256, 0, s, as<int32_t>(R.cells),
@@ -264,7 +305,12 @@ int sort_by_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, 
     CUSCAN_KERNEL(far_rows_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, as<int32_t>(R.cells),
                   as<float>(R.cell_d), n, npiv, count, inv);
     CUSCAN_LAUNCH(ctx, "cell scales");
-    return forest_sort_by_component(ctx, b, x, nullptr, as<int32_t>(R.cells), n, d, s);
+    // within a cell by norm: a 32-column chunk of the screens is bounded by its largest dot product
+    // and its smallest norm, which is tight only when its norms are alike
+    R.cell_levels = CELL_LEVELS;
+    if ((rc = forest_cell_keys(ctx, b, n, R.cell_levels, s))) return rc;
+    return forest_sort_by_component(ctx, b, x, nullptr, as<int32_t>(R.cells), n, d, s,
+                                    as<int32_t>(R.key));
 }
 
 int order_queries(cuscan_ctx *ctx, ForestBuffers &b, const float *pivots, int npiv, const float *q,
@@ -283,12 +329,11 @@ int order_queries(cuscan_ctx *ctx, ForestBuffers &b, const float *pivots, int np
 }
 
 int order_positions(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int32_t *order, cudaStream_t s) {
-    // the sort left its histogram, its scan and the cell of every position; the histogram's array
-    // holds at least 2048 entries and the cells are below kMaxCells
+    // the sort left the scan of its keys and the cell of every position
     int32_t *shift = as<int32_t>(b.fill);  // the sort's cursors, idle now
     CUSCAN_CUDA(ctx, cudaMemsetAsync(order, 0xff, sizeof(int32_t) * padded_queries(n), s));
-    CUSCAN_KERNEL(cell_shift_kernel, 1, (unsigned)kMaxCells, 0, s, as<int32_t>(b.cnt),
-                  as<int32_t>(b.start), as<int32_t>(b.scan_tmp), shift);
+    CUSCAN_KERNEL(cell_shift_kernel, 1, (unsigned)kMaxCells, 0, s, as<int32_t>(b.start),
+                  as<int32_t>(b.scan_tmp), n, b.refined.cell_levels, shift);
     CUSCAN_KERNEL(order_positions_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, as<int32_t>(b.labp),
                   shift, n, order);
     CUSCAN_LAUNCH(ctx, "order_positions_kernel");

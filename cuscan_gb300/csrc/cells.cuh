@@ -22,7 +22,7 @@ int sort_by_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, 
 // Device bytes of sort_by_cells beyond the forest's own buffers.
 inline size_t cells_workspace_bytes(int64_t n, int d) {
     return sizeof(float) * (2 * (size_t)kMaxPivots * d + (size_t)kMaxPivots * kMaxPivots +
-                            2 * kMaxPivots) + 8 * (size_t)n;
+                            2 * kMaxPivots) + 16 * (size_t)n;  // cells, distances, norms, keys
 }
 // Query orders for the pruned sweeps: the rows grouped by cell, every cell padded to whole balls of
 // kBallRows entries with -1, so that no ball straddles two cells. A straddling ball is as wide as

@@ -260,7 +260,7 @@ __global__ void sort_clear_kernel(int32_t *__restrict__ cnt, int32_t *__restrict
                                   unsigned long long *__restrict__ comp_keys, int64_t n,
                                   DevStatus *status) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) {
+    if (i == 0 && status) {
         status->same_pairs = 0.0;
         status->scan_ticket = 0;
     }
@@ -295,6 +295,47 @@ __global__ void hist_kernel(const int32_t *__restrict__ label, int64_t n, int32_
     unsigned peers = __match_any_sync(0xffffffffu, l);
     int lane = threadIdx.x & 31;
     if (l >= 0 && lane == __ffs(peers) - 1) atomicAdd(&cnt[l], __popc(peers));
+}
+
+// Histogram of the labels and flags of the roots (points that carry their own label).
+__global__ void hist_roots_kernel(const int32_t *__restrict__ label, int64_t n,
+                                  int32_t *__restrict__ cnt, int32_t *__restrict__ root) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int32_t l = i < n ? label[i] : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, l);
+    if (l >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&cnt[l], __popc(peers));
+    if (i < n) root[i] = l == (int32_t)i;
+}
+
+// Level of a squared norm within the rows' range.
+__device__ __forceinline__ int norm_level(float p, const unsigned int *range, int levels) {
+    const float lo = __uint_as_float(range[0]), hi = __uint_as_float(range[1]);
+    const float t = (p - lo) / (hi - lo) * (float)levels;  // NaN (one norm, overflow): level 0
+    return t >= (float)levels ? levels - 1 : t > 0.0f ? (int)t : 0;
+}
+
+__global__ void norm_keys_kernel(const int32_t *__restrict__ label, const int32_t *__restrict__ rank,
+                                 const int32_t *__restrict__ sums, const int32_t *__restrict__ cnt,
+                                 const float *__restrict__ rnorm,
+                                 const unsigned int *__restrict__ range, int64_t n, int levels,
+                                 int32_t *__restrict__ key, DevStatus *status) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    double sq = 0.0;
+    if (i < n) {
+        const int32_t l = label[i];
+        key[i] = (rank[l] + sums[l / kScanTile]) * levels + norm_level(rnorm[i], range, levels);
+        sq = (double)cnt[i] * (double)cnt[i];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    if ((threadIdx.x & 31) == 0 && sq != 0.0) atomicAdd(&status->same_pairs, sq);
+}
+
+__global__ void cell_keys_kernel(const int32_t *__restrict__ cell, const float *__restrict__ rnorm,
+                                 const unsigned int *__restrict__ range, int64_t n, int levels,
+                                 int32_t *__restrict__ key) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) key[i] = cell[i] * levels + norm_level(rnorm[i], range, levels);
 }
 
 __global__ void scatter_kernel(const int32_t *__restrict__ label, int64_t n,
@@ -873,8 +914,28 @@ int forest_seed(cuscan_ctx *ctx, ForestBuffers &b, float *core, const int32_t *i
     return resolve_proposals(ctx, b, n, n, nullptr, label, out_src, out_dst, out_w, 0, s);
 }
 
+int forest_norm_keys(cuscan_ctx *ctx, ForestBuffers &b, const int32_t *label, int64_t n,
+                     int64_t components, cudaStream_t s) {
+    RefinedBuffers &R = b.refined;
+    int32_t *cnt = as<int32_t>(b.cnt), *rank = as<int32_t>(b.pos);
+    int rc = ensure(ctx, R.key, sizeof(int32_t) * n, "row keys");
+    if (rc) return rc;
+    CUSCAN_KERNEL(sort_clear_kernel, blocks(n), 256, 0, s, cnt, as<int32_t>(b.fill),
+                  as<unsigned long long>(b.row_keys), as<unsigned long long>(b.comp_keys), n,
+                  b.status);
+    CUSCAN_KERNEL(hist_roots_kernel, blocks(n), 256, 0, s, label, n, cnt, as<int32_t>(b.keep));
+    // ranks of the component roots; the histogram's squares are same_pairs
+    if ((rc = scan_exclusive(ctx, b, as<int32_t>(b.keep), rank, n, nullptr, s))) return rc;
+    CUSCAN_KERNEL(norm_keys_kernel, blocks(n), 256, 0, s, label, rank, as<int32_t>(b.scan_tmp), cnt,
+                  as<float>(R.rnorm), as<unsigned int>(R.norm_range), n,
+                  norm_levels(n, components), as<int32_t>(R.key), b.status);
+    CUSCAN_LAUNCH(ctx, "norm_keys_kernel");
+    return CUSCAN_OK;
+}
+
 int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, const float *core,
-                             const int32_t *label, int64_t n, int d, cudaStream_t s) {
+                             const int32_t *label, int64_t n, int d, cudaStream_t s,
+                             const int32_t *key) {
     int32_t *cnt = as<int32_t>(b.cnt), *start = as<int32_t>(b.start), *fill = as<int32_t>(b.fill);
     if (forest_small(n)) {
         PackFit f = small_fit(b, n, const_cast<int32_t *>(label), nullptr, nullptr, nullptr);
@@ -888,18 +949,28 @@ int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, 
     }
     CUSCAN_KERNEL(sort_clear_kernel, blocks(n), 256, 0, s, cnt, fill,
                   as<unsigned long long>(b.row_keys), as<unsigned long long>(b.comp_keys), n,
-                  b.status);
-    CUSCAN_KERNEL(hist_kernel, blocks(n), 256, 0, s, label, n, cnt);
+                  key ? nullptr : b.status);
+    CUSCAN_KERNEL(hist_kernel, blocks(n), 256, 0, s, key ? key : label, n, cnt);
     CUSCAN_LAUNCH(ctx, "hist_kernel");
     // same_pairs: the sum of squared component sizes, for the work counters
-    int rc = scan_exclusive(ctx, b, cnt, start, n, nullptr, s, &b.status->same_pairs);
+    int rc = scan_exclusive(ctx, b, cnt, start, n, nullptr, s,
+                            key ? nullptr : &b.status->same_pairs);
     if (rc) return rc;
-    CUSCAN_KERNEL(scatter_kernel, blocks(n), 256, 0, s, label, n, start, as<int32_t>(b.scan_tmp),
-                  fill, as<int32_t>(b.perm));
+    CUSCAN_KERNEL(scatter_kernel, blocks(n), 256, 0, s, key ? key : label, n, start,
+                  as<int32_t>(b.scan_tmp), fill, as<int32_t>(b.perm));
     CUSCAN_KERNEL(gather_kernel, blocks(n * d), 256, 0, s, x, core, label, as<int32_t>(b.perm), n, d,
                                                  as<float>(b.xp), as<float>(b.corep),
                                                  as<int32_t>(b.labp));
     CUSCAN_LAUNCH(ctx, "component sort");
+    return CUSCAN_OK;
+}
+
+int forest_cell_keys(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int levels, cudaStream_t s) {
+    RefinedBuffers &R = b.refined;
+    if (int rc = ensure(ctx, R.key, sizeof(int32_t) * n, "row keys")) return rc;
+    CUSCAN_KERNEL(cell_keys_kernel, blocks(n), 256, 0, s, as<int32_t>(R.cells), as<float>(R.rnorm),
+                  as<unsigned int>(R.norm_range), n, levels, as<int32_t>(R.key));
+    CUSCAN_LAUNCH(ctx, "cell_keys_kernel");
     return CUSCAN_OK;
 }
 
@@ -1040,7 +1111,8 @@ int forest_buffers(ForestBuffers &b, Buffer **out) {
                      &r.qthr, &r.xq, &r.pq, &r.mq, &r.cand2, &r.rowcnt2, &r.fallback2,
                      &r.urow, &r.colcnt, &r.colbuf, &r.act_flag, &r.act_idx, &r.act_pos,
                      &r.rowlb, &r.lbtmp, &r.cursor, &r.colp, &r.colc, &r.cmin, &r.pivot_d,
-                     &r.cell_scale, &r.tile_centre, &r.tile_radius, &r.thr0, &r.qorder};
+                     &r.cell_scale, &r.tile_centre, &r.tile_radius, &r.thr0, &r.qorder,
+                     &r.rnorm, &r.norm_range, &r.key};
     static_assert(sizeof(all) / sizeof(all[0]) == kForestBufferCount, "buffer list");
     const int count = (int)(sizeof(all) / sizeof(all[0]));
     if (out)

@@ -26,7 +26,8 @@ struct DevStatus {
 struct RefinedBuffers {
     Buffer xt, pnorm, mnorm, tile_mmax, tile_lo, tile_hi, cand_ids, cand_lb, fallback, count;
     Buffer error, cbound, rowcnt, pivots, cells, cell_d, absmax;
-    Buffer pivot_d, cell_scale;  // pivot distances, per-cell scales (sort_by_cells)
+    // sort_by_cells: pivot distances, per-cell scales, squared norms of the rows and their range
+    Buffer pivot_d, cell_scale, rnorm, norm_range, key;
     // pruned sweeps: tile bounds, first thresholds, padded query order
     Buffer tile_centre, tile_radius, thr0, qorder;
     Buffer qthr, xq, pq, mq, cand2, rowcnt2, fallback2;  // threshold re-screen of kNN rows
@@ -47,6 +48,8 @@ struct RefinedBuffers {
     int64_t screened_rows = 0;  // query rows of the current fit's Borůvka screens
     int64_t symmetric_rounds = 0;  // rounds of the current fit the symmetric screen ran
     bool lb_valid = false;      // rowlb holds bounds of the current fit
+    int cell_levels = 1;        // norm levels per cell of the last sort_by_cells
+    bool pivots_valid = false;  // pivot_d holds distances of the current fit's rows
     // CUDA events around the kNN list screen's launch (created on first use); screen_timed
     // says they hold the current fit's launch
     cudaEvent_t screen_ev[2] = {nullptr, nullptr};
@@ -70,7 +73,7 @@ struct ForestBuffers {
 int forest_reserve(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d);
 void forest_release(ForestBuffers &b);
 // Every device buffer of the forest and of the bf16 screen (out may be null); returns the count.
-constexpr int kForestBufferCount = 70;
+constexpr int kForestBufferCount = 73;
 int forest_buffers(ForestBuffers &b, Buffer **out);
 // Whether a set of n points takes the one-CTA forest steps (fewer than 2048 points).
 bool forest_small(int64_t n);
@@ -80,9 +83,25 @@ int forest_seed(cuscan_ctx *ctx, ForestBuffers &b, float *core, const int32_t *i
                 const float *dsq, int64_t n, int k, int min_samples, int32_t *label,
                 uint32_t *out_src, uint32_t *out_dst, float *out_w, cudaStream_t s);
 // Group points by label: perm, xp, corep, labp; clears the row and component keys. Small sets
-// (forest_small) also get the label range of every 32-row tile.
+// (forest_small) also get the label range of every 32-row tile. With key (below n, n >= 2048) the
+// points are grouped by it instead, which must keep the rows of a label together, and same_pairs is
+// not counted.
 int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, const float *core,
-                             const int32_t *label, int64_t n, int d, cudaStream_t s);
+                             const int32_t *label, int64_t n, int d, cudaStream_t s,
+                             const int32_t *key = nullptr);
+// Keys that order a round's rows by component and then by squared norm (in b.refined.key): the
+// component's rank times `levels` plus the norm's level. Counts same_pairs. Needs
+// b.refined.rnorm and norm_range (sort_by_cells).
+int forest_norm_keys(cuscan_ctx *ctx, ForestBuffers &b, const int32_t *label, int64_t n,
+                     int64_t components, cudaStream_t s);
+// Levels of a norm key: as many as keep components * levels within n, at most 1,024 (a power of 2).
+inline int norm_levels(int64_t n, int64_t groups) {
+    int l = 1;
+    while (l < 1024 && 2 * l * groups <= n) l *= 2;
+    return l;
+}
+// Keys cell * levels + norm level of every row (b.refined.key).
+int forest_cell_keys(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int levels, cudaStream_t s);
 // The same for a fit whose rounds keep the order of sort_by_cells (b.perm, b.xp stay): labels and
 // cores in that order, cleared keys.
 int forest_label_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *core, const int32_t *label,

@@ -2044,6 +2044,7 @@ int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
                                      b.knn_dist_tmp);
     // 1, 2. rows in spatial order (b.perm, b.xp)
     if ((rc = sort_by_cells(ctx, b, x, n, d, s))) return rc;
+    R.pivots_valid = true;
     const float *xs = as<float>(b.xp);
     const int32_t *perm = as<int32_t>(b.perm);
     // 3. screen + exact re-rank in sorted positions, outputs in original rows
@@ -2160,6 +2161,11 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
     R.lb_valid = true;
     CUSCAN_KERNEL(seed_bounds_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, knn_ids, knn_sq, k,
                   core, label, n, as<uint32_t>(R.cbound));
+    // a late component's neighbours are all its own: the pivots bound it (without a bound every
+    // row of it is screened, and every pair appended until the first blocks have found one)
+    if (R.pivots_valid &&
+        (rc = pivot_component_bounds(ctx, b, n, core, label, as<uint32_t>(R.cbound), s)))
+        return rc;
     CUSCAN_KERNEL(init_row_bounds_kernel, (unsigned)ceil_div(n, 256), 256, 0, s,
                   as<uint32_t>(R.cbound), labp, corep, as<float>(R.rowlb), perm, n,
                   as<uint32_t>(R.urow), as<int>(R.count), as<int32_t>(R.act_flag));
