@@ -196,17 +196,18 @@ __global__ void pivot_bounds_kernel(const float *__restrict__ dist, int npiv, in
     if (threadIdx.x == 0 && best < CUSCAN_INF) atomicMin(&cbound[l], __float_as_uint(best));
 }
 
-// Squared norms of the rows and their range (f32 bits; range[0] starts at the largest pattern).
-// Eight lanes per row.
+// Squared norms of the rows, their range and the largest |x| (f32 bits in range[0..2]; range[0] starts
+// at the largest pattern). Eight lanes per row.
 __global__ void row_norms_kernel(const float *__restrict__ x, int64_t n, int d,
                                  float *__restrict__ out, unsigned int *__restrict__ range) {
     const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     const int sub = threadIdx.x & 7;
-    float sq = 0.0f;
+    float sq = 0.0f, most = 0.0f;
     if (r < n)
         for (int f = sub; f < d; f += 8) {
             const float v = x[r * d + f];
             sq = fmaf(v, v, sq);
+            most = fmaxf(most, fabsf(v));
         }
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
@@ -214,16 +215,46 @@ __global__ void row_norms_kernel(const float *__restrict__ x, int64_t n, int d,
     const unsigned bits = __float_as_uint(sq);
     const unsigned lo = __reduce_min_sync(0xffffffffu, r < n ? bits : 0xffffffffu);
     const unsigned hi = __reduce_max_sync(0xffffffffu, r < n ? bits : 0u);
+    const unsigned mx = __reduce_max_sync(0xffffffffu, __float_as_uint(most));
     if ((threadIdx.x & 31) == 0) {
         if (lo < *(volatile unsigned int *)&range[0]) atomicMin(&range[0], lo);
         if (hi > *(volatile unsigned int *)&range[1]) atomicMax(&range[1], hi);
+        if (mx > *(volatile unsigned int *)&range[2]) atomicMax(&range[2], mx);
     }
 }
-__global__ void clear_range_kernel(unsigned int *__restrict__ range, float *__restrict__ scale) {
+// Squared norm of pivot blockIdx.x (one warp); block 0 also clears the range and the cell sums.
+__global__ void pivot_norms_kernel(const float *__restrict__ piv, int d,
+                                   unsigned int *__restrict__ range, float *__restrict__ scale,
+                                   float *__restrict__ norm) {
     const int t = threadIdx.x;
-    if (t == 0) range[0] = 0xffffffffu;
-    if (t == 1) range[1] = 0u;
-    for (int i = t; i < 2 * kMaxPivots; i += blockDim.x) scale[i] = 0.0f;
+    if (blockIdx.x == 0) {
+        if (t < 4) range[t] = t == 0 ? 0xffffffffu : 0u;
+        for (int i = t; i < 2 * kMaxPivots; i += 32) scale[i] = 0.0f;
+    }
+    float sq = 0.0f;
+    for (int f = t; f < d; f += 32) {
+        const float v = piv[(int64_t)blockIdx.x * d + f];
+        sq = fmaf(v, v, sq);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    if (t == 0) norm[blockIdx.x] = sq;
+}
+
+// Rows whose cell is too tight for a screen whose bounds sit `shift` |x|^2 below the distances: the
+// gap that such a row's lists must show between its k-th and their last entry is about
+// H (2 / d) ln(entries / k) where the cell's scale is H and the rows fill d dimensions (fewer
+// make the gap wider). Counted in range[3]. One CTA.
+__global__ void __launch_bounds__(kMaxPivots)
+    tight_rows_kernel(const float *__restrict__ count, const float *__restrict__ inv,
+                      const float *__restrict__ norm, int npiv, float shift, float gap,
+                      unsigned int *__restrict__ range) {
+    const int c = threadIdx.x;
+    unsigned rows = 0;
+    if (c < npiv && inv[c] > 0.0f && shift * norm[c] > gap * (count[c] / inv[c]))
+        rows = (unsigned)count[c];
+    rows = __reduce_add_sync(0xffffffffu, rows);
+    if ((c & 31) == 0 && rows) atomicAdd(&range[3], rows);
 }
 
 // Centre and radius of half blockIdx.y of tile blockIdx.x (simt::RT rows).
@@ -279,7 +310,7 @@ int sort_by_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, 
     if (!rc) rc = ensure(ctx, R.pivot_d, sizeof(float) * npiv * npiv, "pivot distances");
     if (!rc) rc = ensure(ctx, R.cells, sizeof(int32_t) * n, "cells");
     if (!rc) rc = ensure(ctx, R.cell_d, sizeof(float) * n, "cell distances");
-    if (!rc) rc = ensure(ctx, R.cell_scale, sizeof(float) * 2 * kMaxPivots, "cell scales");
+    if (!rc) rc = ensure(ctx, R.cell_scale, sizeof(float) * 3 * kMaxPivots, "cell scales");
     if (rc) return rc;
     float *toured = as<float>(R.pivots), *picked = toured + (size_t)npiv * d;
     CUSCAN_KERNEL(pick_pivots_kernel, (unsigned)ceil_div((int64_t)npiv * d, 256), 256, 0, s, x, n, d,
@@ -295,7 +326,7 @@ int sort_by_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, 
     if ((rc = ensure(ctx, R.rnorm, sizeof(float) * n, "row norms"))) return rc;
     if ((rc = ensure(ctx, R.norm_range, 16, "norm range"))) return rc;
     unsigned int *range = as<unsigned int>(R.norm_range);
-    CUSCAN_KERNEL(clear_range_kernel, 1, 256, 0, s, range, count);
+    CUSCAN_KERNEL(pivot_norms_kernel, npiv, 32, 0, s, toured, d, range, count, inv + kMaxPivots);
     CUSCAN_KERNEL(row_norms_kernel, (unsigned)ceil_div(8 * n, 256), 256, 0, s, x, n, d,
                   as<float>(R.rnorm), range);
     int64_t grid = ceil_div(n, 1024);
@@ -311,6 +342,17 @@ int sort_by_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, 
     if ((rc = forest_cell_keys(ctx, b, n, R.cell_levels, s))) return rc;
     return forest_sort_by_component(ctx, b, x, nullptr, as<int32_t>(R.cells), n, d, s,
                                     as<int32_t>(R.key));
+}
+
+int count_tight_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, float shift, float gap,
+                     cudaStream_t s) {
+    RefinedBuffers &R = b.refined;
+    const float *count = as<float>(R.cell_scale);
+    CUSCAN_KERNEL(tight_rows_kernel, 1, kMaxPivots, 0, s, count, count + kMaxPivots,
+                  count + 2 * kMaxPivots, cell_pivots(n), shift, gap,
+                  as<unsigned int>(R.norm_range));
+    CUSCAN_LAUNCH(ctx, "tight_rows_kernel");
+    return CUSCAN_OK;
 }
 
 int order_queries(cuscan_ctx *ctx, ForestBuffers &b, const float *pivots, int npiv, const float *q,

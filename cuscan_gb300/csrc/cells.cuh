@@ -22,7 +22,7 @@ int sort_by_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, 
 // Device bytes of sort_by_cells beyond the forest's own buffers.
 inline size_t cells_workspace_bytes(int64_t n, int d) {
     return sizeof(float) * (2 * (size_t)kMaxPivots * d + (size_t)kMaxPivots * kMaxPivots +
-                            2 * kMaxPivots) + 16 * (size_t)n;  // cells, distances, norms, keys
+                            3 * kMaxPivots) + 16 * (size_t)n;  // cells, distances, norms, keys
 }
 // Query orders for the pruned sweeps: the rows grouped by cell, every cell padded to whole balls of
 // kBallRows entries with -1, so that no ball straddles two cells. A straddling ball is as wide as
@@ -36,6 +36,10 @@ int order_queries(cuscan_ctx *ctx, ForestBuffers &b, const float *pivots, int np
                   int64_t m, int d, int32_t *order, cudaStream_t s);
 // Of the n positions of the set itself, right after sort_by_cells.
 int order_positions(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int32_t *order, cudaStream_t s);
+// Rows of cells whose scale times gap is below shift times the squared norm of their pivot, counted
+// in word 3 of b.refined.norm_range. Right after sort_by_cells.
+int count_tight_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, float shift, float gap,
+                     cudaStream_t s);
 // cbound[label] (f32 bits, labels by original row) lowered to the weights of edges between pivots
 // of different components. Needs sort_by_cells of the same fit.
 int pivot_component_bounds(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, const float *core,

@@ -126,6 +126,9 @@ constexpr int RESCREEN_MIN_ROWS = 256;  // fewer inconclusive kNN rows go straig
 // A bf16-refined fit whose first kNN screen leaves more than this share of rows inconclusive
 // screens again with tighter operands (split bf16, or scaled fp16 for rows too wide to split).
 constexpr double TIGHTEN_TRIGGER = 0.15;
+// Share of rows that choose_operands_by_cells expects to be inconclusive from which the first
+// screen already uses the tightened operands.
+constexpr double TIGHT_START = 0.25;
 // Status words of a screen: [0] error flag, [2..3] tile pairs (u64), [4] inconclusive rows listed by
 // the re-rank, [5] spare.
 constexpr int SCREEN_STATUS_WORDS = 8;
@@ -1822,13 +1825,26 @@ constexpr double kScreenRangeMax = 3.4028234663852886e38 / 16.0;
 
 // Per fit: the largest |x| (one reduction and one host read) decides whether the screens may run
 // (range_ok) and, when fp16 operands are wanted, their power-of-two scale.
-static int choose_operands(cuscan_ctx *ctx, RefinedBuffers &R, const float *x, int64_t n, int d,
-                           cudaStream_t s) {
-    if (R.have_scale) return CUSCAN_OK;
+static void set_operands(RefinedBuffers &R, int d, unsigned int absmax_bits) {
     R.fp16 = false;
     R.split = false;
     R.scale = 1.0f;
-    R.range_ok = true;
+    float amax;
+    memcpy(&amax, &absmax_bits, sizeof(amax));
+    R.range_ok = std::isfinite(amax) && (double)d * (double)amax * (double)amax <= kScreenRangeMax;
+    R.amax_value = std::isfinite(amax) ? amax : 0.0f;
+    if (R.want_fp16) {
+        const float sc = fp16_scale(amax);
+        if (sc > 0.0f) {
+            R.fp16 = true;
+            R.scale = sc;
+        }
+    }
+    R.have_scale = true;
+}
+static int choose_operands(cuscan_ctx *ctx, RefinedBuffers &R, const float *x, int64_t n, int d,
+                           cudaStream_t s) {
+    if (R.have_scale) return CUSCAN_OK;
     int rc = ensure(ctx, R.absmax, 16, "range reduction");
     if (rc) return rc;
     CUSCAN_CUDA(ctx, cudaMemsetAsync(R.absmax.ptr, 0, sizeof(unsigned int), s));
@@ -1841,18 +1857,29 @@ static int choose_operands(cuscan_ctx *ctx, RefinedBuffers &R, const float *x, i
     unsigned int bits = 0;
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(&bits, R.absmax.ptr, sizeof(bits), cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
-    float amax;
-    memcpy(&amax, &bits, sizeof(amax));
-    R.range_ok = std::isfinite(amax) && (double)d * (double)amax * (double)amax <= kScreenRangeMax;
-    R.amax_value = std::isfinite(amax) ? amax : 0.0f;
-    if (R.want_fp16) {
-        const float sc = fp16_scale(amax);
-        if (sc > 0.0f) {
-            R.fp16 = true;
-            R.scale = sc;
-        }
-    }
-    R.have_scale = true;
+    set_operands(R, d, bits);
+    return CUSCAN_OK;
+}
+
+// The same from what sort_by_cells left (one host read), and whether plain bf16 bounds are so loose
+// against the cells' scales that a first screen with them would only be thrown away: then `tight`
+// is set and the screens start with the tightened operands. The estimate only picks the order of
+// attempts; its factor of two keeps data that passes (unit vectors of 128 features: half the
+// limit) on plain bf16.
+static int choose_operands_by_cells(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d, int d_pad,
+                                    int k, bool &tight, cudaStream_t s) {
+    RefinedBuffers &R = b.refined;
+    float ca, cb, abs_c;
+    error_coefficients(d, d_pad, FMT_BF16, 0.0f, ca, cb, abs_c);
+    const double entries = 2.0 * KNN_LIST;
+    const float gap = (float)(2.0 * (2.0 / d) * std::log(k < entries ? entries / k : 1.0));
+    if (int rc = count_tight_rows(ctx, b, n, ca, gap, s)) return rc;
+    unsigned int words[4] = {0, 0, 0, 0};
+    CUSCAN_CUDA(ctx, cudaMemcpyAsync(words, R.norm_range.ptr, sizeof(words), cudaMemcpyDeviceToHost,
+                                     s));
+    CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
+    set_operands(R, d, words[2]);
+    tight = !R.fp16 && (double)words[3] > TIGHT_START * (double)n;
     return CUSCAN_OK;
 }
 
@@ -2037,24 +2064,17 @@ int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
     RefinedBuffers &R = b.refined;
     Layout L;
     refined_layout(n, d, L);
-    int rc = choose_operands(ctx, R, x, n, d, s);
+    // 1, 2. rows in spatial order (b.perm, b.xp), and the screens' operands
+    bool tight = false;
+    int rc = sort_by_cells(ctx, b, x, n, d, s);
+    if (!rc) rc = choose_operands_by_cells(ctx, b, n, d, L.d_pad, k, tight, s);
     if (rc) return rc;
     if (!R.range_ok)  // values large enough to overflow f32: the exact sweep decides alone
         return launch_exact_knn_fp32(ctx, x, n, x, n, d, k, 1, 0, 1, ids, dist, s, b.knn_ids_tmp,
                                      b.knn_dist_tmp);
-    // 1, 2. rows in spatial order (b.perm, b.xp)
-    if ((rc = sort_by_cells(ctx, b, x, n, d, s))) return rc;
     R.pivots_valid = true;
-    const float *xs = as<float>(b.xp);
-    const int32_t *perm = as<int32_t>(b.perm);
-    // 3. screen + exact re-rank in sorted positions, outputs in original rows
-    int fallbacks = 0;
-    if ((rc = knn_list_pass(ctx, R, L, xs, perm, n, d, k, ids, dist, s, fallbacks))) return rc;
-    if (refined_rows) *refined_rows += n;
-    if (!R.fp16 && !R.split && (double)fallbacks > TIGHTEN_TRIGGER * (double)n) {
-        // the bf16 bound is too loose for this data (norms large against the neighbour
-        // distances): screen again, and run the Borůvka rounds, with split-bf16 operands, or
-        // with scaled fp16 operands where a split tile does not fit the pipeline
+    // the tightened operands: split bf16, or scaled fp16 for rows too wide to split
+    auto tighten = [&]() {
         Layout Ls;
         const float sc = fp16_scale(R.amax_value);
         if (refined_layout(n, d, Ls, true)) {
@@ -2064,6 +2084,18 @@ int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
             R.fp16 = true;
             R.scale = sc;
         }
+    };
+    if (tight) tighten();
+    const float *xs = as<float>(b.xp);
+    const int32_t *perm = as<int32_t>(b.perm);
+    // 3. screen + exact re-rank in sorted positions, outputs in original rows
+    int fallbacks = 0;
+    if ((rc = knn_list_pass(ctx, R, L, xs, perm, n, d, k, ids, dist, s, fallbacks))) return rc;
+    if (refined_rows) *refined_rows += n;
+    if (!R.fp16 && !R.split && (double)fallbacks > TIGHTEN_TRIGGER * (double)n) {
+        // the bf16 bound is too loose for this data (norms large against the neighbour
+        // distances): screen again, and run the Borůvka rounds, with the tightened operands
+        tighten();
         if (R.split || R.fp16)
             if ((rc = knn_list_pass(ctx, R, L, xs, perm, n, d, k, ids, dist, s, fallbacks)))
                 return rc;
