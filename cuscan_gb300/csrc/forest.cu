@@ -371,6 +371,25 @@ __global__ void gather_kernel(const float *__restrict__ x, const float *__restri
     }
 }
 
+// gather_kernel for rows of 16-byte pieces (d a multiple of 4, aligned rows): a thread per piece. What
+// bounds it is HBM and the latency of the row index: 500,000 x 128 107 us against 322 us with
+// a thread per element.
+__global__ void gather4_kernel(const float4 *__restrict__ x, const float *__restrict__ core,
+                               const int32_t *__restrict__ label, const int32_t *__restrict__ perm,
+                               int64_t pieces, unsigned per_row, float4 *__restrict__ xp,
+                               float *__restrict__ corep, int32_t *__restrict__ labp) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= pieces) return;
+    const int64_t pos = e / per_row;
+    const unsigned c = (unsigned)(e - pos * per_row);
+    const int32_t i = perm[pos];
+    xp[e] = x[(int64_t)i * per_row + c];
+    if (c == 0) {
+        if (core) corep[pos] = core[i];
+        labp[pos] = label[i];
+    }
+}
+
 // Per-component minimum of (row weight bits << 32 | row) over component-sorted positions:
 // segmented warp reduction over the contiguous label runs, one atomic per run.
 // Component key of the row at sorted position pos: (weight bits << 32 | row), ~0 for a row
@@ -958,9 +977,14 @@ int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, 
     if (rc) return rc;
     CUSCAN_KERNEL(scatter_kernel, blocks(n), 256, 0, s, key ? key : label, n, start,
                   as<int32_t>(b.scan_tmp), fill, as<int32_t>(b.perm));
-    CUSCAN_KERNEL(gather_kernel, blocks(n * d), 256, 0, s, x, core, label, as<int32_t>(b.perm), n, d,
-                                                 as<float>(b.xp), as<float>(b.corep),
-                                                 as<int32_t>(b.labp));
+    if (d % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0)
+        CUSCAN_KERNEL(gather4_kernel, blocks(n * (d / 4)), 256, 0, s,
+                      reinterpret_cast<const float4 *>(x), core, label, as<int32_t>(b.perm),
+                      n * (d / 4), (unsigned)(d / 4), reinterpret_cast<float4 *>(b.xp.ptr),
+                      as<float>(b.corep), as<int32_t>(b.labp));
+    else
+        CUSCAN_KERNEL(gather_kernel, blocks(n * d), 256, 0, s, x, core, label, as<int32_t>(b.perm), n,
+                      d, as<float>(b.xp), as<float>(b.corep), as<int32_t>(b.labp));
     CUSCAN_LAUNCH(ctx, "component sort");
     return CUSCAN_OK;
 }

@@ -1286,40 +1286,79 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
 
 // Exact squared distance (the reference's order) from the warp's query row q_s (shared) to the
 // candidate row j held by this lane (j < 0: none, returns +inf). The warp first copies the 32
-// candidate rows into its shared staging area row by row, each row read with consecutive
-// addresses, then every lane sums its own row sequentially; the row stride d + 1 keeps the
-// lanes on distinct banks.
+// candidate rows into its shared staging area, then every lane sums its own row sequentially.
+// What bounds it is the copies (32 rows of L2 per 32 candidates). VEC: rows of d % 4 == 0 features
+// on 16-byte boundaries move in 16-byte pieces, 32 / (d / 4) rows per instruction, and are read
+// back as float4 (row stride d + 4: eight lanes cover the 32 banks); other rows move in 4-byte
+// pieces with row stride d + 1. 500,000 x 128 rows, 32 candidates each: 3.1 ms against 4.0 ms
+// in 4-byte pieces.
+template <bool VEC>
 __device__ __forceinline__ float staged_d2(const float *__restrict__ x, int d,
                                            const float *q_s, int32_t j, float *rows_s,
                                            int lane) {
-    // asynchronous 4-byte copies: every row's loads are in flight at once
-    for (int r = 0; r < 32; ++r) {
-        const int32_t jr = __shfl_sync(0xffffffffu, j, r);
-        if (jr < 0) continue;
-        const float *src = x + (int64_t)jr * d;
-        float *dst = rows_s + r * (d + 1);
-        for (int f = lane; f < d; f += 32)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + f)),
-                         "l"(src + f)
-                         : "memory");
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncwarp();
     float acc = CUSCAN_INF;
-    if (j >= 0) {
-        const float *row = rows_s + lane * (d + 1);
-        acc = 0.0f;
-        for (int f = 0; f < d; ++f) {
-            const float t = q_s[f] - row[f];
-            acc = __fmaf_rn(t, t, acc);
+    if (VEC) {
+        const int pieces = d >> 2, total = 32 * pieces, stride = d + 4;
+        for (int p0 = 0; p0 < total; p0 += 32) {
+            const int p = p0 + lane;  // total is a multiple of 32
+            const int r = p / pieces, c = p - r * pieces;
+            const int32_t jr = __shfl_sync(0xffffffffu, j, r);
+            if (jr >= 0)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                 smem_u32(rows_s + r * stride + 4 * c)),
+                             "l"(x + (int64_t)jr * d + 4 * c)
+                             : "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        if (j >= 0) {
+            const float4 *row = reinterpret_cast<const float4 *>(rows_s + lane * stride);
+            const float4 *q = reinterpret_cast<const float4 *>(q_s);
+            acc = 0.0f;
+#pragma unroll 4
+            for (int c = 0; c < pieces; ++c) {
+                const float4 a = q[c], b = row[c];
+                const float t0 = a.x - b.x, t1 = a.y - b.y, t2 = a.z - b.z, t3 = a.w - b.w;
+                acc = __fmaf_rn(t0, t0, acc);
+                acc = __fmaf_rn(t1, t1, acc);
+                acc = __fmaf_rn(t2, t2, acc);
+                acc = __fmaf_rn(t3, t3, acc);
+            }
+        }
+    } else {
+        for (int r = 0; r < 32; ++r) {
+            const int32_t jr = __shfl_sync(0xffffffffu, j, r);
+            if (jr < 0) continue;
+            const float *src = x + (int64_t)jr * d;
+            float *dst = rows_s + r * (d + 1);
+            for (int f = lane; f < d; f += 32)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst + f)),
+                             "l"(src + f)
+                             : "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        if (j >= 0) {
+            const float *row = rows_s + lane * (d + 1);
+            acc = 0.0f;
+            for (int f = 0; f < d; ++f) {
+                const float t = q_s[f] - row[f];
+                acc = __fmaf_rn(t, t, acc);
+            }
         }
     }
     __syncwarp();
     return acc;
 }
 
-// Shared floats one warp of a re-rank kernel stages: 32 candidate rows and the query row.
-__host__ __device__ constexpr int64_t rerank_warp_floats(int d) { return 32 * (d + 1) + d; }
+// Shared floats one warp of a re-rank kernel stages: 32 candidate rows and the query row (a multiple
+// of four with VEC, so that every warp's rows stay on 16-byte boundaries).
+__host__ __device__ constexpr int64_t rerank_warp_floats(int d, bool vec) {
+    return vec ? 32 * (d + 4) + d : 32 * (d + 1) + d;
+}
+static bool rerank_vec(const float *x, int d) {
+    return d % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+}
 constexpr int RERANK_WARPS = 4;
 
 __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
@@ -1345,7 +1384,7 @@ __device__ __forceinline__ float unseen_bound(const int32_t *ids, const float *l
 // kNN re-rank: one warp per row, exact distances of the 2M candidates, top-k by (d, id).
 // x and the candidates are in sorted positions; perm maps a position to its original row, which
 // is the id the reference orders ties by and the row the output goes to.
-template <int M>
+template <int M, bool VEC>
 __global__ void rerank_knn_kernel(const float *__restrict__ x, const int32_t *__restrict__ perm,
                                   int64_t n, int d, int k, const int32_t *__restrict__ cand_ids,
                                   const float *__restrict__ cand_lb, int32_t *__restrict__ ids,
@@ -1356,7 +1395,7 @@ __global__ void rerank_knn_kernel(const float *__restrict__ x, const int32_t *__
     const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= n) return;
-    float *q_s = rerank_smem + (threadIdx.x >> 5) * rerank_warp_floats(d);
+    float *q_s = rerank_smem + (threadIdx.x >> 5) * rerank_warp_floats(d, VEC);
     float *rows_s = q_s + d;
     for (int f = lane; f < d; f += 32) q_s[f] = x[row * d + f];
     __syncwarp();
@@ -1374,7 +1413,7 @@ __global__ void rerank_knn_kernel(const float *__restrict__ x, const int32_t *__
     auto round_key = [&](int first, int count) -> unsigned long long {
         const int h = lane >> 4, o = lane & 15;
         const int32_t j = o < count ? cand_ids[row * W + h * M + first + o] : -1;
-        const float dd = staged_d2(x, d, q_s, j, rows_s, lane);
+        const float dd = staged_d2<VEC>(x, d, q_s, j, rows_s, lane);
         return j < 0 ? ~0ull : ((unsigned long long)__float_as_uint(dd) << 32) | (uint32_t)perm[j];
     };
     key[0] = round_key(0, F);
@@ -1432,6 +1471,7 @@ __global__ void rerank_knn_kernel(const float *__restrict__ x, const int32_t *__
 // bound does not exceed an upper bound of its k-th distance, so the exact top k of its appended
 // candidates by (d, original id) is its exact kNN row. A buffer that overflowed (or a row with
 // fewer than k candidates) sends the row's original index to the exact f32 sweep.
+template <bool VEC>
 __global__ void rerank_knn_threshold_kernel(const float *__restrict__ x,
                                             const int32_t *__restrict__ perm,
                                             const int32_t *__restrict__ qpos, int64_t nq, int d,
@@ -1452,7 +1492,7 @@ __global__ void rerank_knn_threshold_kernel(const float *__restrict__ x,
         return;
     }
     extern __shared__ float rerank_smem[];
-    float *q_s = rerank_smem + (threadIdx.x >> 5) * rerank_warp_floats(d);
+    float *q_s = rerank_smem + (threadIdx.x >> 5) * rerank_warp_floats(d, VEC);
     float *rows_s = q_s + d;
     for (int f = lane; f < d; f += 32) q_s[f] = x[pos * d + f];
     __syncwarp();
@@ -1464,7 +1504,7 @@ __global__ void rerank_knn_threshold_kernel(const float *__restrict__ x,
         if (s < c0 + c1)
             j = s < c0 ? cand_ids[(q * 2) * cap + s] : cand_ids[(q * 2 + 1) * cap + (s - c0)];
         // every lane joins the staging (it is warp-wide), the rounds are uniform per warp
-        const float dd = t * 32 < c0 + c1 ? staged_d2(x, d, q_s, j, rows_s, lane) : CUSCAN_INF;
+        const float dd = t * 32 < c0 + c1 ? staged_d2<VEC>(x, d, q_s, j, rows_s, lane) : CUSCAN_INF;
         key[t] = j < 0 ? ~0ull : ((unsigned long long)__float_as_uint(dd) << 32) | (uint32_t)perm[j];
     }
     for (int r = 0; r < k; ++r) {
@@ -1493,6 +1533,7 @@ __global__ void positions_to_rows_kernel(int32_t *__restrict__ list, int64_t cou
 // both row halves, row minimum (w, original j) into row_keys[original row]. Rows whose buffer
 // overflowed are re-run exactly; rows without candidates keep an empty key (they cannot hold
 // their component's cheapest edge: every pair reaching it is appended).
+template <bool VEC>
 __global__ void rerank_boruvka_kernel(const float *__restrict__ xp, const float *__restrict__ corep,
                                       const int32_t *__restrict__ labp,
                                       const int32_t *__restrict__ perm, int64_t nq,
@@ -1528,7 +1569,7 @@ __global__ void rerank_boruvka_kernel(const float *__restrict__ xp, const float 
     const int total = c0 + c1 + c2;
     if (total == 0) return;  // no candidate: the row keeps an empty key
     extern __shared__ float rerank_smem[];
-    float *q_s = rerank_smem + (threadIdx.x >> 5) * rerank_warp_floats(d);
+    float *q_s = rerank_smem + (threadIdx.x >> 5) * rerank_warp_floats(d, VEC);
     float *rows_s = q_s + d;
     for (int f = lane; f < d; f += 32) q_s[f] = xp[pos * d + f];
     __syncwarp();
@@ -1544,7 +1585,7 @@ __global__ void rerank_boruvka_kernel(const float *__restrict__ xp, const float 
                               : colbuf[pos * capc + (s - c0 - c1)];
             if (labp[j] == li) j = -1;
         }
-        const float d2 = staged_d2(xp, d, q_s, j, rows_s, lane);
+        const float d2 = staged_d2<VEC>(xp, d, q_s, j, rows_s, lane);
         if (j < 0) continue;
         const float w = fmaxf(fmaxf(d2, ci), corep[j]);
         if (w != w) continue;
@@ -1943,13 +1984,18 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
     P.stages = L.stages;
     P.stage_blocks = L.stage_blocks;
     P.cursor = as<unsigned long long>(R.cursor);
-    // parts of at least 128 tiles: the start of a work item (A tile, pipeline fill) stays small
+    // parts of at least 128 tiles in general: the start of a work item (A tile, pipeline fill) stays small
     // against its tiles, and the fits of a serving stream (under 32,768 rows) keep one CTA per
     // block, leaving the other SMs to the fits running beside them
     P.splits = 1;
     if (MODE == MODE_BORUVKA && P.n_qblocks > 0 && P.n_qblocks < ctx->sm_count && !debug_tile) {
         int64_t per = ctx->sm_count / P.n_qblocks;
         if (per > P.n_tiles / 128) per = P.n_tiles / 128;
+        // a round of few blocks may take a quarter of the SMs in parts of at least 16 tiles
+        // (950 rows of 50,000 x 128: eight CTAs took 0.77 ms for the round, in four parts 0.43 ms)
+        int64_t few = ctx->sm_count / (4 * P.n_qblocks);
+        if (few > P.n_tiles / 16) few = P.n_tiles / 16;
+        if (per < few) per = few;
         P.splits = (int)(per < 1 ? 1 : per < 16 ? per : 16);
     }
     float ca, cb, abs_c;
@@ -2043,9 +2089,11 @@ static int knn_list_pass(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, co
         return rc;
     CUSCAN_CUDA(ctx, cudaEventRecord(R.screen_ev[1], s));
     R.screen_timed = true;
-    const size_t rr_smem = sizeof(float) * RERANK_WARPS * (size_t)rerank_warp_floats(d);
-    if (int rc = allow_dynamic_smem(ctx, rerank_knn_kernel<M>, rr_smem)) return rc;
-    CUSCAN_KERNEL(rerank_knn_kernel<M>, (unsigned)ceil_div(n, (int64_t)RERANK_WARPS),
+    const bool vec = rerank_vec(xs, d);
+    const size_t rr_smem = sizeof(float) * RERANK_WARPS * (size_t)rerank_warp_floats(d, vec);
+    const auto rerank = vec ? rerank_knn_kernel<M, true> : rerank_knn_kernel<M, false>;
+    if (int rc = allow_dynamic_smem(ctx, rerank, rr_smem)) return rc;
+    CUSCAN_KERNEL(rerank, (unsigned)ceil_div(n, (int64_t)RERANK_WARPS),
                   32 * RERANK_WARPS, rr_smem, s, xs, perm, n, d,
                   k, as<int32_t>(R.cand_ids), as<float>(R.cand_lb), ids, dist,
                   as<int32_t>(R.fallback), as<float>(R.qthr), as<int>(R.error) + STATUS_FALLBACKS);
@@ -2102,7 +2150,9 @@ int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
     }
     if (fallbacks == 0) return CUSCAN_OK;
     constexpr int M = KNN_LIST;
-    const size_t rr_smem = sizeof(float) * RERANK_WARPS * (size_t)rerank_warp_floats(d);
+    const bool vec = rerank_vec(xs, d);
+    const size_t rr_smem = sizeof(float) * RERANK_WARPS * (size_t)rerank_warp_floats(d, vec);
+    const auto rerank = vec ? rerank_knn_threshold_kernel<true> : rerank_knn_threshold_kernel<false>;
     int32_t *exact_rows = as<int32_t>(R.fallback);
     int exact = fallbacks;
     if (fallbacks >= RESCREEN_MIN_ROWS && k <= 2 * KNN_CAP) {
@@ -2131,8 +2181,8 @@ int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
         if ((rc = run_screen<M, MODE_KNN_THRESHOLD>(ctx, R, L, n, d, nullptr, nullptr, nullptr,
                                                    nullptr, s, nullptr, nullptr, Q)))
             return rc;
-        if ((rc = allow_dynamic_smem(ctx, rerank_knn_threshold_kernel, rr_smem))) return rc;
-        CUSCAN_KERNEL(rerank_knn_threshold_kernel, (unsigned)ceil_div(nq, (int64_t)RERANK_WARPS),
+        if ((rc = allow_dynamic_smem(ctx, rerank, rr_smem))) return rc;
+        CUSCAN_KERNEL(rerank, (unsigned)ceil_div(nq, (int64_t)RERANK_WARPS),
                       32 * RERANK_WARPS, rr_smem, s, xs,
                       perm, as<int32_t>(R.fallback), nq, d, k, as<int32_t>(R.cand2),
                       as<int32_t>(R.rowcnt2), KNN_CAP, ids, dist, as<int32_t>(R.fallback2),
@@ -2260,10 +2310,12 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
     if (rc) return rc;
     R.screened_rows += nq;
     if (sym) ++R.symmetric_rounds;
-    const size_t rr_smem = sizeof(float) * RERANK_WARPS * (size_t)rerank_warp_floats(d);
-    if ((rc = allow_dynamic_smem(ctx, rerank_boruvka_kernel, rr_smem))) return rc;
+    const bool vec = rerank_vec(xp, d);
+    const size_t rr_smem = sizeof(float) * RERANK_WARPS * (size_t)rerank_warp_floats(d, vec);
+    const auto rerank = vec ? rerank_boruvka_kernel<true> : rerank_boruvka_kernel<false>;
+    if ((rc = allow_dynamic_smem(ctx, rerank, rr_smem))) return rc;
     if (nq > 0) {
-        CUSCAN_KERNEL(rerank_boruvka_kernel, (unsigned)ceil_div(nq, (int64_t)RERANK_WARPS),
+        CUSCAN_KERNEL(rerank, (unsigned)ceil_div(nq, (int64_t)RERANK_WARPS),
                       32 * RERANK_WARPS, rr_smem, s, xp, corep, labp, perm, nq, qpos, d,
                       as<int32_t>(R.cand_ids), as<int32_t>(R.rowcnt), BORUVKA_CAP,
                       sym ? as<int32_t>(R.colcnt) : nullptr, as<int32_t>(R.colbuf),
