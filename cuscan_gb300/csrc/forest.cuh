@@ -33,6 +33,7 @@ struct RefinedBuffers {
     Buffer qthr, xq, pq, mq, cand2, rowcnt2, fallback2;  // threshold re-screen of kNN rows
     Buffer urow, colcnt, colbuf;  // symmetric Borůvka: row bounds, column-side buffers
     Buffer act_flag, act_idx, act_pos;  // Borůvka rows that can hold their component's edge
+    Buffer qchunk_lo, qchunk_hi;  // label ranges of the gathered rows' 32-row chunks
     Buffer rowlb, lbtmp;  // lower bounds of each row's cheapest cross edge (original order)
     // operand format of the current fit: fp16 of x * scale (scale a power of two), or bf16
     bool want_fp16 = false;  // requested by the caller's precision
@@ -73,7 +74,7 @@ struct ForestBuffers {
 int forest_reserve(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d);
 void forest_release(ForestBuffers &b);
 // Every device buffer of the forest and of the bf16 screen (out may be null); returns the count.
-constexpr int kForestBufferCount = 73;
+constexpr int kForestBufferCount = 75;
 int forest_buffers(ForestBuffers &b, Buffer **out);
 // Whether a set of n points takes the one-CTA forest steps (fewer than 2048 points).
 bool forest_small(int64_t n);

@@ -96,6 +96,8 @@ struct Params {
     const float *pq, *mq;     // their squared norms and rounded-up norms
     int64_t nq;               // query rows
     const int32_t *qpos;      // position of each query row in the reference order (null: same)
+    const int32_t *qchunk_lo; // Borůvka: label range of 32-row chunks of gathered query rows
+    const int32_t *qchunk_hi;
     const float *qthr;        // threshold mode: per-query upper bound of the k-th distance (raw)
     // symmetric Borůvka: per-row upper bounds of the cheapest cross edge (raw f32 bits) and the
     // per-row buffers that other query blocks append column-side pairs to
@@ -364,24 +366,24 @@ __global__ void __launch_bounds__(PREP_THREADS)
         }
         mmax = fmaxf(mmax, m);
     }
+    if (label && tid < BN) {
+        // a warp per 32-row chunk; chunks past the end have the empty range
+        const int64_t r = row0 + tid;
+        const int32_t l = r < n ? label[rowmap ? (int64_t)rowmap[r] : r] : 0;
+        const int32_t lo = __reduce_min_sync(0xffffffffu, r < n ? l : INT32_MAX);
+        const int32_t hi = __reduce_max_sync(0xffffffffu, r < n ? l : INT32_MIN);
+        if (lane == 0) {
+            range_lo[tid >> 5] = lo;
+            range_hi[tid >> 5] = hi;
+            if (r < n) {
+                chunk_lo[r >> 5] = lo;
+                chunk_hi[r >> 5] = hi;
+            }
+        }
+    }
     if (tile_mmax) {
         mmax = ord2f(__reduce_max_sync(0xffffffffu, f2ord(mmax)));
         if (lane == 0) warp_max[tid >> 5] = mmax;
-        if (label && tid < BN) {
-            // a warp per 32-row chunk; chunks past the end have the empty range
-            const int64_t r = row0 + tid;
-            const int32_t l = r < n ? label[r] : 0;
-            const int32_t lo = __reduce_min_sync(0xffffffffu, r < n ? l : INT32_MAX);
-            const int32_t hi = __reduce_max_sync(0xffffffffu, r < n ? l : INT32_MIN);
-            if (lane == 0) {
-                range_lo[tid >> 5] = lo;
-                range_hi[tid >> 5] = hi;
-                if (r < n) {
-                    chunk_lo[r >> 5] = lo;
-                    chunk_hi[r >> 5] = hi;
-                }
-            }
-        }
         __syncthreads();
         if (tid == 0) {
             float mx = 0.0f;
@@ -514,16 +516,21 @@ __device__ __forceinline__ int64_t block_at(const Params &P, int64_t qi) {
 // Label range of query block qb (4 chunks of 32 rows).
 __device__ __forceinline__ void qblock_range(const Params &P, int64_t qb, int32_t &lo,
                                              int32_t &hi) {
-    if (P.qpos) {  // gathered query rows: no label range (no tile is skipped)
+    // gathered query rows keep the order of their components, so most of their blocks have one
+    // label too and skip their own component's tiles; without label ranges they skip none
+    if (P.qpos && !P.qchunk_lo) {
         lo = INT32_MIN;
         hi = INT32_MAX;
         return;
     }
+    const int32_t *clo = P.qpos ? P.qchunk_lo : P.chunk_lo;
+    const int32_t *chi = P.qpos ? P.qchunk_hi : P.chunk_hi;
+    const int64_t chunks = P.qpos ? (P.nq + 31) / 32 : P.n_chunks;
     lo = INT32_MAX;
     hi = INT32_MIN;
-    for (int64_t c = qb * 4; c < qb * 4 + 4 && c < P.n_chunks; ++c) {
-        lo = min(lo, P.chunk_lo[c]);
-        hi = max(hi, P.chunk_hi[c]);
+    for (int64_t c = qb * 4; c < qb * 4 + 4 && c < chunks; ++c) {
+        lo = min(lo, clo[c]);
+        hi = max(hi, chi[c]);
     }
 }
 
@@ -1807,6 +1814,7 @@ size_t refined_workspace_bytes(int64_t n, int d, int k) {
     // their scan and the gathered positions
     b += 8 * (size_t)n + 4 * (size_t)n * BORUVKA_COL_CAP + 12 * (size_t)n;
     b += 12 * (size_t)n;  // row lower bounds (original order) and per-half screen bounds
+    b += 8 * (size_t)(L.n_pad / 32);  // label ranges of gathered rows
     return b;
 }
 
@@ -1941,6 +1949,7 @@ struct QuerySet {
     const float *pq = nullptr, *mq = nullptr;
     int64_t nq = -1;
     const int32_t *qpos = nullptr;
+    const int32_t *qchunk_lo = nullptr, *qchunk_hi = nullptr;
     const float *qthr = nullptr;
     int32_t *cand_ids = nullptr;
     int32_t *rowcnt = nullptr;
@@ -1966,6 +1975,8 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
     P.mq = Q.mq ? Q.mq : P.mnorm;
     P.nq = Q.nq >= 0 ? Q.nq : n;
     P.qpos = Q.qpos;
+    P.qchunk_lo = Q.qchunk_lo;
+    P.qchunk_hi = Q.qchunk_hi;
     P.qthr = Q.qthr;
     P.core = core;
     P.label = label;
@@ -2256,9 +2267,17 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
                              as<int32_t>(R.count) + 1, s)))
         return rc;
     int counts[2] = {0, 0};  // rows without a component bound, rows that can hold an edge
+    double same_pairs = 0.0;
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(counts, R.count.ptr, sizeof(counts), cudaMemcpyDeviceToHost, s));
+    CUSCAN_CUDA(ctx, cudaMemcpyAsync(&same_pairs, &b.status->same_pairs, sizeof(double),
+                                     cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
     const int64_t active = counts[1];
+    // Gathered blocks look for tiles of their own component only where components hold a fair share
+    // of the pairs: the look costs every tile two loads in each role (4 % of a round at 500,000 x 128,
+    // where 1 to 2 % of the tiles could go; at 100,000 x 64 rounds 3 and 4 run 12 % and 51 % fewer
+    // tiles, 6.1 -> 5.3 ms over the fit's screens).
+    const bool skip_own = same_pairs > 0.06 * (double)n * (double)n;
     // Forms of the round:
     //  * one-sided over the rows that can hold their component's cheapest edge (all rows, or a
     //    gathered subset): it also leaves each screened row a lower bound of its cheapest cross
@@ -2289,15 +2308,21 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
                       as<int32_t>(b.scan_tmp), n, as<int32_t>(R.act_pos));
         CUSCAN_LAUNCH(ctx, "compact_positions_kernel");
         qpos = as<int32_t>(R.act_pos);
-        if ((rc = tile_rows(ctx, R, xp, nq, d, L.d_pad, nq_pad, qpos, as<uint8_t>(R.xq),
-                            as<float>(R.pq), as<float>(R.mq), s)))
-            return rc;
+        rc = ensure(ctx, R.qchunk_lo, sizeof(int32_t) * (nq_pad / 32), "subset labels");
+        if (!rc) rc = ensure(ctx, R.qchunk_hi, sizeof(int32_t) * (nq_pad / 32), "subset labels");
+        if (!rc)
+            rc = tile_rows(ctx, R, xp, nq, d, L.d_pad, nq_pad, qpos, as<uint8_t>(R.xq),
+                           as<float>(R.pq), as<float>(R.mq), s, nullptr, skip_own ? labp : nullptr,
+                           as<int32_t>(R.qchunk_lo), as<int32_t>(R.qchunk_hi));
+        if (rc) return rc;
         QuerySet Q;
         Q.xq = as<uint8_t>(R.xq);
         Q.pq = as<float>(R.pq);
         Q.mq = as<float>(R.mq);
         Q.nq = nq;
         Q.qpos = qpos;
+        Q.qchunk_lo = skip_own ? as<int32_t>(R.qchunk_lo) : nullptr;
+        Q.qchunk_hi = skip_own ? as<int32_t>(R.qchunk_hi) : nullptr;
         Q.rowlb = as<float>(R.lbtmp);
         rc = run_screen<M, MODE_BORUVKA>(ctx, R, L, n, d, corep, labp, clo, chi, s, nullptr, nullptr, Q);
     } else if (sym) {
