@@ -22,7 +22,7 @@ int sort_by_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, 
 // Device bytes of sort_by_cells beyond the forest's own buffers.
 inline size_t cells_workspace_bytes(int64_t n, int d) {
     return sizeof(float) * (2 * (size_t)kMaxPivots * d + (size_t)kMaxPivots * kMaxPivots +
-                            3 * kMaxPivots) + 16 * (size_t)n;  // cells, distances, norms, keys
+                            4 * kMaxPivots) + 16 * (size_t)n;  // cells, distances, norms, keys
 }
 // Query orders for the pruned sweeps: the rows grouped by cell, every cell padded to whole balls of
 // kBallRows entries with -1, so that no ball straddles two cells. A straddling ball is as wide as
@@ -37,7 +37,8 @@ int order_queries(cuscan_ctx *ctx, ForestBuffers &b, const float *pivots, int np
 // Of the n positions of the set itself, right after sort_by_cells.
 int order_positions(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int32_t *order, cudaStream_t s);
 // Rows of cells whose scale times gap is below shift times the squared norm of their pivot, counted
-// in word 3 of b.refined.norm_range. Right after sort_by_cells.
+// in word 3 of b.refined.norm_range, and in word 4 (f32) the pairs of rows in cells too far apart to be
+// neighbours. Right after sort_by_cells.
 int count_tight_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, float shift, float gap,
                      cudaStream_t s);
 // cbound[label] (f32 bits, labels by original row) lowered to the weights of edges between pivots
@@ -55,7 +56,12 @@ struct TileBounds {
     int64_t tiles = 0, stride = 0;  // stride = PARTS * tiles
 };
 int tile_bounds(cuscan_ctx *ctx, const float *x, int64_t n, int d, Buffer &centre, Buffer &radius,
-                TileBounds &out, cudaStream_t s);
+                TileBounds &out, cudaStream_t s, int k = 0, float *thr = nullptr);
+
+// Lists of the 256-row tiles that the 128-row blocks of a kNN screen visit (refined.cu): b.refined.vis
+// and vis_count. Right after sort_by_cells; tiles up to kMaxVisitTiles.
+constexpr int64_t kMaxVisitTiles = 8192;  // 2,097,152 rows: 268 MB of lists
+int visit_lists(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d, int k, cudaStream_t s);
 
 // Exact kNN of query rows against a spatially ordered set (knn.cu): squared distances, the rows
 // and order of launch_exact_knn_fp32, every tile that cannot hold a neighbour left out. ref_ids

@@ -30,6 +30,7 @@ struct RefinedBuffers {
     Buffer pivot_d, cell_scale, rnorm, norm_range, key;
     // pruned sweeps: tile bounds, first thresholds, padded query order
     Buffer tile_centre, tile_radius, thr0, qorder;
+    Buffer ball_thr, vis, vis_count;  // kNN screens over lists of tiles: thresholds, lists, lengths
     Buffer qthr, xq, pq, mq, cand2, rowcnt2, fallback2;  // threshold re-screen of kNN rows
     Buffer urow, colcnt, colbuf;  // symmetric Borůvka: row bounds, column-side buffers
     Buffer act_flag, act_idx, act_pos;  // Borůvka rows that can hold their component's edge
@@ -51,6 +52,7 @@ struct RefinedBuffers {
     bool lb_valid = false;      // rowlb holds bounds of the current fit
     int cell_levels = 1;        // norm levels per cell of the last sort_by_cells
     bool pivots_valid = false;  // pivot_d holds distances of the current fit's rows
+    bool listed = false;        // the current fit's kNN list screens run lists of tiles
     // CUDA events around the kNN list screen's launch (created on first use); screen_timed
     // says they hold the current fit's launch
     cudaEvent_t screen_ev[2] = {nullptr, nullptr};
@@ -74,7 +76,7 @@ struct ForestBuffers {
 int forest_reserve(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d);
 void forest_release(ForestBuffers &b);
 // Every device buffer of the forest and of the bf16 screen (out may be null); returns the count.
-constexpr int kForestBufferCount = 75;
+constexpr int kForestBufferCount = 78;
 int forest_buffers(ForestBuffers &b, Buffer **out);
 // Whether a set of n points takes the one-CTA forest steps (fewer than 2048 points).
 bool forest_small(int64_t n);

@@ -108,6 +108,9 @@ struct Params {
     // one-sided Borůvka: per query row and column half, a lower bound of every cross-component
     // pair weight the row has (raw f32, rounded down)
     float *rowlb;
+    // LIST: the tiles each query block visits ([n_qblocks][n_tiles], in order) and their number
+    const uint16_t *vis;
+    const int32_t *vis_count;
 };
 
 // Screen modes: kNN lists, Borůvka thresholds with shared component bounds, kNN thresholds.
@@ -131,6 +134,14 @@ constexpr double TIGHTEN_TRIGGER = 0.15;
 // Share of rows that choose_operands_by_cells expects to be inconclusive from which the first
 // screen already uses the tightened operands.
 constexpr double TIGHT_START = 0.25;
+// kNN screens over lists of tiles: smallest fit, and the share of row pairs in cells too far apart to
+// hold neighbours from which the lists are made (mixtures of separated clusters have 0.93 to 0.97,
+// unit vectors about 0). At 100,000 x 64, 50 clusters and noise, the blocks visit a fifth of the
+// tiles and the screen takes 1.60 ms instead of 2.46 ms (lists and balls 0.09 ms; the noise
+// blocks visit all); 50,000 x 128: 0.41 instead of 0.65 ms. At 9,001 x 32, where half of the tiles
+// stay, the two launches cost what the screen gains.
+constexpr int64_t LIST_MIN_ROWS = 16384;
+constexpr float LIST_MIN_APART = 0.6f;
 // Status words of a screen: [0] error flag, [2..3] tile pairs (u64), [4] inconclusive rows listed by
 // the re-rank, [5] spare.
 constexpr int SCREEN_STATUS_WORDS = 8;
@@ -558,13 +569,15 @@ __device__ __forceinline__ void list_insert(float (&L)[M], int (&J)[M], float x,
     }
 }
 
-template <int M, int MODE>
+// LIST (kNN lists): the blocks visit the tiles of their lists (visit_lists_kernel), not every tile.
+template <int M, int MODE, bool LIST>
 __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
     constexpr bool BORUVKA = MODE == MODE_BORUVKA || MODE == MODE_BORUVKA_SYM;
     constexpr bool SYM = MODE == MODE_BORUVKA_SYM;
     constexpr bool THRESH = MODE == MODE_KNN_THRESHOLD;
     constexpr bool APPEND = BORUVKA || THRESH;  // threshold modes append to per-row buffers
-    constexpr bool ROT = !BORUVKA;              // kNN sweeps: rotated shared tile order
+    constexpr bool ROT = !BORUVKA && !LIST;     // kNN sweeps: rotated shared tile order
+    constexpr bool CLAIM = !BORUVKA;            // and blocks from a global counter
     // kNN sweeps: the column terms of each tile are copied into the warp's shared slots, where
     // the list insertions read them (Borůvka screens read them from global memory)
     constexpr bool STAGE = !BORUVKA;
@@ -641,7 +654,7 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
             for (uint32_t li = 0; !*abort; ++li) {  // li: this CTA's query step
                 int64_t qi = blockIdx.x + (int64_t)li * gridDim.x;
                 int32_t rot = 0;
-                if (ROT) {
+                if (CLAIM) {
                     // kNN sweeps: blocks come from a global counter, so that CTAs that run faster
                     // take more of them. The block and its rotation of the shared order (the
                     // CTAs' average position: tiles issued so far over the grid) go to the MMA
@@ -651,7 +664,7 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
                     // (6.8 against 4.3 ms for the two sweeps of an anisotropic 100,000 x 64 fit).
                     qi = (int64_t)atomicAdd(P.cursor + 1, 1ull);
                     qi = qi < P.n_qblocks ? P.n_qblocks - 1 - qi : P.n_qblocks;
-                    if (P.n_tiles > WARM && qi < P.n_qblocks) {
+                    if (ROT && P.n_tiles > WARM && qi < P.n_qblocks) {
                         const unsigned long long all = *(volatile unsigned long long *)P.cursor;
                         rot = (int32_t)((all / gridDim.x) % (unsigned long long)(P.n_tiles - WARM));
                     }
@@ -674,11 +687,12 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
                     bulk_g2s(sA + kb * KBLOCK_A, asrc + (uint64_t)kb * KBLOCK_B, KBLOCK_A, a_full);
                 int32_t qlo = 0, qhi = 0;
                 if (BORUVKA) qblock_range(P, qb, qlo, qhi);
-                const int64_t wa = window_start(P, qb);
-                const int64_t nvis = vis_count<SYM>(P, qb);
+                const int64_t wa = LIST ? qb * P.n_tiles : window_start(P, qb);
+                const int64_t nvis = LIST ? P.vis_count[qb] : vis_count<SYM>(P, qb);
                 const int64_t i_hi = (part + 1) * nvis / P.splits;
                 for (int64_t i = part * nvis / P.splits; i < i_hi; ++i) {
-                    const int64_t t = ROT ? (int64_t)knn_tile((int32_t)P.n_tiles, (int32_t)wa, rot, (int32_t)i)
+                    const int64_t t = LIST ? (int64_t)P.vis[wa + i]
+                                      : ROT ? (int64_t)knn_tile((int32_t)P.n_tiles, (int32_t)wa, rot, (int32_t)i)
                                           : vis_tile<SYM>(P, qb, wa, i);
                     if (tile_skipped<BORUVKA>(P, t, qlo, qhi)) continue;
                     const uint8_t *bsrc = P.xt + (uint64_t)t * (uint64_t)b_bytes;
@@ -767,7 +781,7 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
             auto blocks = [&](auto kb_c, auto sb_c, auto split_c) {
                 for (uint32_t li = 0; !*abort; ++li) {
                     int64_t qi = blockIdx.x + (int64_t)li * gridDim.x;
-                    if (ROT) {  // kNN sweeps: the block the producer took
+                    if (CLAIM) {  // the block the producer took
                         const uint32_t rs = li & 3;
                         if (!mbar_wait(&rot_full[rs], (li >> 2) & 1, abort, P.error)) break;
                         qi = *(volatile int64_t *)&rot_blk[rs];
@@ -781,8 +795,8 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
                     fence_after();
                     int32_t qlo = 0, qhi = 0;
                     if (BORUVKA) qblock_range(P, qb, qlo, qhi);
-                    const int64_t wa = window_start(P, qb);
-                    const int64_t nvis = vis_count<SYM>(P, qb);
+                    const int64_t wa = LIST ? 0 : window_start(P, qb);
+                    const int64_t nvis = LIST ? P.vis_count[qb] : vis_count<SYM>(P, qb);
                     const int64_t i_hi = (part + 1) * nvis / P.splits;
                     bool ok = true;
                     for (int64_t i = part * nvis / P.splits; i < i_hi; ++i) {
@@ -837,7 +851,7 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
         for (uint32_t li = 0; !*abort; ++li) {
             int64_t qi = blockIdx.x + (int64_t)li * gridDim.x;
             int32_t rot = 0;
-            if (ROT) {  // kNN sweeps: the block the producer took and its rotation
+            if (CLAIM) {  // the block the producer took and its rotation
                 const uint32_t rs = li & 3;
                 if (!mbar_wait(&rot_full[rs], (li >> 2) & 1, abort, P.error)) break;
                 qi = *(volatile int64_t *)&rot_blk[rs];
@@ -884,8 +898,8 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
             int cnt = 0;
             int32_t qlo = 0, qhi = 0;
             if (BORUVKA) qblock_range(P, qb, qlo, qhi);
-            const int64_t wa = window_start(P, qb);
-            const int64_t nvis = vis_count<SYM>(P, qb);
+            const int64_t wa = LIST ? qb * P.n_tiles : window_start(P, qb);
+            const int64_t nvis = LIST ? P.vis_count[qb] : vis_count<SYM>(P, qb);
             // this work item's part [i_lo, i_hi) of the block's tile order
             const int64_t i_lo = part * nvis / P.splits, i_hi = (part + 1) * nvis / P.splits;
             // symmetric mode: the warp's 32 rows summarised for the column-side block test
@@ -896,8 +910,9 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
                 coremin_w = warp_min_f(valid ? core_i : CUSCAN_INF);
             }
             auto tile_at = [&](int64_t i) -> int64_t {
-                return ROT ? (int64_t)knn_tile((int32_t)P.n_tiles, (int32_t)wa, rot, (int32_t)i)
-                           : vis_tile<SYM>(P, qb, wa, i);
+                return LIST  ? (int64_t)P.vis[wa + i]
+                       : ROT ? (int64_t)knn_tile((int32_t)P.n_tiles, (int32_t)wa, rot, (int32_t)i)
+                             : vis_tile<SYM>(P, qb, wa, i);
             };
             // next visited position i (>= i0) in this block's tile order, and its tile t_at
             int64_t t_at = 0;
@@ -1815,6 +1830,8 @@ size_t refined_workspace_bytes(int64_t n, int d, int k) {
     b += 8 * (size_t)n + 4 * (size_t)n * BORUVKA_COL_CAP + 12 * (size_t)n;
     b += 12 * (size_t)n;  // row lower bounds (original order) and per-half screen bounds
     b += 8 * (size_t)(L.n_pad / 32);  // label ranges of gathered rows
+    if (n >= LIST_MIN_ROWS && L.n_tiles <= kMaxVisitTiles)  // balls, thresholds, lists of tiles
+        b += 2 * (size_t)L.n_qblocks * (4 * (size_t)d + 8 + (size_t)L.n_tiles + 2);
     return b;
 }
 
@@ -1916,19 +1933,22 @@ static int choose_operands(cuscan_ctx *ctx, RefinedBuffers &R, const float *x, i
 // attempts; its factor of two keeps data that passes (unit vectors of 128 features: half the
 // limit) on plain bf16.
 static int choose_operands_by_cells(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d, int d_pad,
-                                    int k, bool &tight, cudaStream_t s) {
+                                    int k, bool &tight, float &apart, cudaStream_t s) {
     RefinedBuffers &R = b.refined;
     float ca, cb, abs_c;
     error_coefficients(d, d_pad, FMT_BF16, 0.0f, ca, cb, abs_c);
     const double entries = 2.0 * KNN_LIST;
     const float gap = (float)(2.0 * (2.0 / d) * std::log(k < entries ? entries / k : 1.0));
     if (int rc = count_tight_rows(ctx, b, n, ca, gap, s)) return rc;
-    unsigned int words[4] = {0, 0, 0, 0};
+    unsigned int words[5] = {0, 0, 0, 0, 0};
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(words, R.norm_range.ptr, sizeof(words), cudaMemcpyDeviceToHost,
                                      s));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
     set_operands(R, d, words[2]);
     tight = !R.fp16 && (double)words[3] > TIGHT_START * (double)n;
+    float pairs;
+    memcpy(&pairs, &words[4], sizeof(pairs));
+    apart = (float)((double)pairs / ((double)n * (double)n));
     return CUSCAN_OK;
 }
 
@@ -1956,7 +1976,7 @@ struct QuerySet {
     float *rowlb = nullptr;  // one-sided Borůvka: per query row and half, the pair lower bound
 };
 
-template <int M, int MODE>
+template <int M, int MODE, bool LIST = false>
 static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64_t n, int d,
                       const float *core, const int32_t *label, const int32_t *chunk_lo,
                       const int32_t *chunk_hi, cudaStream_t s, float *debug_tile = nullptr,
@@ -1995,6 +2015,8 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
     P.stages = L.stages;
     P.stage_blocks = L.stage_blocks;
     P.cursor = as<unsigned long long>(R.cursor);
+    P.vis = reinterpret_cast<const uint16_t *>(R.vis.ptr);
+    P.vis_count = as<int32_t>(R.vis_count);
     // parts of at least 128 tiles in general: the start of a work item (A tile, pipeline fill) stays small
     // against its tiles, and the fits of a serving stream (under 32,768 rows) keep one CTA per
     // block, leaving the other SMs to the fits running beside them
@@ -2059,7 +2081,7 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
                   BORUVKA ? reinterpret_cast<int2 *>(P.rowcnt) : nullptr,
                   P.splits > 1 ? reinterpret_cast<float2 *>(P.rowlb) : nullptr, P.nq);
     CUSCAN_LAUNCH(ctx, "screen_columns_kernel");
-    auto kernel = screen_kernel<M, MODE>;
+    auto kernel = screen_kernel<M, MODE, LIST>;
     if (int rc = allow_dynamic_smem(ctx, kernel, L.smem)) return rc;
     const int64_t items = P.n_qblocks * P.splits;
     int64_t grid = items < ctx->sm_count ? items : ctx->sm_count;
@@ -2096,8 +2118,12 @@ static int knn_list_pass(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, co
     for (cudaEvent_t &e : R.screen_ev)
         if (!e) CUSCAN_CUDA(ctx, cudaEventCreate(&e));
     CUSCAN_CUDA(ctx, cudaEventRecord(R.screen_ev[0], s));
-    if (int rc = run_screen<M, MODE_KNN_LIST>(ctx, R, L, n, d, nullptr, nullptr, nullptr, nullptr, s))
-        return rc;
+    const int rc = R.listed
+                       ? run_screen<M, MODE_KNN_LIST, true>(ctx, R, L, n, d, nullptr, nullptr, nullptr,
+                                                            nullptr, s)
+                       : run_screen<M, MODE_KNN_LIST>(ctx, R, L, n, d, nullptr, nullptr, nullptr,
+                                                      nullptr, s);
+    if (rc) return rc;
     CUSCAN_CUDA(ctx, cudaEventRecord(R.screen_ev[1], s));
     R.screen_timed = true;
     const bool vec = rerank_vec(xs, d);
@@ -2121,17 +2147,24 @@ int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
                                      b.knn_dist_tmp);
     }
     RefinedBuffers &R = b.refined;
+    R.listed = false;
     Layout L;
     refined_layout(n, d, L);
     // 1, 2. rows in spatial order (b.perm, b.xp), and the screens' operands
     bool tight = false;
+    float apart = 0.0f;
     int rc = sort_by_cells(ctx, b, x, n, d, s);
-    if (!rc) rc = choose_operands_by_cells(ctx, b, n, d, L.d_pad, k, tight, s);
+    if (!rc) rc = choose_operands_by_cells(ctx, b, n, d, L.d_pad, k, tight, apart, s);
     if (rc) return rc;
     if (!R.range_ok)  // values large enough to overflow f32: the exact sweep decides alone
         return launch_exact_knn_fp32(ctx, x, n, x, n, d, k, 1, 0, 1, ids, dist, s, b.knn_ids_tmp,
                                      b.knn_dist_tmp);
     R.pivots_valid = true;
+    if (n >= LIST_MIN_ROWS && L.n_tiles <= kMaxVisitTiles && apart > LIST_MIN_APART) {
+        if ((rc = visit_lists(ctx, b, n, d, k, s)) && rc != CUSCAN_MEMORY) return rc;
+        R.listed = rc == CUSCAN_OK;  // without room for the lists every tile is visited
+        if (rc) clear_error(ctx);
+    }
     // the tightened operands: split bf16, or scaled fp16 for rows too wide to split
     auto tighten = [&]() {
         Layout Ls;
