@@ -39,44 +39,45 @@ __global__ void pivot_distances_kernel(const float *__restrict__ piv, int npiv, 
 }
 
 // Greedy tour of the pivots: from each to the nearest one not visited yet, so that the cells of
-// a cluster follow one another and few tiles straddle two clusters. One CTA, a thread per pivot;
-// a step is one row of the distance matrix and a block minimum. Also writes the pivots in tour
-// order, and the order.
+// a cluster follow one another and few tiles straddle two clusters. Also writes the pivots in tour
+// order, and the order. One CTA, a thread per pivot: a step is a serial chain, so the distances sit
+// in shared memory (the lower triangle, 130 KB) and a block minimum is two warp reductions around
+// one barrier: 32-bit keys of a distance's upper bits over the pivot's number. 256 pivots of 64
+// features take 69 us; with a row of the matrix read from L2 and a 64-bit shuffle minimum per
+// step they took 172 us.
+constexpr size_t tour_smem(int npiv) { return sizeof(float) * (size_t)npiv * (npiv - 1) / 2; }
 __global__ void __launch_bounds__(kMaxPivots)
     pivot_tour_kernel(const float *__restrict__ piv, const float *__restrict__ dist, int npiv, int d,
                       float *__restrict__ out, int32_t *__restrict__ tour) {
-    __shared__ unsigned long long best[2];
+    static_assert(kMaxPivots == 256, "a pivot's number takes the low byte of a key");
+    constexpr int WARPS = kMaxPivots / 32;
+    extern __shared__ float tri[];  // [i (i - 1) / 2 + j], j < i
+    __shared__ unsigned best[2][WARPS];
     __shared__ int order[kMaxPivots];
-    const int t = threadIdx.x, lane = t & 31;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+#pragma unroll 8
+    for (int i = 1; i < npiv; ++i)
+        if (t < i) tri[i * (i - 1) / 2 + t] = dist[i * npiv + t];
     bool open = t < npiv && t != 0;
-    if (t == 0) {
-        order[0] = 0;
-        best[0] = best[1] = ~0ull;
-    }
+    if (t == 0) order[0] = 0;
     __syncthreads();
     int at = 0;
     for (int s = 1; s < npiv; ++s) {
-        unsigned long long key = ~0ull;
+        unsigned key = ~0u;
         if (open) {
-            const float v = dist[at * npiv + t];
+            const int i = max(at, t), j = min(at, t);
+            const float v = tri[i * (i - 1) / 2 + j];
             // NaN and infinite distances come last, in index order
-            key = ((unsigned long long)__float_as_uint(v >= 0.0f ? v : CUSCAN_INF) << 32) | (unsigned)t;
+            key = (__float_as_uint(v >= 0.0f ? v : CUSCAN_INF) & ~255u) | (unsigned)t;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long u = __shfl_xor_sync(0xffffffffu, key, o);
-            key = u < key ? u : key;
-        }
-        if (lane == 0 && key != ~0ull) atomicMin(&best[s & 1], key);
-        __syncthreads();
-        at = (int)(uint32_t)best[s & 1];
+        key = __reduce_min_sync(0xffffffffu, key);
+        if (lane == 0) best[s & 1][warp] = key;
+        __syncthreads();  // the other buffer's readers are past it too
+        at = (int)(__reduce_min_sync(0xffffffffu, best[s & 1][lane % WARPS]) & 255u);
         if (t == at) open = false;
-        if (t == 0) {
-            order[s] = at;
-            best[(s + 1) & 1] = ~0ull;
-        }
-        __syncthreads();
+        if (t == 0) order[s] = at;
     }
+    __syncthreads();
     if (t < npiv) tour[t] = order[t];
     for (int64_t e = t; e < (int64_t)npiv * d; e += blockDim.x) {
         const int64_t p = e / d;
@@ -423,7 +424,8 @@ int sort_by_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, 
     CUSCAN_KERNEL(pick_pivots_kernel, (unsigned)ceil_div((int64_t)npiv * d, 256), 256, 0, s, x, n, d,
                   npiv, picked);
     CUSCAN_KERNEL(pivot_distances_kernel, npiv, 256, 0, s, picked, npiv, d, as<float>(R.pivot_d));
-    CUSCAN_KERNEL(pivot_tour_kernel, 1, kMaxPivots, 0, s, picked, as<float>(R.pivot_d), npiv, d,
+    if ((rc = allow_dynamic_smem(ctx, pivot_tour_kernel, tour_smem(kMaxPivots)))) return rc;
+    CUSCAN_KERNEL(pivot_tour_kernel, 1, kMaxPivots, tour_smem(npiv), s, picked, as<float>(R.pivot_d), npiv, d,
                   toured, pivot_tour(R, npiv));
     CUSCAN_LAUNCH(ctx, "cell pivots");
     if ((rc = launch_exact_knn_fp32(ctx, x, n, toured, npiv, d, 1, 0, 0, 1, as<int32_t>(R.cells),
