@@ -159,7 +159,7 @@ class HDBSCAN:
 
     # ---- validation (python/cuscan/hdbscan.py:275-364) ----
     @staticmethod
-    def _input_array(X):
+    def _input_array(X, copy=False):
         try:
             values = np.asarray(X)
         except (TypeError, ValueError) as error:
@@ -172,10 +172,13 @@ class HDBSCAN:
         if values.dtype == np.float32:
             # already the native rows: every finite value fits, so the general path's float64 copy
             # and its gathered finite values have nothing to find (4,096 x 64 rows: 510 us
-            # there, 33 us here). The result may be the caller's own memory.
+            # there, 33 us here). Without copy the result may be the caller's own memory.
             finite = np.isfinite(values)
             finite_rows = (np.ones(values.shape[0], bool) if finite.all() else finite.all(axis=1))
-            return np.ascontiguousarray(values), finite_rows
+            rows = np.ascontiguousarray(values)
+            if copy and np.may_share_memory(rows, values):
+                rows = rows.copy()
+            return rows, finite_rows
         try:
             values64 = np.asarray(values, dtype=np.float64)
         except (TypeError, ValueError, OverflowError) as error:
@@ -259,13 +262,12 @@ class HDBSCAN:
         if fit_params:
             raise NotImplementedError(f"fit parameter {next(iter(fit_params))!r} is not supported")
         self._validate_parameters()
-        x, finite_rows = self._input_array(X)
+        # the fitted state keeps the rows for its predictor
+        x, finite_rows = self._input_array(X, copy=True)
         if x.shape[1] == 0:
             raise ValueError("input must contain at least one feature")
         if not np.any(finite_rows):
             raise ValueError("X must contain at least one fully finite row")
-        if isinstance(X, np.ndarray) and np.may_share_memory(x, X):
-            x = x.copy()  # the fitted state keeps the rows for its predictor
         state = fit_hdbscan(x, finite_rows, **self._native_kwargs())
         self._fitted_state = state
         return self
