@@ -28,7 +28,9 @@ int debug_screen_tile(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t
                       int operands, float *out, float *rows_out, float *chunk_out,
                       float *scale_out, cudaStream_t s);
 int refined_operand_format(const ForestBuffers &b);
-size_t refined_workspace_bytes(int64_t n, int d, int k);
+size_t refined_workspace_bytes(int64_t n, int d, int k, bool lean);
+int64_t fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, int32_t precision, bool lean);
+void set_lean(cuscan_ctx *ctx, bool lean);
 
 // Every device buffer a context holds.
 static int workspace_buffers(FitWorkspace *f, Buffer **out) {
@@ -135,26 +137,40 @@ int cuscan_ctx_release_workspace(cuscan_ctx *ctx) {
     return CUSCAN_OK;
 }
 
-int64_t cuscan_fit_workspace_bytes(int64_t n, int32_t d, int32_t min_samples, int32_t precision) {
+}  // extern "C"
+
+// Upper bound of a fit's device memory. lean: of a fit on a context set lean (see set_lean).
+int64_t cuscan::fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, int32_t precision,
+                                    bool lean) {
     if (n < 2 || d <= 0 || min_samples <= 0) return 0;
     const size_t N = (size_t)n, D = (size_t)d;
     const size_t k = (size_t)((int64_t)min_samples < n - 1 ? min_samples : n - 1);
     size_t b = 4 * N * D + 8 * N * k + 5 * 4 * N;  // input copy, kNN lists, core/label/MST arrays
     b += 18 * 4 * N + 4 * N * D + 16 * N;          // forest arrays, sorted copy, 64-bit keys
     b += 2 * 4 * (N / 32 + 2) + 64 + sizeof(DevStatus) + 4 * (N / 1024 + 2);  // tiles, scan
-    // split-kNN partial lists, one list per query row of every CTA
-    b += 8 * k * simt::QT *
-         (size_t)simt::split_plan_max_ctas(kSMs, ceil_div(n, (int64_t)simt::QT));
+    // partial lists of split kNN sweeps, here and (in the same buffers) of the pruned sweep
+    size_t partials = 8 * k * (size_t)simt::split_max_rows(n, n);
     if (precision == CUSCAN_PRECISION_BF16_REFINED || precision == CUSCAN_PRECISION_FP16_REFINED)
-        b += refined_workspace_bytes(n, d, (int)k);
+        b += refined_workspace_bytes(n, d, (int)k, lean);
     else if (n >= 2048) {  // exact rounds over a row subset: bounds, flags, positions, counts
         b += 7 * 4 * N + 64;
         // rows in spatial order, bounds of their tiles, first thresholds
-        if (worth_pruning(n, n, d))
+        if (!lean && worth_pruning(n, n, d) && knn_pruned_shape(d, (int)k)) {
             b += cells_workspace_bytes(n, d) + 4 * TileBounds::PARTS * (N / simt::RT + 1) * (D + 1) +
-                 8 * (size_t)padded_queries(n) + (size_t)kPrunedPartials;
+                 8 * (size_t)padded_queries(n);
+            const size_t p = (size_t)pruned_partial_bytes(padded_queries(n), n, (int)k);
+            partials = p > partials ? p : partials;
+        }
     }
-    return (int64_t)b + (1 << 20);
+    return (int64_t)(b + partials) + (1 << 20);
+}
+
+void cuscan::set_lean(cuscan_ctx *ctx, bool lean) { ctx->fit->forest.refined.lean = lean; }
+
+extern "C" {
+
+int64_t cuscan_fit_workspace_bytes(int64_t n, int32_t d, int32_t min_samples, int32_t precision) {
+    return fit_workspace_bound(n, d, min_samples, precision, false);
 }
 
 const char *cuscan_last_error(const cuscan_ctx *ctx) { return ctx ? ctx->err : "null context"; }
@@ -311,7 +327,7 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
     b.refined.pivots_valid = false;
     b.refined.screen_timed = false;
 
-    const bool spatial = !refined && knn_pruned_shape(d, k) && worth_pruning(n, n, d);
+    bool spatial = !refined && !b.refined.lean && knn_pruned_shape(d, k) && worth_pruning(n, n, d);
     TileBounds bounds;
     CUSCAN_CUDA(ctx, cudaMemsetAsync(b.status, 0, sizeof(DevStatus), s));
     CUSCAN_CUDA(ctx, cudaEventRecord(ev[0], s));
@@ -322,18 +338,24 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
     else if (spatial) {
         // plain f32 in spatial order: every distance that is formed is the same, and tiles whose
         // every row is too far to matter are left out (here and in the rounds)
-        if ((rc = sort_by_cells(ctx, b, data, n, d, s))) return rc;
-        if ((rc = tile_bounds(ctx, as<float>(b.xp), n, d, b.refined.tile_centre,
-                              b.refined.tile_radius, bounds, s)))
-            return rc;
-        rc = ensure(ctx, b.refined.qorder, sizeof(int32_t) * padded_queries(n), "query order");
+        rc = sort_by_cells(ctx, b, data, n, d, s);
+        if (!rc)
+            rc = tile_bounds(ctx, as<float>(b.xp), n, d, b.refined.tile_centre,
+                             b.refined.tile_radius, bounds, s);
+        if (!rc)
+            rc = ensure(ctx, b.refined.qorder, sizeof(int32_t) * padded_queries(n), "query order");
         if (!rc) rc = order_positions(ctx, b, n, as<int32_t>(b.refined.qorder), s);
         if (!rc)
             rc = launch_knn_pruned(ctx, as<float>(b.xp), padded_queries(n), as<float>(b.xp), n, d, k,
                                    1, knn_ids, knn_sq, s, b.knn_ids_tmp, b.knn_dist_tmp,
                                    b.refined.thr0, bounds, as<int32_t>(b.perm),
                                    as<int32_t>(b.refined.qorder), as<int32_t>(b.perm));
-    } else
+        if (rc == CUSCAN_MEMORY) {  // no room for the order or the partial lists: the plain sweeps
+            clear_error(ctx);
+            spatial = false;
+        }
+    }
+    if (!refined && !spatial)
         rc = launch_exact_knn_fp32(ctx, data, n, data, n, d, k, 1, 0, 1, knn_ids, knn_sq, s,
                                    b.knn_ids_tmp, b.knn_dist_tmp);
     if (rc) return rc;

@@ -71,6 +71,22 @@ int visit_lists(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d, int k, cuda
 // themselves.
 bool knn_pruned_shape(int d, int k);
 constexpr int64_t kPrunedPartials = 256ll << 20;  // most bytes of partial lists
+// Parts of the reference tiles: a query tile among far rows visits every reference tile, one in a
+// cluster a few per cent of them, so the longest CTA sets the end of the launch. Parts of at least 32
+// tiles, 16 at most, within kPrunedPartials of partial lists (100,000 x 64: 16.3 ms in one part,
+// 11.1 ms in 16).
+inline int64_t pruned_parts(int64_t nq, int64_t nr, int k) {
+    const int64_t tiles = ceil_div(nr, (int64_t)simt::RT);
+    int64_t parts = tiles / 32 < 16 ? tiles / 32 : 16;
+    const int64_t room = kPrunedPartials / (8 * nq * k);
+    if (parts > room) parts = room;
+    return parts < 1 ? 1 : parts;
+}
+// Bytes of the partial lists: one part writes its results in place.
+inline int64_t pruned_partial_bytes(int64_t nq, int64_t nr, int k) {
+    const int64_t parts = pruned_parts(nq, nr, k);
+    return parts > 1 ? 8 * parts * nq * k : 0;
+}
 int launch_knn_pruned(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, int64_t nr,
                       int d, int k, int self, int32_t *ids, float *dist, cudaStream_t s,
                       Buffer &scratch_ids, Buffer &scratch_dist, Buffer &thr0,

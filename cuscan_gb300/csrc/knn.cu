@@ -709,7 +709,7 @@ void knn_split_plan(const cuscan_ctx *ctx, int64_t nq, int64_t nr, int64_t &spli
     // every part fills lists of its own: about 4 k merged pairs per row, against 384 d cycles per
     // tile (both per resident CTA)
     simt::split_plan(ctx->sm_count, ceil_div(nq, (int64_t)QT), nr, 2,
-                     1.0 + 2.0 * (double)k / (double)d, splits, chunk);
+                     1.0 + 2.0 * (double)k / (double)d, splits, chunk, simt::split_most(nq));
 }
 
 template <int L>
@@ -765,15 +765,8 @@ int run_knn_pruned(cuscan_ctx *ctx, const float *query, int64_t nq, const float 
     CUSCAN_LAUNCH(ctx, "knn_thresholds_kernel");
     prune.thr0 = as<float>(thr0);
     prune.thr_out = nullptr;
-    // A query tile among far rows visits every reference tile, one in a cluster a few per cent of
-    // them, so the longest CTA sets the end of the launch: parts of at least 32 tiles, 16 at most,
-    // within kPrunedPartials of partial lists (100,000 x 64: 16.3 ms in one part, 11.1 ms in 16).
-    const int64_t tiles = ceil_div(nr, (int64_t)RT);
-    int64_t splits = tiles / 32 < 16 ? tiles / 32 : 16;
-    const int64_t room = kPrunedPartials / (8 * nq * k);
-    if (splits > room) splits = room;
-    if (splits < 1) splits = 1;
-    const int64_t chunk = ceil_div(tiles, splits) * RT;
+    int64_t splits = pruned_parts(nq, nr, k);
+    const int64_t chunk = ceil_div(ceil_div(nr, (int64_t)RT), splits) * RT;
     splits = ceil_div(nr, chunk);
     const dim3 grid(qtiles, (unsigned)splits);
     if (splits == 1) {

@@ -52,6 +52,7 @@ struct cuscan_predictor {
 };
 
 namespace cuscan {
+int64_t predict_workspace_bound(const cuscan_predictor *p, int64_t m, bool lean);
 namespace {
 
 // Work (query rows x training rows x features) of a batch from which its search runs in spatial
@@ -68,8 +69,14 @@ void free_rows(cuscan_predictor &P) {
     P.bounds = TileBounds();
 }
 
-// The spatial copy of the training rows, when a batch of 4,096 queries would use it.
-int build_spatial(cuscan_ctx *ctx, cuscan_predictor &P) {
+bool searches_spatially(const cuscan_predictor &P, int64_t m) {
+    return P.bounds.centre && m >= kSpatialQueries &&
+           (double)m * (double)P.n_finite * (double)P.d >= kSpatialWork;
+}
+
+// The spatial copy of the training rows, when a batch of 4,096 queries would use it. Without room
+// for it the predictor searches its plain rows.
+int copy_spatial(cuscan_ctx *ctx, cuscan_predictor &P) {
     const int64_t n = P.n_finite;
     const int d = P.d;
     if (n < 2048 || !knn_pruned_shape(d, 2 * P.s) ||
@@ -91,6 +98,15 @@ int build_spatial(cuscan_ctx *ctx, cuscan_predictor &P) {
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(P.pivots.ptr, b.refined.pivots.ptr,
                                      sizeof(float) * P.npiv * d, cudaMemcpyDeviceToDevice, s));
     return tile_bounds(ctx, as<float>(P.rows), n, d, P.centre, P.radius, P.bounds, s);
+}
+int build_spatial(cuscan_ctx *ctx, cuscan_predictor &P) {
+    const int rc = copy_spatial(ctx, P);
+    if (rc != CUSCAN_MEMORY) return rc;
+    CUSCAN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // copies into the buffers freed here
+    for (Buffer *b : {&P.rows, &P.ids, &P.pivots, &P.centre, &P.radius}) release(*b);
+    P.bounds = TileBounds();
+    clear_error(ctx);
+    return CUSCAN_OK;
 }
 
 int invalid(cuscan_ctx *ctx, const std::string &msg) {
@@ -693,17 +709,25 @@ int cuscan_predictor_shape(const cuscan_predictor *p, int64_t *n_finite, int32_t
 }
 
 int64_t cuscan_predict_workspace_bytes(const cuscan_predictor *p, int64_t m) {
+    return predict_workspace_bound(p, m, false);
+}
+
+}  // extern "C"
+
+int64_t cuscan::predict_workspace_bound(const cuscan_predictor *p, int64_t m, bool lean) {
     if (!p || m <= 0) return 0;
     const int64_t k = 2 * (int64_t)p->s;
     // query rows, candidate ids and distances, split-search partial lists
-    int64_t split = 8 * k * simt::QT *
-                    simt::split_plan_max_ctas(kSMs, ceil_div(m, (int64_t)simt::QT));
-    const int64_t pruned = 16 * 8 * k * padded_queries(m);  // at most 16 parts
-    if (pruned > split) split = pruned < kPrunedPartials ? pruned : kPrunedPartials;
-    // queries in spatial order: cells, distances, order, first thresholds
-    return (int64_t)sizeof(float) * m * p->d + 8 * m * k + split + 16 * padded_queries(m) +
-           (1 << 20);
+    int64_t bytes = 8 * k * simt::split_max_rows(m, p->n_finite);
+    if (!lean && searches_spatially(*p, m)) {
+        const int64_t pruned = pruned_partial_bytes(padded_queries(m), p->n_finite, (int)k);
+        if (pruned > bytes) bytes = pruned;
+        bytes += 16 * padded_queries(m);  // cells, distances, order, first thresholds
+    }
+    return (int64_t)sizeof(float) * m * p->d + 8 * m * k + bytes + (1 << 20);
 }
+
+extern "C" {
 
 int cuscan_predictor_no_cluster_tree(const cuscan_predictor *p) {
     return p && p->node_id.empty() ? 1 : 0;
@@ -783,8 +807,8 @@ int predict_queries(cuscan_ctx *ctx, const cuscan_predictor *p, const float *que
     if (rc) return rc;
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(f->pred_q.ptr, queries, sizeof(float) * m * p->d,
                                      cudaMemcpyHostToDevice, s));
-    if (p->bounds.centre && m >= kSpatialQueries &&
-        (double)m * (double)p->n_finite * (double)p->d >= kSpatialWork) {
+    bool spatial = !f->forest.refined.lean && searches_spatially(*p, m);
+    if (spatial) {
         rc = ensure(ctx, f->pred_order, sizeof(int32_t) * padded_queries(m), "query order");
         if (!rc)
             rc = order_queries(ctx, f->forest, reinterpret_cast<const float *>(p->pivots.ptr), p->npiv,
@@ -796,7 +820,12 @@ int predict_queries(cuscan_ctx *ctx, const cuscan_predictor *p, const float *que
                                    f->op_knn_ids, f->op_knn_dist, f->forest.refined.thr0, p->bounds,
                                    reinterpret_cast<const int32_t *>(p->ids.ptr),
                                    as<int32_t>(f->pred_order), nullptr);
-    } else {
+        if (rc == CUSCAN_MEMORY) {  // no room for the order or the partial lists: the plain search
+            clear_error(ctx);
+            spatial = false;
+        }
+    }
+    if (!spatial) {
         rc = launch_exact_knn_fp32(ctx, as<float>(f->pred_q), m, p->train, p->n_finite, p->d, k, 0, 0,
                                    1, as<int32_t>(f->pred_ids), as<float>(f->pred_dist), s,
                                    f->op_knn_ids, f->op_knn_dist);

@@ -1808,9 +1808,12 @@ static bool refined_shape_ok(int64_t n, int d, int k) {
     return n >= 2048 && k <= 32 && refined_layout(n, d, L);
 }
 
-size_t refined_workspace_bytes(int64_t n, int d, int k) {
+// Rows wider than this run the exact sweeps on a lean context.
+constexpr int LEAN_MAX_FEATURES = 128;
+
+size_t refined_workspace_bytes(int64_t n, int d, int k, bool lean) {
     Layout L;
-    if (!refined_shape_ok(n, d, k) || !refined_layout(n, d, L)) return 0;
+    if ((lean && d > LEAN_MAX_FEATURES) || !refined_shape_ok(n, d, k) || !refined_layout(n, d, L)) return 0;
     constexpr size_t M = 32;
     // a bf16-refined fit may switch to split copies (twice the columns) when d <= 64
     const size_t copy_cols = (size_t)L.d_pad * (L.d_pad <= 64 ? 2 : 1);
@@ -1830,7 +1833,7 @@ size_t refined_workspace_bytes(int64_t n, int d, int k) {
     b += 8 * (size_t)n + 4 * (size_t)n * BORUVKA_COL_CAP + 12 * (size_t)n;
     b += 12 * (size_t)n;  // row lower bounds (original order) and per-half screen bounds
     b += 8 * (size_t)(L.n_pad / 32);  // label ranges of gathered rows
-    if (n >= LIST_MIN_ROWS && L.n_tiles <= kMaxVisitTiles)  // balls, thresholds, lists of tiles
+    if (!lean && n >= LIST_MIN_ROWS && L.n_tiles <= kMaxVisitTiles)  // balls, thresholds, lists of tiles
         b += 2 * (size_t)L.n_qblocks * (4 * (size_t)d + 8 + (size_t)L.n_tiles + 2);
     return b;
 }
@@ -2141,7 +2144,7 @@ static int knn_list_pass(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, co
 int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, int d, int k,
                        int32_t *ids, float *dist, cudaStream_t s, int64_t *refined_rows,
                        int64_t *fallback_rows, int64_t *rescreened_rows) {
-    if (!refined_shape_ok(n, d, k)) {
+    if (!refined_shape_ok(n, d, k) || (b.refined.lean && d > LEAN_MAX_FEATURES)) {
         // shapes outside the tensor-core tiling run the exact f32 sweep
         return launch_exact_knn_fp32(ctx, x, n, x, n, d, k, 1, 0, 1, ids, dist, s, b.knn_ids_tmp,
                                      b.knn_dist_tmp);
@@ -2160,7 +2163,7 @@ int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
         return launch_exact_knn_fp32(ctx, x, n, x, n, d, k, 1, 0, 1, ids, dist, s, b.knn_ids_tmp,
                                      b.knn_dist_tmp);
     R.pivots_valid = true;
-    if (n >= LIST_MIN_ROWS && L.n_tiles <= kMaxVisitTiles && apart > LIST_MIN_APART) {
+    if (!R.lean && n >= LIST_MIN_ROWS && L.n_tiles <= kMaxVisitTiles && apart > LIST_MIN_APART) {
         if ((rc = visit_lists(ctx, b, n, d, k, s)) && rc != CUSCAN_MEMORY) return rc;
         R.listed = rc == CUSCAN_OK;  // without room for the lists every tile is visited
         if (rc) clear_error(ctx);
@@ -2258,7 +2261,7 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
     const int32_t *perm = as<int32_t>(b.perm);
     unsigned long long *row_keys = as<unsigned long long>(b.row_keys);
     int32_t *clo = as<int32_t>(b.tile_lo), *chi = as<int32_t>(b.tile_hi);
-    if (!refined_shape_ok(n, d, 1))
+    if (!refined_shape_ok(n, d, 1) || (b.refined.lean && d > LEAN_MAX_FEATURES))
         return launch_candidates_fp32(ctx, xp, corep, labp, perm, n, d, row_keys, clo, chi, s);
     RefinedBuffers &R = b.refined;
     Layout L;

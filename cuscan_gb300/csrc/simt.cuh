@@ -219,11 +219,13 @@ __device__ __forceinline__ void sweep(const float *__restrict__ query, const int
 // taken, among those of at most eight waves (partial results grow with the splits). 10,007 x 64 candidates (157 query tiles
 // on 456 slots) took 787 us with at most 4 splits and take 562 us.
 inline void split_plan(int sm_count, int64_t query_tiles, int64_t nr, int64_t min_tiles,
-                       double start_tiles, int64_t &splits, int64_t &chunk) {
+                       double start_tiles, int64_t &splits, int64_t &chunk,
+                       int64_t limit = INT64_MAX) {
     const int64_t slots = (int64_t)CTAS_PER_SM * sm_count, tiles = ceil_div(nr, (int64_t)RT);
     if (query_tiles < 1) query_tiles = 1;
     int64_t most = ceil_div(8 * slots, query_tiles);
     if (most > ceil_div(tiles, min_tiles)) most = ceil_div(tiles, min_tiles);
+    if (most > limit) most = limit;
     splits = 1;
     double best = 0.0;
     for (int64_t s = 1; s <= most; ++s) {
@@ -239,9 +241,14 @@ inline void split_plan(int sm_count, int64_t query_tiles, int64_t nr, int64_t mi
     splits = ceil_div(nr, chunk);
     if (splits < 1) splits = 1;
 }
-// Most CTAs split_plan launches for a number of query tiles.
-inline int64_t split_plan_max_ctas(int64_t sm_count, int64_t query_tiles) {
-    return query_tiles + 8 * (int64_t)CTAS_PER_SM * sm_count;
+// Parts of a kNN sweep keep their partial lists within kSplitRows rows beyond the queries' own, and
+// have at least two tiles.
+constexpr int64_t kSplitRows = 512 * (int64_t)kSMs;
+inline int64_t split_most(int64_t nq) { return (kSplitRows + nq) / nq; }
+// Most rows of partial lists of up to nq queries against nr references.
+inline int64_t split_max_rows(int64_t nq, int64_t nr) {
+    const int64_t parts = nq * ceil_div(ceil_div(nr, (int64_t)RT), (int64_t)2);
+    return kSplitRows + nq < parts ? kSplitRows + nq : parts;
 }
 
 }  // namespace simt
