@@ -83,7 +83,8 @@ int cuscan_ctx_create(int device, cuscan_ctx **out) {
         }
     }
     ctx->fit = new FitWorkspace();
-    if (cudaMallocHost(&ctx->fit->host_status, sizeof(DevStatus)) != cudaSuccess) {
+    if (cudaMallocHost(&ctx->fit->host_status,
+                       sizeof(DevStatus) + sizeof(int) * FitWorkspace::kHostWords) != cudaSuccess) {
         cudaGetLastError();
         cuscan_ctx_destroy(ctx);
         return CUSCAN_MEMORY;

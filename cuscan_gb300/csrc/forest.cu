@@ -1130,7 +1130,7 @@ int forest_buffers(ForestBuffers &b, Buffer **out) {
                      &b.fill, &b.perm, &b.xp, &b.corep, &b.labp, &b.row_keys, &b.comp_keys,
                      &b.tile_lo, &b.tile_hi, &b.status_buf, &b.scan_tmp, &b.knn_ids_tmp,
                      &b.knn_dist_tmp, &r.xt, &r.pnorm, &r.mnorm, &r.tile_mmax, &r.tile_lo,
-                     &r.tile_hi, &r.cand_ids, &r.cand_lb, &r.fallback, &r.count, &r.error,
+                     &r.tile_hi, &r.cand_ids, &r.cand_lb, &r.fallback, &r.error,
                      &r.cbound, &r.rowcnt, &r.pivots, &r.cells, &r.cell_d, &r.absmax,
                      &r.qthr, &r.xq, &r.pq, &r.mq, &r.cand2, &r.rowcnt2, &r.fallback2,
                      &r.urow, &r.colcnt, &r.colbuf, &r.act_flag, &r.act_idx, &r.act_pos,

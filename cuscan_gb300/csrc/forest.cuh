@@ -12,7 +12,7 @@ struct DevStatus {
     double same_pairs;     // sum of squared component sizes entering the current round
     int err_kind;          // 0 ok, 1 numerical weight, 2 index out of range, 4 no progress
     unsigned int scan_ticket;  // blocks of the running scan that have finished (0 between scans)
-    int pad[2];
+    int row_counts[2];     // screened rounds: rows without a component bound, rows that can hold an edge
     double mst_weight;     // f64 total MST weight, written once after the last round
     // kept on the device by packed fits (no host read after every round): the seed's results,
     // rounds run and ordered cross pairs entering them
@@ -24,7 +24,7 @@ struct DevStatus {
 
 // Buffers of the bf16 screening path (refined.cu).
 struct RefinedBuffers {
-    Buffer xt, pnorm, mnorm, tile_mmax, tile_lo, tile_hi, cand_ids, cand_lb, fallback, count;
+    Buffer xt, pnorm, mnorm, tile_mmax, tile_lo, tile_hi, cand_ids, cand_lb, fallback;
     Buffer error, cbound, rowcnt, pivots, cells, cell_d, absmax;
     // sort_by_cells: pivot distances, per-cell scales, squared norms of the rows and their range
     Buffer pivot_d, cell_scale, rnorm, norm_range, key;
@@ -77,7 +77,7 @@ struct ForestBuffers {
 int forest_reserve(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d);
 void forest_release(ForestBuffers &b);
 // Every device buffer of the forest and of the bf16 screen (out may be null); returns the count.
-constexpr int kForestBufferCount = 78;
+constexpr int kForestBufferCount = 77;
 int forest_buffers(ForestBuffers &b, Buffer **out);
 // Whether a set of n points takes the one-CTA forest steps (fewer than 2048 points).
 bool forest_small(int64_t n);

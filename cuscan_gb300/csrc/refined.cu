@@ -33,6 +33,7 @@
 #include "cells.cuh"
 #include "common.cuh"
 #include "forest.cuh"
+#include "workspace.cuh"
 
 namespace cuscan {
 
@@ -1874,7 +1875,6 @@ static int prep(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, const float
     if (!rc) rc = ensure(ctx, R.tile_lo, sizeof(int32_t) * L.n_tiles, "tile labels");
     if (!rc) rc = ensure(ctx, R.tile_hi, sizeof(int32_t) * L.n_tiles, "tile labels");
     if (!rc) rc = ensure(ctx, R.error, sizeof(int) * SCREEN_STATUS_WORDS, "screen status");
-    if (!rc) rc = ensure(ctx, R.count, 16, "row counts");
     if (!rc) rc = ensure(ctx, R.cursor, 16, "tile cursor");
     if (!rc) rc = ensure(ctx, R.fallback, sizeof(int32_t) * n, "fallback rows");
     if (!rc) rc = ensure(ctx, R.qthr, sizeof(float) * n, "fallback thresholds");
@@ -1943,9 +1943,9 @@ static int choose_operands_by_cells(cuscan_ctx *ctx, ForestBuffers &b, int64_t n
     const double entries = 2.0 * KNN_LIST;
     const float gap = (float)(2.0 * (2.0 / d) * std::log(k < entries ? entries / k : 1.0));
     if (int rc = count_tight_rows(ctx, b, n, ca, gap, s)) return rc;
-    unsigned int words[5] = {0, 0, 0, 0, 0};
-    CUSCAN_CUDA(ctx, cudaMemcpyAsync(words, R.norm_range.ptr, sizeof(words), cudaMemcpyDeviceToHost,
-                                     s));
+    unsigned int *words = reinterpret_cast<unsigned int *>(ctx->fit->host_words());
+    CUSCAN_CUDA(ctx, cudaMemcpyAsync(words, R.norm_range.ptr, 5 * sizeof(unsigned int),
+                                     cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
     set_operands(R, d, words[2]);
     tight = !R.fp16 && (double)words[3] > TIGHT_START * (double)n;
@@ -2094,8 +2094,10 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
 }
 
 static int read_screen_status(cuscan_ctx *ctx, RefinedBuffers &R, cudaStream_t s, int &fallbacks) {
-    int status[SCREEN_STATUS_WORDS] = {0};
-    CUSCAN_CUDA(ctx, cudaMemcpyAsync(status, R.error.ptr, sizeof(status), cudaMemcpyDeviceToHost, s));
+    static_assert(SCREEN_STATUS_WORDS <= FitWorkspace::kHostWords, "pinned words");
+    int *status = ctx->fit->host_words();
+    CUSCAN_CUDA(ctx, cudaMemcpyAsync(status, R.error.ptr, sizeof(int) * SCREEN_STATUS_WORDS,
+                                     cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
     if (status[0])
         return fail(ctx, CUSCAN_BACKEND_UNAVAILABLE,
@@ -2286,7 +2288,7 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
     if (rc) return rc;
     CUSCAN_KERNEL(round_clear_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, as<uint32_t>(R.cbound),
                   as<int32_t>(R.colcnt), R.lb_valid ? nullptr : as<float>(R.rowlb),
-                  as<int32_t>(R.count), n);
+                  b.status->row_counts, n);
     R.lb_valid = true;
     CUSCAN_KERNEL(seed_bounds_kernel, (unsigned)ceil_div(n, 256), 256, 0, s, knn_ids, knn_sq, k,
                   core, label, n, as<uint32_t>(R.cbound));
@@ -2297,18 +2299,18 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
         return rc;
     CUSCAN_KERNEL(init_row_bounds_kernel, (unsigned)ceil_div(n, 256), 256, 0, s,
                   as<uint32_t>(R.cbound), labp, corep, as<float>(R.rowlb), perm, n,
-                  as<uint32_t>(R.urow), as<int>(R.count), as<int32_t>(R.act_flag));
+                  as<uint32_t>(R.urow), b.status->row_counts, as<int32_t>(R.act_flag));
     CUSCAN_LAUNCH(ctx, "init_row_bounds_kernel");
     if ((rc = scan_exclusive(ctx, b, as<int32_t>(R.act_flag), as<int32_t>(R.act_idx), n,
-                             as<int32_t>(R.count) + 1, s)))
+                             b.status->row_counts + 1, s)))
         return rc;
-    int counts[2] = {0, 0};  // rows without a component bound, rows that can hold an edge
-    double same_pairs = 0.0;
-    CUSCAN_CUDA(ctx, cudaMemcpyAsync(counts, R.count.ptr, sizeof(counts), cudaMemcpyDeviceToHost, s));
-    CUSCAN_CUDA(ctx, cudaMemcpyAsync(&same_pairs, &b.status->same_pairs, sizeof(double),
+    const DevStatus *hs = ctx->fit->host_status;
+    CUSCAN_CUDA(ctx, cudaMemcpyAsync(ctx->fit->host_status, b.status, sizeof(DevStatus),
                                      cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
-    const int64_t active = counts[1];
+    const int unbounded = hs->row_counts[0];
+    const double same_pairs = hs->same_pairs;
+    const int64_t active = hs->row_counts[1];
     // Gathered blocks look for tiles of their own component only where components hold a fair share
     // of the pairs: the look costs every tile two loads in each role (4 % of a round at 500,000 x 128,
     // where 1 to 2 % of the tiles could go; at 100,000 x 64 rounds 3 and 4 run 12 % and 51 % fewer
@@ -2325,7 +2327,7 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
     //    known bound (rows of components without a bound draw many appends there); it is used
     //    only when nearly every row is screened.
     const bool sym = n >= SYM_MIN_ROWS &&
-                     (double)counts[0] <= SYM_UNBOUNDED_MAX * (double)n &&
+                     (double)unbounded <= SYM_UNBOUNDED_MAX * (double)n &&
                      (double)active > SYM_ACTIVE_MIN * (double)n;
     const bool subset = !sym && active < n;
     CUSCAN_LAUNCH(ctx, "component bounds");
@@ -2416,7 +2418,6 @@ int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, i
     RefinedBuffers &R = b.refined;
     int rc = ensure(ctx, R.cbound, sizeof(uint32_t) * n, "component bounds");
     if (!rc) rc = ensure(ctx, R.urow, sizeof(uint32_t) * n, "row bounds");
-    if (!rc) rc = ensure(ctx, R.count, 16, "row counts");
     if (!rc) rc = ensure(ctx, R.act_flag, sizeof(int32_t) * n, "active rows");
     if (!rc) rc = ensure(ctx, R.act_idx, sizeof(int32_t) * n, "active rows");
     if (!rc) rc = ensure(ctx, R.act_pos, sizeof(int32_t) * n, "active rows");
@@ -2435,16 +2436,17 @@ int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, i
     if (bounds &&
         (rc = pivot_component_bounds(ctx, b, n, core, label, as<uint32_t>(R.cbound), s)))
         return rc;
-    CUSCAN_CUDA(ctx, cudaMemsetAsync(R.count.ptr, 0, 2 * sizeof(int), s));
+    CUSCAN_CUDA(ctx, cudaMemsetAsync(b.status->row_counts, 0, 2 * sizeof(int), s));
     CUSCAN_KERNEL(init_row_bounds_kernel, (unsigned)ceil_div(n, 256), 256, 0, s,
                   as<uint32_t>(R.cbound), labp, corep, as<float>(R.rowlb), perm, n,
-                  as<uint32_t>(R.urow), as<int>(R.count), as<int32_t>(R.act_flag));
+                  as<uint32_t>(R.urow), b.status->row_counts, as<int32_t>(R.act_flag));
     CUSCAN_LAUNCH(ctx, "component bounds");
     if ((rc = scan_exclusive(ctx, b, as<int32_t>(R.act_flag), as<int32_t>(R.act_idx), n,
-                             as<int32_t>(R.count) + 1, s)))
+                             b.status->row_counts + 1, s)))
         return rc;
-    int counts[2] = {0, 0};  // rows without a component bound, rows that can hold an edge
-    CUSCAN_CUDA(ctx, cudaMemcpyAsync(counts, R.count.ptr, sizeof(counts), cudaMemcpyDeviceToHost, s));
+    int *counts = ctx->fit->host_status->row_counts;
+    CUSCAN_CUDA(ctx, cudaMemcpyAsync(counts, b.status->row_counts, 2 * sizeof(int),
+                                     cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
     const int64_t active = counts[1];
     const int32_t *qpos = nullptr;

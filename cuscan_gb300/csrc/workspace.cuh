@@ -18,7 +18,11 @@ struct FitWorkspace {
     Buffer op_keys, op_tiles_lo, op_tiles_hi, op_partials, op_knn_ids, op_knn_dist;
     // approximate_predict queries, their spatial order and their candidates
     Buffer pred_q, pred_order, pred_ids, pred_dist;
-    DevStatus *host_status = nullptr;              // pinned
+    // pinned: the status of the forest, then up to kHostWords words of the running screen (a copy
+    // to pageable memory goes through the driver's own staging and waits for it)
+    DevStatus *host_status = nullptr;
+    static constexpr int kHostWords = 8;
+    int *host_words() { return reinterpret_cast<int *>(host_status + 1); }
     cudaEvent_t ev[6] = {};
     PackWorkspace *pack = nullptr;                 // created by the first packed call
     // per Borůvka round of the last fit: query rows screened, tensor-core tiles run, candidate
