@@ -158,7 +158,7 @@ int64_t cuscan::fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, i
         // rows in spatial order, bounds of their tiles, first thresholds
         if (!lean && worth_pruning(n, n, d) && knn_pruned_shape(d, (int)k)) {
             b += cells_workspace_bytes(n, d) + 4 * TileBounds::PARTS * (N / simt::RT + 1) * (D + 1) +
-                 8 * (size_t)padded_queries(n);
+                 8 * (size_t)padded_queries(n) + mask_bytes(n);
             const size_t p = (size_t)pruned_partial_bytes(padded_queries(n), n, (int)k);
             partials = p > partials ? p : partials;
         }

@@ -16,6 +16,7 @@
 #include "cells.cuh"
 #include "forest.cuh"
 #include "simt.cuh"
+#include "workspace.cuh"
 
 namespace cuscan {
 namespace {
@@ -71,7 +72,77 @@ constexpr size_t kCandSmem =
 struct CandPrune {
     TileBounds bounds;
     const uint32_t *cbound;
+    const uint32_t *masks;  // candidate_masks_kernel, or null
+    int words;              // of a query tile's mask
 };
+
+// Masks of the tiles that 64 query rows (tile blockIdx.x) have to visit: some row's distance to some
+// half of the tile, by the ball around it, does not exceed the bound of the row's component. The
+// rows themselves bound far better than the balls around them that the sweep walks with: in d
+// features a row's offset in its cluster is nearly at right angles to the other cluster, so its
+// centre distance is about sqrt(D^2 + r^2) where the balls leave D - r. At 100,000 x 64 (50
+// clusters, noise) the rounds between clusters visit 41 % of the tiles instead of 78 %.
+// A thread per half tile, the rows transposed in shared memory; 37 us per round at 20,011 x 32, where
+// the sweeps fell from 2.26 to 1.66 ms over three rounds.
+constexpr int MASK_THREADS = 256;
+constexpr size_t mask_smem(int d, int64_t words) {
+    return sizeof(float) * QT * (size_t)(d + 1) + sizeof(uint32_t) * (size_t)words;
+}
+__global__ void __launch_bounds__(MASK_THREADS, 2)
+    candidate_masks_kernel(const float *__restrict__ data, const int32_t *__restrict__ labels, int d,
+                           const int32_t *__restrict__ qmap, int64_t nq, const TileBounds B,
+                           const uint32_t *__restrict__ cbound, int words,
+                           uint32_t *__restrict__ masks) {
+    extern __shared__ __align__(16) float rows_t[];  // [d][QT], the rows' bounds, the mask
+    float *thr = rows_t + (size_t)QT * d;
+    uint32_t *bits = reinterpret_cast<uint32_t *>(thr + QT);
+    const int tid = threadIdx.x;
+    const int64_t q0 = (int64_t)blockIdx.x * QT;
+    // rows past the end repeat the first, with a bound that nothing meets
+    for (int e = tid; e < QT * d; e += MASK_THREADS) {
+        const int r = e / d, f = e - r * d;
+        const int64_t qi = q0 + r < nq ? q0 + r : q0;
+        rows_t[f * QT + r] = data[(qmap ? (int64_t)qmap[qi] : qi) * d + f];
+    }
+    if (tid < QT) {
+        const int64_t qi = q0 + tid;
+        thr[tid] = qi < nq ? __uint_as_float(cbound[labels[qmap ? (int64_t)qmap[qi] : qi]])
+                           : -CUSCAN_INF;
+    }
+    for (int w = tid; w < words; w += MASK_THREADS) bits[w] = 0;
+    __syncthreads();
+    for (int64_t ball = tid; ball < B.stride; ball += MASK_THREADS) {
+        const float radius = B.radius[ball];
+        if (!(radius >= 0.0f)) continue;  // an empty half
+        bool visit = false;
+#pragma unroll 1
+        for (int g = 0; g < QT && !visit; g += 32) {
+            float sq[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) sq[i] = 0.0f;
+            const float *centre = B.centre + ball;
+            for (int f = 0; f < d; ++f) {
+                const float c = *centre;
+                centre += B.stride;
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {
+                    const float4 q = *reinterpret_cast<const float4 *>(rows_t + f * QT + g + i);
+                    const float t0 = q.x - c, t1 = q.y - c, t2 = q.z - c, t3 = q.w - c;
+                    sq[i] = __fmaf_rn(t0, t0, sq[i]);
+                    sq[i + 1] = __fmaf_rn(t1, t1, sq[i + 1]);
+                    sq[i + 2] = __fmaf_rn(t2, t2, sq[i + 2]);
+                    sq[i + 3] = __fmaf_rn(t3, t3, sq[i + 3]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) visit |= !(pruned_bound(sq[i], radius) > thr[g + i]);
+        }
+        const int64_t t = ball % B.tiles;
+        if (visit) atomicOr(&bits[t >> 5], 1u << (int)(t & 31));
+    }
+    __syncthreads();
+    for (int w = tid; w < words; w += MASK_THREADS) masks[(int64_t)blockIdx.x * words + w] = bits[w];
+}
 
 // One CTA: 64 query rows [q0, q0 + 64) against rows [r_begin, r_end) (r_begin a multiple of the
 // reference tile); each query's cheapest cross-component key is folded into row_keys with
@@ -115,6 +186,7 @@ __device__ __forceinline__ void candidates_block(
     if constexpr (PRUNE) {
         simt::query_balls(sh.balls, data, sh.row, d);
         walk.balls = &sh.balls;
+        walk.mask = prune.masks ? prune.masks + (q0 / QT) * prune.words : nullptr;
     }
     const int32_t qlo = sh.q_range[0];
     const bool q_uniform = qlo == sh.q_range[1];
@@ -433,9 +505,24 @@ int launch_candidates_fp32(cuscan_ctx *ctx, const float *data, const float *core
     const dim3 grid((unsigned)qtiles, (unsigned)splits);
     if (bounds) {
         if (int rc = allow_dynamic_smem(ctx, candidates_pruned_kernel, kCandSmem)) return rc;
+        CandPrune prune{*bounds, cbound, nullptr, (int)mask_words(n)};
+        Buffer &masks = ctx->fit->forest.refined.masks;
+        if (const size_t bytes = mask_bytes(n)) {
+            const size_t smem = mask_smem(d, prune.words);
+            int rc = ensure(ctx, masks, bytes, "tile masks");
+            if (!rc) rc = allow_dynamic_smem(ctx, candidate_masks_kernel, smem);
+            if (rc && rc != CUSCAN_MEMORY) return rc;
+            if (rc) {  // no room: the balls alone
+                clear_error(ctx);
+            } else {
+                prune.masks = as<uint32_t>(masks);
+                CUSCAN_KERNEL(candidate_masks_kernel, (unsigned)qtiles, MASK_THREADS, smem, s, data,
+                              labels, d, qmap, nq, *bounds, cbound, prune.words,
+                              as<uint32_t>(masks));
+            }
+        }
         CUSCAN_KERNEL(candidates_pruned_kernel, grid, simt::THREADS, kCandSmem, s, data, core_sq,
-                      labels, ids, n, d, tile_lo, tile_hi, chunk, row_keys, qmap, nq,
-                      CandPrune{*bounds, cbound});
+                      labels, ids, n, d, tile_lo, tile_hi, chunk, row_keys, qmap, nq, prune);
         CUSCAN_LAUNCH(ctx, "candidates_pruned_kernel");
         return CUSCAN_OK;
     }

@@ -63,6 +63,16 @@ int tile_bounds(cuscan_ctx *ctx, const float *x, int64_t n, int d, Buffer &centr
 constexpr int64_t kMaxVisitTiles = 8192;  // 2,097,152 rows: 268 MB of lists
 int visit_lists(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d, int k, cudaStream_t s);
 
+// Masks of the tiles that the pruned candidate sweeps may visit: a bit per 128-row tile for every 64
+// query rows, up to kMaxMaskTiles tiles.
+constexpr int64_t kMaxMaskTiles = 16384;  // 2,097,152 rows: 67 MB of masks
+inline int64_t mask_words(int64_t n) { return ceil_div(ceil_div(n, (int64_t)simt::RT), (int64_t)32); }
+inline size_t mask_bytes(int64_t n) {
+    return ceil_div(n, (int64_t)simt::RT) > kMaxMaskTiles
+               ? 0
+               : sizeof(uint32_t) * (size_t)(ceil_div(n, (int64_t)simt::QT) * mask_words(n));
+}
+
 // Exact kNN of query rows against a spatially ordered set (knn.cu): squared distances, the rows
 // and order of launch_exact_knn_fp32, every tile that cannot hold a neighbour left out. ref_ids
 // maps reference positions to the ids that order ties and leave in `ids` (null: positions). Entry i
@@ -180,10 +190,13 @@ __device__ __forceinline__ void centre_distances(float (&sq)[BALLS], const Query
 // time, one per lane: 8 d multiply-adds per tile against the 8,192 d of the tile itself. The
 // thresholds only fall, so a tile left out once stays out. Called at the same points by every
 // warp, between barriers that keep the thresholds still, so that all warps walk alike.
+// mask: tiles to leave out in any case (a clear bit per tile), null for none.
 struct PrunedWalk {
     const QueryBalls *balls;
     int64_t window = -1;  // first tile of the bounds in lb
     float lb[BALLS];      // this lane's tile, by query ball
+    const uint32_t *mask = nullptr;
+    uint32_t word = ~0u;  // the mask of the window
 
     __device__ __forceinline__ int64_t next(const TileBounds &B, int d, int64_t t, int64_t t_end,
                                             const float *thr) {
@@ -200,6 +213,11 @@ struct PrunedWalk {
         while (t < t_end) {
             const int64_t base = t & ~(int64_t)31;
             if (base != window) {
+                if (mask && !(word = mask[base >> 5])) {
+                    window = -1;
+                    t = base + 32;
+                    continue;
+                }
                 window = base;
                 const int64_t mine = base + lane < B.tiles ? base + lane : B.tiles - 1;
 #pragma unroll
@@ -218,7 +236,7 @@ struct PrunedWalk {
 #pragma unroll
             for (int q = 0; q < BALLS; ++q) near |= !(lb[q] > worst[q]);
             const unsigned visit =
-                __ballot_sync(0xffffffffu, near) & (0xffffffffu << (int)(t - base));
+                __ballot_sync(0xffffffffu, near) & word & (0xffffffffu << (int)(t - base));
             if (visit) {
                 const int64_t to = base + __ffs(visit) - 1;
                 return to < t_end ? to : t_end;

@@ -1137,7 +1137,7 @@ int forest_buffers(ForestBuffers &b, Buffer **out) {
                      &r.rowlb, &r.lbtmp, &r.cursor, &r.colp, &r.colc, &r.cmin, &r.pivot_d,
                      &r.cell_scale, &r.tile_centre, &r.tile_radius, &r.thr0, &r.qorder,
                      &r.rnorm, &r.norm_range, &r.key, &r.qchunk_lo, &r.qchunk_hi,
-                     &r.ball_thr, &r.vis, &r.vis_count};
+                     &r.masks, &r.ball_thr, &r.vis, &r.vis_count};
     static_assert(sizeof(all) / sizeof(all[0]) == kForestBufferCount, "buffer list");
     const int count = (int)(sizeof(all) / sizeof(all[0]));
     if (out)

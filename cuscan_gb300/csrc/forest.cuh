@@ -30,6 +30,7 @@ struct RefinedBuffers {
     Buffer pivot_d, cell_scale, rnorm, norm_range, key;
     // pruned sweeps: tile bounds, first thresholds, padded query order
     Buffer tile_centre, tile_radius, thr0, qorder;
+    Buffer masks;                     // pruned candidate sweeps: tiles of every query tile
     Buffer ball_thr, vis, vis_count;  // kNN screens over lists of tiles: thresholds, lists, lengths
     Buffer qthr, xq, pq, mq, cand2, rowcnt2, fallback2;  // threshold re-screen of kNN rows
     Buffer urow, colcnt, colbuf;  // symmetric Borůvka: row bounds, column-side buffers
@@ -77,7 +78,7 @@ struct ForestBuffers {
 int forest_reserve(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d);
 void forest_release(ForestBuffers &b);
 // Every device buffer of the forest and of the bf16 screen (out may be null); returns the count.
-constexpr int kForestBufferCount = 77;
+constexpr int kForestBufferCount = 78;
 int forest_buffers(ForestBuffers &b, Buffer **out);
 // Whether a set of n points takes the one-CTA forest steps (fewer than 2048 points).
 bool forest_small(int64_t n);
