@@ -1804,17 +1804,20 @@ static bool refined_layout(int64_t n, int d, Layout &L, bool split = false) {
     return true;
 }
 
+// Shapes beyond these run the exact sweeps on a lean context.
+constexpr int LEAN_MAX_FEATURES = 128;
+constexpr int SCREEN_MAX_K = 32;  // longer lists run the exact kNN sweep, and screened rounds
+static bool lean_exact(int d, int k) { return d > LEAN_MAX_FEATURES || k > SCREEN_MAX_K; }
+
 static bool refined_shape_ok(int64_t n, int d, int k) {
     Layout L;
-    return n >= 2048 && k <= 32 && refined_layout(n, d, L);
+    return n >= 2048 && k <= SCREEN_MAX_K && refined_layout(n, d, L);
 }
 
-// Rows wider than this run the exact sweeps on a lean context.
-constexpr int LEAN_MAX_FEATURES = 128;
 
 size_t refined_workspace_bytes(int64_t n, int d, int k, bool lean) {
     Layout L;
-    if ((lean && d > LEAN_MAX_FEATURES) || !refined_shape_ok(n, d, k) || !refined_layout(n, d, L)) return 0;
+    if ((lean && lean_exact(d, k)) || !refined_shape_ok(n, d, 1) || !refined_layout(n, d, L)) return 0;
     constexpr size_t M = 32;
     // a bf16-refined fit may switch to split copies (twice the columns) when d <= 64
     const size_t copy_cols = (size_t)L.d_pad * (L.d_pad <= 64 ? 2 : 1);
@@ -1825,10 +1828,11 @@ size_t refined_workspace_bytes(int64_t n, int d, int k, bool lean) {
     b += 2 * 4 * (size_t)n * 2 * M;                  // candidate ids and bounds (two lists of M)
     b += sizeof(uint32_t) * (size_t)n + 2 * sizeof(int32_t) * (size_t)n;  // cbound, rowcnt
     b += cells_workspace_bytes(n, d);
-    // threshold re-screen of inconclusive kNN rows (at most all n): thresholds, tiles, norms,
-    // candidates, counts, fallback list
-    b += 4 * (size_t)n + (size_t)L.n_pad * copy_cols * 2 + 2 * sizeof(float) * (size_t)L.n_pad;
-    b += 4 * (size_t)n * 2 * KNN_CAP + 8 * (size_t)n + 4 * (size_t)n;
+    // gathered query rows (subset rounds, threshold re-screen): tiles and norms
+    b += (size_t)L.n_pad * copy_cols * 2 + 2 * sizeof(float) * (size_t)L.n_pad;
+    // threshold re-screen of inconclusive kNN rows (at most all n): thresholds, candidates, counts,
+    // fallback list
+    if (k <= SCREEN_MAX_K) b += 4 * (size_t)n + 4 * (size_t)n * 2 * KNN_CAP + 8 * (size_t)n + 4 * (size_t)n;
     // symmetric Borůvka: row bounds, column-side counts and candidates; subset rounds: flags,
     // their scan and the gathered positions
     b += 8 * (size_t)n + 4 * (size_t)n * BORUVKA_COL_CAP + 12 * (size_t)n;
@@ -2146,7 +2150,7 @@ static int knn_list_pass(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, co
 int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, int d, int k,
                        int32_t *ids, float *dist, cudaStream_t s, int64_t *refined_rows,
                        int64_t *fallback_rows, int64_t *rescreened_rows) {
-    if (!refined_shape_ok(n, d, k) || (b.refined.lean && d > LEAN_MAX_FEATURES)) {
+    if (!refined_shape_ok(n, d, k) || (b.refined.lean && lean_exact(d, k))) {
         // shapes outside the tensor-core tiling run the exact f32 sweep
         return launch_exact_knn_fp32(ctx, x, n, x, n, d, k, 1, 0, 1, ids, dist, s, b.knn_ids_tmp,
                                      b.knn_dist_tmp);
@@ -2263,7 +2267,7 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
     const int32_t *perm = as<int32_t>(b.perm);
     unsigned long long *row_keys = as<unsigned long long>(b.row_keys);
     int32_t *clo = as<int32_t>(b.tile_lo), *chi = as<int32_t>(b.tile_hi);
-    if (!refined_shape_ok(n, d, 1) || (b.refined.lean && d > LEAN_MAX_FEATURES))
+    if (!refined_shape_ok(n, d, 1) || (b.refined.lean && lean_exact(d, k)))
         return launch_candidates_fp32(ctx, xp, corep, labp, perm, n, d, row_keys, clo, chi, s);
     RefinedBuffers &R = b.refined;
     Layout L;

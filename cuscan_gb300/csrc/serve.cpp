@@ -43,8 +43,8 @@
 #include "cuscan_gb300.h"
 
 // Library-internal: bounds and execution of a request in less device memory (without the spatial
-// order of plain fits and of query batches, the tile lists and the screens wider than 128
-// features). A request whose full bound exceeds the server's budget runs so when that fits.
+// order of plain fits and of query batches, the tile lists and the screens of more than 128
+// features or 32 neighbours). A request whose full bound exceeds the server's budget runs so when that fits.
 namespace cuscan {
 int64_t fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, int32_t precision, bool lean);
 int64_t predict_workspace_bound(const cuscan_predictor *p, int64_t m, bool lean);

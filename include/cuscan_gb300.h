@@ -459,7 +459,9 @@ int cuscan_ctx_release_workspace(cuscan_ctx *ctx);
  * own CUDA stream, workspace and host thread, as slots and device memory free up: the sum over
  * slots of max(workspace held, cuscan_fit_workspace_bytes of the running request) stays
  * within `budget_bytes`. Idle slots release retained workspace when the head request needs
- * the room; a request whose own bound exceeds the budget finishes at once with CUSCAN_MEMORY.
+ * the room. A request whose own bound exceeds the budget runs without the spatial order of plain
+ * fits and batches, the tile lists and the screens of more than 128 features or 32 neighbours when
+ * it fits so, and finishes at once with CUSCAN_MEMORY otherwise.
  * The fits of different slots overlap on the device. A request's result equals that of the
  * same fit run alone.
  *

@@ -15,7 +15,8 @@ def bound(n, d, min_samples, precision):
 
 
 # (n, d): plain fits in spatial order, screens of wide rows, tile lists
-CASES = [(10_007, 101, _lib.PRECISION_PLAIN, "fp32"), (3001, 200, _lib.PRECISION_BF16_REFINED, "bf16_refined"),
+CASES = [(10_007, 101, _lib.PRECISION_PLAIN, "fp32"),
+         (3001, 200, _lib.PRECISION_BF16_REFINED, "bf16_refined"),
          (16_500, 40, _lib.PRECISION_FP16_REFINED, "fp16_refined")]
 
 
@@ -41,6 +42,16 @@ def test_lean_fits_equal_full_ones(n, d, code, name):
     lean, full = results
     np.testing.assert_array_equal(lean["labels"], full["labels"])
     np.testing.assert_array_equal(lean["probabilities"], full["probabilities"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,d,k", [(2048, 8, 5), (10_007, 101, 33), (16_500, 40, 10), (20_011, 32, 50),
+                                   (9001, 200, 15)])
+@pytest.mark.parametrize("code", [_lib.PRECISION_PLAIN, _lib.PRECISION_BF16_REFINED])
+def test_the_bound_holds_for_every_route(n, d, k, code):
+    ctx = cg.Context(0)
+    ctx.fit_core(synthetic.gaussian_mixture(n, d, 9, seed=n), k, code)
+    assert cg.load().cuscan_ctx_reserved_bytes(ctx.handle) <= bound(n, d, k, code)
 
 
 @pytest.mark.gpu
