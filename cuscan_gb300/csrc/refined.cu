@@ -1983,6 +1983,27 @@ struct QuerySet {
     float *rowlb = nullptr;  // one-sided Borůvka: per query row and half, the pair lower bound
 };
 
+// Parts of every query block's tile order in a one-sided Borůvka screen. The blocks run in waves of one
+// per SM; a last wave that is nearly empty, or a round of few blocks, leaves SMs idle. The count is the
+// one whose waves take the least, a part costing its tiles and PART_START more (its A tile, the
+// pipeline's start, bounds that start anew), with parts of at least PART_MIN tiles. Splitting only
+// rounds of fewer blocks than SMs, a 50,000 x 128 fit took 3.96 ms and now takes 3.63 ms, 9,001 x 32
+// 1.41 -> 1.34 ms, 100,000 x 64 8.90 -> 8.58 ms; a serving stream's p99 stays (12.8 and 12.1 ms).
+constexpr int64_t PART_MIN = 16, PART_START = 6;
+static int screen_parts(int64_t blocks, int64_t tiles, int64_t sms) {
+    int64_t most = tiles / PART_MIN < 16 ? tiles / PART_MIN : 16;
+    if (blocks > 8 * sms) most = 1;  // the last wave is a small share
+    int64_t best = 1, least = 0;
+    for (int64_t s = 1; s <= most || s == 1; ++s) {
+        const int64_t cost = ceil_div(blocks * s, sms) * (ceil_div(tiles, s) + PART_START);
+        if (s == 1 || cost < least) {
+            least = cost;
+            best = s;
+        }
+    }
+    return (int)best;
+}
+
 template <int M, int MODE, bool LIST = false>
 static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64_t n, int d,
                       const float *core, const int32_t *label, const int32_t *chunk_lo,
@@ -2024,20 +2045,9 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
     P.cursor = as<unsigned long long>(R.cursor);
     P.vis = reinterpret_cast<const uint16_t *>(R.vis.ptr);
     P.vis_count = as<int32_t>(R.vis_count);
-    // parts of at least 128 tiles in general: the start of a work item (A tile, pipeline fill) stays small
-    // against its tiles, and the fits of a serving stream (under 32,768 rows) keep one CTA per
-    // block, leaving the other SMs to the fits running beside them
     P.splits = 1;
-    if (MODE == MODE_BORUVKA && P.n_qblocks > 0 && P.n_qblocks < ctx->sm_count && !debug_tile) {
-        int64_t per = ctx->sm_count / P.n_qblocks;
-        if (per > P.n_tiles / 128) per = P.n_tiles / 128;
-        // a round of few blocks may take a quarter of the SMs in parts of at least 16 tiles
-        // (950 rows of 50,000 x 128: eight CTAs took 0.77 ms for the round, in four parts 0.43 ms)
-        int64_t few = ctx->sm_count / (4 * P.n_qblocks);
-        if (few > P.n_tiles / 16) few = P.n_tiles / 16;
-        if (per < few) per = few;
-        P.splits = (int)(per < 1 ? 1 : per < 16 ? per : 16);
-    }
+    if (MODE == MODE_BORUVKA && P.n_qblocks > 0 && !debug_tile)
+        P.splits = screen_parts(P.n_qblocks, P.n_tiles, ctx->sm_count);
     float ca, cb, abs_c;
     error_coefficients(d, L.d_pad, operand_format(R), R.fp16 ? R.amax_value * R.scale : R.amax_value, ca, cb, abs_c);
     P.c_a = ca;
