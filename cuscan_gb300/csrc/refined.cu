@@ -1988,8 +1988,9 @@ struct QuerySet {
 // one whose waves take the least, a part costing its tiles and PART_START more (its A tile, the
 // pipeline's start, bounds that start anew), with parts of at least PART_MIN tiles. Splitting only
 // rounds of fewer blocks than SMs, a 50,000 x 128 fit took 3.96 ms and now takes 3.63 ms, 9,001 x 32
-// 1.41 -> 1.34 ms, 100,000 x 64 8.90 -> 8.58 ms; a serving stream's p99 stays (12.8 and 12.1 ms).
-constexpr int64_t PART_MIN = 16, PART_START = 6;
+// 1.41 -> 1.27 ms, 100,000 x 64 8.90 -> 8.58 ms (parts of 16 tiles and a start of 6: 1.34 ms at 9,001
+// rows, 3 and 3 no better than 6 and 4). A serving stream's p99 stays at 12.4 to 12.7 ms.
+constexpr int64_t PART_MIN = 6, PART_START = 4;
 static int screen_parts(int64_t blocks, int64_t tiles, int64_t sms) {
     int64_t most = tiles / PART_MIN < 16 ? tiles / PART_MIN : 16;
     if (blocks > 8 * sms) most = 1;  // the last wave is a small share
