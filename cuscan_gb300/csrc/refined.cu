@@ -2158,7 +2158,7 @@ static int knn_list_pass(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, co
     return read_screen_status(ctx, R, s, fallbacks);
 }
 
-int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, int d, int k,
+static int knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, int d, int k,
                        int32_t *ids, float *dist, cudaStream_t s, int64_t *refined_rows,
                        int64_t *fallback_rows, int64_t *rescreened_rows) {
     if (!refined_shape_ok(n, d, k) || (b.refined.lean && lean_exact(d, k))) {
@@ -2268,7 +2268,24 @@ int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
     return CUSCAN_OK;
 }
 
-int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d,
+// Wide rows take more device memory on the screens than in the exact sweeps: without room for it the
+// fit goes on with those.
+int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, int d, int k,
+                       int32_t *ids, float *dist, cudaStream_t s, int64_t *refined_rows,
+                       int64_t *fallback_rows, int64_t *rescreened_rows) {
+    b.refined.no_room = false;
+    const int rc =
+        knn_refined(ctx, b, x, n, d, k, ids, dist, s, refined_rows, fallback_rows, rescreened_rows);
+    if (rc != CUSCAN_MEMORY || d <= LEAN_MAX_FEATURES) return rc;
+    clear_error(ctx);
+    b.refined.no_room = true;
+    for (int64_t *rows : {refined_rows, fallback_rows, rescreened_rows})
+        if (rows) *rows = 0;
+    return launch_exact_knn_fp32(ctx, x, n, x, n, d, k, 1, 0, 1, ids, dist, s, b.knn_ids_tmp,
+                                 b.knn_dist_tmp);
+}
+
+static int candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d,
                               const int32_t *knn_ids, const float *knn_sq, int k,
                               const float *core, const int32_t *label, cudaStream_t s,
                               int64_t *fallback_rows) {
@@ -2278,7 +2295,7 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
     const int32_t *perm = as<int32_t>(b.perm);
     unsigned long long *row_keys = as<unsigned long long>(b.row_keys);
     int32_t *clo = as<int32_t>(b.tile_lo), *chi = as<int32_t>(b.tile_hi);
-    if (!refined_shape_ok(n, d, 1) || (b.refined.lean && lean_exact(d, k)))
+    if (!refined_shape_ok(n, d, 1) || b.refined.no_room || (b.refined.lean && lean_exact(d, k)))
         return launch_candidates_fp32(ctx, xp, corep, labp, perm, n, d, row_keys, clo, chi, s);
     RefinedBuffers &R = b.refined;
     Layout L;
@@ -2410,9 +2427,20 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
     return CUSCAN_OK;
 }
 
-// The per-row terms of the bound for the debug entry point: (ps, pb, cm, m) with
-// ps = (1 - C_B) p - abs_c, pb = (1 - C_B) p, cm = C_A m, so that the screen's bound of entry
-// (r, c) is fmaf(-cm_r, m_c, fmaf(-2, acc_rc, pb_c) + ps_r) (screen units).
+// As launch_knn_refined: every buffer of a round is there before its first kernel writes a key.
+int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d,
+                              const int32_t *knn_ids, const float *knn_sq, int k,
+                              const float *core, const int32_t *label, cudaStream_t s,
+                              int64_t *fallback_rows) {
+    int rc = candidates_refined(ctx, b, n, d, knn_ids, knn_sq, k, core, label, s, fallback_rows);
+    if (rc == CUSCAN_MEMORY && d > LEAN_MAX_FEATURES) {
+        clear_error(ctx);
+        b.refined.no_room = true;
+        rc = candidates_refined(ctx, b, n, d, knn_ids, knn_sq, k, core, label, s, fallback_rows);
+    }
+    return rc;
+}
+
 // An exact (plain f32) Borůvka round over the rows that can hold their component's cheapest
 // edge. The rows are chosen as in the screened rounds: every component gets an upper bound of
 // its cheapest cross edge from the kNN pairs (seed_bounds_kernel), and a row is skipped when its
@@ -2488,6 +2516,9 @@ int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, i
     return CUSCAN_OK;
 }
 
+// The per-row terms of the bound for the debug entry point: (ps, pb, cm, m) with
+// ps = (1 - C_B) p - abs_c, pb = (1 - C_B) p, cm = C_A m, so that the screen's bound of entry
+// (r, c) is fmaf(-cm_r, m_c, fmaf(-2, acc_rc, pb_c) + ps_r) (screen units).
 __global__ void debug_rows_kernel(const float *__restrict__ pnorm, const float *__restrict__ mnorm,
                                   int64_t n, float one_minus_cb, float abs_c, float c_a,
                                   float *__restrict__ rows) {
