@@ -254,15 +254,17 @@ __global__ void relabel_kernel(int32_t *__restrict__ label, const int32_t *__res
 }
 
 // Start of a component sort: empty histogram and cursors, empty row and component keys for the
-// round that follows, the pair sum and the scan's ticket.
+// round that follows, the scan's ticket and, where the sort counts them, the pair sum. The ticket
+// is cleared by every sort: sorts outside a fit (sort_by_cells of a set's kNN or of a predictor's
+// rows) run on a status block that nothing else has written.
 __global__ void sort_clear_kernel(int32_t *__restrict__ cnt, int32_t *__restrict__ fill,
                                   unsigned long long *__restrict__ row_keys,
                                   unsigned long long *__restrict__ comp_keys, int64_t n,
-                                  DevStatus *status) {
+                                  DevStatus *status, bool counts_pairs) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0 && status) {
-        status->same_pairs = 0.0;
+    if (i == 0) {
         status->scan_ticket = 0;
+        if (counts_pairs) status->same_pairs = 0.0;
     }
     if (i >= n) return;
     cnt[i] = 0;
@@ -941,7 +943,7 @@ int forest_norm_keys(cuscan_ctx *ctx, ForestBuffers &b, const int32_t *label, in
     if (rc) return rc;
     CUSCAN_KERNEL(sort_clear_kernel, blocks(n), 256, 0, s, cnt, as<int32_t>(b.fill),
                   as<unsigned long long>(b.row_keys), as<unsigned long long>(b.comp_keys), n,
-                  b.status);
+                  b.status, true);
     CUSCAN_KERNEL(hist_roots_kernel, blocks(n), 256, 0, s, label, n, cnt, as<int32_t>(b.keep));
     // ranks of the component roots; the histogram's squares are same_pairs
     if ((rc = scan_exclusive(ctx, b, as<int32_t>(b.keep), rank, n, nullptr, s))) return rc;
@@ -968,7 +970,7 @@ int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, 
     }
     CUSCAN_KERNEL(sort_clear_kernel, blocks(n), 256, 0, s, cnt, fill,
                   as<unsigned long long>(b.row_keys), as<unsigned long long>(b.comp_keys), n,
-                  key ? nullptr : b.status);
+                  b.status, !key);
     CUSCAN_KERNEL(hist_kernel, blocks(n), 256, 0, s, key ? key : label, n, cnt);
     CUSCAN_LAUNCH(ctx, "hist_kernel");
     // same_pairs: the sum of squared component sizes, for the work counters
@@ -1003,7 +1005,7 @@ int forest_label_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *core, con
     int32_t *cnt = as<int32_t>(b.cnt);
     CUSCAN_KERNEL(sort_clear_kernel, blocks(n), 256, 0, s, cnt, as<int32_t>(b.fill),
                   as<unsigned long long>(b.row_keys), as<unsigned long long>(b.comp_keys), n,
-                  b.status);
+                  b.status, true);
     CUSCAN_KERNEL(label_cells_kernel, blocks(n), 256, 0, s, label, core, as<int32_t>(b.perm), n, cnt,
                   as<int32_t>(b.labp), as<float>(b.corep));
     CUSCAN_LAUNCH(ctx, "label_cells_kernel");

@@ -11,7 +11,7 @@ struct DevStatus {
     unsigned long long edges;       // MST edges emitted so far
     double same_pairs;     // sum of squared component sizes entering the current round
     int err_kind;          // 0 ok, 1 numerical weight, 2 index out of range, 4 no progress
-    unsigned int scan_ticket;  // blocks of the running scan that have finished (0 between scans)
+    unsigned int scan_ticket;  // blocks of the running scan that have finished (every sort clears it)
     int row_counts[2];     // screened rounds: rows without a component bound, rows that can hold an edge
     double mst_weight;     // f64 total MST weight, written once after the last round
     // kept on the device by packed fits (no host read after every round): the seed's results,

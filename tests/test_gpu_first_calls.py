@@ -1,0 +1,71 @@
+"""Operations that order rows on a context that no fit has run on, in device memory that held something
+else: the first exact_knn of a set against itself, and the first predictor, on a new context and
+after release_workspace."""
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import cuscan_gb300 as cg
+from cuscan_gb300 import _lib, synthetic
+from oracle import oracle as O
+from tests.test_gpu_ops import bits, gpu_knn
+
+pytestmark = pytest.mark.gpu
+
+
+def fill_free_memory(pattern=0x5A):
+    """Small and large device blocks filled with a pattern and given back, so that the allocations
+    that follow are handed memory that is not zero."""
+    cuda = C.CDLL("libcuda.so.1")
+    blocks = []
+    for size, count in ((64, 512), (256, 512), (512, 256), (8 << 10, 256), (64 << 10, 64),
+                        (1 << 20, 32), (16 << 20, 4)):
+        for _ in range(count):
+            at = C.c_uint64(0)
+            assert cuda.cuMemAlloc_v2(C.byref(at), C.c_size_t(size)) == 0
+            assert cuda.cuMemsetD8_v2(at, C.c_ubyte(pattern), C.c_size_t(size)) == 0
+            blocks.append(at)
+    assert cuda.cuCtxSynchronize() == 0
+    for at in blocks:
+        assert cuda.cuMemFree_v2(at) == 0
+
+
+@pytest.mark.parametrize("n,d,k", [(2048, 32, 5), (5003, 64, 10), (2600, 200, 15)])
+@pytest.mark.parametrize("released", [False, True])
+def test_exact_knn_needs_no_fit_before_it(gpu_ctx, n, d, k, released):
+    x = synthetic.gaussian_mixture(n, d, 9, seed=n)
+    ctx = _lib.Context(0)
+    if released:
+        ctx.fit_core(x[:2100], 5, _lib.PRECISION_BF16_REFINED)
+        ctx.release_workspace()
+    fill_free_memory()
+    for _ in range(2):
+        ids, ds = gpu_knn(ctx, x, x, k)
+        eids, eds = O.exact_neighbors(x, x, k)
+        np.testing.assert_array_equal(ids, eids)
+        np.testing.assert_array_equal(bits(ds), bits(eds))
+
+
+@pytest.mark.parametrize("restored", [False, True])
+def test_a_predictor_needs_no_fit_before_it(restored):
+    n, d, m = 8000, 64, 4096
+    x = synthetic.gaussian_mixture(n + m, d, 10, seed=3)
+    model = cg.HDBSCAN(min_cluster_size=50, min_samples=5, precision="fp16_refined").fit(x[:n])
+    if restored:
+        arrays, meta = model.to_predictor()._predictor.export_state()
+        ctx = _lib.Context(0)
+        fill_free_memory()
+        predict = cg.prediction.Predictor.from_state(arrays, meta, ctx).predict
+    else:
+        cg.context(0).release_workspace()
+        fill_free_memory()
+        predict = model.to_predictor()._predictor.predict
+    # a batch large enough for the spatial search, against pieces searched plainly
+    assert float(m) * n * d >= 2e9
+    whole = predict(x[n:])
+    parts = [predict(x[a:a + 200]) for a in range(n, n + m, 200)]
+    for got, exp in zip(whole, zip(*parts)):
+        np.testing.assert_array_equal(got, np.concatenate(exp))
