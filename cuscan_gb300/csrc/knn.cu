@@ -745,7 +745,8 @@ void knn_split_plan(const cuscan_ctx *ctx, int64_t nq, int64_t nr, int64_t &spli
 template <int L>
 int run_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, int64_t nr, int d,
             int k, int exclude_self, int64_t query_offset, int squared, int32_t *ids, float *dist,
-            cudaStream_t s, Buffer &scratch_ids, Buffer &scratch_dist, const int32_t *qmap) {
+            cudaStream_t s, Buffer &scratch_ids, Buffer &scratch_dist, const int32_t *qmap,
+            int64_t *launches) {
     const float pad = squared ? std::numeric_limits<float>::infinity() : 3.40282346638528859812e+38f;
     int64_t splits = 1, chunk = 0;
     knn_split_plan(ctx, nq, nr, splits, chunk, d, k);
@@ -758,6 +759,7 @@ int run_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, i
         CUSCAN_KERNEL(knn_fp32_kernel<L>, grid, simt::THREADS, smem, s, query, nq, ref, nr, d, k,
                       exclude_self, query_offset, pad, chunk, ids, dist, 0, squared ? 0 : 1, qmap);
         CUSCAN_LAUNCH(ctx, "knn_fp32_kernel");
+        if (launches) *launches += 1;
         return CUSCAN_OK;
     }
     const int64_t stride = nq * k;
@@ -774,6 +776,7 @@ int run_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, i
                   32 * MERGE_WARPS, 0, s, as<int32_t>(scratch_ids), as<float>(scratch_dist), nq, k,
                   (int)splits, stride, pad, nr, squared ? 0 : 1, ids, dist, qmap, nullptr);
     CUSCAN_LAUNCH(ctx, "knn_merge_kernel");
+    if (launches) *launches += 2;
     return CUSCAN_OK;
 }
 
@@ -825,7 +828,8 @@ int run_knn_pruned(cuscan_ctx *ctx, const float *query, int64_t nq, const float 
 int launch_exact_knn_fp32(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref,
                           int64_t nr, int d, int k, int exclude_self, int64_t query_offset,
                           int squared, int32_t *ids, float *dist, cudaStream_t s,
-                          Buffer &scratch_ids, Buffer &scratch_dist, const int32_t *qmap) {
+                          Buffer &scratch_ids, Buffer &scratch_dist, const int32_t *qmap,
+                          int64_t *launches) {
     if (nq == 0) return CUSCAN_OK;
     if (d > CUSCAN_PACK_MAX_FEATURES)
         return fail(ctx, CUSCAN_CAPACITY,
@@ -839,6 +843,7 @@ int launch_exact_knn_fp32(cuscan_ctx *ctx, const float *query, int64_t nq, const
         CUSCAN_KERNEL(knn_fp32_wide_kernel, (unsigned)ceil_div(nq, WIDE_Q), WIDE_Q, smem, s,
             query, nq, ref, nr, d, k, exclude_self, query_offset, pad, ids, dist);
         CUSCAN_LAUNCH(ctx, "knn_fp32_wide_kernel");
+        if (launches) *launches += squared ? 1 : 2;
         if (!squared) {
             CUSCAN_KERNEL(sqrt_rows_kernel, (unsigned)ceil_div(nq * k, 256), 256, 0, s, dist, nq * k);
             CUSCAN_LAUNCH(ctx, "sqrt_rows_kernel");
@@ -847,7 +852,7 @@ int launch_exact_knn_fp32(cuscan_ctx *ctx, const float *query, int64_t nq, const
     }
 #define CUSCAN_RUN_KNN(L)                                                                        \
     run_knn<L>(ctx, query, nq, ref, nr, d, k, exclude_self, query_offset, squared, ids, dist, s, \
-               scratch_ids, scratch_dist, qmap)
+               scratch_ids, scratch_dist, qmap, launches)
     if (k == 1) return CUSCAN_RUN_KNN(0);
     if (k <= 32) return CUSCAN_RUN_KNN(1);
     if (k <= 64) return CUSCAN_RUN_KNN(2);

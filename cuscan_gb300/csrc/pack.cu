@@ -28,7 +28,7 @@
 // same pointer-doubling step counts, so every output is bit identical to cuscan_fit_core's.
 // Splitting the reference range differently does not change the lists: the kNN merge and the
 // candidate keys are exact minima in a total order. Fits with k > 32 take the per-fit kNN
-// launch (the wide kernel, as alone).
+// launch, as alone.
 //
 // The reference has no counterpart: its serving layer does not exist and its small fits run
 // one host-driven round at a time.
@@ -320,12 +320,11 @@ extern "C" int cuscan_fit_core_packed(cuscan_ctx *ctx, cuscan_fit_item *items, i
         return rc;
     for (int i = 0; i < count; ++i) {
         if (item_k(items[i]) <= kGroupedMaxK) continue;
-        Buffer unused_ids, unused_dist;  // the wide kernel keeps no partial lists
         const PackFit &f = host_fits[i];
+        ForestBuffers &b = ctx->fit->forest;  // partial lists in the buffers of a fit alone
         if ((rc = launch_exact_knn_fp32(ctx, f.x, f.n, f.x, f.n, f.d, f.k, 1, 0, 1, f.ids, f.dsq,
-                                        s, unused_ids, unused_dist)))
+                                        s, b.knn_ids_tmp, b.knn_dist_tmp, nullptr, &P.launches)))
             return rc;
-        ++P.launches;
     }
     CUSCAN_CUDA(ctx, cudaEventRecord(P.ev[1], s));
     if ((rc = pack_seed(ctx, fits, count, more, s))) return rc;
