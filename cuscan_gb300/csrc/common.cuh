@@ -134,6 +134,15 @@ inline cudaStream_t pick_stream(cuscan_ctx *ctx, void *stream) {
     return stream ? (cudaStream_t)stream : ctx->stream;
 }
 
+inline bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) != cudaSuccess) {
+        cudaGetLastError();  // (the legacy stream beside a capture: the launch reports it)
+        return false;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 // Ensure a buffer holds at least `bytes`; contents are not preserved.
 inline int ensure(cuscan_ctx *ctx, Buffer &b, size_t bytes, const char *what) {
     if (bytes == 0) bytes = 16;

@@ -750,6 +750,24 @@ int run_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, i
     const float pad = squared ? std::numeric_limits<float>::infinity() : 3.40282346638528859812e+38f;
     int64_t splits = 1, chunk = 0;
     knn_split_plan(ctx, nq, nr, splits, chunk, d, k);
+    const int64_t stride = nq * k;
+    const size_t list_bytes = (size_t)(stride * splits) * sizeof(float);
+    // A captured sweep allocates nothing, and one of more than 32 neighbours leaves no pointer to the
+    // workspace in the graph, which a later call could free.
+    if (splits > 1 && capturing(s) &&
+        (L > 1 || scratch_ids.bytes < list_bytes || scratch_dist.bytes < list_bytes))
+        splits = 1;
+    if (splits > 1) {
+        int rc = ensure(ctx, scratch_ids, list_bytes, "kNN partial ids");
+        if (!rc) rc = ensure(ctx, scratch_dist, list_bytes, "kNN partial distances");
+        if (rc && rc != CUSCAN_MEMORY) return rc;
+        if (rc) {  // no room for the partial lists: the references in one part
+            clear_error(ctx);
+            release(scratch_ids);
+            release(scratch_dist);
+            splits = 1;
+        }
+    }
     const size_t smem = knn_smem_bytes(k);
     if (int rc = allow_dynamic_smem(ctx, knn_fp32_kernel<L>, smem)) return rc;
     const dim3 grid((unsigned)ceil_div(nq, (int64_t)QT), (unsigned)splits);
@@ -757,16 +775,11 @@ int run_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, i
         if (!squared && qmap)
             return fail(ctx, CUSCAN_INVALID_INPUT, "row-subset kNN is squared only");
         CUSCAN_KERNEL(knn_fp32_kernel<L>, grid, simt::THREADS, smem, s, query, nq, ref, nr, d, k,
-                      exclude_self, query_offset, pad, chunk, ids, dist, 0, squared ? 0 : 1, qmap);
+                      exclude_self, query_offset, pad, nr, ids, dist, 0, squared ? 0 : 1, qmap);
         CUSCAN_LAUNCH(ctx, "knn_fp32_kernel");
         if (launches) *launches += 1;
         return CUSCAN_OK;
     }
-    const int64_t stride = nq * k;
-    int rc = ensure(ctx, scratch_ids, (size_t)(stride * splits) * sizeof(int32_t), "kNN partial ids");
-    if (rc) return rc;
-    rc = ensure(ctx, scratch_dist, (size_t)(stride * splits) * sizeof(float), "kNN partial distances");
-    if (rc) return rc;
     CUSCAN_KERNEL(knn_fp32_kernel<L>, grid, simt::THREADS, smem, s, query, nq, ref, nr, d, k,
                   exclude_self, query_offset, pad, chunk, as<int32_t>(scratch_ids),
                   as<float>(scratch_dist), stride, 0, qmap);

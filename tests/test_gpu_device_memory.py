@@ -2,10 +2,15 @@
 given back with it."""
 from __future__ import annotations
 
+from contextlib import contextmanager
+
 import numpy as np
 import pytest
 
 from cuscan_gb300 import _lib, synthetic
+from oracle import oracle as O
+from tests.test_gpu_fit import assert_fit_equal
+from tests.test_gpu_ops import bits
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -14,6 +19,18 @@ pytestmark = pytest.mark.gpu
 def free_bytes():
     torch.cuda.synchronize()
     return torch.cuda.mem_get_info()[0]
+
+
+@contextmanager
+def little_memory(left):
+    """All but about `left` bytes of the device taken."""
+    torch.cuda.empty_cache()
+    filler = torch.empty(free_bytes() - left, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del filler
+        torch.cuda.empty_cache()
 
 
 def test_repeated_packs_with_wide_lists_hold_no_more_memory():
@@ -36,3 +53,43 @@ def test_packs_count_every_launch_of_wide_lists():
     before = _lib.launch_count()
     ctx.fit_core_packed(fits)
     assert _lib.launch_count() - before == ctx.packed_launch_stats()["launches"]
+
+
+@pytest.mark.parametrize("squared", [True, False])
+def test_exact_knn_of_wide_lists_runs_without_room_for_partial_lists(squared):
+    m, n, d, k = 3000, 60_000, 16, 200
+    x = synthetic.gaussian_mixture(m + n, d, 9, seed=1)
+    q, r = torch.from_numpy(x[:m]).cuda(), torch.from_numpy(x[m:]).cuda()
+    ids = torch.empty((m, k), dtype=torch.int32, device="cuda")
+    ds = torch.empty((m, k), dtype=torch.float32, device="cuda")
+
+    def run(ctx):
+        ids.fill_(-1)
+        torch.cuda.synchronize()
+        ctx.exact_knn(q.data_ptr(), m, r.data_ptr(), n, d, k, False, 0, squared, ids.data_ptr(),
+                      ds.data_ptr())
+        torch.cuda.synchronize()
+        return ids.cpu().numpy(), ds.cpu().numpy()
+
+    left = 24 << 20
+    ctx = _lib.Context(0)
+    ids0, ds0 = run(ctx)
+    assert ctx.reserved_bytes() > left  # the lists of the parts
+    ctx.close()
+    with little_memory(left):
+        ids1, ds1 = run(_lib.Context(0))
+    np.testing.assert_array_equal(ids1, ids0)
+    np.testing.assert_array_equal(bits(ds1), bits(ds0))
+
+
+def test_plain_fits_with_wide_lists_run_without_room_for_partial_lists():
+    x = synthetic.gaussian_mixture(5003, 64, 9, seed=2)
+    left = 32 << 20
+    warm = _lib.Context(0)
+    warm.fit_core(x, 250, _lib.PRECISION_PLAIN)
+    assert warm.reserved_bytes() > left
+    warm.close()
+    ctx = _lib.Context(0)
+    with little_memory(left):
+        got = ctx.fit_core(x, 250, _lib.PRECISION_PLAIN)
+    assert_fit_equal(got, O.fit_core(x, 250))
