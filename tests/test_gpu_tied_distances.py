@@ -51,7 +51,7 @@ def test_ties_cost_no_list_insertions(gpu_ctx, kind, k, squared):
     n, d = 10_000, 16
     ids = torch.empty((n, k), dtype=torch.int32, device="cuda")
     ds = torch.empty((n, k), dtype=torch.float32, device="cuda")
-    stream = torch.cuda.current_stream().cuda_stream
+    legacy_stream = 1  # the events' stream
 
     def fastest(rows):
         q = torch.from_numpy(rows).cuda()
@@ -61,7 +61,7 @@ def test_ties_cost_no_list_insertions(gpu_ctx, kind, k, squared):
             a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
             a.record()
             gpu_ctx.exact_knn(q.data_ptr(), n, r.data_ptr(), n, d, k, False, 0, squared,
-                              ids.data_ptr(), ds.data_ptr(), stream)
+                              ids.data_ptr(), ds.data_ptr(), legacy_stream)
             b.record()
             torch.cuda.synchronize()
             times.append(a.elapsed_time(b))
