@@ -195,9 +195,10 @@ int cuscan_exact_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const floa
     // The kNN of a point set against itself (the fit's core-distance sweep) takes the tensor-core
     // screen with exact re-rank, whose rows equal the exact sweep's bit for bit; it falls back to
     // the exact sweep itself for shapes outside the screen's tiling (fewer than 2048 rows,
-    // k > 32, more than 256 features, values that overflow f32).
+    // k > 32, more than 256 features, values that overflow f32). The screen reads its status on the
+    // host, which a stream that is being captured does not allow: captures hold the exact sweep.
     if (query == reference && nq == nr && query_offset == 0 && exclude_self && squared &&
-        nr >= 2048 && k <= 32 && refined_available()) {
+        nr >= 2048 && k <= 32 && refined_available() && !capturing(s)) {
         ForestBuffers &b = ctx->fit->forest;
         int rc = forest_reserve(ctx, b, nr, d);
         if (rc) return rc;

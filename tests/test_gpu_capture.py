@@ -45,3 +45,18 @@ def test_wide_lists_are_captured_without_a_call_before(k, squared):
     eids, eds = O.exact_neighbors(x, x, k, squared=squared)
     np.testing.assert_array_equal(ids, eids)
     np.testing.assert_array_equal(bits(ds), bits(eds))
+
+
+@pytest.mark.parametrize("n,d,k", [(2048, 129, 5), (2500, 256, 15), (2100, 40, 10)])
+def test_a_set_against_itself_is_captured(n, d, k):
+    x = synthetic.gaussian_mixture(n, d, 7, seed=d)
+    q = torch.from_numpy(x).cuda()
+    ctx = _lib.Context(0)
+    eids, eds = O.exact_neighbors(x, x, k)
+    for _ in range(2):  # before and after a call outside a capture
+        ids, ds = captured_knn(ctx, q, q, k, True, True)
+        np.testing.assert_array_equal(ids, eids)
+        np.testing.assert_array_equal(bits(ds), bits(eds))
+        ids, ds = gpu_knn(ctx, x, x, k)
+        np.testing.assert_array_equal(ids, eids)
+        np.testing.assert_array_equal(bits(ds), bits(eds))
