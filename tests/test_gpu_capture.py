@@ -7,6 +7,7 @@ import pytest
 
 from cuscan_gb300 import _lib, synthetic
 from oracle import oracle as O
+from tests.test_gpu_first_calls import self_knn
 from tests.test_gpu_ops import bits, gpu_knn
 
 torch = pytest.importorskip("torch")
@@ -57,6 +58,6 @@ def test_a_set_against_itself_is_captured(n, d, k):
         ids, ds = captured_knn(ctx, q, q, k, True, True)
         np.testing.assert_array_equal(ids, eids)
         np.testing.assert_array_equal(bits(ds), bits(eds))
-        ids, ds = gpu_knn(ctx, x, x, k)
+        ids, ds = self_knn(ctx, x, k)
         np.testing.assert_array_equal(ids, eids)
         np.testing.assert_array_equal(bits(ds), bits(eds))
