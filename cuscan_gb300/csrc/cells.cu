@@ -118,8 +118,10 @@ __global__ void far_rows_kernel(int32_t *__restrict__ cell, const float *__restr
                                 const float *__restrict__ inv) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int32_t c = cell[i];
-    if (dist[i] * inv[c] > FAR_ROWS * count[c]) cell[i] = c + npiv;
+    // A row without a distance to any pivot (not a number somewhere) got the number past the last
+    // cell, where the order has no entry; the last cell takes it.
+    const int32_t c = min(cell[i], npiv - 1);
+    cell[i] = dist[i] * inv[c] > FAR_ROWS * count[c] ? c + npiv : c;
 }
 
 // Start of every cell in a padded order (kMaxCells threads), from its row count.
@@ -141,7 +143,7 @@ __device__ __forceinline__ int padded_start(int count, int *warp_sums) {
 
 // Padded order of m query rows by cell, one CTA; the order within a cell is free.
 __global__ void __launch_bounds__(kMaxCells)
-    order_queries_kernel(const int32_t *__restrict__ cell, int64_t m, int64_t padded,
+    order_queries_kernel(const int32_t *__restrict__ cell, int64_t m, int npiv, int64_t padded,
                          int32_t *__restrict__ order) {
     __shared__ int start[kMaxCells];
     __shared__ int warp_sums[kMaxCells / 32];
@@ -149,12 +151,13 @@ __global__ void __launch_bounds__(kMaxCells)
     start[t] = 0;
     for (int64_t i = t; i < padded; i += kMaxCells) order[i] = -1;
     __syncthreads();
-    for (int64_t i = t; i < m; i += kMaxCells) atomicAdd(&start[cell[i]], 1);
+    for (int64_t i = t; i < m; i += kMaxCells) atomicAdd(&start[min(cell[i], npiv - 1)], 1);
     __syncthreads();
     const int at = padded_start(start[t], warp_sums);
     start[t] = at;
     __syncthreads();
-    for (int64_t i = t; i < m; i += kMaxCells) order[atomicAdd(&start[cell[i]], 1)] = (int32_t)i;
+    for (int64_t i = t; i < m; i += kMaxCells)
+        order[atomicAdd(&start[min(cell[i], npiv - 1)], 1)] = (int32_t)i;
 }
 
 // The same of a sorted set's positions: shift[c] is what a position of cell c moves by. The cells
@@ -475,7 +478,7 @@ int order_queries(cuscan_ctx *ctx, ForestBuffers &b, const float *pivots, int np
                                     as<float>(R.cell_d), s, b.knn_ids_tmp, b.knn_dist_tmp)))
         return rc;
     CUSCAN_KERNEL(order_queries_kernel, 1, (unsigned)kMaxCells, 0, s, as<int32_t>(R.cells), m,
-                  padded_queries(m), order);
+                  npiv, padded_queries(m), order);
     CUSCAN_LAUNCH(ctx, "order_queries_kernel");
     return CUSCAN_OK;
 }
