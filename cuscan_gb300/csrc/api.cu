@@ -90,6 +90,7 @@ int cuscan_ctx_create(int device, cuscan_ctx **out) {
         return CUSCAN_MEMORY;
     }
     for (auto &ev : ctx->fit->ev) cudaEventCreate(&ev);
+    cudaEventCreateWithFlags(&ctx->last_use, cudaEventDisableTiming);
     *out = ctx;
     return CUSCAN_OK;
 }
@@ -98,6 +99,7 @@ void cuscan_ctx_destroy(cuscan_ctx *ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    if (ctx->in_use) cudaEventSynchronize(ctx->last_use);
     if (ctx->fit) {
         FitWorkspace *f = ctx->fit;
         Buffer *all[kWorkspaceBufferCount];
@@ -112,6 +114,7 @@ void cuscan_ctx_destroy(cuscan_ctx *ctx) {
             if (ev) cudaEventDestroy(ev);
         delete f;
     }
+    if (ctx->last_use) cudaEventDestroy(ctx->last_use);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -130,6 +133,7 @@ int cuscan_ctx_release_workspace(cuscan_ctx *ctx) {
     clear_error(ctx);
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (ctx->in_use) CUSCAN_CUDA(ctx, cudaEventSynchronize(ctx->last_use));
     Buffer *all[kWorkspaceBufferCount];
     const int count = workspace_buffers(ctx->fit, all);
     for (int i = 0; i < count; ++i) release(*all[i]);
@@ -192,6 +196,7 @@ int cuscan_exact_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const floa
         return fail(ctx, CUSCAN_INVALID_INPUT, "exact_knn received a null pointer");
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = pick_stream(ctx, stream);
+    CUSCAN_TURN(ctx, s);
     // The kNN of a point set against itself (the fit's core-distance sweep) takes the tensor-core
     // screen with exact re-rank, whose rows equal the exact sweep's bit for bit; it falls back to
     // the exact sweep itself for shapes outside the screen's tiling (fewer than 2048 rows,
@@ -225,6 +230,7 @@ int cuscan_boruvka_candidates(cuscan_ctx *ctx, const float *data, const float *c
     if (n > INT32_MAX - 1) return fail(ctx, CUSCAN_OVERFLOW, "Boruvka row indices");
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = pick_stream(ctx, stream);
+    CUSCAN_TURN(ctx, s);
     FitWorkspace *f = ctx->fit;
     int rc = ensure(ctx, f->op_keys, sizeof(unsigned long long) * n, "candidate keys");
     if (!rc) rc = ensure(ctx, f->op_tiles_lo, sizeof(int32_t) * (ceil_div(n, 32) + 1), "tiles");
@@ -249,9 +255,11 @@ int cuscan_component_reduce(cuscan_ctx *ctx, const float *weights, const int32_t
         return fail(ctx, CUSCAN_INVALID_INPUT, "component_reduce received inconsistent sizes");
     if (n > INT32_MAX) return fail(ctx, CUSCAN_OVERFLOW, "component member index");
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
+    cudaStream_t s = pick_stream(ctx, stream);
+    CUSCAN_TURN(ctx, s);
     return launch_component_reduce(ctx, weights, indices, members, tile_starts, tile_ends,
                                    partial_offsets, n, p, c, win_weights, win_meta,
-                                   ctx->fit->op_partials, pick_stream(ctx, stream));
+                                   ctx->fit->op_partials, s);
 }
 
 static int read_status(cuscan_ctx *ctx, DevStatus *dev, DevStatus *host, cudaStream_t s) {
@@ -310,6 +318,7 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
         return fail(ctx, CUSCAN_INVALID_INPUT, "fit_core_device received a null pointer");
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = pick_stream(ctx, stream);
+    CUSCAN_TURN(ctx, s);
     FitWorkspace *f = ctx->fit;
     ForestBuffers &b = f->forest;
     int rc = forest_reserve(ctx, b, n, d);
@@ -434,6 +443,7 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
                                      cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaEventRecord(ev[3], s));
     CUSCAN_CUDA(ctx, cudaEventSynchronize(ev[3]));
+    turn.finished();
     if ((int64_t)hs->edges != n - 1)
         return fail(ctx, CUSCAN_NUMERICAL, "Boruvka produced an incomplete spanning tree");
     if (n_edges) *n_edges = (int64_t)hs->edges;
@@ -475,6 +485,7 @@ int cuscan_fit_core(cuscan_ctx *ctx, const float *data, int64_t n, int32_t d,
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     FitWorkspace *f = ctx->fit;
     cudaStream_t s = ctx->stream;
+    CUSCAN_TURN(ctx, s);
     const int64_t k = (int64_t)min_samples < n - 1 ? min_samples : n - 1;
     int rc = ensure(ctx, f->x, sizeof(float) * n * d, "input rows");
     if (!rc) rc = ensure(ctx, f->ids, sizeof(int32_t) * n * k, "kNN ids");
@@ -502,6 +513,7 @@ int cuscan_fit_core(cuscan_ctx *ctx, const float *data, int64_t n, int32_t d,
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(mst_dst, f->dst.ptr, sizeof(uint32_t) * m, cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(mst_wsq, f->w.ptr, sizeof(float) * m, cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
+    turn.finished();
     if (n_edges) *n_edges = m;
     return CUSCAN_OK;
 }
@@ -534,6 +546,7 @@ int cuscan_shard_seed(cuscan_ctx *ctx, int64_t n, int32_t d, int32_t min_samples
         return fail(ctx, CUSCAN_INVALID_INPUT, "null buffer");
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = pick_stream(ctx, stream);
+    CUSCAN_TURN(ctx, s);
     FitWorkspace *f = ctx->fit;
     ForestBuffers &b = f->forest;
     int rc = forest_reserve(ctx, b, n, d);
@@ -562,6 +575,7 @@ int cuscan_shard_round_keys(cuscan_ctx *ctx, const float *data, const float *cor
     if (n > INT32_MAX - 1) return fail(ctx, CUSCAN_OVERFLOW, "row indices");
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = pick_stream(ctx, stream);
+    CUSCAN_TURN(ctx, s);
     FitWorkspace *f = ctx->fit;
     int rc = ensure(ctx, f->op_tiles_lo, sizeof(int32_t) * (ceil_div(n, 32) + 1), "tiles");
     if (!rc) rc = ensure(ctx, f->op_tiles_hi, sizeof(int32_t) * (ceil_div(n, 32) + 1), "tiles");
@@ -584,6 +598,7 @@ int cuscan_shard_round_merge(cuscan_ctx *ctx, const float *data, const float *co
     if (n < 2 || d <= 0 || !row_keys) return fail(ctx, CUSCAN_INVALID_INPUT, "bad round input");
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = pick_stream(ctx, stream);
+    CUSCAN_TURN(ctx, s);
     FitWorkspace *f = ctx->fit;
     ForestBuffers &b = f->forest;
     if (!b.status) return fail(ctx, CUSCAN_INVALID_INPUT, "no shard seed on this context");
@@ -623,6 +638,7 @@ int cuscan_debug_screen_tile_operands(cuscan_ctx *ctx, const float *data, int64_
         return fail(ctx, CUSCAN_INVALID_INPUT, "unknown operand format");
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = pick_stream(ctx, stream);
+    CUSCAN_TURN(ctx, s);
     int rc = forest_reserve(ctx, ctx->fit->forest, n, d);
     if (rc) return rc;
     return debug_screen_tile(ctx, ctx->fit->forest, data, n, d, operands, tile_out, rows_out,

@@ -38,6 +38,10 @@ struct cuscan_ctx {
     char err[1024] = {0};
     int sm_count = cuscan::kSMs;
     cuscan::FitWorkspace *fit = nullptr;
+    // the latest call's work: recorded on its stream where the call returned before its end
+    cudaEvent_t last_use = nullptr;
+    cudaStream_t last_stream = nullptr;
+    bool in_use = false;
 };
 
 namespace cuscan {
@@ -142,6 +146,35 @@ inline bool capturing(cudaStream_t s) {
     }
     return status != cudaStreamCaptureStatusNone;
 }
+
+// A call's turn at the context's workspace. Calls may be given different streams, and most of them
+// return before their work has run: each waits on its stream for the work of the call before it.
+// Captured calls do neither, because a graph runs at other times than the calls around its capture.
+class Turn {
+  public:
+    Turn(cuscan_ctx *ctx, cudaStream_t s) : ctx_(ctx), s_(s), captured_(capturing(s)) {
+        if (captured_ || !ctx->in_use || (s == ctx->stream && s == ctx->last_stream)) return;
+        const cudaError_t e = cudaStreamWaitEvent(s, ctx->last_use, 0);
+        if (e != cudaSuccess) status = cuda_fail(ctx, e, "wait for the context's previous call");
+    }
+    ~Turn() {
+        if (captured_) return;
+        ctx_->in_use = !finished_ && cudaEventRecord(ctx_->last_use, s_) == cudaSuccess;
+        ctx_->last_stream = s_;
+    }
+    Turn(const Turn &) = delete;
+    Turn &operator=(const Turn &) = delete;
+    void finished() { finished_ = true; }  // the call waited for its work
+    int status = CUSCAN_OK;
+
+  private:
+    cuscan_ctx *ctx_;
+    cudaStream_t s_;
+    bool captured_, finished_ = false;
+};
+#define CUSCAN_TURN(ctx, s)        \
+    ::cuscan::Turn turn((ctx), (s)); \
+    if (turn.status) return turn.status
 
 // Ensure a buffer holds at least `bytes`; contents are not preserved.
 inline int ensure(cuscan_ctx *ctx, Buffer &b, size_t bytes, const char *what) {

@@ -293,6 +293,7 @@ extern "C" int cuscan_fit_core_packed(cuscan_ctx *ctx, cuscan_fit_item *items, i
     const int64_t splits = pack_splits(ctx, count, n_max);
     const PackLayout L = make_layout(items, count, splits);
     cudaStream_t s = ctx->stream;
+    CUSCAN_TURN(ctx, s);
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
     if ((rc = ensure(ctx, P.arena, L.total, "packed fits"))) return rc;
     if (P.staging_bytes < L.out_end) {
@@ -349,6 +350,7 @@ extern "C" int cuscan_fit_core_packed(cuscan_ctx *ctx, cuscan_fit_item *items, i
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(stg + L.more, base + L.more, L.out_end - L.more,
                                      cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
+    turn.finished();
 
     // results
     const float knn_ms = elapsed_ms(P.ev[0], P.ev[1]);

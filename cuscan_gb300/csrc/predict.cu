@@ -404,6 +404,7 @@ static int create_predictor(cuscan_ctx *ctx, const float *train, int64_t n_finit
     if (train && clustered) {
         CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
         cudaStream_t s = ctx->stream;
+        CUSCAN_TURN(ctx, s);
         const size_t bytes = sizeof(float) * (size_t)n_finite * d;
         cudaError_t e = cudaMalloc(&P->train, bytes);
         if (e != cudaSuccess) {
@@ -438,6 +439,7 @@ static int create_predictor(cuscan_ctx *ctx, const float *train, int64_t n_finit
             }
         }
         CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
+        turn.finished();
         guard.release();
     } else if (!prediction_core) {
         P->cores.assign(n_finite, 0.0);  // no cluster tree: cores are never read
@@ -676,6 +678,8 @@ int cuscan_predictor_from_state(cuscan_ctx *ctx, const float *geometry, int64_t 
     if (!all_finite(geometry, n_finite * (int64_t)d))
         return finish(invalid(ectx, "predictor geometry must be finite"));
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
+    Turn turn(ctx, ctx->stream);
+    if (turn.status) return finish(turn.status);
     const size_t bytes = sizeof(float) * (size_t)n_finite * d;
     cudaError_t e = cudaMalloc(&P->train, bytes);
     if (e != cudaSuccess) {
@@ -695,6 +699,7 @@ int cuscan_predictor_from_state(cuscan_ctx *ctx, const float *geometry, int64_t 
         free_rows(*P);
         return finish(cuda_fail(ctx, e, "predictor geometry upload"));
     }
+    turn.finished();
     *out = P.release();
     return CUSCAN_OK;
 }
@@ -799,6 +804,7 @@ int predict_queries(cuscan_ctx *ctx, const cuscan_predictor *p, const float *que
         return fail(ctx, CUSCAN_INVALID_INPUT, "X must contain only finite values");
     CUSCAN_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
+    CUSCAN_TURN(ctx, s);
     FitWorkspace *f = ctx->fit;
     const int k = 2 * p->s;
     int rc = ensure(ctx, f->pred_q, sizeof(float) * m * p->d, "query rows");
@@ -838,6 +844,7 @@ int predict_queries(cuscan_ctx *ctx, const cuscan_predictor *p, const float *que
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(sq.data(), f->pred_dist.ptr, sizeof(float) * sq.size(),
                                      cudaMemcpyDeviceToHost, s));
     CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
+    turn.finished();
     std::vector<double> dist((size_t)k);
     for (int64_t q = 0; q < m; ++q) {
         for (int c = 0; c < k; ++c)

@@ -27,7 +27,9 @@
  *    returns.
  *  - `stream` is a cudaStream_t passed as void*; NULL means the context's own stream. Device
  *    entry points only enqueue work on that stream, except where a function states it
- *    synchronises.
+ *    synchronises. The calls of one context share its workspace: a call on another stream than
+ *    the one before it waits on the device for that one's work (calls that are captured into a
+ *    graph do not; order the graph's launches around the context's other calls).
  *  - Row-major float32 data, int32 ids, n < 2^31 rows.
  */
 #ifndef CUSCAN_GB300_H
