@@ -7,6 +7,7 @@ from contextlib import contextmanager
 import numpy as np
 import pytest
 
+import cuscan_gb300 as cg
 from cuscan_gb300 import _lib, synthetic
 from oracle import oracle as O
 from tests.test_gpu_fit import assert_fit_equal
@@ -93,3 +94,50 @@ def test_plain_fits_with_wide_lists_run_without_room_for_partial_lists():
     with little_memory(left):
         got = ctx.fit_core(x, 250, _lib.PRECISION_PLAIN)
     assert_fit_equal(got, O.fit_core(x, 250))
+
+
+def spatial_model(n, d, m):
+    x = synthetic.gaussian_mixture(n + m, d, 10, seed=5)
+    x[n // 2:n // 2 + 50] = x[:50]  # ties between rows with different ids
+    x[n:n + min(m, 20)] = x[:min(m, 20)]
+    return cg.HDBSCAN(min_cluster_size=50, min_samples=5, precision="fp16_refined").fit(x[:n]), x
+
+
+def test_predictors_leave_no_workspace_and_copy_their_rows_only_with_ample_room():
+    n, d, m = 100_000, 64, 4096
+    model, x = spatial_model(n, d, m)
+    assert 4096.0 * n * d >= 2e9  # a copy in spatial order
+    arrays, meta = model.to_predictor()._predictor.export_state()
+    np.testing.assert_array_equal(arrays["geometry"].reshape(n, d), x[:n])
+    rows = 4 * n * d
+    results = []
+    for left, copies in ((None, 2), (6 * rows, 1)):
+        # on a context that has run nothing, whose workspace stays empty
+        ctx = _lib.Context(0)
+
+        def restore():
+            free = free_bytes()
+            predictor = cg.prediction.Predictor.from_state(arrays, meta, ctx)
+            # (ids, bounds and up to 2 MiB of rounding per allocation beside the rows)
+            assert copies * rows <= free - free_bytes() < (copies + 0.5) * rows
+            assert ctx.reserved_bytes() == 0
+            results.append(predictor.predict(x[n:]))
+
+        if left is None:
+            restore()
+        else:
+            with little_memory(left):
+                restore()
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("m", [1, 130, 1500])
+def test_batches_against_rows_in_spatial_order_equal_the_oracle(m):
+    n, d = 8000, 64
+    model, x = spatial_model(n, d, m)
+    assert 4096.0 * n * d >= 2e9
+    got = model.to_predictor().approximate_predict(x[n:], True)
+    exp = O.approximate_predict(model.condensed_tree_, model.labels_, np.arange(n), 5, x[:n], x[n:])
+    for a, b in zip(got, exp):
+        np.testing.assert_array_equal(a, b)
