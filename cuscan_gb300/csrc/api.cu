@@ -29,8 +29,8 @@ int debug_screen_tile(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t
                       float *scale_out, cudaStream_t s);
 int refined_operand_format(const ForestBuffers &b);
 size_t refined_workspace_bytes(int64_t n, int d, int k, bool lean);
-int64_t fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, int32_t precision, bool lean);
-void set_lean(cuscan_ctx *ctx, bool lean);
+int64_t fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, int32_t precision, int lean);
+void set_lean(cuscan_ctx *ctx, int lean);
 
 // Every device buffer a context holds.
 static int workspace_buffers(FitWorkspace *f, Buffer **out) {
@@ -144,9 +144,9 @@ int cuscan_ctx_release_workspace(cuscan_ctx *ctx) {
 
 }  // extern "C"
 
-// Upper bound of a fit's device memory. lean: of a fit on a context set lean (see set_lean).
+// Upper bound of a fit's device memory. lean: of a fit on a context set to that level (serve.cpp).
 int64_t cuscan::fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, int32_t precision,
-                                    bool lean) {
+                                    int lean) {
     if (n < 2 || d <= 0 || min_samples <= 0) return 0;
     const size_t N = (size_t)n, D = (size_t)d;
     const size_t k = (size_t)((int64_t)min_samples < n - 1 ? min_samples : n - 1);
@@ -156,7 +156,7 @@ int64_t cuscan::fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, i
     // partial lists of split kNN sweeps, here and (in the same buffers) of the pruned sweep
     size_t partials = 8 * k * (size_t)simt::split_max_rows(n, n);
     if (precision == CUSCAN_PRECISION_BF16_REFINED || precision == CUSCAN_PRECISION_FP16_REFINED)
-        b += refined_workspace_bytes(n, d, (int)k, lean);
+        b += refined_workspace_bytes(n, d, (int)k, lean > 0);
     else if (n >= 2048) {  // exact rounds over a row subset: bounds, flags, positions, counts
         b += 7 * 4 * N + 64;
         // rows in spatial order, bounds of their tiles, first thresholds
@@ -170,12 +170,12 @@ int64_t cuscan::fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, i
     return (int64_t)(b + partials) + (1 << 20);
 }
 
-void cuscan::set_lean(cuscan_ctx *ctx, bool lean) { ctx->fit->forest.refined.lean = lean; }
+void cuscan::set_lean(cuscan_ctx *ctx, int lean) { ctx->fit->forest.refined.lean = lean; }
 
 extern "C" {
 
 int64_t cuscan_fit_workspace_bytes(int64_t n, int32_t d, int32_t min_samples, int32_t precision) {
-    return fit_workspace_bound(n, d, min_samples, precision, false);
+    return fit_workspace_bound(n, d, min_samples, precision, 0);
 }
 
 const char *cuscan_last_error(const cuscan_ctx *ctx) { return ctx ? ctx->err : "null context"; }

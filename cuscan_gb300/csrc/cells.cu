@@ -7,6 +7,8 @@
 // but the order of work depends on it; every result is decided by exact distances.
 #include "cells.cuh"
 
+#include "workspace.cuh"
+
 namespace cuscan {
 namespace {
 
@@ -465,6 +467,16 @@ int count_tight_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, float shift, 
                   count + 2 * kMaxPivots, as<float>(R.pivot_d), pivot_tour(R, npiv), npiv, shift,
                   gap, as<unsigned int>(R.norm_range));
     CUSCAN_LAUNCH(ctx, "tight_rows_kernel");
+    return CUSCAN_OK;
+}
+
+int read_apart(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, float &apart, cudaStream_t s) {
+    if (int rc = count_tight_rows(ctx, b, n, 0.0f, 1.0f, s)) return rc;
+    float *pairs = reinterpret_cast<float *>(ctx->fit->host_words());
+    CUSCAN_CUDA(ctx, cudaMemcpyAsync(pairs, as<float>(b.refined.norm_range) + 4, sizeof(float),
+                                     cudaMemcpyDeviceToHost, s));
+    CUSCAN_CUDA(ctx, cudaStreamSynchronize(s));
+    apart = (float)((double)*pairs / ((double)n * (double)n));
     return CUSCAN_OK;
 }
 

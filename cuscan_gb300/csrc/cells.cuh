@@ -41,6 +41,9 @@ int order_positions(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int32_t *order
 // neighbours. Right after sort_by_cells.
 int count_tight_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, float shift, float gap,
                      cudaStream_t s);
+// The share of the n x n row pairs that lie in cells too far apart to be neighbours, read on the host.
+// Right after sort_by_cells.
+int read_apart(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, float &apart, cudaStream_t s);
 // cbound[label] (f32 bits, labels by original row) lowered to the weights of edges between pivots
 // of different components. Needs sort_by_cells of the same fit.
 int pivot_component_bounds(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, const float *core,

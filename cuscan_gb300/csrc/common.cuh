@@ -239,12 +239,13 @@ struct TileBounds;  // cells.cuh
 // kNN (knn.cu). All pointers are device pointers. With qmap (squared, k <= 256 only), query row
 // i is row qmap[i] of `query`, excludes reference qmap[i] as itself and is written to output
 // row qmap[i]. The scratch buffers take the partial lists of split sweeps and outlive the call.
-// The launches made are added to *launches.
+// The launches made are added to *launches. one_part: the references are not split (no scratch).
 int launch_exact_knn_fp32(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref,
                           int64_t nr, int d, int k, int exclude_self, int64_t query_offset,
                           int squared, int32_t *ids, float *dist, cudaStream_t s,
                           Buffer &scratch_ids, Buffer &scratch_dist,
-                          const int32_t *qmap = nullptr, int64_t *launches = nullptr);
+                          const int32_t *qmap = nullptr, int64_t *launches = nullptr,
+                          bool one_part = false);
 
 // Borůvka candidates (boruvka.cu): per-row 64-bit keys (weight bits << 32 | reference id),
 // minimised atomically into row_keys[] (which the caller fills with ~0 first). Rows are

@@ -54,7 +54,8 @@ struct RefinedBuffers {
     int cell_levels = 1;        // norm levels per cell of the last sort_by_cells
     bool pivots_valid = false;  // pivot_d holds distances of the current fit's rows
     bool no_room = false;       // the current fit's wide rows run the exact sweeps for want of memory
-    bool lean = false;          // no spatial order of plain fits or batches, no lists, no wide screens
+    int lean = 0;               // 1 and up: no spatial order of plain fits or batches, no lists, no wide
+                                // screens; 2: batches searched in one part
     bool listed = false;        // the current fit's kNN list screens run lists of tiles
     // CUDA events around the kNN list screen's launch (created on first use); screen_timed
     // says they hold the current fit's launch

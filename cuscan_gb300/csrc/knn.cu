@@ -746,7 +746,7 @@ template <int L>
 int run_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, int64_t nr, int d,
             int k, int exclude_self, int64_t query_offset, int squared, int32_t *ids, float *dist,
             cudaStream_t s, Buffer &scratch_ids, Buffer &scratch_dist, const int32_t *qmap,
-            int64_t *launches) {
+            int64_t *launches, bool one_part) {
     const float pad = squared ? std::numeric_limits<float>::infinity() : 3.40282346638528859812e+38f;
     int64_t splits = 1, chunk = 0;
     knn_split_plan(ctx, nq, nr, splits, chunk, d, k);
@@ -756,7 +756,8 @@ int run_knn(cuscan_ctx *ctx, const float *query, int64_t nq, const float *ref, i
     // workspace in the graph, which a later call could free.
     if (splits > 1 && capturing(s) &&
         (L > 1 || scratch_ids.bytes < list_bytes || scratch_dist.bytes < list_bytes))
-        splits = 1;
+        one_part = true;
+    if (one_part) splits = 1;
     if (splits > 1) {
         int rc = ensure(ctx, scratch_ids, list_bytes, "kNN partial ids");
         if (!rc) rc = ensure(ctx, scratch_dist, list_bytes, "kNN partial distances");
@@ -842,7 +843,7 @@ int launch_exact_knn_fp32(cuscan_ctx *ctx, const float *query, int64_t nq, const
                           int64_t nr, int d, int k, int exclude_self, int64_t query_offset,
                           int squared, int32_t *ids, float *dist, cudaStream_t s,
                           Buffer &scratch_ids, Buffer &scratch_dist, const int32_t *qmap,
-                          int64_t *launches) {
+                          int64_t *launches, bool one_part) {
     if (nq == 0) return CUSCAN_OK;
     if (d > CUSCAN_PACK_MAX_FEATURES)
         return fail(ctx, CUSCAN_CAPACITY,
@@ -865,7 +866,7 @@ int launch_exact_knn_fp32(cuscan_ctx *ctx, const float *query, int64_t nq, const
     }
 #define CUSCAN_RUN_KNN(L)                                                                        \
     run_knn<L>(ctx, query, nq, ref, nr, d, k, exclude_self, query_offset, squared, ids, dist, s, \
-               scratch_ids, scratch_dist, qmap, launches)
+               scratch_ids, scratch_dist, qmap, launches, one_part)
     if (k == 1) return CUSCAN_RUN_KNN(0);
     if (k <= 32) return CUSCAN_RUN_KNN(1);
     if (k <= 64) return CUSCAN_RUN_KNN(2);

@@ -45,26 +45,35 @@ struct cuscan_predictor {
     std::vector<double> cores;   // prediction core distances (Euclidean, f64)
     float *train = nullptr;      // device copy of the finite training rows [n_finite, d]
     // the same rows in spatial order, their compact ids, the toured pivots and the tile bounds: large
-    // batches search only the tiles near their queries (empty below kSpatialWork and where the copy
+    // batches search only the tiles near their queries (empty where none would, and where the copy
     // would take a large share of the free memory, kSpatialShare). Small batches search the rows in
     // the order of their ids: 63 queries against 100,000 x 64 rows 166 us, against the spatial copy
     // 218 us. Large batches that gather the rows of the order instead of a copy: 4,096 queries
     // 1.83 ms against 1.70 ms.
     cuscan::Buffer rows, ids, pivots, centre, radius;
     int npiv = 0;
+    float apart = 0.0f;          // share of row pairs in cells too far apart to hold neighbours
     cuscan::TileBounds bounds;
 };
 
 namespace cuscan {
-int64_t predict_workspace_bound(const cuscan_predictor *p, int64_t m, bool lean);
+int64_t predict_workspace_bound(const cuscan_predictor *p, int64_t m, int lean);
 namespace {
 
-// Work (query rows x training rows x features) of a batch from which its search runs in spatial
-// order. Ordering the batch costs about 50 us, the plain search about 1 s per 13e12:
-// 4,096 queries against 100,000 x 64 rows (2.6e10) take 1.1 ms instead of 2.4 ms, 63 queries
-// (4e8) 0.09 ms in the plain search.
-constexpr double kSpatialWork = 2e9;
-constexpr int64_t kSpatialQueries = 256;  // fewer queries are few tiles, each spread over the data
+// Where a batch is searched in spatial order. The order pads the queries of every cell to whole balls
+// and adds thresholds and bounds before the first distance; what it leaves out depends on how far the
+// training rows' cells lie apart (`apart`: the share of row pairs in cells too far apart to hold
+// neighbours). Batches through the predictor, plain search against spatial search, us, k = 10:
+//   apart 0.97 (40 clusters), 100,000 x 64: 1,024 queries 898, 1,346; 2,048: 1,586, 1,293; 4,096: 2,876, 1,623
+//                             100,000 x 16: 2,048 queries 865, 858; 4,096: 1,453, 1,143
+//                             300,000 x 64: 1,024 queries 2,019, 2,081; 2,048: 3,718, 2,420
+//   apart 0.66 (3 clusters),  100,000 x 64: 2,048 queries 1,581, 1,754; 4,096: 2,869, 2,578
+//   apart 0 (overlapping),    100,000 x 64: 4,096 queries 2,884, 3,885; 300,000 x 64: 256 queries 667, 3,837
+// and with fewer than 256 cells (30,000 x 128, k = 30, apart 0.97): 4,096 queries 2,866, 2,903.
+constexpr int64_t kSpatialRows = 256 * (int64_t)kMaxPivots;  // training rows with every cell
+constexpr float kSpatialApart = 0.6f, kSpatialFarApart = 0.9f;
+constexpr int64_t kSpatialQueries = 4096, kSpatialFarQueries = 2048;  // 16 and 8 of a cell
+constexpr double kSpatialWork = 3e9;  // queries x rows x features
 // The spatial copy takes at most this share of the free device memory, so that a predictor whose rows
 // are large against the device holds them once.
 constexpr double kSpatialShare = 1.0 / 8.0;
@@ -77,11 +86,12 @@ void free_rows(cuscan_predictor &P) {
 }
 
 bool searches_spatially(const cuscan_predictor &P, int64_t m) {
-    return P.bounds.centre && m >= kSpatialQueries &&
+    return P.bounds.centre &&
+           m >= (P.apart >= kSpatialFarApart ? kSpatialFarQueries : kSpatialQueries) &&
            (double)m * (double)P.n_finite * (double)P.d >= kSpatialWork;
 }
 
-// The spatial copy of the training rows.
+// The spatial copy of the training rows, where their cells lie apart.
 int copy_spatial(cuscan_ctx *ctx, cuscan_predictor &P) {
     const int64_t n = P.n_finite;
     const int d = P.d;
@@ -89,6 +99,8 @@ int copy_spatial(cuscan_ctx *ctx, cuscan_predictor &P) {
     cudaStream_t s = ctx->stream;
     int rc = forest_reserve(ctx, b, n, d);
     if (!rc) rc = sort_by_cells(ctx, b, P.train, n, d, s);
+    if (!rc) rc = read_apart(ctx, b, n, P.apart, s);
+    if (rc || P.apart < kSpatialApart) return rc;
     P.npiv = cell_pivots(n);
     if (!rc) rc = ensure(ctx, P.rows, sizeof(float) * n * d, "predictor rows");
     if (!rc) rc = ensure(ctx, P.ids, sizeof(int32_t) * n, "predictor ids");
@@ -102,12 +114,12 @@ int copy_spatial(cuscan_ctx *ctx, cuscan_predictor &P) {
                                      sizeof(float) * P.npiv * d, cudaMemcpyDeviceToDevice, s));
     return tile_bounds(ctx, as<float>(P.rows), n, d, P.centre, P.radius, P.bounds, s);
 }
-// The same when a batch of 4,096 queries would use it and there is ample room. Without the copy the
+// The same when a batch of kSpatialQueries would use it and there is ample room. Without the copy the
 // predictor searches its plain rows. The workspace that the order took beyond what the context held
 // is given back.
 int build_spatial(cuscan_ctx *ctx, cuscan_predictor &P) {
-    if (P.n_finite < 2048 || !knn_pruned_shape(P.d, 2 * P.s) ||
-        4096.0 * (double)P.n_finite * (double)P.d < kSpatialWork)
+    if (P.n_finite < kSpatialRows || !knn_pruned_shape(P.d, 2 * P.s) ||
+        (double)kSpatialQueries * (double)P.n_finite * (double)P.d < kSpatialWork)
         return CUSCAN_OK;
     size_t room = 0, total = 0;
     CUSCAN_CUDA(ctx, cudaMemGetInfo(&room, &total));
@@ -736,16 +748,16 @@ int cuscan_predictor_shape(const cuscan_predictor *p, int64_t *n_finite, int32_t
 }
 
 int64_t cuscan_predict_workspace_bytes(const cuscan_predictor *p, int64_t m) {
-    return predict_workspace_bound(p, m, false);
+    return predict_workspace_bound(p, m, 0);
 }
 
 }  // extern "C"
 
-int64_t cuscan::predict_workspace_bound(const cuscan_predictor *p, int64_t m, bool lean) {
+int64_t cuscan::predict_workspace_bound(const cuscan_predictor *p, int64_t m, int lean) {
     if (!p || m <= 0) return 0;
     const int64_t k = 2 * (int64_t)p->s;
-    // query rows, candidate ids and distances, split-search partial lists
-    int64_t bytes = 8 * k * simt::split_max_rows(m, p->n_finite);
+    // query rows, candidate ids and distances, lists of the search's parts
+    int64_t bytes = lean >= 2 ? 0 : 8 * k * simt::split_max_rows(m, p->n_finite);
     if (!lean && searches_spatially(*p, m)) {
         const int64_t pruned = pruned_partial_bytes(padded_queries(m), p->n_finite, (int)k);
         if (pruned > bytes) bytes = pruned;
@@ -856,7 +868,8 @@ int predict_queries(cuscan_ctx *ctx, const cuscan_predictor *p, const float *que
     if (!spatial) {
         rc = launch_exact_knn_fp32(ctx, as<float>(f->pred_q), m, p->train, p->n_finite, p->d, k, 0, 0,
                                    1, as<int32_t>(f->pred_ids), as<float>(f->pred_dist), s,
-                                   f->op_knn_ids, f->op_knn_dist);
+                                   f->op_knn_ids, f->op_knn_dist, nullptr, nullptr,
+                                   f->forest.refined.lean >= 2);
     }
     if (rc) return rc;
     std::vector<int32_t> ids((size_t)m * k);

@@ -42,13 +42,14 @@
 
 #include "cuscan_gb300.h"
 
-// Library-internal: bounds and execution of a request in less device memory (without the spatial
-// order of plain fits and of query batches, the tile lists and the screens of more than 128
-// features or 32 neighbours). A request whose full bound exceeds the server's budget runs so when that fits.
+// Library-internal: bounds and execution of a request in less device memory. Level 1 does without the
+// spatial order of plain fits and of query batches, the tile lists and the screens of more than 128
+// features or 32 neighbours; level 2 also searches query batches in one part. A request whose full
+// bound exceeds the server's budget runs at the first level that fits.
 namespace cuscan {
-int64_t fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, int32_t precision, bool lean);
-int64_t predict_workspace_bound(const cuscan_predictor *p, int64_t m, bool lean);
-void set_lean(cuscan_ctx *ctx, bool lean);
+int64_t fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, int32_t precision, int lean);
+int64_t predict_workspace_bound(const cuscan_predictor *p, int64_t m, int lean);
+void set_lean(cuscan_ctx *ctx, int lean);
 }  // namespace cuscan
 
 namespace {
@@ -76,8 +77,8 @@ struct Request {
     int32_t precision = 0;
     cuscan_extract_config cfg{};
     int64_t bytes = 0;  // admission bound
-    int64_t lean_bytes = 0;
-    bool lean = false;
+    int64_t lean_bytes[2] = {0, 0};  // the same at levels 1 and 2
+    int lean = 0;
     Clock::time_point t_submit, t_admit, t_done;
     double prep_ms = 0, fit_ms = 0, extract_ms = 0;  // host wall time of the three phases
     int slot = -1;
@@ -494,10 +495,11 @@ struct cuscan_server {
         *request_id = r->id;
         ++submitted;
         Request *raw = r.get();
-        if (raw->bytes > budget && raw->lean_bytes < raw->bytes) {
-            raw->lean = true;
-            raw->bytes = raw->lean_bytes;
-        }
+        for (int level = 1; level <= 2 && raw->bytes > budget; ++level)
+            if (raw->lean_bytes[level - 1] < raw->bytes) {
+                raw->lean = level;
+                raw->bytes = raw->lean_bytes[level - 1];
+            }
         requests.emplace(r->id, std::move(r));
         if (raw->bytes > budget) {
             raw->status = CUSCAN_MEMORY;
@@ -645,7 +647,9 @@ int cuscan_server_submit_fit(cuscan_server *s, const float *data, int64_t n, int
     r->precision = precision;
     r->cfg = *config;
     r->bytes = cuscan_fit_workspace_bytes(n < 2 ? 2 : n, d, min_samples, precision);
-    r->lean_bytes = cuscan::fit_workspace_bound(n < 2 ? 2 : n, d, min_samples, precision, true);
+    for (int level = 1; level <= 2; ++level)
+        r->lean_bytes[level - 1] =
+            cuscan::fit_workspace_bound(n < 2 ? 2 : n, d, min_samples, precision, level);
     r->t_submit = Clock::now();
     return s->enqueue(std::move(r), request_id);
 }
@@ -667,7 +671,8 @@ int cuscan_server_submit_predict(cuscan_server *s, const cuscan_predictor *predi
     r->d = d;
     r->min_samples = ms;
     r->bytes = cuscan_predict_workspace_bytes(predictor, m);
-    r->lean_bytes = cuscan::predict_workspace_bound(predictor, m, true);
+    for (int level = 1; level <= 2; ++level)
+        r->lean_bytes[level - 1] = cuscan::predict_workspace_bound(predictor, m, level);
     r->t_submit = Clock::now();
     return s->enqueue(std::move(r), request_id);
 }

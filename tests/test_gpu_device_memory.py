@@ -10,6 +10,7 @@ import pytest
 import cuscan_gb300 as cg
 from cuscan_gb300 import _lib, synthetic
 from oracle import oracle as O
+from tests.test_gpu_first_calls import searches_spatially
 from tests.test_gpu_fit import assert_fit_equal
 from tests.test_gpu_ops import bits
 
@@ -106,7 +107,6 @@ def spatial_model(n, d, m):
 def test_predictors_leave_no_workspace_and_copy_their_rows_only_with_ample_room():
     n, d, m = 100_000, 64, 4096
     model, x = spatial_model(n, d, m)
-    assert 4096.0 * n * d >= 2e9  # a copy in spatial order
     arrays, meta = model.to_predictor()._predictor.export_state()
     np.testing.assert_array_equal(arrays["geometry"].reshape(n, d), x[:n])
     rows = 4 * n * d
@@ -120,6 +120,7 @@ def test_predictors_leave_no_workspace_and_copy_their_rows_only_with_ample_room(
             predictor = cg.prediction.Predictor.from_state(arrays, meta, ctx)
             # (ids, bounds and up to 2 MiB of rounding per allocation beside the rows)
             assert copies * rows <= free - free_bytes() < (copies + 0.5) * rows
+            assert searches_spatially(predictor, m) == (copies == 2)
             assert ctx.reserved_bytes() == 0
             results.append(predictor.predict(x[n:]))
 
@@ -132,12 +133,3 @@ def test_predictors_leave_no_workspace_and_copy_their_rows_only_with_ample_room(
         np.testing.assert_array_equal(a, b)
 
 
-@pytest.mark.parametrize("m", [1, 130, 1500])
-def test_batches_against_rows_in_spatial_order_equal_the_oracle(m):
-    n, d = 8000, 64
-    model, x = spatial_model(n, d, m)
-    assert 4096.0 * n * d >= 2e9
-    got = model.to_predictor().approximate_predict(x[n:], True)
-    exp = O.approximate_predict(model.condensed_tree_, model.labels_, np.arange(n), 5, x[:n], x[n:])
-    for a, b in zip(got, exp):
-        np.testing.assert_array_equal(a, b)

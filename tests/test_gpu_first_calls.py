@@ -47,6 +47,16 @@ def self_knn(ctx, x, k):
     return ids.cpu().numpy(), ds.cpu().numpy()
 
 
+def searches_spatially(predictor, m):
+    """Whether a batch of m queries is searched in spatial order: its bound has the order's arrays."""
+    k, n = 2 * predictor.min_samples, predictor.n_finite
+    lists = 8 * k * min(512 * 152 + m, m * -(-(-(-n // 128)) // 2))
+    plain = 4 * m * predictor.n_features_in_ + 8 * m * k + lists + (1 << 20)
+    bound = cg.load().cuscan_predict_workspace_bytes(predictor.handle, m)
+    assert bound >= plain
+    return bound > plain
+
+
 @pytest.mark.parametrize("n,d,k", [(2048, 32, 5), (5003, 64, 10), (2600, 200, 15)])
 @pytest.mark.parametrize("released", [False, True])
 def test_exact_knn_needs_no_fit_before_it(gpu_ctx, n, d, k, released):
@@ -65,21 +75,21 @@ def test_exact_knn_needs_no_fit_before_it(gpu_ctx, n, d, k, released):
 
 @pytest.mark.parametrize("restored", [False, True])
 def test_a_predictor_needs_no_fit_before_it(restored):
-    n, d, m = 8000, 64, 4096
+    n, d, m = 66_000, 16, 4096
     x = synthetic.gaussian_mixture(n + m, d, 10, seed=3)
     model = cg.HDBSCAN(min_cluster_size=50, min_samples=5, precision="fp16_refined").fit(x[:n])
     if restored:
         arrays, meta = model.to_predictor()._predictor.export_state()
         ctx = _lib.Context(0)
         fill_free_memory()
-        predict = cg.prediction.Predictor.from_state(arrays, meta, ctx).predict
+        predictor = cg.prediction.Predictor.from_state(arrays, meta, ctx)
     else:
         cg.context(0).release_workspace()
         fill_free_memory()
-        predict = model.to_predictor()._predictor.predict
+        predictor = model.to_predictor()._predictor
     # a batch large enough for the spatial search, against pieces searched plainly
-    assert float(m) * n * d >= 2e9
-    whole = predict(x[n:])
-    parts = [predict(x[a:a + 200]) for a in range(n, n + m, 200)]
+    assert searches_spatially(predictor, m) and not searches_spatially(predictor, 200)
+    whole = predictor.predict(x[n:])
+    parts = [predictor.predict(x[a:a + 200]) for a in range(n, n + m, 200)]
     for got, exp in zip(whole, zip(*parts)):
         np.testing.assert_array_equal(got, np.concatenate(exp))
