@@ -21,8 +21,9 @@ int sort_by_cells(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, 
                   cudaStream_t s);
 // Device bytes of sort_by_cells beyond the forest's own buffers.
 inline size_t cells_workspace_bytes(int64_t n, int d) {
-    return sizeof(float) * (2 * (size_t)kMaxPivots * d + (size_t)kMaxPivots * kMaxPivots +
-                            4 * kMaxPivots) + 16 * (size_t)n;  // cells, distances, norms, keys
+    const size_t npiv = (size_t)cell_pivots(n);
+    return sizeof(float) * (2 * npiv * d + (npiv + 1) * npiv + 3 * kMaxPivots) + 32 +
+           16 * (size_t)n;  // cells, distances, norms, keys
 }
 // Query orders for the pruned sweeps: the rows grouped by cell, every cell padded to whole balls of
 // kBallRows entries with -1, so that no ball straddles two cells. A straddling ball is as wide as

@@ -128,6 +128,7 @@ constexpr int64_t SYM_MIN_ROWS = 131072;     // smallest point set for the symme
 constexpr double SYM_ACTIVE_MIN = 0.9;  // smallest share of screened rows for the symmetric screen
 constexpr int KNN_CAP = 512;  // threshold-mode candidate slots per row half
 constexpr int KNN_LIST = 22;  // kNN list entries per row half
+static_assert(KNN_LIST <= BORUVKA_CAP, "the candidate buffer of the rounds holds the lists");
 constexpr int RESCREEN_MIN_ROWS = 256;  // fewer inconclusive kNN rows go straight to exact f32
 // A bf16-refined fit whose first kNN screen leaves more than this share of rows inconclusive
 // screens again with tighter operands (split bf16, or scaled fp16 for rows too wide to split).
@@ -1818,14 +1819,14 @@ static bool refined_shape_ok(int64_t n, int d, int k) {
 size_t refined_workspace_bytes(int64_t n, int d, int k, bool lean) {
     Layout L;
     if ((lean && lean_exact(d, k)) || !refined_shape_ok(n, d, 1) || !refined_layout(n, d, L)) return 0;
-    constexpr size_t M = 32;
     // a bf16-refined fit may switch to split copies (twice the columns) when d <= 64
     const size_t copy_cols = (size_t)L.d_pad * (L.d_pad <= 64 ? 2 : 1);
     size_t b = (size_t)L.n_pad * copy_cols * 2 + 2 * sizeof(float) * (size_t)L.n_pad;  // xt, norms
     b += 3 * sizeof(float) * (size_t)L.n_tiles + 64;          // tile stats, flags, cursor
     b += 2 * sizeof(float) * (size_t)L.n_pad + sizeof(float) * (size_t)L.n_pad / 16;  // column terms
     b += sizeof(int32_t) * (size_t)n;                                                 // fallback
-    b += 2 * 4 * (size_t)n * 2 * M;                  // candidate ids and bounds (two lists of M)
+    // candidates of both row halves, and with lists their bounds
+    b += 4 * (size_t)n * 2 * BORUVKA_CAP + (k <= SCREEN_MAX_K ? 4 * (size_t)n * 2 * KNN_LIST : 0);
     b += sizeof(uint32_t) * (size_t)n + 2 * sizeof(int32_t) * (size_t)n;  // cbound, rowcnt
     b += cells_workspace_bytes(n, d);
     // gathered query rows (subset rounds, threshold re-screen): tiles and norms
@@ -2013,7 +2014,8 @@ static int run_screen(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, int64
                       const QuerySet &Q = QuerySet()) {
     constexpr bool BORUVKA = MODE == MODE_BORUVKA || MODE == MODE_BORUVKA_SYM;
     int rc = ensure(ctx, R.cand_ids, sizeof(int32_t) * n * 2 * M, "screen candidates");
-    if (!rc) rc = ensure(ctx, R.cand_lb, sizeof(float) * n * 2 * M, "screen bounds");
+    if (!rc && MODE == MODE_KNN_LIST)  // the lists; other forms append candidates without bounds
+        rc = ensure(ctx, R.cand_lb, sizeof(float) * n * 2 * M, "screen bounds");
     if (rc) return rc;
     Params P{};
     P.xt = as<uint8_t>(R.xt);
