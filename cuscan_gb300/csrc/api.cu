@@ -24,6 +24,7 @@ int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, i
                                  const int32_t *knn_ids, const float *knn_sq, int k,
                                  const float *core, const int32_t *label, cudaStream_t s,
                                  int64_t *screened_rows, const TileBounds *bounds);
+int reserve_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n);
 int debug_screen_tile(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, int d,
                       int operands, float *out, float *rows_out, float *chunk_out,
                       float *scale_out, cudaStream_t s);
@@ -280,6 +281,8 @@ static int status_error(cuscan_ctx *ctx, int kind) {
     }
 }
 
+// Plain fits of fewer rows scan every row in every round (see the rounds).
+constexpr int64_t EXACT_ROWS_MIN = 2048;
 // Fewer norm levels than this per component do not narrow a 32-row chunk's norms.
 constexpr int NORM_LEVELS_MIN = 8;
 // Rounds of fewer rows are bound by their launches, of which the norm keys are five.
@@ -323,6 +326,7 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
     ForestBuffers &b = f->forest;
     int rc = forest_reserve(ctx, b, n, d);
     if (!rc) rc = ensure(ctx, f->label, sizeof(int32_t) * n, "point labels");
+    if (!rc && !refined && n >= EXACT_ROWS_MIN) rc = reserve_exact_rows(ctx, b, n);
     if (rc) return rc;
     const int k = (int)((int64_t)min_samples < n - 1 ? min_samples : n - 1);
     int32_t *label = as<int32_t>(f->label);
@@ -364,6 +368,8 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
         if (rc == CUSCAN_MEMORY) {  // no room for the order or the partial lists: the plain sweeps
             clear_error(ctx);
             spatial = false;
+            forest_release_refined(b);
+            if ((rc = reserve_exact_rows(ctx, b, n))) return rc;
         }
     }
     if (!refined && !spatial)
@@ -386,7 +392,7 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
     f->round_count = 0;
     // exact rounds of fits of at least 2048 rows scan only the rows that can hold their
     // component's cheapest edge (smaller fits scan every row: one host read per round fewer)
-    const bool exact_rows = !refined && n >= 2048;
+    const bool exact_rows = !refined && n >= EXACT_ROWS_MIN;
     while (components > 1) {
         const int64_t rows0 = b.refined.screened_rows, tiles0 = b.refined.tile_pairs;
         if (rounds > 64) return fail(ctx, CUSCAN_NUMERICAL, "Boruvka did not converge");

@@ -1120,6 +1120,7 @@ int forest_reserve(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d) {
     RES(tile_lo, sizeof(int32_t) * (size_t)(ceil_div(n, 32) + 1), "tile label ranges");
     RES(tile_hi, sizeof(int32_t) * (size_t)(ceil_div(n, 32) + 1), "tile label ranges");
     RES(status_buf, sizeof(DevStatus), "fit status");
+    RES(scan_tmp, sizeof(int32_t) * (size_t)ceil_div(n, SCAN_TILE), "scan tile sums");
 #undef RES
     b.status = as<DevStatus>(b.status_buf);
     return CUSCAN_OK;
@@ -1145,6 +1146,14 @@ int forest_buffers(ForestBuffers &b, Buffer **out) {
     if (out)
         for (int i = 0; i < count; ++i) out[i] = all[i];
     return count;
+}
+
+void forest_release_refined(ForestBuffers &b) {
+    Buffer *all[kForestBufferCount];
+    const int count = forest_buffers(b, all);
+    int first = 0;
+    while (all[first] != &b.knn_ids_tmp) ++first;  // the list above: the rest follows the forest's own
+    for (int i = first; i < count; ++i) release(*all[i]);
 }
 
 void forest_release(ForestBuffers &b) {

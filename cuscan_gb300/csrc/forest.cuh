@@ -56,6 +56,7 @@ struct RefinedBuffers {
     bool no_room = false;       // the current fit's wide rows run the exact sweeps for want of memory
     int lean = 0;               // 1 and up: no spatial order of plain fits or batches, no lists, no wide
                                 // screens; 2: batches searched in one part
+    bool no_lists = false;      // the current fit's screens visit every tile for want of memory
     bool listed = false;        // the current fit's kNN list screens run lists of tiles
     // CUDA events around the kNN list screen's launch (created on first use); screen_timed
     // says they hold the current fit's launch
@@ -79,6 +80,9 @@ struct ForestBuffers {
 
 int forest_reserve(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int d);
 void forest_release(ForestBuffers &b);
+// The buffers beyond the forest's own, and the partial lists of its kNN sweeps: what a fit that goes on
+// with the plain exact sweeps can give back.
+void forest_release_refined(ForestBuffers &b);
 // Every device buffer of the forest and of the bf16 screen (out may be null); returns the count.
 constexpr int kForestBufferCount = 78;
 int forest_buffers(ForestBuffers &b, Buffer **out);

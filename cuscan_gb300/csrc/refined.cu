@@ -2160,6 +2160,17 @@ static int knn_list_pass(cuscan_ctx *ctx, RefinedBuffers &R, const Layout &L, co
     return read_screen_status(ctx, R, s, fallbacks);
 }
 
+// Whether there was something to release.
+static bool release_lists(RefinedBuffers &R) {
+    bool held = false;
+    for (Buffer *b : {&R.ball_thr, &R.vis, &R.vis_count, &R.tile_centre, &R.tile_radius}) {
+        held |= b->ptr != nullptr;
+        release(*b);
+    }
+    R.listed = false;
+    return held;
+}
+
 static int knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, int d, int k,
                        int32_t *ids, float *dist, cudaStream_t s, int64_t *refined_rows,
                        int64_t *fallback_rows, int64_t *rescreened_rows) {
@@ -2182,10 +2193,13 @@ static int knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
         return launch_exact_knn_fp32(ctx, x, n, x, n, d, k, 1, 0, 1, ids, dist, s, b.knn_ids_tmp,
                                      b.knn_dist_tmp);
     R.pivots_valid = true;
-    if (!R.lean && n >= LIST_MIN_ROWS && L.n_tiles <= kMaxVisitTiles && apart > LIST_MIN_APART) {
+    if (!R.lean && !R.no_lists && n >= LIST_MIN_ROWS && L.n_tiles <= kMaxVisitTiles && apart > LIST_MIN_APART) {
         if ((rc = visit_lists(ctx, b, n, d, k, s)) && rc != CUSCAN_MEMORY) return rc;
         R.listed = rc == CUSCAN_OK;  // without room for the lists every tile is visited
-        if (rc) clear_error(ctx);
+        if (rc) {
+            release_lists(R);
+            clear_error(ctx);
+        }
     }
     // the tightened operands: split bf16, or scaled fp16 for rows too wide to split
     auto tighten = [&]() {
@@ -2270,17 +2284,30 @@ static int knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_
     return CUSCAN_OK;
 }
 
-// Wide rows take more device memory on the screens than in the exact sweeps: without room for it the
-// fit goes on with those.
+// Lists of tiles are given up where the screens' own buffers have no room beside them. Wide rows take
+// more device memory on the screens than in the exact sweeps: without room for it the fit goes on with
+// those.
 int launch_knn_refined(cuscan_ctx *ctx, ForestBuffers &b, const float *x, int64_t n, int d, int k,
                        int32_t *ids, float *dist, cudaStream_t s, int64_t *refined_rows,
                        int64_t *fallback_rows, int64_t *rescreened_rows) {
     b.refined.no_room = false;
-    const int rc =
-        knn_refined(ctx, b, x, n, d, k, ids, dist, s, refined_rows, fallback_rows, rescreened_rows);
+    b.refined.no_lists = false;
+    auto screens = [&]() {
+        for (int64_t *rows : {refined_rows, fallback_rows, rescreened_rows})
+            if (rows) *rows = 0;
+        return knn_refined(ctx, b, x, n, d, k, ids, dist, s, refined_rows, fallback_rows,
+                           rescreened_rows);
+    };
+    int rc = screens();
+    if (rc == CUSCAN_MEMORY && release_lists(b.refined)) {
+        clear_error(ctx);
+        b.refined.no_lists = true;
+        rc = screens();
+    }
     if (rc != CUSCAN_MEMORY || d <= LEAN_MAX_FEATURES) return rc;
     clear_error(ctx);
     b.refined.no_room = true;
+    forest_release_refined(b);
     for (int64_t *rows : {refined_rows, fallback_rows, rescreened_rows})
         if (rows) *rows = 0;
     return launch_exact_knn_fp32(ctx, x, n, x, n, d, k, 1, 0, 1, ids, dist, s, b.knn_ids_tmp,
@@ -2435,11 +2462,29 @@ int launch_candidates_refined(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int 
                               const float *core, const int32_t *label, cudaStream_t s,
                               int64_t *fallback_rows) {
     int rc = candidates_refined(ctx, b, n, d, knn_ids, knn_sq, k, core, label, s, fallback_rows);
+    if (rc == CUSCAN_MEMORY && release_lists(b.refined)) {
+        clear_error(ctx);
+        rc = candidates_refined(ctx, b, n, d, knn_ids, knn_sq, k, core, label, s, fallback_rows);
+    }
     if (rc == CUSCAN_MEMORY && d > LEAN_MAX_FEATURES) {
         clear_error(ctx);
         b.refined.no_room = true;
+        b.refined.pivots_valid = false;
+        forest_release_refined(b);
         rc = candidates_refined(ctx, b, n, d, knn_ids, knn_sq, k, core, label, s, fallback_rows);
     }
+    return rc;
+}
+
+// Device memory of the exact rounds (a fit takes it before the spatial order, which it can do without).
+int reserve_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n) {
+    RefinedBuffers &R = b.refined;
+    int rc = ensure(ctx, R.cbound, sizeof(uint32_t) * n, "component bounds");
+    if (!rc) rc = ensure(ctx, R.urow, sizeof(uint32_t) * n, "row bounds");
+    if (!rc) rc = ensure(ctx, R.act_flag, sizeof(int32_t) * n, "active rows");
+    if (!rc) rc = ensure(ctx, R.act_idx, sizeof(int32_t) * n, "active rows");
+    if (!rc) rc = ensure(ctx, R.act_pos, sizeof(int32_t) * n, "active rows");
+    if (!rc) rc = ensure(ctx, R.rowlb, sizeof(float) * n, "row lower bounds");
     return rc;
 }
 
@@ -2461,12 +2506,7 @@ int launch_candidates_exact_rows(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, i
     unsigned long long *row_keys = as<unsigned long long>(b.row_keys);
     int32_t *clo = as<int32_t>(b.tile_lo), *chi = as<int32_t>(b.tile_hi);
     RefinedBuffers &R = b.refined;
-    int rc = ensure(ctx, R.cbound, sizeof(uint32_t) * n, "component bounds");
-    if (!rc) rc = ensure(ctx, R.urow, sizeof(uint32_t) * n, "row bounds");
-    if (!rc) rc = ensure(ctx, R.act_flag, sizeof(int32_t) * n, "active rows");
-    if (!rc) rc = ensure(ctx, R.act_idx, sizeof(int32_t) * n, "active rows");
-    if (!rc) rc = ensure(ctx, R.act_pos, sizeof(int32_t) * n, "active rows");
-    if (!rc) rc = ensure(ctx, R.rowlb, sizeof(float) * n, "row lower bounds");
+    int rc = reserve_exact_rows(ctx, b, n);
     if (rc) return rc;
     if (!R.lb_valid) {  // first round of the fit: no bounds yet
         CUSCAN_CUDA(ctx, cudaMemsetAsync(R.rowlb.ptr, 0, sizeof(float) * n, s));

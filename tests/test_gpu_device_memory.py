@@ -133,3 +133,26 @@ def test_predictors_leave_no_workspace_and_copy_their_rows_only_with_ample_room(
         np.testing.assert_array_equal(a, b)
 
 
+
+
+@pytest.mark.parametrize("n,d,k,precision,left", [
+    # in spatial order 400 MB; the plain sweeps take 113 MB in blocks of 2 MiB. (With 300 to 320 MiB
+    # the order, the balls and the partial lists fit, but not the rounds' arrays beside them.)
+    (600_000, 2, 5, _lib.PRECISION_PLAIN, 200 << 20), (600_000, 2, 5, _lib.PRECISION_PLAIN, 310 << 20),
+    (600_000, 2, 5, _lib.PRECISION_PLAIN, 320 << 20),
+    # screens of wide rows 155 MB, the exact sweeps 40 MB
+    (20_000, 200, 15, _lib.PRECISION_BF16_REFINED, 60 << 20),
+])
+def test_fits_run_where_only_the_plain_sweeps_fit(n, d, k, precision, left):
+    x = synthetic.gaussian_mixture(n, d, 30, seed=7)
+    warm = _lib.Context(0)
+    full = warm.fit_core(x, k, precision)
+    assert warm.reserved_bytes() > left
+    warm.close()
+    ctx = _lib.Context(0)
+    with little_memory(left):
+        got = ctx.fit_core(x, k, precision)
+    for key in ("knn_ids", "src", "dst"):
+        np.testing.assert_array_equal(got[key], full[key])
+    for key in ("knn_sq", "core_sq", "wsq"):
+        np.testing.assert_array_equal(bits(got[key]), bits(full[key]))
