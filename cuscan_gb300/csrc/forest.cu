@@ -575,12 +575,19 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 // where the sequences have kernel boundaries, on arrays in shared memory. What bounds them is the
 // chain of dependent loads and barriers (two per pointer-doubling or path-halving step, 24 steps
 // at 2,000 points), so the arrays sit where a load takes tens of cycles instead of an L2 trip, and
-// 1,024 threads take two nodes each. Measured in a pack of eight fits of 500 to 2,047 rows on a
-// GB300, against 256 threads on global arrays: seed 16.4 us (41.0), sort 10.9 us (18.6), merge
-// 11.2 us (26.3).
+// 1,024 threads (256 up to 512 rows) take two nodes each. Measured in a pack of eight fits of 500 to
+// 2,047 rows on a GB300, against 256 threads on global arrays: seed 16.4 us (41.0), sort 10.9 us
+// (18.6), merge 11.2 us (26.3).
 constexpr int64_t SMALL_ROWS = 2048;  // nodes the arrays hold; fits of fewer points take this form
 constexpr int SMALL_THREADS = 1024;
 constexpr int SMALL_ITEMS = (int)(SMALL_ROWS / SMALL_THREADS);
+// Fits of few rows take fewer threads, whose barriers cost less: a pack of 5, 9 and 30 rows 191 us
+// instead of 201 us, eight fits of 250 rows 359 us instead of 371 us (128 threads 192 and 370 us).
+constexpr int TINY_THREADS = 256;
+constexpr int64_t TINY_ROWS = SMALL_ITEMS * (int64_t)TINY_THREADS;
+inline int small_threads(int64_t n) { return n <= TINY_ROWS ? TINY_THREADS : SMALL_THREADS; }
+// The instance of a one-CTA kernel for fits of up to n rows.
+#define CUSCAN_SMALL(kernel, n) ((n) <= TINY_ROWS ? kernel<TINY_THREADS> : kernel<SMALL_THREADS>)
 
 struct SmallForest {
     unsigned long long *comp_keys;
@@ -617,6 +624,7 @@ __device__ __forceinline__ SmallForest small_forest(void *smem) {
 // Cycle breaking, emit and union of the proposals in F.next/esrc/edst/ew (resolve_proposals).
 // The points' labels are F.label, which are also the active labels of a round; the seed
 // (active_label null) starts from labels 0..n-1. New labels leave to point_label.
+template <int T>
 __device__ __forceinline__ void resolve_block(const SmallForest &F, const int32_t *active_label,
                                               int32_t *__restrict__ point_label, int64_t n,
                                               int steps, DevStatus *status,
@@ -624,14 +632,14 @@ __device__ __forceinline__ void resolve_block(const SmallForest &F, const int32_
                                               uint32_t *__restrict__ out_dst,
                                               float *__restrict__ out_w, int64_t capacity,
                                               int require_progress) {
-    __shared__ int warp_sums[SMALL_THREADS / 32];
+    __shared__ int warp_sums[T / 32];
     const int tid = threadIdx.x;
     int32_t *ja = F.ja, *ma = F.ma, *jb = F.jb, *mb = F.mb;
     // cycle breaking: pointer doubling with a running maximum, ping-pong buffers
-    for (int64_t s = tid; s < n; s += SMALL_THREADS) dbl_init_at(s, F.next, active_label, ja, ma);
+    for (int64_t s = tid; s < n; s += T) dbl_init_at(s, F.next, active_label, ja, ma);
     __syncthreads();
     for (int t = 0; t < steps; ++t) {
-        for (int64_t s = tid; s < n; s += SMALL_THREADS)
+        for (int64_t s = tid; s < n; s += T)
             dbl_step_at(s, ja, ma, active_label, jb, mb);
         __syncthreads();
         int32_t *tj = ja, *tm = ma;
@@ -640,7 +648,7 @@ __device__ __forceinline__ void resolve_block(const SmallForest &F, const int32_
         jb = tj;
         mb = tm;
     }
-    for (int64_t s = tid; s < n; s += SMALL_THREADS)
+    for (int64_t s = tid; s < n; s += T)
         keep_at(s, F.next, ja, ma, active_label, F.keep, F.parent);
     __syncthreads();
     // exclusive scan of keep in node order: thread t holds nodes [t SMALL_ITEMS, +SMALL_ITEMS)
@@ -653,7 +661,7 @@ __device__ __forceinline__ void resolve_block(const SmallForest &F, const int32_
         sum += v[u];
     }
     int total;
-    int prefix = block_exclusive_scan<SMALL_THREADS>(sum, warp_sums, total);
+    int prefix = block_exclusive_scan<T>(sum, warp_sums, total);
 #pragma unroll
     for (int u = 0; u < SMALL_ITEMS; ++u) {
         if (base + u < n) F.pos[base + u] = prefix;
@@ -662,7 +670,7 @@ __device__ __forceinline__ void resolve_block(const SmallForest &F, const int32_
     __syncthreads();
     // append the kept edges in node order after the edges emitted so far
     const int64_t edges = (int64_t)status->edges;
-    for (int64_t s = tid; s < n; s += SMALL_THREADS)
+    for (int64_t s = tid; s < n; s += T)
         emit_at(s, F.keep, F.pos, F.esrc, F.edst, F.ew, edges, out_src, out_dst, out_w, capacity);
     __syncthreads();
     if (tid == 0) {
@@ -672,17 +680,17 @@ __device__ __forceinline__ void resolve_block(const SmallForest &F, const int32_
     }
     // union: path halving, smallest point of every tree, relabel, count the components
     for (int t = 0; t < steps; ++t) {
-        for (int64_t s = tid; s < n; s += SMALL_THREADS) jump_at(s, F.parent, active_label);
+        for (int64_t s = tid; s < n; s += T) jump_at(s, F.parent, active_label);
         __syncthreads();
     }
-    for (int64_t s = tid; s < n; s += SMALL_THREADS)
+    for (int64_t s = tid; s < n; s += T)
         minlab_init_at(s, F.parent, active_label, F.minlab);
     __syncthreads();
-    for (int64_t s = tid; s < n; s += SMALL_THREADS)
+    for (int64_t s = tid; s < n; s += T)
         minlab_reduce_at(s, F.parent, active_label, F.minlab);
     __syncthreads();
     int roots = 0;
-    for (int64_t i0 = 0; i0 < n; i0 += SMALL_THREADS) {
+    for (int64_t i0 = 0; i0 < n; i0 += T) {
         const int64_t i = i0 + tid;
         int32_t l = -1;
         if (i < n) {
@@ -695,40 +703,42 @@ __device__ __forceinline__ void resolve_block(const SmallForest &F, const int32_
 }
 
 // Core column, seed proposals and their merge (core_kernel, seed_kernel, resolve_proposals).
+template <int T>
 __device__ __forceinline__ void small_seed(const PackFit &f, void *smem) {
     const SmallForest F = small_forest(smem);
     const int64_t n = f.n;
-    for (int64_t i = threadIdx.x; i < n; i += SMALL_THREADS)
+    for (int64_t i = threadIdx.x; i < n; i += T)
         core_at(i, f.dsq, n, f.k, f.min_samples, f.core);
     __syncthreads();
-    for (int64_t i = threadIdx.x; i < n; i += SMALL_THREADS)
+    for (int64_t i = threadIdx.x; i < n; i += T)
         seed_at(i, f.core, f.ids, f.dsq, n, f.k, F.next, F.esrc, F.edst, F.ew, f.status);
     __syncthreads();
-    resolve_block(F, nullptr, f.label, n, log2_ceil_dev(n > 1 ? n : 2) + 1, f.status, f.src, f.dst,
+    resolve_block<T>(F, nullptr, f.label, n, log2_ceil_dev(n > 1 ? n : 2) + 1, f.status, f.src, f.dst,
                   f.w, n - 1, 0);
 }
 
 // Start of a round: counting sort by label (histogram, sum of squared sizes, exclusive scan and
 // scatter; the order of points within a label is free, as in scatter_kernel), the sorted labels
 // and core distances, cleared row keys and the label range of every 32-row tile.
+template <int T>
 __device__ __forceinline__ void small_sort(const PackFit &f, void *smem) {
     const SmallForest F = small_forest(smem);
     int32_t *cnt = F.next, *start = F.ja, *fill = F.ma, *perm = F.jb, *labp = F.mb;
-    __shared__ int warp_sums[SMALL_THREADS / 32];
-    __shared__ double pair_sums[SMALL_THREADS / 32];
+    __shared__ int warp_sums[T / 32];
+    __shared__ double pair_sums[T / 32];
     const int tid = threadIdx.x;
     const int64_t n = f.n;
-    for (int64_t i = tid; i < n; i += SMALL_THREADS) {
+    for (int64_t i = tid; i < n; i += T) {
         cnt[i] = 0;
         fill[i] = 0;
         F.label[i] = f.label[i];
     }
     __syncthreads();
-    for (int64_t i = tid; i < n; i += SMALL_THREADS) atomicAdd(&cnt[F.label[i]], 1);
+    for (int64_t i = tid; i < n; i += T) atomicAdd(&cnt[F.label[i]], 1);
     __syncthreads();
     // sum of squared sizes (exact in f64: integers below 2^53)
     double v = 0.0;
-    for (int64_t i = tid; i < n; i += SMALL_THREADS) {
+    for (int64_t i = tid; i < n; i += T) {
         const double c = (double)cnt[i];
         v += c * c;
     }
@@ -744,7 +754,7 @@ __device__ __forceinline__ void small_sort(const PackFit &f, void *smem) {
         sum += c[u];
     }
     int total;
-    int prefix = block_exclusive_scan<SMALL_THREADS>(sum, warp_sums, total);
+    int prefix = block_exclusive_scan<T>(sum, warp_sums, total);
 #pragma unroll
     for (int u = 0; u < SMALL_ITEMS; ++u) {
         if (base + u < n) start[base + u] = prefix;
@@ -752,16 +762,16 @@ __device__ __forceinline__ void small_sort(const PackFit &f, void *smem) {
     }
     if (tid == 0) {
         double t = 0.0;
-        for (int w = 0; w < SMALL_THREADS / 32; ++w) t += pair_sums[w];
+        for (int w = 0; w < T / 32; ++w) t += pair_sums[w];
         f.status->same_pairs = t;
     }
     __syncthreads();
-    for (int64_t i = tid; i < n; i += SMALL_THREADS) {
+    for (int64_t i = tid; i < n; i += T) {
         const int32_t l = F.label[i];
         perm[start[l] + atomicAdd(&fill[l], 1)] = (int32_t)i;
     }
     __syncthreads();
-    for (int64_t p = tid; p < n; p += SMALL_THREADS) {
+    for (int64_t p = tid; p < n; p += T) {
         const int32_t i = perm[p], l = F.label[i];
         labp[p] = l;
         f.perm[p] = i;
@@ -771,7 +781,7 @@ __device__ __forceinline__ void small_sort(const PackFit &f, void *smem) {
     }
     __syncthreads();
     const int64_t tiles = ceil_div(n, SMALL_RANGE);
-    for (int64_t t = tid; t < tiles; t += SMALL_THREADS) {
+    for (int64_t t = tid; t < tiles; t += T) {
         const int64_t a = t * SMALL_RANGE, b = a + SMALL_RANGE < n ? a + SMALL_RANGE : n;
         int32_t mn = labp[a], mx = mn;
         for (int64_t i = a + 1; i < b; ++i) {
@@ -786,40 +796,44 @@ __device__ __forceinline__ void small_sort(const PackFit &f, void *smem) {
 
 // End of a round: the per-component minimum key (component_min_kernel's keys, reduced with
 // shared atomics), the winners (winner_kernel), then resolve_block over `components` components.
+template <int T>
 __device__ __forceinline__ void small_merge(const PackFit &f, int64_t components, void *smem) {
     const SmallForest F = small_forest(smem);
     const int tid = threadIdx.x;
     const int64_t n = f.n;
-    for (int64_t i = tid; i < n; i += SMALL_THREADS) {
+    for (int64_t i = tid; i < n; i += T) {
         F.comp_keys[i] = ~0ull;
         F.label[i] = f.label[i];
     }
     __syncthreads();
-    for (int64_t p = tid; p < n; p += SMALL_THREADS) {
+    for (int64_t p = tid; p < n; p += T) {
         const unsigned long long v = comp_key_at(p, f.perm, f.row_keys, f.status, f.allow_empty);
         if (v != ~0ull) atomicMin(&F.comp_keys[f.labp[p]], v);
     }
     __syncthreads();
-    for (int64_t i = tid; i < n; i += SMALL_THREADS)
+    for (int64_t i = tid; i < n; i += T)
         winner_at(i, F.label, F.comp_keys, f.row_keys, n, F.next, F.esrc, F.edst, F.ew, f.status);
     __syncthreads();
-    resolve_block(F, F.label, f.label, n, log2_ceil_dev(components > 1 ? components : 2) + 1,
+    resolve_block<T>(F, F.label, f.label, n, log2_ceil_dev(components > 1 ? components : 2) + 1,
                   f.status, f.src, f.dst, f.w, n - 1, 1);
 }
 
 // One fit alone: its descriptor is a kernel argument.
-__global__ void __launch_bounds__(SMALL_THREADS) small_seed_kernel(const PackFit f) {
+template <int T>
+__global__ void __launch_bounds__(T) small_seed_kernel(const PackFit f) {
     extern __shared__ __align__(16) unsigned char small_smem[];
-    small_seed(f, small_smem);
+    small_seed<T>(f, small_smem);
 }
-__global__ void __launch_bounds__(SMALL_THREADS) small_sort_kernel(const PackFit f) {
+template <int T>
+__global__ void __launch_bounds__(T) small_sort_kernel(const PackFit f) {
     extern __shared__ __align__(16) unsigned char small_smem[];
-    small_sort(f, small_smem);
+    small_sort<T>(f, small_smem);
 }
-__global__ void __launch_bounds__(SMALL_THREADS)
+template <int T>
+__global__ void __launch_bounds__(T)
     small_merge_kernel(const PackFit f, int64_t components) {
     extern __shared__ __align__(16) unsigned char small_smem[];
-    small_merge(f, components, small_smem);
+    small_merge<T>(f, components, small_smem);
 }
 // Sorted copy of the rows only (labels and cores: small_sort).
 __global__ void gather_rows_kernel(const float *__restrict__ x, const int32_t *__restrict__ perm,
@@ -921,8 +935,9 @@ int forest_seed(cuscan_ctx *ctx, ForestBuffers &b, float *core, const int32_t *i
         f.core = core;
         f.ids = const_cast<int32_t *>(ids);
         f.dsq = const_cast<float *>(dsq);
-        if (int rc = allow_dynamic_smem(ctx, small_seed_kernel, kSmallSmem)) return rc;
-        CUSCAN_KERNEL(small_seed_kernel, 1, SMALL_THREADS, kSmallSmem, s, f);
+        const auto kernel = CUSCAN_SMALL(small_seed_kernel, n);
+        if (int rc = allow_dynamic_smem(ctx, kernel, kSmallSmem)) return rc;
+        CUSCAN_KERNEL(kernel, 1, small_threads(n), kSmallSmem, s, f);
         CUSCAN_LAUNCH(ctx, "small_seed_kernel");
         return CUSCAN_OK;
     }
@@ -961,8 +976,9 @@ int forest_sort_by_component(cuscan_ctx *ctx, ForestBuffers &b, const float *x, 
     if (forest_small(n)) {
         PackFit f = small_fit(b, n, const_cast<int32_t *>(label), nullptr, nullptr, nullptr);
         f.core = const_cast<float *>(core);
-        if (int rc = allow_dynamic_smem(ctx, small_sort_kernel, kSmallSmem)) return rc;
-        CUSCAN_KERNEL(small_sort_kernel, 1, SMALL_THREADS, kSmallSmem, s, f);
+        const auto kernel = CUSCAN_SMALL(small_sort_kernel, n);
+        if (int rc = allow_dynamic_smem(ctx, kernel, kSmallSmem)) return rc;
+        CUSCAN_KERNEL(kernel, 1, small_threads(n), kSmallSmem, s, f);
         CUSCAN_KERNEL(gather_rows_kernel, blocks(n * d), 256, 0, s, x, as<int32_t>(b.perm), n * d, d,
                       as<float>(b.xp));
         CUSCAN_LAUNCH(ctx, "component sort");
@@ -1019,8 +1035,9 @@ int forest_round(cuscan_ctx *ctx, ForestBuffers &b, int64_t n, int64_t component
     if (forest_small(n)) {
         PackFit f = small_fit(b, n, label, out_src, out_dst, out_w);
         f.allow_empty = allow_empty;
-        if (int rc = allow_dynamic_smem(ctx, small_merge_kernel, kSmallSmem)) return rc;
-        CUSCAN_KERNEL(small_merge_kernel, 1, SMALL_THREADS, kSmallSmem, s, f, components);
+        const auto kernel = CUSCAN_SMALL(small_merge_kernel, n);
+        if (int rc = allow_dynamic_smem(ctx, kernel, kSmallSmem)) return rc;
+        CUSCAN_KERNEL(kernel, 1, small_threads(n), kSmallSmem, s, f, components);
         CUSCAN_LAUNCH(ctx, "small_merge_kernel");
         return CUSCAN_OK;
     }
@@ -1168,7 +1185,8 @@ namespace {
 
 // Fit blockIdx.x: core column, seed proposals, labels and the seed's merge (small_seed, as a fit
 // alone). Block 0 also clears the pack's per-round counters.
-__global__ void __launch_bounds__(SMALL_THREADS)
+template <int T>
+__global__ void __launch_bounds__(T)
     pack_seed_kernel(const PackFit *__restrict__ fits, int *more) {
     extern __shared__ __align__(16) unsigned char small_smem[];
     const PackFit f = fits[blockIdx.x];
@@ -1180,7 +1198,7 @@ __global__ void __launch_bounds__(SMALL_THREADS)
         f.kept_total[1] = 0;
     }
     __syncthreads();
-    small_seed(f, small_smem);
+    small_seed<T>(f, small_smem);
     if (tid == 0) {
         st->seed_edges = st->edges;
         st->components_after_seed = st->components;
@@ -1190,7 +1208,8 @@ __global__ void __launch_bounds__(SMALL_THREADS)
 // Start of round r of fit blockIdx.x: whether it runs (more than one component, no error,
 // within the round limit: the host driver's checks), then small_sort (pack_gather_kernel copies
 // the rows).
-__global__ void __launch_bounds__(SMALL_THREADS) pack_sort_kernel(const PackFit *__restrict__ fits) {
+template <int T>
+__global__ void __launch_bounds__(T) pack_sort_kernel(const PackFit *__restrict__ fits) {
     extern __shared__ __align__(16) unsigned char small_smem[];
     const PackFit f = fits[blockIdx.x];
     DevStatus *st = f.status;
@@ -1206,7 +1225,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) pack_sort_kernel(const PackFit 
     }
     __syncthreads();
     if (!run) return;
-    small_sort(f, small_smem);
+    small_sort<T>(f, small_smem);
 }
 
 // Sorted copy of the rows of fit blockIdx.y whose round runs (gather_kernel's copy), spread over
@@ -1227,7 +1246,8 @@ __global__ void pack_gather_kernel(const PackFit *__restrict__ fits) {
 
 // End of round r of fit blockIdx.x: winners and merge (small_merge), then the round's
 // bookkeeping (rounds run, ordered cross pairs entering it) and whether another round is due.
-__global__ void __launch_bounds__(SMALL_THREADS)
+template <int T>
+__global__ void __launch_bounds__(T)
     pack_merge_kernel(const PackFit *__restrict__ fits, int r, int *more) {
     extern __shared__ __align__(16) unsigned char small_smem[];
     const PackFit f = fits[blockIdx.x];
@@ -1237,7 +1257,7 @@ __global__ void __launch_bounds__(SMALL_THREADS)
     DevStatus *st = f.status;
     const int64_t comps = (int64_t)st->components;
     __syncthreads();  // every thread has the count before the merge rewrites it
-    small_merge(f, comps, small_smem);
+    small_merge<T>(f, comps, small_smem);
     if (tid == 0) {
         st->rounds += 1;
         st->cross_pairs += (double)n * (double)n - st->same_pairs;
@@ -1284,24 +1304,28 @@ int pack_knn(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int
     return launch_pack_knn(ctx, fits, count, n_max, d_max, k_max, splits, s, launches);
 }
 
-int pack_seed(cuscan_ctx *ctx, const PackFit *fits, int count, int *more, cudaStream_t s) {
-    if (int rc = allow_dynamic_smem(ctx, pack_seed_kernel, kSmallSmem)) return rc;
-    CUSCAN_KERNEL(pack_seed_kernel, count, SMALL_THREADS, kSmallSmem, s, fits, more);
+int pack_seed(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int *more,
+              cudaStream_t s) {
+    const auto kernel = CUSCAN_SMALL(pack_seed_kernel, n_max);
+    if (int rc = allow_dynamic_smem(ctx, kernel, kSmallSmem)) return rc;
+    CUSCAN_KERNEL(kernel, count, small_threads(n_max), kSmallSmem, s, fits, more);
     CUSCAN_LAUNCH(ctx, "pack_seed_kernel");
     return CUSCAN_OK;
 }
 
 int pack_round(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int d_max,
                int splits, int r, int *more, cudaStream_t s) {
-    if (int rc = allow_dynamic_smem(ctx, pack_sort_kernel, kSmallSmem)) return rc;
-    if (int rc = allow_dynamic_smem(ctx, pack_merge_kernel, kSmallSmem)) return rc;
-    CUSCAN_KERNEL(pack_sort_kernel, count, SMALL_THREADS, kSmallSmem, s, fits);
+    const auto sort = CUSCAN_SMALL(pack_sort_kernel, n_max);
+    const auto merge = CUSCAN_SMALL(pack_merge_kernel, n_max);
+    if (int rc = allow_dynamic_smem(ctx, sort, kSmallSmem)) return rc;
+    if (int rc = allow_dynamic_smem(ctx, merge, kSmallSmem)) return rc;
+    CUSCAN_KERNEL(sort, count, small_threads(n_max), kSmallSmem, s, fits);
     CUSCAN_LAUNCH(ctx, "pack_sort_kernel");
     const dim3 gg((unsigned)std::min<int64_t>(ceil_div(n_max * d_max, 256), 128), (unsigned)count);
     CUSCAN_KERNEL(pack_gather_kernel, gg, 256, 0, s, fits);
     CUSCAN_LAUNCH(ctx, "pack_gather_kernel");
     if (int rc = launch_pack_candidates(ctx, fits, count, n_max, d_max, splits, s)) return rc;
-    CUSCAN_KERNEL(pack_merge_kernel, count, SMALL_THREADS, kSmallSmem, s, fits, r, more);
+    CUSCAN_KERNEL(merge, count, small_threads(n_max), kSmallSmem, s, fits, r, more);
     CUSCAN_LAUNCH(ctx, "pack_merge_kernel");
     return CUSCAN_OK;
 }

@@ -163,7 +163,8 @@ int pack_knn(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int
              int k_max, int splits, cudaStream_t s, int64_t &launches);
 // Core column, kNN seed and its merge (forest_core + forest_seed) of every fit; zeroes the
 // fits' status blocks and the pack's per-round counters more[0, kPackMaxRounds + 2).
-int pack_seed(cuscan_ctx *ctx, const PackFit *fits, int count, int *more, cudaStream_t s);
+int pack_seed(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int *more,
+              cudaStream_t s);
 // One Borůvka round r of every fit that still has more than one component: the component
 // sort, the sorted copy of the rows, the exact candidate sweep, the winners and the merge.
 // more[r] counts the fits that need another round after it.

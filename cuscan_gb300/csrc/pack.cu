@@ -328,7 +328,7 @@ extern "C" int cuscan_fit_core_packed(cuscan_ctx *ctx, cuscan_fit_item *items, i
             return rc;
     }
     CUSCAN_CUDA(ctx, cudaEventRecord(P.ev[1], s));
-    if ((rc = pack_seed(ctx, fits, count, more, s))) return rc;
+    if ((rc = pack_seed(ctx, fits, count, n_max, more, s))) return rc;
     ++P.launches;
     int r = 0;
     for (int batch = kFirstBatch; r < kPackMaxRounds + 2; batch = kNextBatch) {
