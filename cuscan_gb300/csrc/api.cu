@@ -285,8 +285,11 @@ static int status_error(cuscan_ctx *ctx, int kind) {
 constexpr int64_t EXACT_ROWS_MIN = 2048;
 // Fewer norm levels than this per component do not narrow a 32-row chunk's norms.
 constexpr int NORM_LEVELS_MIN = 8;
-// Rounds of fewer rows are bound by their launches, of which the norm keys are five.
-// (9,001 x 32: 1.353 against 1.361 ms, 20,000 x 200: 2.46 against 2.52 ms).
+// Rounds of fewer rows are bound by their launches, of which the norm keys are five; what they save
+// grows with the tiles. Fits with and without them, ms, runs within 1 %: 5,000 x 32 1.06, 1.03;
+// 9,001 x 32 1.32, 1.31; 20,000 x 200 unit vectors 2.28, 2.23; 20,000 x 64 mixture 1.66, 1.74;
+// 33,000 x 64 anisotropic 2.20 to 2.67, 2.31 to 2.91; 33,000 x 128 unit vectors 2.50, 2.45;
+// 50,000 x 128 mixture 3.75, 3.84; 100,000 x 64 anisotropic 8.4 to 8.9, 10.4 to 11.4.
 constexpr int64_t NORM_KEYS_MIN_ROWS = 32768;
 
 static float elapsed(cudaEvent_t a, cudaEvent_t b) {

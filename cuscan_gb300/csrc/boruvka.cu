@@ -62,13 +62,15 @@ constexpr size_t kCandSmem =
     sizeof(float) * simt::STAGES * simt::STAGE_FLOATS + sizeof(CandShared);
 
 // A pruned sweep: bounds of the reference tiles and the components' upper bounds (f32 bits, by
-// label). A pair is left out only when its weight exceeds both its query's best so far and the
-// bound of the query's component, so a query's key is its exact cheapest edge unless that exceeds
-// the component's bound (such a key, or none, cannot win the component).
+// label). A pair is left out only when its weight exceeds the smaller of its query's best so far and
+// the bound of the query's component. A pair above the best is not the query's cheapest edge, and a
+// query whose cheapest edge lies above the component's bound cannot win the component: its key is
+// then some larger weight, or none. So every query's cheapest weight is at least the smaller of its
+// key's and the bound, and its key is exact where that is at most the bound.
 // The component bounds stay as the round starts with them: lowering them as the sweep finds
-// edges prunes more of a round (31.2 -> 26.3 ms at 100,000 x 64, round 2), but then fewer rows
-// leave a lower bound above their component's next bound, and the rounds after it scan more rows
-// (18,539 -> 75,251 in round 4): 66.6 ms became 74.7 ms over the fit's rounds.
+// edges prunes more of a round (31.2 -> 26.3 ms in the second round at 100,000 x 64), but then fewer
+// rows leave a lower bound above their component's next bound, and the rounds after it scan more
+// rows (18,539 -> 75,251 in the fourth): 66.6 ms became 74.7 ms over the fit's rounds.
 struct CandPrune {
     TileBounds bounds;
     const uint32_t *cbound;

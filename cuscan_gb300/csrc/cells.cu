@@ -336,7 +336,7 @@ constexpr int VISIT_THREADS = 256;
 __global__ void __launch_bounds__(VISIT_THREADS)
     visit_lists_kernel(const TileBounds balls, const float *__restrict__ ball_thr, int d, int n_tiles,
                        uint16_t *__restrict__ list, int32_t *__restrict__ counts) {
-    __shared__ float centre[CUSCAN_PACK_MAX_FEATURES][2];
+    __shared__ alignas(8) float centre[CUSCAN_PACK_MAX_FEATURES][2];  // read as float2
     __shared__ uint32_t bits[kMaxVisitTiles / 32];
     __shared__ int warp_sums[VISIT_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

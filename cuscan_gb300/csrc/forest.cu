@@ -1299,11 +1299,6 @@ __global__ void __launch_bounds__(kWeightThreads)
 
 }  // namespace
 
-int pack_knn(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int d_max,
-             int k_max, int splits, cudaStream_t s, int64_t &launches) {
-    return launch_pack_knn(ctx, fits, count, n_max, d_max, k_max, splits, s, launches);
-}
-
 int pack_seed(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int *more,
               cudaStream_t s) {
     const auto kernel = CUSCAN_SMALL(pack_seed_kernel, n_max);

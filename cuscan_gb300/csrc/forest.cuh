@@ -158,11 +158,11 @@ struct PackFit {
 constexpr int kPackMaxRounds = 64;  // the host driver's round limit (api.cu)
 constexpr int kPackErrNoConvergence = 8;
 // Exact kNN lists of every fit whose k is at most 32 (squared distances, self excluded), the
-// reference range of each fit split in `splits` chunks (partial lists merged when > 1).
-int pack_knn(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int d_max,
-             int k_max, int splits, cudaStream_t s, int64_t &launches);
-// Core column, kNN seed and its merge (forest_core + forest_seed) of every fit; zeroes the
-// fits' status blocks and the pack's per-round counters more[0, kPackMaxRounds + 2).
+// reference range of each fit split in `splits` chunks (partial lists merged when > 1; knn.cu).
+int launch_pack_knn(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int d_max,
+                    int k_max, int splits, cudaStream_t s, int64_t &launches);
+// Core column, kNN seed and its merge (forest_seed) of every fit; zeroes the fits' status blocks
+// and the pack's per-round counters more[0, kPackMaxRounds + 2).
 int pack_seed(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int *more,
               cudaStream_t s);
 // One Borůvka round r of every fit that still has more than one component: the component
@@ -172,9 +172,7 @@ int pack_round(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, i
                int splits, int r, int *more, cudaStream_t s);
 // status->mst_weight of every fit without an error (forest_mst_weight's order).
 int pack_weight(cuscan_ctx *ctx, const PackFit *fits, int count, cudaStream_t s);
-// Grouped launches inside other translation units (knn.cu, boruvka.cu).
-int launch_pack_knn(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max, int d_max,
-                    int k_max, int splits, cudaStream_t s, int64_t &launches);
+// Grouped candidate sweep of a round (boruvka.cu).
 int launch_pack_candidates(cuscan_ctx *ctx, const PackFit *fits, int count, int64_t n_max,
                            int d_max, int splits, cudaStream_t s);
 

@@ -35,8 +35,8 @@ constexpr int GROUPED_K = 32;     // largest k of the packed fits' kernels
 constexpr int TILED_K = 256;      // largest k of the tiled kernel
 constexpr int SEEDED_K = 32;      // largest k whose first thresholds come from group minima
 
-// Shared memory of one CTA after the sweep's stages (k entries per list). Up to k = 54 three
-// CTAs fit an SM (52 with the ball of a pruned sweep).
+// Shared memory of one CTA after the sweep's stages (k entries per list). Up to k = 57 three
+// CTAs fit the 228 KB of an SM (49 with the balls of a pruned sweep).
 struct KnnShared {
     float *thr;        // [QT] upper bound of the row's k-th distance
     int32_t *row;      // [QT] query row in the query array

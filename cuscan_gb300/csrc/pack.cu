@@ -317,7 +317,7 @@ extern "C" int cuscan_fit_core_packed(cuscan_ctx *ctx, cuscan_fit_item *items, i
     CUSCAN_CUDA(ctx, cudaEventRecord(P.ev[0], s));
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(base, stg, L.in_bytes, cudaMemcpyHostToDevice, s));
     if (k_max > 0 &&
-        (rc = pack_knn(ctx, fits, count, n_max, d_max, k_max, (int)splits, s, P.launches)))
+        (rc = launch_pack_knn(ctx, fits, count, n_max, d_max, k_max, (int)splits, s, P.launches)))
         return rc;
     for (int i = 0; i < count; ++i) {
         if (item_k(items[i]) <= kGroupedMaxK) continue;

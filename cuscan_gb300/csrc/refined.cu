@@ -53,7 +53,7 @@ constexpr int PB_STRIDE = 4 * HALF;       // kNN modes, per epilogue warp: [2][H
 constexpr int BORUVKA_CAP = 32;           // Borůvka candidate slots per row half
 
 struct Params {
-    const uint8_t *xt;        // 16-bit tiles, pre-swizzled (see tile_16bit_kernel)
+    const uint8_t *xt;        // 16-bit tiles, pre-swizzled (see prep_rows_kernel)
     int nbk;                  // K blocks per tile row of the copy: kblocks, or 2 kblocks (split)
     int split;                // split bf16: blocks [0, kblocks) hold hi, [kblocks, 2 kblocks) lo
     // kNN sweeps: [0] tiles issued by all CTAs so far (see knn_tile), [1] query blocks taken
@@ -74,9 +74,9 @@ struct Params {
     const int32_t *tile_hi;
     int64_t n, n_tiles, n_qblocks, n_chunks;
     int kblocks, stages, stage_blocks;  // stage_blocks: K blocks per ring stage (divides nbk)
-    // one-sided Borůvka with fewer query blocks than SMs: CTAs per query block, each running one
-    // contiguous part of the block's tile order (work item qi = block qi / splits, part qi %
-    // splits; appends then take their slots with atomics and the row bounds are min-reduced)
+    // one-sided Borůvka: parts of every query block's tile order (screen_parts), each a work item of
+    // its own (item qi = block qi / splits, part qi % splits; with several parts appends take their
+    // slots with atomics and the row bounds are min-reduced)
     int splits;
     float c_a, one_minus_cb;
     int32_t *cand_ids;        // [n][M]
@@ -520,12 +520,6 @@ __device__ __forceinline__ int64_t vis_tile(const Params &P, int64_t qb, int64_t
     return SYM ? (qb >> 1) + i : tile_order(P, wa, i);
 }
 
-// The query block a CTA takes at its qi-th step (blocks in order, strided over the CTAs).
-template <bool SYM>
-__device__ __forceinline__ int64_t block_at(const Params &P, int64_t qi) {
-    return qi;
-}
-
 // Label range of query block qb (4 chunks of 32 rows).
 __device__ __forceinline__ void qblock_range(const Params &P, int64_t qb, int32_t &lo,
                                              int32_t &hi) {
@@ -677,7 +671,7 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
                     mbar_arrive(&rot_full[rs]);
                 }
                 if (qi >= P.n_qblocks * P.splits) break;
-                const int64_t qb = block_at<SYM>(P, qi / P.splits);
+                const int64_t qb = qi / P.splits;
                 const int64_t part = qi % P.splits;
                 if (!mbar_wait(a_empty, a_phase ^ 1, abort, P.error)) break;
                 a_issued = 2u | a_phase;
@@ -790,7 +784,7 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
                         mbar_arrive(&rot_empty[rs]);
                     }
                     if (qi >= P.n_qblocks * P.splits) break;
-                    const int64_t qb = block_at<SYM>(P, qi / P.splits);
+                    const int64_t qb = qi / P.splits;
                     const int64_t part = qi % P.splits;
                     if (!mbar_wait(a_full, a_phase, abort, P.error)) break;
                     a_phase ^= 1;
@@ -862,7 +856,7 @@ __global__ void __launch_bounds__(THREADS, 1) screen_kernel(const Params P) {
                 if (lane == 0) mbar_arrive(&rot_empty[rs]);
             }
             if (qi >= P.n_qblocks * P.splits) break;
-            const int64_t qb = block_at<SYM>(P, qi / P.splits);
+            const int64_t qb = qi / P.splits;
             const int64_t part = qi % P.splits;
             // the debug entry point dumps query block 0 against tile 0 (its first tile)
             const bool debug = P.debug_tile != nullptr && qb == 0;
@@ -1415,7 +1409,7 @@ __global__ void rerank_knn_kernel(const float *__restrict__ x, const int32_t *__
                                   float *__restrict__ dist, int32_t *__restrict__ fallback,
                                   float *__restrict__ fallback_thr,
                                   int *__restrict__ fallback_count) {
-    extern __shared__ float rerank_smem[];
+    extern __shared__ __align__(16) float rerank_smem[];
     const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= n) return;
@@ -1515,7 +1509,7 @@ __global__ void rerank_knn_threshold_kernel(const float *__restrict__ x,
         if (lane == 0) fallback[atomicAdd(fallback_count, 1)] = (int32_t)orow;
         return;
     }
-    extern __shared__ float rerank_smem[];
+    extern __shared__ __align__(16) float rerank_smem[];
     float *q_s = rerank_smem + (threadIdx.x >> 5) * rerank_warp_floats(d, VEC);
     float *rows_s = q_s + d;
     for (int f = lane; f < d; f += 32) q_s[f] = x[pos * d + f];
@@ -1592,7 +1586,7 @@ __global__ void rerank_boruvka_kernel(const float *__restrict__ xp, const float 
     }
     const int total = c0 + c1 + c2;
     if (total == 0) return;  // no candidate: the row keeps an empty key
-    extern __shared__ float rerank_smem[];
+    extern __shared__ __align__(16) float rerank_smem[];
     float *q_s = rerank_smem + (threadIdx.x >> 5) * rerank_warp_floats(d, VEC);
     float *rows_s = q_s + d;
     for (int f = lane; f < d; f += 32) q_s[f] = xp[pos * d + f];
@@ -1695,7 +1689,7 @@ __global__ void row_lb_from_keys_kernel(const unsigned long long *__restrict__ r
     const int32_t orow = perm[pos];
     const unsigned long long key = row_keys[orow];  // keys are kept by original row
     float w = key == ~0ull ? CUSCAN_INF : __uint_as_float((uint32_t)(key >> 32));
-    // a pruned round left out pairs above both the row's best and its component's bound
+    // a pruned round left out pairs above the smaller of the row's best and its component's bound
     if (cbound) w = fminf(w, __uint_as_float(cbound[labp[pos]]));
     rowlb[orow] = fmaxf(rowlb[orow], w);
 }
