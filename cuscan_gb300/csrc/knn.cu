@@ -295,7 +295,8 @@ __device__ __forceinline__ void knn_block(
             // A bucket that was full is rare but for rows with many equal distances (duplicates,
             // overflow), whose ties would all be pushed and merged; a thread that met them there
             // looks for them at once from then on. 10,000 equal rows of 16 features, k = 8: 6,116 us
-            // without, 384 us. (Looking at ties in every test costs sweeps without them 2 to 11 %.)
+            // without, 384 us. (Looking at ties in every test costs sweeps without them 2 to 11 %;
+            // this form at most 1.5 %, pruned sweeps of 50 neighbours 2.4 %.)
             if ((again || tied) && hits) {
                 const unsigned long long left = without_ties(acc, r0, hits);
                 tied |= left != hits;
@@ -335,7 +336,8 @@ __device__ __forceinline__ void knn_block(
                     x = sh.bucket_d[q * BUCKET + lane];
                     j = (int32_t)(r0 + sh.bucket_r[q * BUCKET + lane]);
                     if (PRUNE && prune.ids) j = prune.ids[j];
-                    pass = knn_better(x, j, ld[k - 1], li[k - 1]);
+                    // (the look costs the pruned sweeps of up to 32 neighbours 1 %)
+                    pass = (PRUNE && L == 1) || knn_better(x, j, ld[k - 1], li[k - 1]);
                 }
                 const unsigned enter = __ballot_sync(0xffffffffu, pass);
                 if (enter) merge_hits<L>(ld, li, k, x, j, enter);
