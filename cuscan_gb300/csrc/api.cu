@@ -32,6 +32,7 @@ int refined_operand_format(const ForestBuffers &b);
 size_t refined_workspace_bytes(int64_t n, int d, int k, bool lean);
 int64_t fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, int32_t precision, int lean);
 void set_lean(cuscan_ctx *ctx, int lean);
+void set_served(cuscan_ctx *ctx);
 
 // Every device buffer a context holds.
 static int workspace_buffers(FitWorkspace *f, Buffer **out) {
@@ -172,6 +173,7 @@ int64_t cuscan::fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, i
 }
 
 void cuscan::set_lean(cuscan_ctx *ctx, int lean) { ctx->fit->forest.refined.lean = lean; }
+void cuscan::set_served(cuscan_ctx *ctx) { ctx->fit->served = true; }
 
 extern "C" {
 

@@ -57,7 +57,7 @@ struct cuscan_predictor {
 };
 
 namespace cuscan {
-int64_t predict_workspace_bound(const cuscan_predictor *p, int64_t m, int lean);
+int64_t predict_workspace_bound(const cuscan_predictor *p, int64_t m, int lean, bool served);
 namespace {
 
 // Where a batch is searched in spatial order. The order pads the queries of every cell to whole balls
@@ -74,6 +74,13 @@ constexpr int64_t kSpatialRows = 256 * (int64_t)kMaxPivots;  // training rows wi
 constexpr float kSpatialApart = 0.6f, kSpatialFarApart = 0.9f;
 constexpr int64_t kSpatialQueries = 4096, kSpatialFarQueries = 2048;  // 16 and 8 of a cell
 constexpr double kSpatialWork = 3e9;  // queries x rows x features
+// On a server's slots the other requests wait for the SMs that a plain search fills, so batches of fewer
+// queries are searched in spatial order where that is less work, although it takes longer alone. The
+// mixed stream (fits and batches of 1 to 4,096 queries against 100,000 x 64 rows, eight slots):
+// prediction p50 0.33 ms and p99 2.36 to 2.46 ms, with the rule above 0.36 to 0.38 and 2.9 to 3.2 ms;
+// from 1,024 queries 0.34 and 2.35 to 2.56 ms.
+constexpr int64_t kServedQueries = 512;
+constexpr double kServedWork = 2e9;
 // The spatial copy takes at most this share of the free device memory, so that a predictor whose rows
 // are large against the device holds them once.
 constexpr double kSpatialShare = 1.0 / 8.0;
@@ -85,10 +92,12 @@ void free_rows(cuscan_predictor &P) {
     P.bounds = TileBounds();
 }
 
-bool searches_spatially(const cuscan_predictor &P, int64_t m) {
-    return P.bounds.centre &&
-           m >= (P.apart >= kSpatialFarApart ? kSpatialFarQueries : kSpatialQueries) &&
-           (double)m * (double)P.n_finite * (double)P.d >= kSpatialWork;
+bool searches_spatially(const cuscan_predictor &P, int64_t m, bool served) {
+    if (!P.bounds.centre) return false;
+    const double work = (double)m * (double)P.n_finite * (double)P.d;
+    if (served && P.apart >= kSpatialFarApart) return m >= kServedQueries && work >= kServedWork;
+    return m >= (P.apart >= kSpatialFarApart ? kSpatialFarQueries : kSpatialQueries) &&
+           work >= kSpatialWork;
 }
 
 // The spatial copy of the training rows, where their cells lie apart.
@@ -748,17 +757,18 @@ int cuscan_predictor_shape(const cuscan_predictor *p, int64_t *n_finite, int32_t
 }
 
 int64_t cuscan_predict_workspace_bytes(const cuscan_predictor *p, int64_t m) {
-    return predict_workspace_bound(p, m, 0);
+    return predict_workspace_bound(p, m, 0, false);
 }
 
 }  // extern "C"
 
-int64_t cuscan::predict_workspace_bound(const cuscan_predictor *p, int64_t m, int lean) {
+int64_t cuscan::predict_workspace_bound(const cuscan_predictor *p, int64_t m, int lean,
+                                        bool served) {
     if (!p || m <= 0) return 0;
     const int64_t k = 2 * (int64_t)p->s;
     // query rows, candidate ids and distances, lists of the search's parts
     int64_t bytes = lean >= 2 ? 0 : 8 * k * simt::split_max_rows(m, p->n_finite);
-    if (!lean && searches_spatially(*p, m)) {
+    if (!lean && searches_spatially(*p, m, served)) {
         const int64_t pruned = pruned_partial_bytes(padded_queries(m), p->n_finite, (int)k);
         if (pruned > bytes) bytes = pruned;
         bytes += 16 * padded_queries(m);  // cells, distances, order, first thresholds
@@ -847,7 +857,7 @@ int predict_queries(cuscan_ctx *ctx, const cuscan_predictor *p, const float *que
     if (rc) return rc;
     CUSCAN_CUDA(ctx, cudaMemcpyAsync(f->pred_q.ptr, queries, sizeof(float) * m * p->d,
                                      cudaMemcpyHostToDevice, s));
-    bool spatial = !f->forest.refined.lean && searches_spatially(*p, m);
+    bool spatial = !f->forest.refined.lean && searches_spatially(*p, m, f->served);
     if (spatial) {
         rc = ensure(ctx, f->pred_order, sizeof(int32_t) * padded_queries(m), "query order");
         if (!rc)

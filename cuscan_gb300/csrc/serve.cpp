@@ -48,8 +48,10 @@
 // bound exceeds the server's budget runs at the first level that fits.
 namespace cuscan {
 int64_t fit_workspace_bound(int64_t n, int32_t d, int32_t min_samples, int32_t precision, int lean);
-int64_t predict_workspace_bound(const cuscan_predictor *p, int64_t m, int lean);
+int64_t predict_workspace_bound(const cuscan_predictor *p, int64_t m, int lean, bool served);
 void set_lean(cuscan_ctx *ctx, int lean);
+// The context is one of several that share the device: batches are searched in the form of least work.
+void set_served(cuscan_ctx *ctx);
 }  // namespace cuscan
 
 namespace {
@@ -557,6 +559,7 @@ int start_server(cuscan_server *s, int32_t slots, char *err, size_t err_len) {
                 s->slots.clear();
                 return rc;
             }
+            if (slots > 1) cuscan::set_served(slot->ctx);
         }
         s->slots.push_back(std::move(slot));
     }
@@ -670,9 +673,10 @@ int cuscan_server_submit_predict(cuscan_server *s, const cuscan_predictor *predi
     cuscan_predictor_shape(predictor, &nf, &d, &ms);
     r->d = d;
     r->min_samples = ms;
-    r->bytes = cuscan_predict_workspace_bytes(predictor, m);
+    r->bytes = cuscan::predict_workspace_bound(predictor, m, 0, s->slots.size() > 1);
     for (int level = 1; level <= 2; ++level)
-        r->lean_bytes[level - 1] = cuscan::predict_workspace_bound(predictor, m, level);
+        r->lean_bytes[level - 1] =
+            cuscan::predict_workspace_bound(predictor, m, level, s->slots.size() > 1);
     r->t_submit = Clock::now();
     return s->enqueue(std::move(r), request_id);
 }

@@ -24,6 +24,7 @@ struct FitWorkspace {
     static constexpr int kHostWords = 8;
     int *host_words() { return reinterpret_cast<int *>(host_status + 1); }
     cudaEvent_t ev[6] = {};
+    bool served = false;                           // a server's slot: other contexts share the device
     PackWorkspace *pack = nullptr;                 // created by the first packed call
     // per Borůvka round of the last fit: query rows screened, tensor-core tiles run, candidate
     // kernel time (ms), ordered cross-component pairs entering the round

@@ -97,3 +97,22 @@ def test_requests_run_at_the_first_level_whose_bound_fits():
     for other in results[1:]:
         for name in ("labels", "strengths", "connecting_points"):
             np.testing.assert_array_equal(other[name], results[0][name])
+
+
+@pytest.mark.parametrize("slots,m,spatial", [(2, 600, True), (2, 511, False), (1, 600, False)])
+def test_slots_that_share_the_device_search_smaller_batches_in_spatial_order(slots, m, spatial):
+    from cuscan_gb300 import _lib
+    from cuscan_gb300.serving import FitServer
+
+    n, d = 70_000, 64
+    _, predictor, x = fitted(n, d, 40, 1.0, 5, m)
+    assert not searches_spatially(predictor._predictor, m)
+    alone = predictor.approximate_predict(x[n:], True)
+    plain = cg.load().cuscan_predict_workspace_bytes(predictor._predictor.handle, m)
+    with FitServer(slots=slots, budget_bytes=8 << 30) as srv:
+        rid = srv.submit_predict(predictor, x[n:])
+        info = srv.wait(rid, 60.0)
+        got = srv.result(rid, timeout=60.0)
+    assert info["status"] == _lib.OK and (info["workspace_bound_bytes"] > plain) == spatial
+    for name, value in zip(("labels", "strengths", "connecting_points"), alone):
+        np.testing.assert_array_equal(got[name], value)
