@@ -331,8 +331,16 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
     ForestBuffers &b = f->forest;
     int rc = forest_reserve(ctx, b, n, d);
     if (!rc) rc = ensure(ctx, f->label, sizeof(int32_t) * n, "point labels");
-    if (!rc && !refined && n >= EXACT_ROWS_MIN) rc = reserve_exact_rows(ctx, b, n);
     if (rc) return rc;
+    // the rounds' arrays before what the fit can do without (fits whose seed connects every point
+    // run no round: they ask for the arrays again where they need them)
+    auto reserve_rounds = [&]() {
+        if (refined || n < EXACT_ROWS_MIN) return true;
+        const bool room = reserve_exact_rows(ctx, b, n) == CUSCAN_OK;
+        if (!room) clear_error(ctx);
+        return room;
+    };
+    const bool room = reserve_rounds();
     const int k = (int)((int64_t)min_samples < n - 1 ? min_samples : n - 1);
     int32_t *label = as<int32_t>(f->label);
     cudaEvent_t *ev = f->ev;
@@ -347,7 +355,8 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
     b.refined.pivots_valid = false;
     b.refined.screen_timed = false;
 
-    bool spatial = !refined && !b.refined.lean && knn_pruned_shape(d, k) && worth_pruning(n, n, d);
+    bool spatial = !refined && room && !b.refined.lean && knn_pruned_shape(d, k) &&
+                   worth_pruning(n, n, d);
     TileBounds bounds;
     CUSCAN_CUDA(ctx, cudaMemsetAsync(b.status, 0, sizeof(DevStatus), s));
     CUSCAN_CUDA(ctx, cudaEventRecord(ev[0], s));
@@ -374,7 +383,7 @@ int cuscan_fit_core_device(cuscan_ctx *ctx, const float *data, int64_t n, int32_
             clear_error(ctx);
             spatial = false;
             forest_release_refined(b);
-            if ((rc = reserve_exact_rows(ctx, b, n))) return rc;
+            reserve_rounds();
         }
     }
     if (!refined && !spatial)
